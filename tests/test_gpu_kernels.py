@@ -618,6 +618,33 @@ def test_gemm_tcgen05_many_tiles_and_row_invariance():
     assert torch.equal(part, out[300:370])
 
 
+@pytest.mark.parametrize("m,n,k", [(129, 256, 64), (256, 300, 456), (257, 264, 1032), (383, 1000, 72), (4097, 776, 520)])
+def test_gemm_tcgen05_pairs_of_blocks(m, n, k):
+    """Tiles of 256 rows on two blocks against tiles of 128 on one: edges of both tiles, fewer and more slabs than the ring
+    holds, rows beyond one group of the walk.  The sums are the same chains, so the results are the same bits."""
+    o = ops()
+    x = torch.randn(m, k, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(2 * n, k, device=DEV) * 0.1).to(torch.bfloat16)
+    got = {}
+    try:
+        for rows in (128, 256):
+            o.set_tuning(o.Tuning(gemm_tile_rows=rows))
+            out, acc = torch.full((m, n), 7.0, device=DEV), torch.ones(m, n, device=DEV)
+            gated = torch.empty(m, n, device=DEV, dtype=torch.bfloat16)
+            o.gemm_tcgen05(out, x, w[:n].contiguous())
+            o.gemm_tcgen05(acc, x, w[:n].contiguous(), "accumulate")
+            o.gemm_tcgen05(gated, x, w, "swiglu", up_rows=n)
+            got[rows] = (out, acc, gated)
+    finally:
+        o.set_tuning(o.Tuning())
+    o.check_error_flag(DEV)
+    want = f64(x) @ f64(w[:n]).T
+    assert rel(got[256][0], want) < 1e-5
+    assert rel(got[256][1], want + 1.0) < 1e-5
+    for single, pair in zip(got[128], got[256]):
+        assert torch.equal(single, pair)
+
+
 @pytest.mark.parametrize("m,inner,k", [(128, 128, 64), (130, 203, 104), (300, 136, 96)])
 def test_gemm_tcgen05_swiglu(m, inner, k):
     x = torch.randn(m, k, device=DEV).to(torch.bfloat16)

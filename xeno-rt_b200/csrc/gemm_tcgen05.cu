@@ -7,13 +7,14 @@
 // so both operands are K-major and no transposition is needed.  The reference's own CUDA matmul_kernel
 // (crates/xrt-cuda/src/lib.rs:636-772) is a 16x16-tile scalar kernel; this is its Blackwell counterpart.
 //
-// A persistent block (one a multiprocessor) walks output tiles of 128 x 256.  Six warps:
-//   warp 0     producer: for each 64-wide slab of K, one TMA load of the X tile (128 x 64) and two of
-//              the W tile (2 x 128 x 64) into the next free stage of a four-stage ring; the loads
-//              complete on the stage's "full" mbarrier.  Tiles that reach beyond M, N or K are
-//              zero-filled by TMA, so any M and N and any K that is a multiple of 8 work.
-//   warp 1     allocates 512 TMEM columns (two accumulators of 128 lanes x 256 columns) and issues the
-//              MMAs: four tcgen05.mma (128 x 256 x 16) a stage, then tcgen05.commit to the stage's
+// A persistent block, or a pair of blocks as one (TcShape), one block a multiprocessor, walks output tiles of 128 x 256 (a
+// pair: 256 x 256).  Six warps a block:
+//   warp 0     producer: for each 64-wide slab of K, TMA loads of the block's 128 rows of X and of its 256 rows of W (in a
+//              pair: 128 of them) into the next free stage of a ring; the loads complete on the stage's "full" mbarrier.
+//              Tiles that reach beyond M, N or K are zero-filled by TMA, so any M and N and any K that is a multiple
+//              of 8 work.
+//   warp 1     allocates 512 TMEM columns (two accumulators of 128 lanes x 256 columns) and issues the MMAs (in a pair the
+//              first block's does, for both): four tcgen05.mma a stage, then tcgen05.commit to the stage's
 //              "empty" mbarrier; after the last slab, tcgen05.commit to the accumulator's "full" mbarrier.
 //   warps 2-5  epilogue: each warp reads its 32 TMEM lanes (rows) with tcgen05.ld, 32 columns at a
 //              time, and stores, adds into the 32-bit residual stream, or applies SwiGLU (the W
@@ -29,21 +30,24 @@ namespace xrt {
 using namespace sm100;
 
 constexpr int TC_BM = 128, TC_BN = 256, TC_BK = 64, TC_UMMA_K = 16;
-constexpr int TC_A_BYTES = TC_BM * TC_BK * 2;        // 16 KB: 128 rows of X, one slab of K
-constexpr int TC_B_BYTES = TC_BN * TC_BK * 2;        // 32 KB
-// MT = 1: tiles of 128 x 256, four stages, two accumulators (the epilogue of a tile overlaps the MMAs
-// of the next).  MT = 2: tiles of 256 x 256 (two MMAs a slab share the W tile: a third fewer operand
-// bytes per flop, which is what bounds this kernel), three stages, one accumulator of all 512 TMEM
-// columns and eight epilogue warps to drain it.
-template <int MT> struct TcShape {
-  static constexpr int STAGES = MT == 1 ? 4 : 3;
-  static constexpr int STAGE_BYTES = MT * TC_A_BYTES + TC_BN * TC_BK * 2;
-  static constexpr int ACC_SETS = MT == 1 ? 2 : 1;
-  static constexpr int EPI_WARPS = 4 * MT;
-  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
-  static constexpr int STAGING_BYTES = EPI_WARPS * 32 * 33 * 4;    // a 32 x 32 patch (padded) an epilogue warp
+constexpr int TC_A_BYTES = TC_BM * TC_BK * 2;        // 16 KB: 128 rows of X (or of W), one slab of K
+// PAIR: two neighbouring blocks (a cluster of two, each on its own multiprocessor) work on one tile of 256 x 256 with
+// tcgen05.mma of cta_group::2.  Each block stages its own 128 rows of X and HALF of the W tile (128 of its 256 rows)
+// and keeps its own 128 rows of the accumulator: an MMA reads a third less shared memory and a slab brings a third
+// fewer bytes from the L2 per flop than two single blocks would, which is what bounds this kernel (and what it spends
+// of the power limit).  The first block of the pair issues all MMAs.
+// Measured back to back, microseconds, single blocks -> pairs (rows x outputs x inputs): 2,048 x 4,096 x 14,336 added into
+// the residual 222 -> 205; 7,999 x 6,144 x 4,096 stored 350 -> 330 (1,220 of 1,621 TFLOP/s); 17,000 x 14,336 (gated)
+// x 4,096 3,028 -> 2,955.
+template <bool PAIR> struct TcShape {
+  static constexpr int B_BYTES = PAIR ? TC_A_BYTES : 2 * TC_A_BYTES;  // of the W tile, in one block
+  static constexpr int STAGES = PAIR ? 6 : 4;
+  static constexpr int STAGE_BYTES = TC_A_BYTES + B_BYTES;
+  static constexpr int THREADS = 192;
+  static constexpr int STAGING_BYTES = 4 * 32 * 33 * 4;    // a 32 x 32 patch (padded) an epilogue warp
   static constexpr int SMEM = STAGES * STAGE_BYTES + STAGING_BYTES + 256 + 1024;  // + barriers + alignment slack
 };
+constexpr int TC_ACC_SETS = 2;  // the epilogue of a tile overlaps the MMAs of the next
 constexpr int TC_TMEM_COLS = 512;
 
 // Four consecutive outputs of one row: 16 bytes of float32 (stored, or added into the residual
@@ -67,21 +71,38 @@ __device__ __forceinline__ void store_quad(__nv_bfloat16* dst, float a, float b,
   *reinterpret_cast<uint2*>(dst) = packed;
 }
 
+// Where a tile lies.  Tiles that run at the same time should share operands in the L2: the walk goes down TC_GROUP_ROWS
+// rows of X, then to the next column of tiles, and only after the last column to the next such group of rows, so that
+// about 150 multiprocessors work on a block of the output that is nearly square.  Without groups (all rows of a column of
+// tiles first) 17,000 rows x 4,096 inputs came from memory once for every column of tiles: 3,850 us for 14,336 gated outputs
+// against 3,028, 911 against 721 for 6,144; up to 4,096 rows the walk is the same.  Groups of 2,048 rows: 2 percent slower.
+constexpr int TC_GROUP_ROWS = 4096;
+template <int TILE_ROWS>
+__device__ __forceinline__ void tile_place(int tile, int tiles_m, int tiles_n, int& m_blk, int& n_blk) {
+  constexpr int GROUP = TC_GROUP_ROWS / TILE_ROWS;
+  const int per_group = GROUP * tiles_n;
+  const int group = tile / per_group, in_group = tile - group * per_group;
+  const int rows = min(GROUP, tiles_m - group * GROUP);
+  n_blk = in_group / rows;
+  m_blk = group * GROUP + (in_group - n_blk * rows);
+}
+
 // MODE 0: store, 1: add into float out, 2: SwiGLU.  n_tiles_n counts tiles of 256 output columns
 // (SwiGLU: of 128, each computed from 128 gate rows and 128 up rows of W).
-template <int MODE, int MT, typename TO>
-__global__ void __launch_bounds__(TcShape<MT>::THREADS, 1)
+template <int MODE, bool PAIR, typename TO>
+__global__ void __launch_bounds__(TcShape<PAIR>::THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     TO* __restrict__ out, int M, int N, int K, int ldo, int up_rows, int* __restrict__ error_flag,
                     const NormEmit emit, const RowScale scale) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int TC_STAGES = TcShape<MT>::STAGES, ACC_SETS = TcShape<MT>::ACC_SETS;
-  constexpr int STAGE_A = MT * TC_A_BYTES;
+  constexpr int TC_STAGES = TcShape<PAIR>::STAGES, ACC_SETS = TC_ACC_SETS;
+  constexpr int STAGE_A = TC_A_BYTES, STAGE_B = TcShape<PAIR>::B_BYTES;
+  constexpr int TILE_ROWS = (PAIR ? 2 : 1) * TC_BM;
   unsigned char* a_stages = smem;
   unsigned char* b_stages = smem + TC_STAGES * STAGE_A;
-  float* staging = reinterpret_cast<float*>(smem + TC_STAGES * TcShape<MT>::STAGE_BYTES);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TC_STAGES * TcShape<MT>::STAGE_BYTES + TcShape<MT>::STAGING_BYTES);
+  float* staging = reinterpret_cast<float*>(smem + TC_STAGES * TcShape<PAIR>::STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TC_STAGES * TcShape<PAIR>::STAGE_BYTES + TcShape<PAIR>::STAGING_BYTES);
   uint64_t* full = bars;                       // [TC_STAGES]
   uint64_t* empty = bars + TC_STAGES;          // [TC_STAGES]
   uint64_t* acc_full = bars + 2 * TC_STAGES;   // [ACC_SETS] (room for two)
@@ -91,23 +112,31 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int N_PER_TILE = MODE == 2 ? TC_BN / 2 : TC_BN;  // output columns a tile
-  const int tiles_m = (M + MT * TC_BM - 1) / (MT * TC_BM);
+  const int tiles_m = (M + TILE_ROWS - 1) / TILE_ROWS;
   const int tiles_n = (N + N_PER_TILE - 1) / N_PER_TILE;
   const int n_tiles = tiles_m * tiles_n;
   const int k_iters = (K + TC_BK - 1) / TC_BK;
+  const int rank = PAIR ? (int)(blockIdx.x & 1) : 0;  // the block's place in its pair
+  const int unit = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, units = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; ++s) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(smem_u32(&acc_full[a]), 1); mbar_init(smem_u32(&acc_empty[a]), 32 * TcShape<MT>::EPI_WARPS); }
+    for (int a = 0; a < 2; ++a) { mbar_init(smem_u32(&acc_full[a]), 1); mbar_init(smem_u32(&acc_empty[a]), PAIR ? 256 : 128); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {  // the MMA warp owns the TMEM allocation
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TC_TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TC_TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TC_TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
   }
   fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();  // the other block's barriers stand before anything arrives on them
   fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -118,67 +147,82 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
       int it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const int m_blk = tile % tiles_m, n_blk = tile / tiles_m;
+      for (int tile = unit; tile < n_tiles && ok; tile += units) {
+        int m_blk, n_blk;
+        tile_place<TILE_ROWS>(tile, tiles_m, tiles_n, m_blk, n_blk);
         for (int kb = 0; kb < k_iters; ++kb, ++it) {
           const int s = it % TC_STAGES;
           ok = mbar_wait(smem_u32(&empty[s]), ((it / TC_STAGES) & 1) ^ 1, abort_flag);
           if (!ok) break;
-          const uint32_t bar = smem_u32(&full[s]);
-          mbar_arrive_expect_tx(bar, STAGE_A + TC_B_BYTES);
-#pragma unroll
-          for (int h = 0; h < MT; ++h)
-            tma_load_2d(smem_u32(a_stages + s * STAGE_A + h * TC_A_BYTES), &map_x, kb * TC_BK,
-                           (m_blk * MT + h) * TC_BM, bar);
+          const uint32_t a_dst = smem_u32(a_stages + s * STAGE_A), b_dst = smem_u32(b_stages + s * STAGE_B);
           const int w_row0 = n_blk * N_PER_TILE;
           const int w_row1 = MODE == 2 ? up_rows + w_row0 : w_row0 + 128;
-          tma_load_2d(smem_u32(b_stages + s * TC_B_BYTES), &map_w, kb * TC_BK, w_row0, bar);
-          tma_load_2d(smem_u32(b_stages + s * TC_B_BYTES + TC_B_BYTES / 2), &map_w, kb * TC_BK, w_row1, bar);
+          if (PAIR) {
+            // both blocks' copies complete on the first block's barrier, which alone the MMAs wait for; the bytes of
+            // both are announced there once (a copy of the second block may complete before that: the phase cannot end
+            // without the one arrival, and the second block reuses a stage only after the MMAs have released it)
+            const uint32_t bar = first_block_address(smem_u32(&full[s]));
+            if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full[s]), 2 * (STAGE_A + STAGE_B));
+            tma_load_2d_pair(a_dst, &map_x, kb * TC_BK, m_blk * TILE_ROWS + rank * TC_BM, bar);
+            tma_load_2d_pair(b_dst, &map_w, kb * TC_BK, rank == 0 ? w_row0 : w_row1, bar);
+          } else {
+            const uint32_t bar = smem_u32(&full[s]);
+            mbar_arrive_expect_tx(bar, STAGE_A + STAGE_B);
+            tma_load_2d(a_dst, &map_x, kb * TC_BK, m_blk * TC_BM, bar);
+            tma_load_2d(b_dst, &map_w, kb * TC_BK, w_row0, bar);
+            tma_load_2d(b_dst + STAGE_B / 2, &map_w, kb * TC_BK, w_row1, bar);
+          }
         }
       }
+      // a block of a pair leaves only when the other's MMAs have let go of its last stages
+      for (int j = 0; PAIR && ok && j < TC_STAGES; ++j, ++it)
+        ok = mbar_wait(smem_u32(&empty[it % TC_STAGES]), ((it / TC_STAGES) & 1) ^ 1, abort_flag);
       if (!ok) { *abort_flag = 1; if (error_flag != nullptr) atomicExch(error_flag, 3); }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issue
-    if (lane == 0) {
-      constexpr uint32_t idesc = instr_desc(TC_BM, TC_BN);
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = instr_desc(TILE_ROWS, TC_BN);
       int it = 0, tile_i = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++tile_i) {
+      for (int tile = unit; tile < n_tiles && ok; tile += units, ++tile_i) {
         const int a = tile_i % ACC_SETS;
         ok = mbar_wait(smem_u32(&acc_empty[a]), ((tile_i / ACC_SETS) & 1) ^ 1, abort_flag);
         if (!ok) break;
         fence_after();
-        const uint32_t tmem_d = tmem_base + a * MT * TC_BN;
+        const uint32_t tmem_d = tmem_base + a * TC_BN;
         for (int kb = 0; kb < k_iters; ++kb, ++it) {
           const int s = it % TC_STAGES;
           ok = mbar_wait(smem_u32(&full[s]), (it / TC_STAGES) & 1, abort_flag);
           if (!ok) break;
           fence_after();
-          const uint64_t desc_b = desc_k_major(smem_u32(b_stages + s * TC_B_BYTES));
+          const uint64_t desc_a = desc_k_major(smem_u32(a_stages + s * STAGE_A));
+          const uint64_t desc_b = desc_k_major(smem_u32(b_stages + s * STAGE_B));
 #pragma unroll
-          for (int h = 0; h < MT; ++h) {
-            const uint64_t desc_a = desc_k_major(smem_u32(a_stages + s * STAGE_A + h * TC_A_BYTES));
-#pragma unroll
-            for (int k = 0; k < TC_BK / TC_UMMA_K; ++k)  // 32 bytes further along K inside the swizzle atom
-              mma_f16(tmem_d + h * TC_BN, desc_a + 2 * k, desc_b + 2 * k, idesc, (kb | k) != 0);
+          for (int k = 0; k < TC_BK / TC_UMMA_K; ++k) {  // 32 bytes further along K inside the swizzle atom
+            if (PAIR) mma_f16_pair(tmem_d, desc_a + 2 * k, desc_b + 2 * k, idesc, (kb | k) != 0);
+            else mma_f16(tmem_d, desc_a + 2 * k, desc_b + 2 * k, idesc, (kb | k) != 0);
           }
-          commit(smem_u32(&empty[s]));
+          if (PAIR) commit_pair(smem_u32(&empty[s]));
+          else commit(smem_u32(&empty[s]));
         }
-        if (ok) commit(smem_u32(&acc_full[a]));
+        if (ok) {
+          if (PAIR) commit_pair(smem_u32(&acc_full[a]));
+          else commit(smem_u32(&acc_full[a]));
+        }
       }
       if (!ok) { *abort_flag = 1; if (error_flag != nullptr) atomicExch(error_flag, 3); }
     }
   } else {
     // ---------------------------------------------------------------- epilogue
     const int quarter = warp & 3;  // the TMEM lanes this warp may read: 32 * quarter ..
-    const int half = (warp - 2) / 4;  // which 128 rows of the tile (always 0 for tiles of 128 rows)
     int tile_i = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++tile_i) {
-      const int m_blk = tile % tiles_m, n_blk = tile / tiles_m;
+    for (int tile = unit; tile < n_tiles && ok; tile += units, ++tile_i) {
+      int m_blk, n_blk;
+      tile_place<TILE_ROWS>(tile, tiles_m, tiles_n, m_blk, n_blk);
       const int a = tile_i % ACC_SETS;
-      const int row0 = (m_blk * MT + half) * TC_BM + quarter * 32;  // the warp's first row
+      const int row0 = m_blk * TILE_ROWS + rank * TC_BM + quarter * 32;  // the warp's first row
       // a pending norm of the input (RowScale): this lane's row's 1 / rms, from the parts the product before
       // this one left, added in part order while the tile's products still run
       float row_inv = 1.f;
@@ -191,7 +235,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       ok = mbar_wait(smem_u32(&acc_full[a]), (tile_i / ACC_SETS) & 1, abort_flag);
       if (!ok) break;
       fence_after();
-      const uint32_t tmem_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (a * MT + half) * TC_BN;
+      const uint32_t tmem_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + a * TC_BN;
       const int col0 = n_blk * N_PER_TILE;
       // A thread holds one ROW of the accumulator; written as it is, every store instruction of the
       // warp would touch 32 lines.  The warp turns each 32 x 32 patch around in shared memory and
@@ -293,16 +337,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         }
       }
       fence_before();
-      mbar_arrive(smem_u32(&acc_empty[a]));
+      if (PAIR) mbar_arrive_remote(first_block_address(smem_u32(&acc_empty[a])));
+      else mbar_arrive(smem_u32(&acc_empty[a]));
     }
     if (!ok && lane == 0) { *abort_flag = 1; if (error_flag != nullptr) atomicExch(error_flag, 3); }
   }
 
   fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();  // neither block leaves while the other may still arrive on its barriers or read its shared memory
   if (warp == 1) {
     fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TC_TMEM_COLS));
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TC_TMEM_COLS));
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TC_TMEM_COLS));
   }
 }
 
@@ -311,29 +358,39 @@ static bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int
   return sm100::make_map_bf16_2d(map, base, rows, cols, ld, 128);
 }
 
-template <int MODE, int MT, typename TO>
+template <int MODE, bool PAIR, typename TO>
 int launch_tcgen05_tiled(void* out, const CUtensorMap& map_x, const CUtensorMap& map_w, int M, int N, int K, int ldo,
                          int up_rows, int* error_flag, int sm_count, const NormEmit& emit, const RowScale& scale,
                          cudaStream_t stream) {
-  auto kernel = gemm_tcgen05_kernel<MODE, MT, TO>;
+  auto kernel = gemm_tcgen05_kernel<MODE, PAIR, TO>;
   static bool allowed = false;
   if (!allowed) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TcShape<MT>::SMEM);
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TcShape<PAIR>::SMEM);
     if (err != cudaSuccess) return (int)err;
     allowed = true;
   }
-  constexpr int n_per_tile = MODE == 2 ? TC_BN / 2 : TC_BN;
-  const int tiles = ((M + MT * TC_BM - 1) / (MT * TC_BM)) * ((N + n_per_tile - 1) / n_per_tile);
-  const int blocks = tiles < sm_count ? tiles : sm_count;
+  constexpr int n_per_tile = MODE == 2 ? TC_BN / 2 : TC_BN, tile_rows = (PAIR ? 2 : 1) * TC_BM;
+  const int tiles = ((M + tile_rows - 1) / tile_rows) * ((N + n_per_tile - 1) / n_per_tile);
+  const int units = PAIR ? sm_count / 2 : sm_count;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((tiles < units ? tiles : units) * (PAIR ? 2 : 1));
+  config.blockDim = dim3(TcShape<PAIR>::THREADS);
+  config.dynamicSmemBytes = TcShape<PAIR>::SMEM;
+  config.stream = stream;
   // (no programmatic dependent launch: see attention_prefill_tcgen05.cu's launcher)
-  kernel<<<blocks, TcShape<MT>::THREADS, TcShape<MT>::SMEM, stream>>>(map_x, map_w, (TO*)out, M, N, K, ldo, up_rows,
-                                                                      error_flag, emit, scale);
+  cudaLaunchAttribute attrs[1];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = 2; attrs[0].val.clusterDim.y = 1; attrs[0].val.clusterDim.z = 1;
+  config.attrs = attrs;
+  config.numAttrs = PAIR ? 1 : 0;
+  cudaLaunchKernelEx(&config, kernel, map_x, map_w, (TO*)out, M, N, K, ldo, up_rows, error_flag, emit, scale);
   return launch_status();
 }
 
-// Tiles of 256 rows for products of few tiles, when they keep the multiprocessors about as busy as
-// tiles of 128 rows would (the larger tile moves a third fewer operand bytes per flop and drains its
-// accumulator with twice the warps; with many tiles the overlap of the small tile's two accumulators wins).
+// Pairs of blocks, except where their tiles of 256 rows take more rounds of the multiprocessors (600 rows, 14,336 gated
+// outputs: 155 us against 137), or pad the rows by more than a tenth beyond tiles of 128 (600 rows, 6,144 outputs: 35
+// against 31), then only if single blocks would leave four multiprocessors in ten without a tile (600 rows, 4,096 outputs,
+// 14,336 inputs: 94 against 114).
 // Tuning::gemm_tile_rows = 128 or 256 forces one, for comparison.
 template <int MODE, typename TO>
 int launch_tcgen05(void* out, const CUtensorMap& map_x, const CUtensorMap& map_w, int M, int N, int K, int ldo,
@@ -341,15 +398,16 @@ int launch_tcgen05(void* out, const CUtensorMap& map_x, const CUtensorMap& map_w
                    cudaStream_t stream) {
   constexpr int n_per_tile = MODE == 2 ? TC_BN / 2 : TC_BN;
   const long long tiles_n = (N + n_per_tile - 1) / n_per_tile;
-  auto busy = [&](long long tiles) { return (double)tiles / (double)(((tiles + sm_count - 1) / sm_count) * sm_count); };
-  const long long small_tiles = ((M + 127) / 128) * tiles_n;
-  const double small = busy(small_tiles), large = 1.25 * busy(((M + 255) / 256) * tiles_n);
+  const long long rows_128 = (M + 127) / 128 * 128, rows_256 = (M + 255) / 256 * 256;
+  const long long tiles_128 = rows_128 / 128 * tiles_n, tiles_256 = rows_256 / 256 * tiles_n;
+  auto rounds = [](long long tiles, int units) { return (tiles + units - 1) / units; };
   const int forced = tuning().gemm_tile_rows;
-  // measured at 2,048 and 8,192 rows: the large tile wins where the small one leaves under two rounds of work
-  const bool use_large = forced == 256 || (forced != 128 && M > 128 && small_tiles <= 2 * sm_count && large > small);
-  if (use_large)
-    return launch_tcgen05_tiled<MODE, 2, TO>(out, map_x, map_w, M, N, K, ldo, up_rows, error_flag, sm_count, emit, scale, stream);
-  return launch_tcgen05_tiled<MODE, 1, TO>(out, map_x, map_w, M, N, K, ldo, up_rows, error_flag, sm_count, emit, scale, stream);
+  const bool pair = forced == 256 || (forced != 128 && M > 128 && sm_count >= 2 &&
+                                      rounds(tiles_256, sm_count / 2) <= rounds(tiles_128, sm_count) &&
+                                      (rows_256 * 10 <= rows_128 * 11 || tiles_128 * 10 < 6ll * sm_count));
+  if (pair)
+    return launch_tcgen05_tiled<MODE, true, TO>(out, map_x, map_w, M, N, K, ldo, up_rows, error_flag, sm_count, emit, scale, stream);
+  return launch_tcgen05_tiled<MODE, false, TO>(out, map_x, map_w, M, N, K, ldo, up_rows, error_flag, sm_count, emit, scale, stream);
 }
 
 }  // namespace xrt

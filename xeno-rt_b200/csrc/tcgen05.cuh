@@ -59,6 +59,26 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
                ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar), "l"(policy) : "memory");
 }
 
+// Two blocks as one (cta_group::2): the pair is a cluster of two, block 0 of it issues the MMAs, and both blocks' copies
+// complete on block 0's barriers.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of the same place in the first block's shared memory, as the cluster sees it.
+__device__ __forceinline__ uint32_t first_block_address(uint32_t addr) {
+  uint32_t mapped;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(mapped) : "r"(addr));
+  return mapped;
+}
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+// A tile into this block's shared memory that completes on a barrier of either block of the pair.  No multicast.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t cluster_bar) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(cluster_bar) : "memory");
+}
+
 // Shared-memory matrix descriptor of a K-major operand: rows of 128 bytes (64 bfloat16 of the
 // contraction), 128-byte swizzle, groups of eight rows 1024 bytes apart (stride byte offset, bits
 // [32, 46)), start address in bits [0, 14), descriptor version 1 in bits [46, 48), layout type
@@ -93,6 +113,18 @@ __device__ __forceinline__ void mma_f16_a_tmem(uint32_t tmem_d, uint32_t tmem_a,
   asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
                " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
                ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// One MMA of the pair: A is 2 x 128 rows, B 2 halves of N, each half in its block's shared memory at the same place;
+// each block's tensor memory gets its 128 rows of D.
+__device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+               " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
+               ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// One arrival on the barrier at this place in BOTH blocks when every MMA of the pair issued so far has completed.
+__device__ __forceinline__ void commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 // The barrier gets one arrival when every tcgen05.mma issued so far by this thread has completed.
 __device__ __forceinline__ void commit(uint32_t bar) {
