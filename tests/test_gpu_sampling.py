@@ -135,3 +135,48 @@ def test_small_top_k_over_a_big_vocabulary_gathered_or_not():
     assert set(got.tolist()) <= set(ids.tolist())
     top = int(ids[np.argmax(probs)])
     assert abs((got == top).mean() - probs.max()) < 4 * np.sqrt(probs.max() * (1 - probs.max()) / 4000) + 1e-3
+
+
+# one block a row, two, eight; a slice that just fits the blocks' shared memory and one that does not; rows of whole 16 bytes or not
+@pytest.mark.parametrize("vocab", [1, 33, 4096, 4097, 16390, 128256, 327680, 327685])
+@pytest.mark.parametrize("temperature,top_k,top_p", [(0.8, 40, 0.95), (1.0, 300, 0.9), (1.0, 0, 0.9), (0.7, 0, 1.0)])
+def test_a_draw_lands_where_the_mass_says(vocab, temperature, top_k, top_p):
+    """The id of a draw u is the one whose share of the kept mass, walked in index order, covers u.  The kernel's masses are
+    rounded down to 2^-32 of the largest, and 32-bit exponentials are off by 2e-7 of their value: the walk may be off by
+    vocab * 2^-32 + 1e-6; an id at the edge of the kept set, which either rounding may put in or out, holds less than 1e-5."""
+    from xeno_rt_b200.sampling import sequence_key
+    rng = np.random.default_rng(vocab + top_k)
+    logits = (rng.normal(size=vocab) * 2.0).astype(np.float32)
+    if vocab > 1000:
+        logits[rng.random(vocab) < 0.3] = -np.inf
+    n, mask = 24, (1 << 64) - 1
+    got = run_sampler(logits, n, temperature, top_k, top_p, 1.0, seed=3)
+    ids, probs = ps.candidate_distribution(logits.astype(np.float64), (), temperature, top_k, top_p, 1.0)
+    order = np.argsort(ids)
+    upper = dict(zip(ids[order].tolist(), np.cumsum(probs[order]).tolist()))
+    share = dict(zip(ids.tolist(), probs.tolist()))
+
+    def splitmix(x):
+        x = (x + 0x9E3779B97F4A7C15) & mask
+        x = ((x ^ (x >> 30)) * 0xBF58476D1CE4E5B9) & mask
+        x = ((x ^ (x >> 27)) * 0x94D049BB133111EB) & mask
+        return x ^ (x >> 31)
+
+    slack = vocab * 2.0 ** -32 + 1.2e-5
+    for i, token in enumerate(got.tolist()):
+        u = (splitmix((sequence_key(3 * 100003 + i) + 0x9E3779B97F4A7C15) & mask) >> 32) / 2.0 ** 32
+        assert token in upper
+        assert upper[token] - share[token] - slack <= u <= upper[token] + slack
+
+
+def test_rows_without_a_finite_maximum_and_with_nan():
+    """Only ids above minus infinity are drawn; one infinity takes the row; a row without any value gives its first id."""
+    for vocab in (300, 20001):
+        logits = np.full(vocab, -np.inf, dtype=np.float32)
+        assert set(run_sampler(logits, 8, 1.0, 40, 0.9, 1.0).tolist()) == {0}
+        logits[[7, vocab - 2]] = 1.0
+        assert set(run_sampler(logits, 64, 1.0, 40, 1.0, 1.0).tolist()) == {7, vocab - 2}
+        assert set(run_sampler(logits, 64, 1.0, 0, 0.99, 1.0).tolist()) == {7, vocab - 2}
+        logits[5] = np.nan
+        assert set(run_sampler(logits, 64, 1.0, 2, 1.0, 1.0).tolist()) == {7, vocab - 2}
+        assert set(run_sampler(logits, 8, 0.0, 0, 1.0, 1.0).tolist()) == {7}

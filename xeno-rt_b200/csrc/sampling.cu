@@ -1,4 +1,4 @@
-// Sampling on the device, one thread block per row of 32-bit logits.
+// Sampling on the device, one team of thread blocks per row of 32-bit logits.
 //
 // What the reference's sampler computes (crates/xrt-runtime/src/sampler.rs):
 //   repetition penalty p > 1 on every id seen in the history: l > 0 ? l / p : l * p      :77-91, 110-125
@@ -16,12 +16,28 @@
 // splitmix64(key[slot] + (counter[slot] + 1) * 0x9E3779B97F4A7C15), counter[slot] += 1 a draw.
 // Probability mass is summed as 64-bit integers (probability * 2^32), so sums do not depend on
 // the order in which threads add and a seed gives the same tokens on every run.
+//
+// A row is worked on by a team of up to eight blocks (one thread-block cluster), each with a contiguous slice of the
+// vocabulary: a row of 128,256 logits is half a megabyte, and one block alone was bound by the latency of its passes over it.
+// A block reads its slice once, applies the penalty and keeps the values in shared memory.  A small top_k leaves few
+// candidates, which the first block finishes by itself; without one, the team goes through the
+// selects together, meeting once a pass.
+// Measured, microseconds, one block a row -> teams: 128,256 logits, top_k 40, top_p 0.95, 1 row 137 -> 22, 64 rows 145 -> 59; top_p
+// alone 463 -> 58 and 483 -> 162; greedy 16 -> 5 and 17 -> 14; 4 rows of 256 logits 45 -> 10.  64 rows: bound by the
+// multiprocessors' instructions (16,032 logits a block, three and a half blocks on each); memory would take 5.
 #include "common.cuh"
 
 namespace xrt {
 
-constexpr int SAMPLE_THREADS = 1024;
-constexpr int HIST_COPIES = SAMPLE_THREADS / 64;  // private histograms of the radix select
+constexpr int SAMPLE_THREADS = 512, SAMPLE_WARPS = SAMPLE_THREADS / 32;
+constexpr int SAMPLE_TEAM = 8;                             // blocks of a team at most
+constexpr int SAMPLE_HIST_COPIES = SAMPLE_THREADS / 64;    // private histograms of the radix select
+constexpr int SAMPLE_FINE_BINS = 4096;                     // of the first histogram: the order key's top 12 bits
+constexpr int SAMPLE_HIST_BYTES = SAMPLE_FINE_BINS * 4;    // also room for the private histograms, and for a block's candidates
+constexpr int SAMPLE_CANDIDATES = 4096;                    // of a small top_k, all blocks together
+constexpr int SAMPLE_NARROW = 192;                         // so many candidates are cut down once more
+constexpr int SAMPLE_CACHED_BYTES = 160 * 1024;            // of logits a block keeps at most
+static_assert(SAMPLE_HIST_COPIES * 256 * 8 <= SAMPLE_HIST_BYTES && SAMPLE_CANDIDATES * 8 <= 32 * 1024, "the regions hold");
 
 __device__ __forceinline__ uint64_t sm64(uint64_t x) {
   x += 0x9E3779B97F4A7C15ull;
@@ -82,310 +98,516 @@ __device__ uint64_t block_exclusive_scan(uint64_t v, uint64_t* warp_totals, uint
   return warp_totals[warp] + inc - v;
 }
 
-// The first index, in index order, at which the running sum of weight(i) exceeds `target`;
-// -1 if the whole sum does not.  Each thread owns a contiguous segment of indices.
-template <typename F>
-__device__ int ordered_pick(F weight, int n, uint64_t target, uint64_t* scan_scratch, int* result) {
-  const int seg = (n + blockDim.x - 1) / blockDim.x;
-  const int lo = min(n, (int)threadIdx.x * seg), hi = min(n, lo + seg);
+// ------------------------------------------------------------------------------------------ the team
+__device__ __forceinline__ void team_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void team_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ void team_sync() { team_arrive(); team_wait(); }
+// The same variable in the shared memory of block `rank` of the team.
+template <typename T>
+__device__ __forceinline__ T* of_block(T* p, int rank) {
+  uint64_t mapped;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(mapped) : "l"(reinterpret_cast<uint64_t>(p)), "r"(rank));
+  return reinterpret_cast<T*>(mapped);
+}
+
+struct SampleShared {
+  uint64_t scan[33];
+  uint64_t exchange[2][SAMPLE_TEAM];   // a number from every block, two meetings in turn
+  uint64_t best[SAMPLE_TEAM];          // every block's largest value and where
+  unsigned long long merged[2][256];   // this block's histogram of a pass, two passes in turn
+  uint64_t selected_inside, selected_at;
+  uint32_t selected_prefix;
+  int selected;
+  int count;                           // this block's candidates, -1: too many
+  int cut;
+  int irregular;                       // a NaN among this block's logits
+  unsigned int draw;
+  long long pick;
+  int warp_count[SAMPLE_WARPS];
+};
+
+struct Team {
+  SampleShared* sh;
+  uint32_t* hist;  // SAMPLE_HIST_BYTES
+  int size, rank, turn;
+};
+
+// Exclusive prefix sum of one value a thread over the team, blocks in rank order, threads in thread order; *total gets the sum.
+template <bool TEAM>
+__device__ uint64_t team_exclusive_scan(uint64_t v, Team& team, uint64_t* total) {
+  uint64_t before = block_exclusive_scan(v, team.sh->scan, total);
+  if (TEAM) {
+    uint64_t* mine = team.sh->exchange[team.turn];
+    team.turn ^= 1;
+    if ((int)threadIdx.x < team.size) of_block(mine, threadIdx.x)[team.rank] = *total;
+    team_sync();
+    uint64_t sum = 0;
+    for (int r = 0; r < team.size; ++r) {
+      if (r == team.rank) before += sum;
+      sum += mine[r];
+    }
+    *total = sum;
+  }
+  return before;
+}
+
+// The first place, in index order, at which the running sum of weight(i) exceeds `target`; -1 if the whole sum does not.
+// Places of a block's elements count from `base`.  A warp owns a contiguous run of elements, its lanes side by side.
+template <bool TEAM, typename F>
+__device__ long long ordered_pick(F weight, int n, int base, uint64_t target, Team& team) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int run = ((n + SAMPLE_WARPS - 1) / SAMPLE_WARPS + 31) & ~31;
+  const int lo = min(n, warp * run), hi = min(n, lo + run);
   uint64_t local = 0;
-#pragma unroll 4
-  for (int i = lo; i < hi; ++i) local += weight(i);
-  if (threadIdx.x == 0) *result = -1;
+  for (int i = lo + lane; i < hi; i += 32) local += weight(i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, (unsigned long long)local, o);
+  if (threadIdx.x == 0) team.sh->pick = -1;
   uint64_t total;
-  const uint64_t before = block_exclusive_scan(local, scan_scratch, &total);
-  if (before <= target && target < before + local) {
-    uint64_t c = before;
-    for (int i = lo; i < hi; ++i) {
-      c += weight(i);
-      if (c > target) { *result = i; break; }
+  uint64_t before = team_exclusive_scan<TEAM>(lane == 0 ? local : 0, team, &total);
+  before = __shfl_sync(0xffffffffu, (unsigned long long)before, 0);
+  if (before <= target && target < before + local) {  // one warp of the team
+    for (int i0 = lo; i0 < hi; i0 += 32) {
+      const int i = i0 + lane;
+      uint64_t inc = i < hi ? weight(i) : 0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t up = shfl_up64(inc, d);
+        if (lane >= d) inc += up;
+      }
+      const unsigned reached = __ballot_sync(0xffffffffu, before + inc > target);
+      if (reached) {
+        const long long place = (long long)base + i0 + (__ffs(reached) - 1);
+        if (TEAM) {
+          if (lane < team.size) *of_block(&team.sh->pick, lane) = place;
+        } else if (lane == 0) {
+          team.sh->pick = place;
+        }
+        break;
+      }
+      before += __shfl_sync(0xffffffffu, (unsigned long long)inc, 31);
     }
   }
-  __syncthreads();
-  const int found = *result;
-  __syncthreads();  // the next call resets *result
+  if (TEAM) team_sync();
+  else __syncthreads();
+  const long long found = team.sh->pick;
+  __syncthreads();  // the next call resets it
   return found;
 }
 
-// Radix select from the top: the largest key K such that the weight of {key >= K} reaches `want`.
+// Radix select from the top: the largest key K such that the weight of {key >= K} reaches `want` (>= 1).
 // Returns the key; *inside gets want minus the weight of {key > K} (what the keys equal to K still
-// have to supply, >= 1 if want >= 1) and *at_key the weight of {key == K}.  If the whole weight is
-// below `want`, returns 0 with *inside = 0.
-template <typename A, typename F>
-__device__ uint32_t radix_select(A adjusted, F weight, int n, uint64_t want, unsigned long long* hist,
-                                 uint64_t* inside, uint64_t* at_key, uint32_t* shared_prefix) {
+// have to supply) and *at_key the weight of {key == K}.  If the whole weight is below `want`, returns 0 with *inside = 0.
+// weight <= 2^32.  `wide`: so many elements that a bin's sum of 16-bit halves could pass 32 bits.
+template <bool TEAM, typename A, typename F>
+__device__ uint32_t radix_select(A adjusted, F weight, int n, uint64_t want, bool wide, Team& team, uint64_t* inside,
+                                 uint64_t* at_key) {
+  SampleShared* sh = team.sh;
   uint32_t prefix = 0, mask = 0;
   uint64_t remaining = want;
   for (int pass = 3; pass >= 0; --pass) {
     const int shift = pass * 8;
-    // HIST_COPIES private histograms (a pair of warps shares one): logits crowd into a few bins
-    // of the leading byte, and a thousand threads adding to the same shared-memory word serialise
-    unsigned long long* mine = hist + 258 + (threadIdx.x >> 6) * 256;
-    for (int b = threadIdx.x; b < HIST_COPIES * 256; b += blockDim.x) hist[258 + b] = 0ull;
+    // private histograms (a pair of warps shares one): logits crowd into a few bins of the leading byte.  A bin is two
+    // 32-bit sums, of the weights' low and high 16 bits: adding 64 bits to shared memory is a compare-and-swap loop.
+    uint32_t* mine = team.hist + (threadIdx.x >> 6) * 512;
+    for (int b = threadIdx.x; b < SAMPLE_HIST_COPIES * 512; b += SAMPLE_THREADS) team.hist[b] = 0u;
+    if (threadIdx.x == 0) sh->selected = 0;
     __syncthreads();
-    auto count = [&](int i, float a) {
+    for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) {
+      const float a = adjusted(i);
       const uint32_t k = order_key(a);
       if ((k & mask) == prefix) {
         const uint64_t w = weight(i, a);
-        if (w) atomicAdd(&mine[(k >> shift) & 255u], (unsigned long long)w);
-      }
-    };
-    {
-      // four loads in flight a thread; the histogram updates follow them
-      int i = threadIdx.x;
-      for (; i + 3 * (int)blockDim.x < n; i += 4 * blockDim.x) {
-        float a[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) a[u] = adjusted(i + u * blockDim.x);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) count(i + u * blockDim.x, a[u]);
-      }
-      for (; i < n; i += blockDim.x) count(i, adjusted(i));
-    }
-    __syncthreads();
-    for (int b = threadIdx.x; b < 256; b += blockDim.x) {
-      unsigned long long sum = 0ull;
-#pragma unroll
-      for (int c = 0; c < HIST_COPIES; ++c) sum += hist[258 + c * 256 + b];
-      hist[b] = sum;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      uint64_t above = 0;
-      int bin = 255;
-      for (; bin >= 0; --bin) {
-        if (above + hist[bin] >= remaining) break;
-        above += hist[bin];
-      }
-      if (bin < 0) {  // not enough weight in all: keep everything
-        shared_prefix[0] = 0u; shared_prefix[1] = 1u;
-        hist[256] = 0ull; hist[257] = 0ull;
-      } else {
-        shared_prefix[0] = prefix | ((uint32_t)bin << shift); shared_prefix[1] = 0u;
-        hist[256] = remaining - above; hist[257] = hist[bin];
+        const uint32_t bin = (k >> shift) & 255u;
+        if (wide) {
+          if (w) atomicAdd(reinterpret_cast<unsigned long long*>(mine) + bin, (unsigned long long)w);
+        } else {
+          const uint32_t low = (uint32_t)w & 0xffffu, high = (uint32_t)(w >> 16);
+          if (low) atomicAdd(&mine[2 * bin], low);
+          if (high) atomicAdd(&mine[2 * bin + 1], high);
+        }
       }
     }
     __syncthreads();
-    if (shared_prefix[1]) { *inside = 0; *at_key = 0; __syncthreads(); return 0u; }
-    prefix = shared_prefix[0];
+    unsigned long long* merged = sh->merged[pass & 1];
+    unsigned long long sum = 0ull;
+    const int bin = 255 - (int)threadIdx.x;  // from the top
+    if (bin >= 0) {
+#pragma unroll
+      for (int c = 0; c < SAMPLE_HIST_COPIES; ++c) {
+        if (wide) sum += reinterpret_cast<unsigned long long*>(team.hist)[c * 256 + bin];
+        else sum += (unsigned long long)team.hist[c * 512 + 2 * bin] + ((unsigned long long)team.hist[c * 512 + 2 * bin + 1] << 16);
+      }
+    }
+    if (TEAM) {
+      if (bin >= 0) merged[bin] = sum;
+      team_sync();
+      sum = 0ull;
+      if (bin >= 0)
+        for (int r = 0; r < team.size; ++r) sum += of_block(merged, r)[bin];
+    }
+    uint64_t total;
+    const uint64_t above = block_exclusive_scan(sum, sh->scan, &total);
+    if (above < remaining && remaining <= above + sum) {  // one thread, unless there is not enough weight in all
+      sh->selected = 1;
+      sh->selected_prefix = prefix | ((uint32_t)bin << shift);
+      sh->selected_inside = remaining - above;
+      sh->selected_at = sum;
+    }
+    __syncthreads();
+    if (!sh->selected) {
+      *inside = 0; *at_key = 0;
+      __syncthreads();
+      return 0u;
+    }
+    prefix = sh->selected_prefix;
     mask |= 255u << shift;
-    remaining = hist[256];
-    *at_key = hist[257];
+    remaining = sh->selected_inside;
+    *at_key = sh->selected_at;
     __syncthreads();
   }
   *inside = remaining;
   return prefix;
 }
 
-constexpr int SAMPLE_CANDIDATES = 4096;                      // room for the candidates of a small top_k
-constexpr int SAMPLE_DYNAMIC_BYTES = SAMPLE_CANDIDATES * 8;  // their ids and values; first the 4,096-bin histogram
-
-__global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int vocab,
-              const int* __restrict__ row_slot, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const float* __restrict__ top_p,
-              const float* __restrict__ penalty, const uint32_t* __restrict__ seen, int seen_words,
-              const unsigned long long* __restrict__ rng_key, unsigned int* __restrict__ rng_counter) {
-  __shared__ unsigned long long hist[258 + HIST_COPIES * 256];  // merged bins, two result words, private copies
-  __shared__ uint64_t scan_scratch[33];
-  __shared__ float red_val[32];
-  __shared__ int red_idx[32];
-  __shared__ uint32_t shared_prefix[2];
-  __shared__ int pick_result;
-  __shared__ float bcast_max;
-  __shared__ int bcast_arg;
-  __shared__ int cut_bin, cut_count;
-  extern __shared__ __align__(16) unsigned char dynamic[];
-  int* cand_id = reinterpret_cast<int*>(dynamic);
-  float* cand_val = reinterpret_cast<float*>(dynamic + SAMPLE_CANDIDATES * 4);
-  unsigned int* fine_hist = reinterpret_cast<unsigned int*>(dynamic);  // 4,096 bins, before the candidates are written
-
-  pdl_trigger();
-  pdl_wait(logits, row_slot, temperature, top_k, top_p, penalty, seen);
-  const int row = blockIdx.x;
-  const int slot = row_slot[row];
-  if (slot < 0) { if (threadIdx.x == 0) out_ids[row] = -1; return; }
-  RowView view;
-  view.logits = logits + (size_t)row * vocab;
-  view.penalty = penalty[row];
-  view.seen = (seen != nullptr && view.penalty > 1.0f) ? seen + (size_t)slot * seen_words : nullptr;
-  const float temp = temperature[row];
-  const int k = top_k[row];
-
-  // A small top_k first gathers its candidates: one pass counts the adjusted logits into 4,096 bins
-  // of the order key's top 12 bits, the bin that holds the k-th largest is found, and every element
-  // of that bin or above (k plus what shares the bin) is copied to shared memory IN INDEX ORDER
-  // (a thread owns a contiguous run of ids; its offset comes from a scan of the counts).  All later
-  // steps run over these few candidates instead of the vocabulary: the kept set, its masses and the
-  // draw are the same, since they only ever look at elements at or above the top_k threshold.
-  int n = vocab;  // elements the later steps walk: the vocabulary, or the candidates
-  bool compact = false;
-  if (temp > 1e-5f && k > 0 && k < vocab) {
-    for (int b = threadIdx.x; b < 4096; b += blockDim.x) fine_hist[b] = 0u;
-    __syncthreads();
-    {
-      int i = threadIdx.x;
-      for (; i + 7 * (int)blockDim.x < vocab; i += 8 * blockDim.x) {
-        float a[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) a[u] = view.adjusted(i + u * blockDim.x);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) atomicAdd(&fine_hist[order_key(a[u]) >> 20], 1u);
-      }
-      for (; i < vocab; i += blockDim.x) atomicAdd(&fine_hist[order_key(view.adjusted(i)) >> 20], 1u);
-    }
-    __syncthreads();
-    {
-      // thread t looks at bins 4095 - 4t .. 4092 - 4t (from the top); a scan tells how many lie above them
-      uint64_t local = 0;
-      if (threadIdx.x == 0) { cut_bin = 0; cut_count = vocab; }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) local += fine_hist[4095 - 4 * (int)threadIdx.x - j];
-      uint64_t total;
-      const uint64_t before = block_exclusive_scan(local, scan_scratch, &total);
-      if (before < (uint64_t)k && (uint64_t)k <= before + local) {
-        uint64_t above = before;
-        for (int j = 0; j < 4; ++j) {
-          const int bin = 4095 - 4 * (int)threadIdx.x - j;
-          above += fine_hist[bin];
-          if (above >= (uint64_t)k) { cut_bin = bin; cut_count = (int)above; break; }
-        }
-      }
-      __syncthreads();
-    }
-    if (cut_count <= SAMPLE_CANDIDATES) {
-      const uint32_t cut = (uint32_t)cut_bin;
-      const int total_kept = cut_count;
-      const int seg = (vocab + blockDim.x - 1) / blockDim.x;
-      const int lo = min(vocab, (int)threadIdx.x * seg), hi = min(vocab, lo + seg);
-      uint64_t mine = 0;
-      for (int i = lo; i < hi; ++i) mine += (order_key(view.adjusted(i)) >> 20) >= cut;
-      uint64_t total;
-      uint64_t at = block_exclusive_scan(mine, scan_scratch, &total);  // also: every thread is done with the histogram
-      for (int i = lo; i < hi && mine > 0; ++i) {
-        const float a = view.adjusted(i);
-        if ((order_key(a) >> 20) >= cut) { cand_id[at] = i; cand_val[at] = a; ++at; }
-      }
-      __syncthreads();
-      compact = true;
-      n = total_kept;
-    } else {
-      __syncthreads();
-    }
-  }
-  auto adjusted = [&](int j) { return compact ? cand_val[j] : view.adjusted(j); };
-  auto id_of = [&](int j) { return compact ? cand_id[j] : j; };
-
-  // maximum and its first index
-  float best = -INFINITY; int best_i = 0x7fffffff;
-  {
-    // eight loads in flight a thread: a row is read once and the pass is bound by load latency
-    constexpr int UNROLL = 8;
-    int i = threadIdx.x;
-    for (; i + (UNROLL - 1) * (int)blockDim.x < n; i += UNROLL * blockDim.x) {
-      float a[UNROLL];
-#pragma unroll
-      for (int u = 0; u < UNROLL; ++u) a[u] = adjusted(i + u * blockDim.x);
-#pragma unroll
-      for (int u = 0; u < UNROLL; ++u)
-        if (a[u] > best) { best = a[u]; best_i = i + u * blockDim.x; }  // indices rise: the first maximum is kept
-    }
-    for (; i < n; i += blockDim.x) {
-      const float a = adjusted(i);
-      if (a > best) { best = a; best_i = i; }
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-    if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
-  }
-  if ((threadIdx.x & 31) == 0) { red_val[threadIdx.x >> 5] = best; red_idx[threadIdx.x >> 5] = best_i; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float b = red_val[0]; int bi = red_idx[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-      if (red_val[w] > b || (red_val[w] == b && red_idx[w] < bi)) { b = red_val[w]; bi = red_idx[w]; }
-    bcast_max = b; bcast_arg = bi == 0x7fffffff ? 0 : bi;
-  }
-  __syncthreads();
-  const float row_max = bcast_max;
-  const int row_arg = id_of(bcast_arg);
-
-  unsigned int counter = 0;
-  if (threadIdx.x == 0) { counter = rng_counter[slot]; rng_counter[slot] = counter + 1; }
-  if (temp <= 1e-5f) { if (threadIdx.x == 0) out_ids[row] = row_arg; return; }
-
-  auto key_of = [&](int i) { return order_key(adjusted(i)); };
-  // this thread's share of the sum of weight(i, adjusted(i)) over the elements, four loads in flight
-  auto strided_sum = [&](auto weight) {
-    uint64_t local = 0;
-    int i = threadIdx.x;
-    for (; i + 3 * (int)blockDim.x < n; i += 4 * blockDim.x) {
-      float a[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) a[u] = adjusted(i + u * blockDim.x);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) local += weight(i + u * blockDim.x, a[u]);
-    }
-    for (; i < n; i += blockDim.x) local += weight(i, adjusted(i));
-    return local;
-  };
-
-  // top-k: threshold key and the last index kept among equal keys
-  uint32_t k_key = 0u; int k_last = n;  // kept: key > k_key, or key == k_key and i <= k_last
-  if (k > 0 && k < n) {
+// From the values to the id: top_k, top_p and the draw over `n` elements of this block, whose places count from `base`.
+// TEAM: over the elements of all blocks.  Returns the place of the id, -1 if no mass was left.
+template <bool TEAM, typename A>
+__device__ long long sample_place(A adjusted, int n, int base, long long n_all, int k, float temp, float p, float row_max,
+                                  bool wide, Team& team) {
+  // top-k: threshold key and the last place kept among equal keys
+  uint32_t k_key = 0u; long long k_last = n_all;  // kept: key > k_key, or key == k_key and place <= k_last
+  if (k > 0 && k < n_all) {
     uint64_t inside, at_key;
     auto one = [&](int, float) { return (uint64_t)1; };
-    k_key = radix_select(adjusted, one, n, (uint64_t)k, hist, &inside, &at_key, shared_prefix);
+    k_key = radix_select<TEAM>(adjusted, one, n, (uint64_t)k, wide, team, &inside, &at_key);
     if (at_key > inside) {
-      auto tie = [&](int i) { return (uint64_t)(key_of(i) == k_key); };
-      k_last = ordered_pick(tie, n, inside - 1, scan_scratch, &pick_result);
+      auto tie = [&](int i) { return (uint64_t)(order_key(adjusted(i)) == k_key); };
+      k_last = ordered_pick<TEAM>(tie, n, base, inside - 1, team);
     }
   }
   const float inv_temp = 1.0f / temp;
   auto mass_of = [&](int i, float a) -> uint64_t {
     const uint32_t key = order_key(a);
-    if (key < k_key || (key == k_key && i > k_last)) return 0ull;
+    if (key < k_key || (key == k_key && base + i > k_last)) return 0ull;
     return (uint64_t)(expf((a - row_max) * inv_temp) * 4294967296.0f);
   };
-  auto mass = [&](int i) -> uint64_t { return mass_of(i, adjusted(i)); };
-
   // top-p: threshold by probability mass
-  uint32_t p_key = 0u; int p_last = n;
-  const float p = top_p[row];
+  uint32_t p_key = 0u; long long p_last = n_all;
   if (p < 1.0f) {
-    const uint64_t local = strided_sum(mass_of);
-    uint64_t total;
-    block_exclusive_scan(local, scan_scratch, &total);
+    uint64_t local = 0, total;
+    for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) local += mass_of(i, adjusted(i));
+    team_exclusive_scan<TEAM>(local, team, &total);
     uint64_t want = (uint64_t)ceil((double)p * (double)total);
     if (want < 1) want = 1;
     uint64_t inside, at_key;
-    p_key = radix_select(adjusted, mass_of, n, want, hist, &inside, &at_key, shared_prefix);
+    p_key = radix_select<TEAM>(adjusted, mass_of, n, want, wide, team, &inside, &at_key);
     if (at_key > inside) {
       // equal keys have equal mass: how many of them the remaining mass needs
-      auto tie_mass = [&](int i) { return key_of(i) == p_key ? mass(i) : 0ull; };
-      p_last = ordered_pick(tie_mass, n, inside - 1, scan_scratch, &pick_result);
+      auto tie_mass = [&](int i) { const float a = adjusted(i); return order_key(a) == p_key ? mass_of(i, a) : 0ull; };
+      p_last = ordered_pick<TEAM>(tie_mass, n, base, inside - 1, team);
     }
   }
-  auto kept_mass_of = [&](int i, float a) -> uint64_t {
+  auto kept_mass = [&](int i) -> uint64_t {
+    const float a = adjusted(i);
     const uint32_t key = order_key(a);
-    if (key < p_key || (key == p_key && i > p_last)) return 0ull;
+    if (key < p_key || (key == p_key && base + i > p_last)) return 0ull;
     return mass_of(i, a);
   };
-  auto kept_mass = [&](int i) -> uint64_t { return kept_mass_of(i, adjusted(i)); };
+  uint64_t local = 0, total;
+  for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) local += kept_mass(i);
+  team_exclusive_scan<TEAM>(local, team, &total);
+  const uint64_t target = __umul64hi((uint64_t)team.sh->draw << 32, total);  // floor(u / 2^32 * total)
+  return total > 0 ? ordered_pick<TEAM>(kept_mass, n, base, target, team) : -1;
+}
 
-  const uint64_t local = strided_sum(kept_mass_of);
-  uint64_t total;
-  block_exclusive_scan(local, scan_scratch, &total);
-  __shared__ unsigned int shared_u;
-  if (threadIdx.x == 0)
-    shared_u = (unsigned int)(sm64(rng_key[slot] + ((uint64_t)counter + 1ull) * 0x9E3779B97F4A7C15ull) >> 32);
+// `hist` holds, by the top 12 bits of their order keys, numbers that say: at least so many elements lie in this bin.  Cuts
+// at the bin where they reach k from the top (at 0 if they don't) and copies every element from there upwards to
+// out_id / out_val, in index order, if there are no more than `cap`.  Returns how many there are.  The outputs may be the
+// histogram's own room.
+template <typename A, typename I>
+__device__ int cut_and_gather(A adjusted, I id_of, int n, int k, int cap, const uint32_t* hist, SampleShared* sh, int* out_id,
+                              float* out_val) {
+  constexpr int BINS = SAMPLE_FINE_BINS / SAMPLE_THREADS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t local = 0, total;
+  if (threadIdx.x == 0) sh->cut = 0;
+#pragma unroll
+  for (int j = 0; j < BINS; ++j) local += hist[SAMPLE_FINE_BINS - 1 - BINS * (int)threadIdx.x - j];
+  uint64_t above = block_exclusive_scan(local, sh->scan, &total);
+  if (above < (uint64_t)k && (uint64_t)k <= above + local) {
+    for (int j = 0; j < BINS; ++j) {
+      const int bin = SAMPLE_FINE_BINS - 1 - BINS * (int)threadIdx.x - j;
+      above += hist[bin];
+      if (above >= (uint64_t)k) { sh->cut = bin; break; }
+    }
+  }
   __syncthreads();
-  const uint64_t target = __umul64hi((uint64_t)shared_u << 32, total);  // floor(u / 2^32 * total)
-  const int pick = total > 0 ? ordered_pick(kept_mass, n, target, scan_scratch, &pick_result) : -1;
-  if (threadIdx.x == 0) out_ids[row] = pick >= 0 ? id_of(pick) : row_arg;
+  const uint32_t cut = (uint32_t)sh->cut;
+  if (cut == 0 && n > cap) return n;
+  const int run = ((n + SAMPLE_WARPS - 1) / SAMPLE_WARPS + 31) & ~31;
+  const int lo = min(n, warp * run), hi = min(n, lo + run);
+  int mine = 0;
+  for (int i0 = lo; i0 < hi; i0 += 32) {
+    const int i = i0 + lane;
+    mine += __popc(__ballot_sync(0xffffffffu, i < hi && (order_key(adjusted(i)) >> 20) >= cut));
+  }
+  if (lane == 0) sh->warp_count[warp] = mine;
+  __syncthreads();  // also: everybody is done with the histogram
+  int at = 0, count = 0;
+  for (int w = 0; w < SAMPLE_WARPS; ++w) {
+    if (w == warp) at = count;
+    count += sh->warp_count[w];
+  }
+  if (count <= cap) {
+    for (int i0 = lo; i0 < hi && mine > 0; i0 += 32) {
+      const int i = i0 + lane;
+      const float a = i < hi ? adjusted(i) : 0.f;
+      const bool in = i < hi && (order_key(a) >> 20) >= cut;
+      const unsigned mask = __ballot_sync(0xffffffffu, in);
+      if (in) {
+        const int place = at + __popc(mask & ((1u << lane) - 1u));
+        out_id[place] = id_of(i);
+        out_val[place] = a;
+      }
+      at += __popc(mask);
+    }
+  }
+  __syncthreads();
+  return count;
+}
+
+// The same choice as sample_place over no more candidates than threads, each thread its own: its rank is the number of
+// candidates before it by falling value (equal values in index order), the mass before it theirs.  `order` and `mass`:
+// shared memory for SAMPLE_THREADS numbers each.
+__device__ long long ranked_place(float a, int n, int k, float temp, float p, float row_max, uint64_t* order, uint64_t* mass,
+                                  Team& team) {
+  const int i = threadIdx.x;
+  const uint64_t mine = ((uint64_t)order_key(a) << 32) | (uint32_t)~(uint32_t)i;
+  if (i < n) order[i] = mine;
+  if (i == 0) team.sh->pick = -1;
+  __syncthreads();
+  int rank = n;
+  if ((i & ~31) < n) {
+    rank = 0;
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) rank += order[j] > mine;
+  }
+  const uint64_t m = i < n && rank < k ? (uint64_t)(expf((a - row_max) * (1.0f / temp)) * 4294967296.0f) : 0ull;
+  if (i < n) mass[i] = m;
+  uint64_t total;
+  block_exclusive_scan(m, team.sh->scan, &total);
+  uint64_t kept = m;
+  if (p < 1.0f) {
+    uint64_t want = (uint64_t)ceil((double)p * (double)total);
+    if (want < 1) want = 1;
+    uint64_t before = 0;
+    if (__any_sync(0xffffffffu, m != 0)) {
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) before += order[j] > mine ? mass[j] : 0ull;
+    }
+    if (before >= want) kept = 0;
+  }
+  const uint64_t below = block_exclusive_scan(kept, team.sh->scan, &total);
+  const uint64_t target = __umul64hi((uint64_t)team.sh->draw << 32, total);  // floor(u / 2^32 * total)
+  if (total > 0 && below <= target && target < below + kept) team.sh->pick = i;
+  __syncthreads();
+  return team.sh->pick;
+}
+
+// CACHED: a block's slice of the row fits its shared memory (else the passes read it from the L2 again).
+// VEC: rows are whole 16 bytes.
+template <bool CACHED, bool VEC>
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int vocab, int per_block, int values_bytes,
+              const int* __restrict__ row_slot, const float* __restrict__ temperature,
+              const int* __restrict__ top_k, const float* __restrict__ top_p,
+              const float* __restrict__ penalty, const uint32_t* __restrict__ seen, int seen_words,
+              const unsigned long long* __restrict__ rng_key, unsigned int* __restrict__ rng_counter, int team_size) {
+  __shared__ SampleShared sh;
+  extern __shared__ __align__(16) unsigned char dynamic[];
+  float* values = reinterpret_cast<float*>(dynamic);  // the slice; in the first block later the candidates' ids and values
+  uint32_t* hist = reinterpret_cast<uint32_t*>(dynamic + values_bytes);
+
+  pdl_trigger();
+  team_arrive();
+  pdl_wait(logits, row_slot, temperature, top_k, top_p, penalty, seen);
+  Team team = {&sh, hist, team_size, (int)(blockIdx.x % team_size), 0};
+  const int row = blockIdx.x / team_size, rank = team.rank;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int slot = row_slot[row];
+  if (slot < 0) {  // the whole team
+    team_wait();
+    if (rank == 0 && threadIdx.x == 0) out_ids[row] = -1;
+    return;
+  }
+  const int base = (int)min((long long)vocab, (long long)rank * per_block);
+  const int n = min(per_block, vocab - base);
+  RowView view;
+  view.logits = logits + (size_t)row * vocab + base;
+  view.penalty = penalty[row];
+  view.seen = (seen != nullptr && view.penalty > 1.0f) ? seen + (size_t)slot * seen_words + base / 32 : nullptr;
+  const float temp = temperature[row];
+  const int k = top_k[row];
+  const bool few = temp > 1e-5f && k > 0 && k < vocab;  // candidates are gathered first
+
+  // The one pass over the logits: penalty, and every thread's largest value (the first of equals).  For a small top_k a
+  // histogram of the order keys' top 12 bits says where to cut: of the threads' largest values if they are at least twice
+  // as many as k (there are then k elements at or above the cut, and hardly more), else of all values.
+  const bool of_largest = k <= SAMPLE_THREADS / 2;
+  if (few)
+    for (int b = threadIdx.x; b < SAMPLE_FINE_BINS; b += SAMPLE_THREADS) hist[b] = 0u;
+  if (few) __syncthreads();
+  float best = -INFINITY; int best_i = -1, nan_seen = 0;
+  auto take = [&](int i, float a) {
+    if (CACHED) values[i] = a;
+    if (a > best) { best = a; best_i = i; }  // indices rise: the first maximum is kept
+    nan_seen |= a != a;
+    if (few && !of_largest) atomicAdd(&hist[order_key(a) >> 20], 1u);
+  };
+  if (VEC) {
+    constexpr int UNROLL = 4;  // loads in flight a thread
+    const int quads = n / 4;
+    const float4* src = reinterpret_cast<const float4*>(view.logits);
+    for (int q0 = threadIdx.x; q0 < quads; q0 += UNROLL * SAMPLE_THREADS) {
+      float4 v[UNROLL]; uint32_t bits[UNROLL];
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        const int q = q0 + u * SAMPLE_THREADS;
+        v[u] = q < quads ? src[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+        bits[u] = (q < quads && view.seen != nullptr) ? view.seen[q >> 3] >> (4 * (q & 7)) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        const int q = q0 + u * SAMPLE_THREADS;
+        if (q < quads) {
+          float a[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if ((bits[u] >> e) & 1u) a[e] = a[e] > 0.f ? a[e] / view.penalty : a[e] * view.penalty;
+            take(4 * q + e, a[e]);
+          }
+        }
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) take(i, view.adjusted(i));
+  }
+  auto adjusted = [&](int i) { return CACHED ? values[i] : view.adjusted(i); };
+
+  if (few && of_largest) atomicAdd(&hist[best_i < 0 ? 0 : order_key(best) >> 20], 1u);
+  // (larger value, smaller place) as one number; 0 where nothing lies above minus infinity
+  uint64_t packed = best_i < 0 ? 0ull : ((uint64_t)order_key(best + 0.0f) << 32) | (uint32_t)~(uint32_t)(base + best_i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const uint64_t other = __shfl_xor_sync(0xffffffffu, (unsigned long long)packed, o);
+    packed = other > packed ? other : packed;
+  }
+  if (lane == 0) sh.scan[warp] = packed;
+  const int irregular_here = __syncthreads_or(nan_seen);
+  if (threadIdx.x == 0) sh.irregular = irregular_here;
+  if (threadIdx.x < SAMPLE_TEAM) {
+    for (int w = 0; w < SAMPLE_WARPS; ++w) packed = sh.scan[w] > packed ? sh.scan[w] : packed;
+  }
+  __syncthreads();
+
+  // This block's candidates, in index order.  (What the row keeps lies at or above its k-th largest value, which is no
+  // smaller than any block's k-th largest.)
+  int* my_id = reinterpret_cast<int*>(hist);
+  const int quota = min(SAMPLE_CANDIDATES / team_size, SAMPLE_HIST_BYTES / 8);
+  float* my_val = reinterpret_cast<float*>(hist) + quota;
+  if (few) {
+    const int count = cut_and_gather(adjusted, [&](int i) { return base + i; }, n, k, quota, hist, &sh, my_id, my_val);
+    if (threadIdx.x == 0) sh.count = count <= quota ? count : -1;
+  }
+
+  team_wait();  // every block of the team runs: its shared memory may be written
+  if ((int)threadIdx.x < team_size) {
+    of_block(sh.best, threadIdx.x)[rank] = packed;
+    if (rank == 0) {
+      const unsigned int counter = rng_counter[slot];
+      __syncwarp(__activemask());
+      if (threadIdx.x == 0) rng_counter[slot] = counter + 1;
+      *of_block(&sh.draw, threadIdx.x) =
+          (unsigned int)(sm64(rng_key[slot] + ((uint64_t)counter + 1ull) * 0x9E3779B97F4A7C15ull) >> 32);
+    }
+  }
+  team_sync();
+  packed = 0;
+  for (int r = 0; r < team_size; ++r) packed = sh.best[r] > packed ? sh.best[r] : packed;
+  const uint32_t best_key = (uint32_t)(packed >> 32);
+  const float row_max = packed == 0 ? -INFINITY
+                                    : __uint_as_float((best_key & 0x80000000u) ? (best_key & 0x7fffffffu) : ~best_key);
+  const int row_arg = packed == 0 ? 0 : (int)~(uint32_t)packed;
+  if (temp <= 1e-5f || packed == 0) {  // (a row without a value above minus infinity has no probabilities: its first id)
+    if (rank == 0 && threadIdx.x == 0) out_ids[row] = row_arg;
+    return;
+  }
+
+  bool compact = few;
+  int counts[SAMPLE_TEAM];
+  int all = 0;
+  // masses beyond 2^32 (of a NaN, or of an infinity against another) are summed in 64 bits
+  bool wide = n > 65535 * SAMPLE_HIST_COPIES || !(fabsf(row_max) < INFINITY);
+#pragma unroll
+  for (int r = 0; r < SAMPLE_TEAM; ++r) {
+    counts[r] = (few && r < team_size) ? *of_block(&sh.count, r) : 0;
+    if (r < team_size) wide = wide || *of_block(&sh.irregular, r) != 0;
+    compact = compact && counts[r] >= 0;
+    all += counts[r];
+  }
+  const float p = top_p[row];
+  if (compact) {
+    if (rank == 0) {
+      int* ids = reinterpret_cast<int*>(values);
+      float* vals = values + SAMPLE_CANDIDATES;
+      int at = 0;
+#pragma unroll
+      for (int r = 0; r < SAMPLE_TEAM; ++r) {
+        if (r < team_size) {
+          const int* from_id = of_block(my_id, r);
+          const float* from_val = of_block(my_val, r);
+          for (int i = threadIdx.x; i < counts[r]; i += SAMPLE_THREADS) {
+            ids[at + i] = from_id[i];
+            vals[at + i] = from_val[i];
+          }
+        }
+        at += counts[r];
+      }
+      team_sync();  // the candidates are here: the other blocks may leave
+      if (all > SAMPLE_NARROW && k <= SAMPLE_THREADS / 2 && !wide) {
+        for (int b = threadIdx.x; b < SAMPLE_FINE_BINS; b += SAMPLE_THREADS) hist[b] = 0u;
+        __syncthreads();
+        for (int i = threadIdx.x; i < all; i += SAMPLE_THREADS) atomicAdd(&hist[order_key(vals[i]) >> 20], 1u);
+        __syncthreads();
+        int* few_id = reinterpret_cast<int*>(hist);
+        float* few_val = reinterpret_cast<float*>(hist) + SAMPLE_THREADS;
+        const int count = cut_and_gather([&](int i) { return vals[i]; }, [&](int i) { return ids[i]; }, all, k, SAMPLE_THREADS,
+                                         hist, &sh, few_id, few_val);
+        if (count <= SAMPLE_THREADS) {
+          ids = few_id;
+          vals = few_val;
+          all = count;
+        }
+      }
+      long long place;
+      if (all <= SAMPLE_THREADS && !wide) {
+        uint64_t* order = reinterpret_cast<uint64_t*>(hist) + SAMPLE_THREADS;  // beyond the candidates that may lie there
+        place = ranked_place(threadIdx.x < all ? vals[threadIdx.x] : 0.f, all, k, temp, p, row_max, order,
+                             order + SAMPLE_THREADS, team);
+      } else {
+        place = sample_place<false>([&](int i) { return vals[i]; }, all, 0, all, k, temp, p, row_max, wide, team);
+      }
+      if (threadIdx.x == 0) out_ids[row] = place >= 0 ? ids[place] : row_arg;
+    } else {
+      team_sync();
+    }
+    return;
+  }
+  team_sync();  // the counts are read; the histograms start anew
+  const long long place = sample_place<true>(adjusted, n, base, vocab, k, temp, p, row_max, wide, team);
+  if (rank == 0 && threadIdx.x == 0) out_ids[row] = place >= 0 ? (int)place : row_arg;
+  team_sync();  // nobody leaves while its sums may still be read
 }
 
 // Marks token ids as seen in their slot's bitmap (the history the repetition penalty looks at).
@@ -410,15 +632,37 @@ XRT_EXPORT int xrt_sample(int* out_ids, const float* logits, int n_rows, int voc
   if (n_rows < 0 || vocab <= 0) return XRT_ERR_ARGUMENT;
   if (seen != nullptr && seen_words * 32 < vocab) return XRT_ERR_ARGUMENT;
   if (n_rows == 0) return XRT_OK;
-  static bool allowed = false;
-  if (!allowed) {  // static and dynamic shared memory together pass 48 KB
-    cudaError_t err = cudaFuncSetAttribute(xrt::sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           xrt::SAMPLE_DYNAMIC_BYTES);
-    if (err != cudaSuccess) return (int)err;
-    allowed = true;
-  }
-  xrt::launch_kernel(xrt::sample_kernel, dim3(n_rows), dim3(xrt::SAMPLE_THREADS), xrt::SAMPLE_DYNAMIC_BYTES, stream, out_ids, logits, vocab,
-                     row_slot, temperature, top_k, top_p, penalty, (const uint32_t*)seen, seen_words, rng_key, rng_counter);
+  // blocks of a team: slices of 4,096 logits or more (smaller ones are read in less time than a team takes to meet); half as
+  // many while the rows alone bring more than four blocks a multiprocessor
+  int team = 1;
+  while (team < xrt::SAMPLE_TEAM && (long long)team * 4096 < vocab) team *= 2;
+  while (team > 2 && (long long)team * n_rows > 4 * 148) team /= 2;
+  const long long per = ((long long)vocab + team * 32 - 1) / (team * 32) * 32;
+  const bool cached = per * 4 <= xrt::SAMPLE_CACHED_BYTES;
+  const bool vec = vocab % 4 == 0 && ((uintptr_t)logits & 15) == 0;
+  int values_bytes = cached ? (int)per * 4 : 0;
+  if (values_bytes < xrt::SAMPLE_CANDIDATES * 8) values_bytes = xrt::SAMPLE_CANDIDATES * 8;
+  const size_t smem = (size_t)values_bytes + xrt::SAMPLE_HIST_BYTES;
+  auto kernel = cached ? (vec ? xrt::sample_kernel<true, true> : xrt::sample_kernel<true, false>)
+                       : (vec ? xrt::sample_kernel<false, true> : xrt::sample_kernel<false, false>);
+  // one limit for every launch: setting a smaller one beside a launch of another thread would take it its room
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               xrt::SAMPLE_CACHED_BYTES + xrt::SAMPLE_HIST_BYTES);
+  if (err != cudaSuccess) return (int)err;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)n_rows * team);
+  config.blockDim = dim3(xrt::SAMPLE_THREADS);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = team; attrs[0].val.clusterDim.y = 1; attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attrs;
+  config.numAttrs = xrt::pdl_enabled() ? 2 : 1;
+  cudaLaunchKernelEx(&config, kernel, out_ids, logits, vocab, (int)per, values_bytes, row_slot, temperature, top_k, top_p,
+                     penalty, (const uint32_t*)seen, seen_words, rng_key, rng_counter, team);
   return xrt::launch_status();
 }
 
