@@ -28,8 +28,10 @@ def close(got, want, tol=2e-5):
 
 
 # heads, q/k heads, key size, value size: key sizes on every lane layout of the kernel (8, 16 and 32 rows a
-# lane, 1 to 8 lanes a column), value sizes below, at and above a block's columns, sizes that are no power of two
-SCAN_SIZES = [(2, 2, 8, 8), (3, 1, 16, 24), (4, 2, 48, 40), (1, 1, 130, 100), (2, 1, 256, 16), (2, 2, 32, 64)]
+# lane, 1 to 8 lanes a column), value sizes below, at and above a block's columns, sizes that are no power of two; the last
+# four: the kernel of four tokens at a time, with two columns a lane and (many heads) with four
+SCAN_SIZES = [(2, 2, 8, 8), (3, 1, 16, 24), (4, 2, 48, 40), (1, 1, 130, 100), (2, 1, 256, 16), (2, 2, 32, 64),
+              (2, 1, 128, 20), (4, 4, 64, 36), (20, 10, 128, 36), (20, 10, 64, 68)]
 
 
 @pytest.mark.parametrize("delta", [False, True])

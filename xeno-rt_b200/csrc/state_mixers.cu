@@ -44,6 +44,7 @@ struct ScanArgs {
   int n_heads, heads_per_qk, dim, vdim;
   float q_scale;
   int parts, cols, tile_tokens, stage_floats;
+  int stages;  // the wide kernel's ring
 };
 
 // VEC: 16-byte copies (dim, vdim, cols and every row stride are multiples of 4 floats, every base 16-byte aligned).
@@ -275,6 +276,252 @@ __global__ void __launch_bounds__(128) state_scan_kernel(const ScanArgs a) {
       }
     }
   }
+}
+
+// The scan for keys of 64 or 128 floats whose rows can be copied 16 bytes at a time; plain or delta rule.
+// What bounds the general kernel above is shared memory: every lane reads 12 bytes for each element of the state and token,
+// and a multiprocessor delivers 128 bytes a clock, whatever the lanes share.  Here a lane holds R rows of C2 neighbouring
+// columns, so that what it reads of q, k and a serves C2 columns, and what one prompt has of heads and columns is cut
+// finely enough to give every scheduler of the device a warp or two.  What is left is the chain from token to token, so
+// four tokens go together:
+//   the read-outs of four tokens are summed over the lanes in one go (lane_sums);
+//   with the delta rule, all the sums that four tokens' writes need are formed before the first write: with D_i the
+//   state decayed to token i without these writes, token i sees k_i^T D_i + sum over j < i of (k_i^T w_ij) u_j, where
+//   w_ij is k_j decayed from token j to i.  One round of shuffles instead of four.  The writes and read-outs then
+//   follow token by token as in the general kernel.
+// A ring of WIDE_STAGES tiles of WIDE_TOKENS tokens is filled by cp.async.
+// Measured, microseconds, general kernel -> this one: one prompt of 2,000 tokens, plain, 8 heads of 128 x 256 897 -> 281
+// (32 heads of 128 x 128 897 -> 400; 8 heads of 64 x 64 565 -> 216); delta rule, 16 heads of 128 x 128 1,046 -> 461 (four
+// prompts of 1,024 539 -> 433); 64 single tokens 27 -> 24.  Bound by the latency of its own chain of instructions: with two
+// warps a scheduler 0.4 instructions a clock, a third of the waiting for shared memory and shuffles.
+constexpr int WIDE_TOKENS = 8, WIDE_STAGES = 4, WIDE_GROUP = 4;
+
+template <int R, int PARTS, int C2, int THREADS, bool DELTA>
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 3) state_scan_wide_kernel(const ScanArgs a) {
+  constexpr int P = R / 2, DIM = PARTS * R, COLS = THREADS / PARTS * C2, G = WIDE_GROUP;
+  extern __shared__ float4 tile4[];
+  float* tile = reinterpret_cast<float*>(tile4);
+  pdl_trigger();
+  const int TT = a.tile_tokens, vdim = a.vdim;
+  const int vec_floats = TT * DIM;  // a stage: q | k | a, each [TT][DIM]; v [TT][COLS]; b [TT], padded to 16 bytes
+  const int part = threadIdx.x % PARTS, jl = (threadIdx.x / PARTS) * C2;
+  pdl_wait();
+  const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * COLS;
+  const int slot = a.seq_slot[s];
+  const int begin = a.cu_seqlens[s], end = a.cu_seqlens[s + 1];
+  if (slot < 0 || end <= begin) return;
+  const int j = col0 + jl, qh = h / a.heads_per_qk;
+
+  auto issue = [&](int t0, int stage) {
+    float* sq = tile + stage * a.stage_floats;
+    const int nt = min(TT, end - t0);
+    constexpr int PER = DIM / 4;
+    const int d = (threadIdx.x % PER) * 4;
+    for (int tt = threadIdx.x / PER; tt < nt; tt += THREADS / PER) {
+      const size_t t = (size_t)(t0 + tt);
+      cp_async<16>(sq + tt * DIM + d, a.q + t * a.q_stride + qh * DIM + d);
+      cp_async<16>(sq + vec_floats + tt * DIM + d, a.k + t * a.k_stride + qh * DIM + d);
+      cp_async<16>(sq + 2 * vec_floats + tt * DIM + d, a.decay + t * a.decay_stride + h * DIM + d);
+    }
+    float* sv = sq + 3 * vec_floats;
+    constexpr int VPER = COLS / 4;
+    const int c = (threadIdx.x % VPER) * 4;
+    if (col0 + c < vdim)
+      for (int tt = threadIdx.x / VPER; tt < nt; tt += THREADS / VPER)
+        cp_async<16>(sv + tt * COLS + c, a.v + (size_t)(t0 + tt) * a.v_stride + h * vdim + col0 + c);
+    if (DELTA && (int)threadIdx.x < nt)
+      cp_async<4>(sv + TT * COLS + threadIdx.x, a.beta + (size_t)(t0 + threadIdx.x) * a.beta_stride + h);
+  };
+
+  // a lane's rows: every PARTS-th group of four, as in the general kernel
+  auto rows_of = [&](const float* row, float2 (&out)[P]) {
+#pragma unroll
+    for (int g = 0; g < R / 4; ++g) {
+      const float4 t = reinterpret_cast<const float4*>(row)[g * PARTS + part];
+      out[2 * g] = make_float2(t.x, t.y);
+      out[2 * g + 1] = make_float2(t.z, t.w);
+    }
+  };
+  auto dot = [](const float2 (&x)[P], const float2 (&y)[P]) {
+    float2 sum = __fmul2_rn(x[0], y[0]);
+#pragma unroll
+    for (int i = 1; i < P; ++i) sum = __ffma2_rn(x[i], y[i], sum);
+    return sum.x + sum.y;
+  };
+  float2 S[C2][P];
+  float* sp = a.state + (((size_t)slot * a.n_heads + h) * vdim + j) * DIM;
+#pragma unroll
+  for (int c = 0; c < C2; ++c) {
+    if (j + c < vdim) {
+      rows_of(sp + (size_t)c * DIM, S[c]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < P; ++i) S[c][i] = make_float2(0.f, 0.f);
+    }
+  }
+  // the write of u into the state decayed by `aa`
+  auto write = [&](const float2 (&aa)[P], const float2 (&kk)[P], const float (&u)[C2]) {
+#pragma unroll
+    for (int c = 0; c < C2; ++c)
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        if (DELTA) S[c][i] = __ffma2_rn(kk[i], make_float2(u[c], u[c]), __fmul2_rn(S[c][i], aa[i]));
+        else S[c][i] = __ffma2_rn(S[c][i], aa[i], __fmul2_rn(kk[i], make_float2(u[c], u[c])));
+      }
+  };
+  // sum number `value` of a group of tokens that begins at token t belongs to this lane
+  auto store = [&](int t, int value, int per_value, float sum) {
+    const int tt = value / C2, c = value % C2;
+    if (part % per_value == 0 && j + c < vdim)
+      a.out[(size_t)(t + tt) * a.n_heads * vdim + h * vdim + j + c] = sum * a.q_scale;
+  };
+
+  const int n_tiles = (end - begin + TT - 1) / TT, stages = a.stages;
+  for (int p = 0; p < stages - 1; ++p) {
+    if (p < n_tiles) issue(begin + p * TT, p);
+    cp_async_commit();
+  }
+  for (int tile_i = 0; tile_i < n_tiles; ++tile_i) {
+    const int t0 = begin + tile_i * TT, nt = min(TT, end - t0), stage = tile_i % stages;
+    if (stages == 1) {
+      if (tile_i > 0) __syncthreads();  // (a sequence is longer than the caller said: one tile after another)
+      issue(t0, 0);
+      cp_async_commit();
+      cp_async_wait<0>();
+    } else {
+      cp_async_wait<WIDE_STAGES - 2>();
+    }
+    const float* sq = tile + stage * a.stage_floats;
+    const float* sk = sq + vec_floats;
+    const float* sa = sk + vec_floats;
+    float* sv = tile + stage * a.stage_floats + 3 * vec_floats;
+    float* sb = sv + TT * COLS;
+    if (DELTA && (int)threadIdx.x < nt)  // b = sigmoid(raw), once a tile, by the thread whose own copy brought the raw value
+      sb[threadIdx.x] = sigmoidf_(sb[threadIdx.x]);
+    __syncthreads();  // the tile is there, and everybody has left the stage that the next copies overwrite
+    if (stages > 1) {
+      if (tile_i + stages - 1 < n_tiles) issue(t0 + (stages - 1) * TT, (tile_i + stages - 1) % stages);
+      cp_async_commit();
+    }
+    auto group = [&](int tt) {
+      float2 kk[G][P], aa[G][P], qq[G][P];
+      float u[G][C2];
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        rows_of(sk + (tt + g) * DIM, kk[g]);
+        rows_of(sa + (tt + g) * DIM, aa[g]);
+#pragma unroll
+        for (int c = 0; c < C2; ++c) u[g][c] = sv[(tt + g) * COLS + jl + c];
+      }
+#pragma unroll
+      for (int g = 0; g < G; ++g) rows_of(sq + (tt + g) * DIM, qq[g]);
+      if (DELTA) {
+        constexpr int CROSS = G * (G - 1) / 2, N = G * C2 + CROSS;  // k_i^T D_i by token and column, then k_i^T w_ij
+        float sums[N];
+        float2 D[C2][P], w[G][P];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+#pragma unroll
+          for (int c = 0; c < C2; ++c) {
+#pragma unroll
+            for (int i = 0; i < P; ++i) D[c][i] = __fmul2_rn(g == 0 ? S[c][i] : D[c][i], aa[g][i]);
+            sums[g * C2 + c] = dot(D[c], kk[g]);
+          }
+#pragma unroll
+          for (int e = 0; e < g; ++e) {
+#pragma unroll
+            for (int i = 0; i < P; ++i) w[e][i] = __fmul2_rn(w[e][i], aa[g][i]);
+            sums[G * C2 + g * (g - 1) / 2 + e] = dot(w[e], kk[g]);
+          }
+#pragma unroll
+          for (int i = 0; i < P; ++i) w[g][i] = kk[g][i];
+        }
+        all_lane_sums<PARTS>(sums, part);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const float b = sb[tt + g];
+#pragma unroll
+          for (int c = 0; c < C2; ++c) {
+            float seen = sums[g * C2 + c];
+#pragma unroll
+            for (int e = 0; e < g; ++e) seen = fmaf(sums[G * C2 + g * (g - 1) / 2 + e], u[e][c], seen);
+            u[g][c] = b * (u[g][c] - seen);
+          }
+        }
+      }
+      float read[G * C2];
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        write(aa[g], kk[g], u[g]);
+#pragma unroll
+        for (int c = 0; c < C2; ++c) read[g * C2 + c] = dot(S[c], qq[g]);
+      }
+      store(t0 + tt, part * (G * C2) / PARTS, PARTS / (G * C2), lane_sums<PARTS>(read, part));
+    };
+    int tt = 0;
+    if (nt == WIDE_TOKENS) {  // the usual tile in one piece: the second group's loads do not wait for the first's sums
+#pragma unroll
+      for (; tt < WIDE_TOKENS; tt += G) group(tt);
+    } else {
+#pragma unroll 1
+      for (; tt + G <= nt; tt += G) group(tt);
+    }
+#pragma unroll 1
+    for (; tt < nt; ++tt) {
+      float2 kk[P], aa[P], qq[P];
+      rows_of(sk + tt * DIM, kk);
+      rows_of(sa + tt * DIM, aa);
+      rows_of(sq + tt * DIM, qq);
+      float u[C2], read[C2];
+#pragma unroll
+      for (int c = 0; c < C2; ++c) u[c] = sv[tt * COLS + jl + c];
+      if (DELTA) {
+        float seen[C2];
+#pragma unroll
+        for (int c = 0; c < C2; ++c) {
+          float2 D[P];
+#pragma unroll
+          for (int i = 0; i < P; ++i) D[i] = __fmul2_rn(S[c][i], aa[i]);
+          seen[c] = dot(D, kk);
+        }
+#pragma unroll
+        for (int o = PARTS / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int c = 0; c < C2; ++c) seen[c] += __shfl_xor_sync(0xffffffffu, seen[c], o);
+        const float b = sb[tt];
+#pragma unroll
+        for (int c = 0; c < C2; ++c) u[c] = b * (u[c] - seen[c]);
+      }
+      write(aa, kk, u);
+#pragma unroll
+      for (int c = 0; c < C2; ++c) read[c] = dot(S[c], qq);
+      store(t0 + tt, part * C2 / PARTS, PARTS / C2, lane_sums<PARTS>(read, part));
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < C2; ++c)
+#pragma unroll
+    for (int g = 0; g < R / 4; ++g)
+      if (j + c < vdim)
+        reinterpret_cast<float4*>(sp + (size_t)c * DIM)[g * PARTS + part] =
+            make_float4(S[c][2 * g].x, S[c][2 * g].y, S[c][2 * g + 1].x, S[c][2 * g + 1].y);
+}
+
+template <int R, int PARTS, int C2, int THREADS, bool DELTA>
+int launch_state_scan_wide(ScanArgs a, int n_seqs, int max_new, cudaStream_t stream) {
+  constexpr int DIM = PARTS * R, COLS = THREADS / PARTS * C2;
+  auto kernel = state_scan_wide_kernel<R, PARTS, C2, THREADS, DELTA>;
+  a.tile_tokens = max_new < WIDE_TOKENS ? max_new : WIDE_TOKENS;
+  a.stages = max_new <= WIDE_TOKENS ? 1 : WIDE_STAGES;
+  a.stage_floats = 3 * a.tile_tokens * DIM + a.tile_tokens * COLS + ((a.tile_tokens + 3) & ~3);
+  const size_t smem = (size_t)a.stages * a.stage_floats * sizeof(float);
+  constexpr int most = WIDE_STAGES * (WIDE_TOKENS * (3 * DIM + COLS + 1)) * (int)sizeof(float);
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (err != cudaSuccess) return (int)err;
+  const dim3 grid(n_seqs, a.n_heads, (a.vdim + COLS - 1) / COLS);
+  if (max_new > 1) launch_kernel_alone(kernel, grid, dim3(THREADS), smem, stream, a);
+  else launch_kernel(kernel, grid, dim3(THREADS), smem, stream, a);
+  return launch_status();
 }
 
 // ------------------------------------------------------------------------------------------ convolution
@@ -689,7 +936,23 @@ XRT_EXPORT int xrt_state_scan(float* out, const float* q, int q_stride, const fl
   xrt::ScanArgs a = {out, q, k, v, decay, beta, unit, removal, unit_stride, removal_stride,
                      q_stride, k_stride, v_stride, decay_stride, beta_stride, state,
                      cu_seqlens, seq_slot, n_heads, n_heads / n_qk_heads, dim, vdim, q_scale, parts, cols, tile_tokens,
-                     stage_floats(tile_tokens)};
+                     stage_floats(tile_tokens), 1};
+  if (vec && mode != 2 && (dim == 128 || dim == 64)) {
+    // four columns a lane once their blocks cover the multiprocessors (16 prompts of 500 tokens, 8 heads of 128 x 256, plain:
+    // 360 us against 370 with two columns); else two, and half the rows a lane (one prompt: 281 against 290)
+    const long long blocks_4 = (long long)n_seqs * n_heads * ((vdim + 31) / 32);
+    const bool four = blocks_4 >= 148;
+#define XRT_SCAN_WIDE(DD)                                                                                    \
+  do {                                                                                                       \
+    if (dim == 128 && four) return xrt::launch_state_scan_wide<8, 16, 4, 128, DD>(a, n_seqs, max_new, stream); \
+    if (dim == 128) return xrt::launch_state_scan_wide<4, 32, 2, 256, DD>(a, n_seqs, max_new, stream);         \
+    if (four) return xrt::launch_state_scan_wide<4, 16, 4, 128, DD>(a, n_seqs, max_new, stream);               \
+    return xrt::launch_state_scan_wide<4, 16, 2, 128, DD>(a, n_seqs, max_new, stream);                         \
+  } while (0)
+    if (delta) XRT_SCAN_WIDE(true);
+    XRT_SCAN_WIDE(false);
+#undef XRT_SCAN_WIDE
+  }
   const dim3 grid(n_seqs, n_heads, (vdim + cols - 1) / cols), block(parts * groups);
 #define XRT_SCAN(RR, CC, DD, VV)                                                                                  \
   do {                                                                                                                \
