@@ -98,7 +98,8 @@ def _ssd_inputs(rng, n, heads, vdim, state, groups):
 
 
 @pytest.mark.parametrize("heads,vdim,state,groups", [(3, 8, 16, 1), (4, 20, 5, 2), (2, 64, 128, 2), (6, 4, 48, 6),
-                                                     (1, 40, 200, 1)])
+                                                     (1, 40, 200, 1),
+                                                     (4, 36, 128, 2), (28, 36, 128, 2)])  # two and four columns a lane
 def test_scan_of_a_prompt_equals_single_tokens_and_the_plain_recurrence(heads, vdim, state, groups):
     from xeno_rt_b200.csrc import ops
     rng = np.random.default_rng(3)

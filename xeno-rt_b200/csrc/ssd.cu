@@ -11,7 +11,7 @@
 // padding rows of a captured step leave every state alone.  The state is kept [slot][head][vdim][state]: a column
 // of S is contiguous.  A token's arithmetic is the same whether it comes alone or inside a prompt, so results do
 // not depend on how a sequence was cut into steps.
-#include "common.cuh"
+#include "recurrence.cuh"
 
 namespace xrt {
 
@@ -31,13 +31,6 @@ struct SsdArgs {
 // the read-out's sum over rows is finished by a butterfly among those lanes, so its order is fixed.  Tiles of
 // `tile_tokens` tokens' b, c, x and raw step sizes are brought into shared memory by cp.async, two tiles in flight:
 // the next tile lands while this one is worked on.
-template <int BYTES>
-__device__ __forceinline__ void ssd_cp_async(float* smem, const float* global) {
-  const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
-  if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(global) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(global) : "memory");
-}
-
 // VEC: 16-byte copies (n_state, cols, vdim and every row stride are multiples of 4 floats, every base 16-byte aligned).
 template <int R, bool VEC>
 __global__ void __launch_bounds__(128) ssd_scan_kernel(const SsdArgs a) {
@@ -78,25 +71,25 @@ __global__ void __launch_bounds__(128) ssd_scan_kernel(const SsdArgs a) {
       const int d = (threadIdx.x % per) * E;
       for (int tt = threadIdx.x / per; tt < nt; tt += blockDim.x / per) {
         const size_t at = (size_t)(t0 + tt) * a.bc_stride + g * n_state + d;
-        ssd_cp_async<B>(sb + tt * padded + d, a.b + at);
-        ssd_cp_async<B>(sc + tt * padded + d, a.c + at);
+        cp_async<B>(sb + tt * padded + d, a.b + at);
+        cp_async<B>(sc + tt * padded + d, a.c + at);
       }
     } else {
       for (int e = threadIdx.x; e < nt * per; e += blockDim.x) {
         const int tt = e / per, d = (e - tt * per) * E;
         const size_t at = (size_t)(t0 + tt) * a.bc_stride + g * n_state + d;
-        ssd_cp_async<B>(sb + tt * padded + d, a.b + at);
-        ssd_cp_async<B>(sc + tt * padded + d, a.c + at);
+        cp_async<B>(sb + tt * padded + d, a.b + at);
+        cp_async<B>(sc + tt * padded + d, a.c + at);
       }
     }
     const int xper = cols / E;
     for (int e = threadIdx.x; e < nt * xper; e += blockDim.x) {
       const int tt = e / xper, cc = (e - tt * xper) * E;
-      if (col0 + cc < vdim) ssd_cp_async<B>(sx + tt * cols + cc, a.x + (size_t)(t0 + tt) * a.x_stride + h * vdim + col0 + cc);
+      if (col0 + cc < vdim) cp_async<B>(sx + tt * cols + cc, a.x + (size_t)(t0 + tt) * a.x_stride + h * vdim + col0 + cc);
     }
     for (int tt = threadIdx.x; tt < nt; tt += blockDim.x)
-      ssd_cp_async<4>(sraw + tt, a.dt + (size_t)(t0 + tt) * a.dt_stride + h);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+      cp_async<4>(sraw + tt, a.dt + (size_t)(t0 + tt) * a.dt_stride + h);
+    cp_async_commit();
   };
 
   float S[R];
@@ -112,9 +105,9 @@ __global__ void __launch_bounds__(128) ssd_scan_kernel(const SsdArgs a) {
     const int nt = min(TT, end - t0);
     if (t0 + TT < end) {
       issue(t0 + TT, stage ^ 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      cp_async_wait<1>();
     } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      cp_async_wait<0>();
     }
     __syncthreads();
     const float* sb = tile + stage * stage_floats;
@@ -166,6 +159,158 @@ __global__ void __launch_bounds__(128) ssd_scan_kernel(const SsdArgs a) {
     const int row = row_of(i);
     if (live && row < n_state) sp[row] = S[i];
   }
+}
+
+// The scan of prompts whose state has 128 rows: 16 lanes a column of the state as above, 8 rows each, but C2 neighbouring
+// columns a lane.  The kernel above is bound by shared memory (every lane reads 8 bytes of b and c for each element of the
+// state and token; a multiprocessor delivers 128 bytes a clock) and by its butterflies; here what a lane reads serves C2
+// columns, the multiply-adds are the packed 2 x fp32 ones, and the read-outs of four tokens are summed over the lanes
+// together (lane_sums).  Each sum has the same terms in the same order as above, so a token's result is the same bit for
+// bit.  A ring of SSD_STAGES tiles of SSD_TOKENS tokens is filled by cp.async.
+// Measured, microseconds, the kernel above -> this one, 64 heads of 64 x 128: one prompt of 2,000 tokens 719 -> 319, prompts of
+// 1,000 and 1,100 tokens 741 -> 271, 16 of 300 1,230 -> 406.  At two columns a lane shared memory was 78 percent busy (301 us for
+// the two prompts).
+constexpr int SSD_TOKENS = 16, SSD_STAGES = 3, SSD_GROUP = 4;
+
+template <int C2>
+__global__ void __launch_bounds__(128) ssd_scan_wide_kernel(const SsdArgs a) {
+  constexpr int PARTS = 16, ROWS = 128, COLS = 128 / PARTS * C2, TT = SSD_TOKENS;
+  constexpr int STAGE = 2 * TT * ROWS + TT * COLS + TT;  // b | c, each [TT][ROWS]; x [TT][COLS]; raw step sizes [TT]
+  extern __shared__ __align__(16) float tile[];
+  __shared__ float sdt[TT], sdecay[TT];
+  pdl_trigger();
+  pdl_wait();
+  const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * COLS;
+  const int slot = a.seq_slot[s];
+  const int begin = a.cu_seqlens[s], end = a.cu_seqlens[s + 1];
+  if (slot < 0 || end <= begin) return;
+  const int vdim = a.vdim;
+  const int part = threadIdx.x % PARTS, jl = (threadIdx.x / PARTS) * C2, j = col0 + jl;
+  const int g = h / a.heads_per_group;
+  const float rate = expf(a.a_log[h]), dt_bias = a.dt_bias[h], d_skip = a.d_skip[h];
+
+  auto issue = [&](int t0, int stage) {
+    float* sb = tile + stage * STAGE;
+    const int nt = min(TT, end - t0);
+    const int d = (threadIdx.x % 32) * 4;
+    for (int tt = threadIdx.x / 32; tt < nt; tt += 4) {
+      const size_t at = (size_t)(t0 + tt) * a.bc_stride + g * ROWS + d;
+      cp_async<16>(sb + tt * ROWS + d, a.b + at);
+      cp_async<16>(sb + TT * ROWS + tt * ROWS + d, a.c + at);
+    }
+    constexpr int XPER = COLS / 4;
+    const int c = (threadIdx.x % XPER) * 4;
+    if (col0 + c < vdim)
+      for (int tt = threadIdx.x / XPER; tt < nt; tt += 128 / XPER)
+        cp_async<16>(sb + 2 * TT * ROWS + tt * COLS + c, a.x + (size_t)(t0 + tt) * a.x_stride + h * vdim + col0 + c);
+    if ((int)threadIdx.x < nt)
+      cp_async<4>(sb + 2 * TT * ROWS + TT * COLS + threadIdx.x, a.dt + (size_t)(t0 + threadIdx.x) * a.dt_stride + h);
+  };
+
+  float2 S[C2][4];
+  float* sp = a.state + (((size_t)slot * a.n_heads + h) * vdim + j) * ROWS;
+#pragma unroll
+  for (int c = 0; c < C2; ++c)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (j + c < vdim) t = *reinterpret_cast<const float4*>(sp + (size_t)c * ROWS + 4 * (i * PARTS + part));
+      S[c][2 * i] = make_float2(t.x, t.y);
+      S[c][2 * i + 1] = make_float2(t.z, t.w);
+    }
+
+  // one token: its write into the state; `read` gets this lane's part of what the token reads, column by column
+  auto token = [&](const float* sb, int tt, float (&read)[C2]) {
+    const float4* pb = reinterpret_cast<const float4*>(sb + tt * ROWS) + part;
+    const float4* pc = reinterpret_cast<const float4*>(sb + TT * ROWS + tt * ROWS) + part;
+    const float4 b0 = pb[0], b1 = pb[PARTS], c0 = pc[0], c1 = pc[PARTS];
+    const float2 bb[4] = {{b0.x, b0.y}, {b0.z, b0.w}, {b1.x, b1.y}, {b1.z, b1.w}};
+    const float2 cc[4] = {{c0.x, c0.y}, {c0.z, c0.w}, {c1.x, c1.y}, {c1.z, c1.w}};
+    const float dt = sdt[tt], decay = sdecay[tt];
+    const float* sx = sb + 2 * TT * ROWS + tt * COLS + jl;
+    float xv[C2];
+    if constexpr (C2 == 4) {
+      const float4 x4 = *reinterpret_cast<const float4*>(sx);
+      xv[0] = x4.x; xv[1] = x4.y; xv[2] = x4.z; xv[3] = x4.w;
+    } else {
+#pragma unroll
+      for (int c = 0; c < C2; ++c) xv[c] = sx[c];
+    }
+#pragma unroll
+    for (int c = 0; c < C2; ++c) {
+      const float u = dt * xv[c];
+      float2 y = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        S[c][i] = __ffma2_rn(make_float2(decay, decay), S[c][i], __fmul2_rn(make_float2(u, u), bb[i]));
+        y = __ffma2_rn(S[c][i], cc[i], y);
+      }
+      read[c] = y.x + y.y;
+    }
+  };
+  // sum number `value` of a group of tokens that begins at place tt of the tile belongs to this lane
+  auto store = [&](const float* sb, int t0, int tt, int value, int per_value, float sum) {
+    const int at = tt + value / C2, c = value % C2;
+    if (part % per_value == 0 && j + c < vdim)
+      a.out[(size_t)(t0 + at) * a.n_heads * vdim + h * vdim + j + c] = fmaf(d_skip, sb[2 * TT * ROWS + at * COLS + jl + c], sum);
+  };
+
+  const int n_tiles = (end - begin + TT - 1) / TT;
+  for (int p = 0; p < SSD_STAGES - 1; ++p) {
+    if (p < n_tiles) issue(begin + p * TT, p);
+    cp_async_commit();
+  }
+  for (int tile_i = 0; tile_i < n_tiles; ++tile_i) {
+    const int t0 = begin + tile_i * TT, nt = min(TT, end - t0);
+    cp_async_wait<SSD_STAGES - 2>();
+    const float* sb = tile + (tile_i % SSD_STAGES) * STAGE;
+    __syncthreads();  // the tile is there, and everybody has left the tile before it
+    if ((int)threadIdx.x < nt) {
+      const float dt = softplusf_(sb[2 * TT * ROWS + TT * COLS + threadIdx.x] + dt_bias);
+      sdt[threadIdx.x] = dt;
+      sdecay[threadIdx.x] = expf(-rate * dt);
+    }
+    if (tile_i + SSD_STAGES - 1 < n_tiles) issue(t0 + (SSD_STAGES - 1) * TT, (tile_i + SSD_STAGES - 1) % SSD_STAGES);
+    cp_async_commit();
+    __syncthreads();
+    int tt = 0;
+#pragma unroll 1
+    for (; tt + SSD_GROUP <= nt; tt += SSD_GROUP) {
+      float read[SSD_GROUP * C2];
+#pragma unroll
+      for (int i = 0; i < SSD_GROUP; ++i) {
+        float one[C2];
+        token(sb, tt + i, one);
+#pragma unroll
+        for (int c = 0; c < C2; ++c) read[i * C2 + c] = one[c];
+      }
+      const float sum = lane_sums<PARTS>(read, part);
+      store(sb, t0, tt, part * (SSD_GROUP * C2) / PARTS, PARTS / (SSD_GROUP * C2), sum);
+    }
+#pragma unroll 1
+    for (; tt < nt; ++tt) {
+      float read[C2];
+      token(sb, tt, read);
+      store(sb, t0, tt, part * C2 / PARTS, PARTS / C2, lane_sums<PARTS>(read, part));
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < C2; ++c)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (j + c < vdim)
+        *reinterpret_cast<float4*>(sp + (size_t)c * ROWS + 4 * (i * PARTS + part)) =
+            make_float4(S[c][2 * i].x, S[c][2 * i].y, S[c][2 * i + 1].x, S[c][2 * i + 1].y);
+}
+
+template <int C2>
+int launch_ssd_scan_wide(const SsdArgs& a, int n_seqs, cudaStream_t stream) {
+  constexpr int COLS = 8 * C2;
+  constexpr size_t smem = (size_t)SSD_STAGES * (2 * SSD_TOKENS * 128 + SSD_TOKENS * COLS + SSD_TOKENS) * sizeof(float);
+  const cudaError_t err = cudaFuncSetAttribute(ssd_scan_wide_kernel<C2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err != cudaSuccess) return (int)err;
+  launch_kernel_alone(ssd_scan_wide_kernel<C2>, dim3(n_seqs, a.n_heads, (a.vdim + COLS - 1) / COLS), dim3(128), smem, stream, a);
+  return launch_status();
 }
 
 // v = y * silu(z); each of `groups` stretches of the row by its own root mean square; times w.  One block a
@@ -227,6 +372,11 @@ XRT_EXPORT int xrt_ssd_scan(float* out, const float* x, int x_stride, const floa
   const size_t smem = floats(a.tile_tokens) * sizeof(float);
   const bool vec = n_state % 4 == 0 && a.cols % 4 == 0 && vdim % 4 == 0 && x_stride % 4 == 0 && bc_stride % 4 == 0 &&
                    (((uintptr_t)x | (uintptr_t)b | (uintptr_t)c) & 15) == 0;
+  if (max_new > 1 && vec && n_state == 128 && ((uintptr_t)state & 15) == 0) {
+    // four columns a lane where their blocks still reach two thirds of the multiprocessors, two else
+    if ((long long)n_seqs * n_heads * ((vdim + 31) / 32) >= 100) return xrt::launch_ssd_scan_wide<4>(a, n_seqs, stream);
+    return xrt::launch_ssd_scan_wide<2>(a, n_seqs, stream);
+  }
   dim3 grid(n_seqs, n_heads, (vdim + a.cols - 1) / a.cols);
 #define XRT_SSD(R)                                                                                              \
   do {                                                                                                                 \
