@@ -112,7 +112,7 @@ gemm_decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   const int acc_cols = GROUPS * shape.nb;  // TMEM columns of one accumulator set
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) { mbar_init(smem_u32(&full[s]), 2); mbar_init(smem_u32(&empty[s]), 1); }
+    for (int s = 0; s < stages; ++s) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(smem_u32(&acc_full[a]), 1); mbar_init(smem_u32(&acc_empty[a]), 128); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -136,24 +136,30 @@ gemm_decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
       // Blocks that work at the same time start their walk over K at different slabs (a rotation that
       // depends on the tile only, so the order of the sum is fixed per output element): otherwise every
       // block asks the L2 for the same few lines of X at the same moment.
+      // One thread does all of this for every 16 KB of weights, and was the bound of products of one group of weight
+      // rows (780 clocks a slab, most of them divisions; 1 row x 128,256 outputs x 4,096 inputs 172 us): nothing in the walk
+      // or in the ring's turn divides but the step to another item (157 us, 6,690 GB/s; 4,096 x 14,336 26.3 -> 21.6).
       struct Walk {
-        int item, i, span, kb0, rotate, tile;
+        int item, left, kb, kb0, kb1, tile;  // slabs left of the item, the next one, the item's range
         __device__ void enter(const DecodeGemmShape& sh, int k_total) {
           tile = item / sh.splits;
-          kb0 = (item % sh.splits) * sh.k_per_split;
-          span = max(0, min(k_total, kb0 + sh.k_per_split) - kb0);
-          rotate = span > 0 ? (tile * 5) % span : 0;
-          i = 0;
+          kb0 = (item - tile * sh.splits) * sh.k_per_split;
+          kb1 = max(kb0, min(k_total, kb0 + sh.k_per_split));
+          left = kb1 - kb0;
+          kb = left > 0 ? kb0 + (tile * 5) % left : kb0;
         }
         __device__ bool settle(const DecodeGemmShape& sh, int k_total, int n_items, int stride) {
           while (item < n_items) {  // skips items without slabs (a split beyond K)
-            if (i < span) return true;
+            if (left > 0) return true;
             item += stride;
             if (item < n_items) enter(sh, k_total);
           }
           return false;
         }
-        __device__ int kb() const { return kb0 + (i + rotate) % span; }
+        __device__ void next() {
+          --left;
+          if (++kb == kb1) kb = kb0;
+        }
       };
       Walk walk;
       walk.item = blockIdx.x;
@@ -163,44 +169,43 @@ gemm_decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
       // (activations, the residual, the partial sums, the kernels' code) stays (measured at the
       // 8B shape, context 4096: 4 to 7 percent of a step of 17 to 64 sequences)
       const uint64_t once = policy_evict_first();
+      const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty), stage0 = smem_u32(smem);
       auto load_w = [&](const Walk& at, int s) {
-        const uint32_t bar = smem_u32(&full[s]);
-        unsigned char* stage = smem + (size_t)s * stage_bytes;
-        mbar_arrive_expect_tx(bar, w_bytes);
-        tma_load_2d(smem_u32(stage), &map_w, at.kb() * DG_BK, at.tile * DG_ROWS, bar, once);
-        if (MODE == 2) tma_load_2d(smem_u32(stage + DG_W_BYTES), &map_w, at.kb() * DG_BK, shape.up_rows + at.tile * DG_ROWS, bar, once);
+        const uint32_t bar = full0 + s * 8, stage = stage0 + s * stage_bytes;
+        tma_load_2d(stage, &map_w, at.kb * DG_BK, at.tile * DG_ROWS, bar, once);
+        if (MODE == 2) tma_load_2d(stage + DG_W_BYTES, &map_w, at.kb * DG_BK, shape.up_rows + at.tile * DG_ROWS, bar, once);
       };
       auto load_x = [&](const Walk& at, int s) {
-        const uint32_t bar = smem_u32(&full[s]);
-        mbar_arrive_expect_tx(bar, x_bytes);
-        tma_load_2d(smem_u32(smem + (size_t)s * stage_bytes + GROUPS * DG_W_BYTES), &map_x, at.kb() * DG_BK, 0, bar);
+        tma_load_2d(stage0 + s * stage_bytes + GROUPS * DG_W_BYTES, &map_x, at.kb * DG_BK, 0, full0 + s * 8);
       };
       // The weights do not depend on the step: the whole ring is filled with them while the kernel
       // before this one finishes.  X does: its loads follow once that kernel has completed.  A stage's
-      // barrier takes two arrivals (weights asked for, X asked for) and the bytes of both.
+      // barrier hears of the bytes of its weights first, and of those of X with the one arrival.
       Walk ahead = walk;
       int filled = 0;
       while (filled < stages && ahead.settle(shape, k_iters_total, n_items, gridDim.x)) {
+        mbar_expect_tx(full0 + filled * 8, w_bytes);
         load_w(ahead, filled);
-        ++ahead.i;
+        ahead.next();
         ++filled;
       }
       pdl_wait();
-      int it = 0;
-      bool ok = true;
-      while (it < filled && walk.settle(shape, k_iters_total, n_items, gridDim.x)) {
-        load_x(walk, it);
-        ++walk.i;
-        ++it;
+      for (int s = 0; s < filled && walk.settle(shape, k_iters_total, n_items, gridDim.x); ++s) {
+        mbar_arrive_expect_tx(full0 + s * 8, x_bytes);
+        load_x(walk, s);
+        walk.next();
       }
-      while (ok && walk.settle(shape, k_iters_total, n_items, gridDim.x)) {
-        const int s = it % stages;
-        ok = mbar_wait(smem_u32(&empty[s]), ((it / stages) & 1) ^ 1, abort_flag);
+      bool ok = true;
+      int s = 0;
+      uint32_t turn = 0;  // the parity of the ring's turn that has to be used up
+      while (ok && walk.settle(shape, k_iters_total, n_items, gridDim.x)) {  // (only once the whole ring was filled)
+        ok = mbar_wait(empty0 + s * 8, turn, abort_flag);
         if (!ok) break;
+        mbar_arrive_expect_tx(full0 + s * 8, w_bytes + x_bytes);
         load_w(walk, s);
         load_x(walk, s);
-        ++walk.i;
-        ++it;
+        walk.next();
+        if (++s == stages) { s = 0; turn ^= 1; }
       }
       if (!ok) { *abort_flag = 1; if (error_flag != nullptr) atomicExch(error_flag, 4); }
     }
@@ -209,7 +214,8 @@ gemm_decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
     // ---------------------------------------------------------------- MMA issue
     if (lane == 0) {
       const uint32_t idesc = instr_desc(DG_ROWS, shape.nb);
-      int it = 0, item_i = 0;
+      int s = 0, item_i = 0;
+      uint32_t turn = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++item_i) {
         const int split = item % shape.splits;
@@ -220,9 +226,8 @@ gemm_decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
         if (!ok) break;
         fence_after();
         const uint32_t tmem_d = tmem_base + a * acc_cols;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {  // the slabs arrive in the producer's rotated order
-          const int s = it % stages;
-          ok = mbar_wait(smem_u32(&full[s]), (it / stages) & 1, abort_flag);
+        for (int kb = kb0; kb < kb1; ++kb) {  // the slabs arrive in the producer's rotated order
+          ok = mbar_wait(smem_u32(&full[s]), turn, abort_flag);
           if (!ok) break;
           fence_after();
           unsigned char* stage = smem + (size_t)s * stage_bytes;
@@ -235,6 +240,7 @@ gemm_decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
               mma_f16(tmem_d + gr * shape.nb, desc_w + 2 * k, desc_x + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           }
           commit(smem_u32(&empty[s]));
+          if (++s == stages) { s = 0; turn ^= 1; }
         }
         if (ok) commit(smem_u32(&acc_full[a]));
       }
