@@ -23,6 +23,7 @@ def aligned(x, weight) -> bool:
 
 
 ACCUMULATE_MIN_K_9_ROWS = 8192  # a product of 9 to 16 rows that adds into the residual stream takes the tcgen05 kernel from here on
+ACCUMULATE_LONG_K = 12288       # one of any number of rows does from here on
 STREAM_BLOCKS_PER_SM = 4        # blocks of the cp.async kernel that a multiprocessor holds at once (registers)
 
 
@@ -42,16 +43,25 @@ def stream_kernel_waves(sms: int, n: int, accumulate: bool = False) -> float:
 def tcgen05_for_few_rows(sms: int, rows: int, n: int, k: int, mode: str) -> bool:
     """Up to 16 rows both decode kernels take the product.  The tcgen05 kernel runs its items one a
     multiprocessor in rounds: it wins where they fill the rounds (one round at least 0.6 full, or
-    several at least 0.85 full).  Products that add into the residual stream stay on the cp.async
-    kernel up to 8 rows, and from 9 rows on below K = 8,192 (its time grows with the rows, the tcgen05
-    kernel's does not), unless its own rounds of blocks are badly filled.  Measured alone and back to
-    back, cp.async against tcgen05 in microseconds at 1 / 8 / 16 rows: N 4,096, K 4,096: 7.6 / 8.6 / 10.3
-    against 11.5; K 14,336: 22.7 / 26.1 / 29.2 against 26.4; N 5,120, K 8,192: 15.0 / 16.6 / 21.4 against
-    21.2; K 25,600: 44.7 / 48.4 / 66.7 against 55.0."""
+    several at least 0.85 full), but for up to 8 rows of a product that is only stored and takes several
+    rounds (an output matrix): the cp.async kernel reads whole rows of the weight, which the memory answers faster.
+    Products that add into the residual stream stay on the cp.async kernel up to 8 rows, and from 9 rows
+    on below K = 8,192 (its time grows with the rows, the tcgen05 kernel's does not), unless its own rounds of blocks
+    are badly filled, or K is long enough for the tcgen05 kernel's fixed costs not to count.  Measured alone and back to
+    back, cp.async against tcgen05 in microseconds at 1 / 8 / 16 rows: added, N 4,096, K 4,096: 7.8 / 8.2 / 9.8
+    against 10.0; K 12,288: 19.8 / 21.7 / 23.5 against 19.3; K 14,336: 22.7 / 24.7 / 26.9 against 21.8; N 5,120, K 8,192:
+    14.7 / 15.9 / 20.6 against 17.6; K 25,600: 44.0 / 46.6 / 63.6 against 43.9; N 2,048, K 8,192: 13.5 / 14.5 / 15.6
+    against 10.8.  Stored, N 128,256, K 4,096: 146 / 151 / 167 against 162 / 164 / 166; N 151,936: 173 / 178 / 198
+    against 196 / 196 / 202."""
     rounds, fill, reduction = ops.gemm_decode_tcgen05_plan(sms, rows, n, k, mode)
     fills = fill >= 0.6 and (rounds == 1 or fill >= 0.85)
+    if mode == "accumulate" and fills and (k >= ACCUMULATE_LONG_K or (
+            k >= ACCUMULATE_MIN_K_9_ROWS and -(-n // 8) < 2 * sms)):
+        return True
     if mode == "accumulate" and (rows <= 8 or k < ACCUMULATE_MIN_K_9_ROWS):
         return fills and fill > stream_kernel_waves(sms, n, accumulate=True) + 0.2
+    if mode == "store" and rows <= 8 and rounds > 1:
+        return False
     if mode == "store" and reduction == "scratch":
         # splits that the device does not hold as clusters end in one block that merges a tile: the cp.async
         # kernel with 16 weight rows a block is faster then (N 6,144, K 4,096, alone at 1 / 8 / 16 rows: 8.4 /
