@@ -387,8 +387,9 @@ int launch_tcgen05_tiled(void* out, const CUtensorMap& map_x, const CUtensorMap&
   return launch_status();
 }
 
-// Pairs of blocks, except where their tiles of 256 rows take more rounds of the multiprocessors (600 rows, 14,336 gated
-// outputs: 155 us against 137), or pad the rows by more than a tenth beyond tiles of 128 (600 rows, 6,144 outputs: 35
+// Pairs of blocks, except where their tiles of 256 rows take more rounds of the multiprocessors, by more than the one in 25
+// that a pair's round is shorter (600 rows, 14,336 gated outputs: 5 against 4, 155 us against 137; 7,999 rows: 49 against
+// 48, 1,402 against 1,430), or pad the rows by more than a tenth beyond tiles of 128 (600 rows, 6,144 outputs: 35
 // against 31), then only if single blocks would leave four multiprocessors in ten without a tile (600 rows, 4,096 outputs,
 // 14,336 inputs: 94 against 114).
 // Tuning::gemm_tile_rows = 128 or 256 forces one, for comparison.
@@ -403,7 +404,7 @@ int launch_tcgen05(void* out, const CUtensorMap& map_x, const CUtensorMap& map_w
   auto rounds = [](long long tiles, int units) { return (tiles + units - 1) / units; };
   const int forced = tuning().gemm_tile_rows;
   const bool pair = forced == 256 || (forced != 128 && M > 128 && sm_count >= 2 &&
-                                      rounds(tiles_256, sm_count / 2) <= rounds(tiles_128, sm_count) &&
+                                      24 * rounds(tiles_256, sm_count / 2) <= 25 * rounds(tiles_128, sm_count) &&
                                       (rows_256 * 10 <= rows_128 * 11 || tiles_128 * 10 < 6ll * sm_count));
   if (pair)
     return launch_tcgen05_tiled<MODE, true, TO>(out, map_x, map_w, M, N, K, ldo, up_rows, error_flag, sm_count, emit, scale, stream);
