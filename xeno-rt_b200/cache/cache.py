@@ -228,6 +228,8 @@ class Cache:
         length moves only with ``advance``.  Raises if the slot is not open, the sequence would
         pass the model's positions, or the pool has no block left."""
         start = self.length(slot)
+        if 0 < n_new <= self._n_seq_blocks[slot] * BLOCK_TOKENS - start and start + n_new <= self.max_positions:
+            return start  # the last block has room
         if n_new <= 0:
             raise CacheError(f"slot {slot}: a step must bring at least one token, got {n_new}")
         if start + n_new > self.max_positions:
@@ -280,6 +282,8 @@ class Cache:
             raise CacheError(f"slot {slot}: advancing by {n_new} passes what was reserved")
         self.lengths[slot] += n_new
         for group in self.kv_groups:
+            if group.need.window is None:  # nothing ever falls behind
+                continue
             done = min(group.blocks_behind_the_window(self.lengths[slot]), self._n_seq_blocks[slot])
             first = max(group.first_block[slot], min(group.kept_blocks, self._n_seq_blocks[slot]))
             if done > first:

@@ -31,6 +31,6 @@ class PinnedRing:
 
     def copied(self, i: int) -> None:
         if self.pinned:
-            event = torch.cuda.Event()
-            event.record()
-            self.events[i] = event
+            if self.events[i] is None:
+                self.events[i] = torch.cuda.Event()
+            self.events[i].record()

@@ -161,6 +161,21 @@ class _DecodeGraph:
             ctx.captured = True
             self.logits = model.forward(ctx, cache, self.rows)
         self.launches = ops.launch_count() - before
+        self.views = {k: self.static[lay[k][0]:lay[k][1]] for k in ("ids", "pos", "slot", "cu", "seq_slot", "seq_start")}
+        self.rows_of = {}  # views of the first n ids and the first n rows of the logits, made once for each n
+
+    def first(self, n: int):
+        if n not in self.rows_of:
+            self.rows_of[n] = (self.static[:n], self.logits[:n])
+        return self.rows_of[n]
+
+    def context(self, starts, max_context: int, mean_context: int, dtype) -> StepContext:
+        """What ``context_from`` makes of a step of one token for each of ``starts``, over the views kept here."""
+        v = self.views
+        return StepContext(
+            n_tokens=self.bucket, n_seqs=self.bucket, token_ids=v["ids"], tok_pos=v["pos"], tok_slot=v["slot"],
+            cu_seqlens=v["cu"], seq_slot=v["seq_slot"], seq_start=v["seq_start"], new_lens=[1] * len(starts),
+            starts=starts, all_single=True, max_new=1, max_context=max_context, mean_context=mean_context, dtype=dtype)
 
 
 class Engine:
@@ -204,7 +219,9 @@ class Engine:
         use_graph = self.use_graphs if graph is None else (graph and self.model.graph_safe)
         if (use_graph and pad_to is None and len(entries) <= GRAPH_MAX_BATCH
                 and all(len(e.tokens) == 1 for e in entries)):
-            return self._graph_step(entries)
+            _check_entries(entries, model.vocab_size)
+            return self._graph_step([e.slot for e in entries], [int(e.tokens[0]) for e in entries],
+                                    [i for i, e in enumerate(entries) for _ in e.want])
         ctx, want_rows = build_context(entries, self.cache, model.vocab_size, model.dtype, model.device, pad_to,
                                        self.staging)
         self.cache.flush_tables()
@@ -221,19 +238,22 @@ class Engine:
         the ids when the step cannot be replayed from a graph."""
         n = len(slots)
         if self.use_graphs and n <= GRAPH_MAX_BATCH:
-            return self._graph_step([StepEntry(s, [0], [0]) for s in slots], ids_device=ids)
+            slots = list(slots)
+            if n == 0 or len(set(slots)) != n:
+                _check_entries([StepEntry(s, [0], [0]) for s in slots], self.model.vocab_size)  # raises
+            return self._graph_step(slots, [0] * n, list(range(n)), ids_device=ids)
         tokens = ids[:n].tolist()
         return self.step([StepEntry(s, [int(t)], [0]) for s, t in zip(slots, tokens)])
 
-    def _graph_step(self, entries, ids_device=None):
-        model = self.model
-        _check_entries(entries, model.vocab_size)
-        n = len(entries)
+    def _graph_step(self, slots, tokens, wanted, ids_device=None):
+        """One token for each of ``slots`` (checked by the caller); ``wanted``: the rows whose logits are returned."""
+        model, n = self.model, len(slots)
         bucket = batch_bucket(n)
-        starts = self.cache.reserve_all([e.slot for e in entries], [1] * n)
+        starts = self.cache.reserve_all(slots, [1] * n)
         # launch shapes follow the longest context and, where lengths are unequal, the mean one (both by
         # powers of two): attention cuts its keys finer when most sequences are far shorter than the longest
-        key = (bucket, context_bucket(max(starts) + 1), context_bucket(mean_context_of(starts, [1] * n, bucket)))
+        longest, mean = max(starts) + 1, -(-(sum(starts) + n) // bucket)
+        key = (bucket, context_bucket(longest), context_bucket(mean))
         g = self._graphs.get(key)
         if g is None:
             while len(self._graphs) >= GRAPH_KEEP:  # a batch that shrinks while its contexts grow meets many keys
@@ -242,19 +262,22 @@ class Engine:
             g = self._graphs[key] = _DecodeGraph(self, *key)
         self._graphs.move_to_end(key)
         turn, host = self.staging.take(g.size)
-        wanted = fill_arrays(host.numpy(), entries, starts, bucket, bucket)
+        zero, gone = [0] * (bucket - n), [-1] * (bucket - n)  # the padding rows; the arrays as ``layout`` orders them
+        host.numpy()[:] = (tokens + zero + starts + zero + slots + gone + list(range(n)) + [n] * (bucket - n + 1)
+                           + slots + gone + starts + zero)
         g.static.copy_(host, non_blocking=True)
         self.staging.copied(turn)
+        ids, logits = g.first(n)
         if ids_device is not None:  # the ids are the first array of the layout
-            g.static[:n].copy_(ids_device[:n], non_blocking=True)
+            ids.copy_(ids_device[:n], non_blocking=True)
         self.cache.flush_tables()
-        self.last_context = context_from(g.static, bucket, bucket, [1] * n, starts, model.dtype)
+        self.last_context = g.context(starts, longest, mean, model.dtype)
         g.graph.replay()
         ops.add_launches(g.launches)
-        for e in entries:
-            self.cache.advance(e.slot, 1)
+        for slot in slots:
+            self.cache.advance(slot, 1)
         if not wanted:
             return None
         if wanted == list(range(n)):
-            return g.logits[:n].clone()
+            return logits.clone()
         return g.logits[torch.tensor(wanted, dtype=torch.int64, device=model.device)]

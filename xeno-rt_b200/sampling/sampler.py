@@ -64,10 +64,10 @@ class Sampler:
                 params[1, i] = np.int32(c.top_k).view(np.float32)
                 params[2, i] = c.top_p
                 params[3, i] = c.repetition_penalty
-            self._options = torch.from_numpy(params).to(self.device)
+            dev = torch.from_numpy(params).to(self.device)
+            self._options = (dev[0], dev[1].view(torch.int32), dev[2], dev[3])
             self._options_key = key
-        dev = self._options
         out = torch.empty(n, dtype=torch.int32, device=self.device)
-        ops.sample(out, logits, row_slot, dev[0], dev[1].view(torch.int32), dev[2], dev[3], self.seen,
+        ops.sample(out, logits, row_slot, *self._options, self.seen,
                    self.rng_key, self.rng_counter)
         return out
