@@ -223,6 +223,18 @@ def test_gemm_reference(xd, wd, od, m, n, k):
         assert rel(acc, f64(base) + want) < 2e-6
 
 
+@pytest.mark.parametrize("k", [1, 63, 64, 65, 200])
+def test_gemm_reference_large_and_small_tiles_give_the_same_bits(k):
+    """100 tiles of 64 x 64 (large tiles) against some of the rows alone (tiles of 16 x 16), and both against float64."""
+    x = torch.randn(640, k, device=DEV)
+    w = torch.randn(640, k, device=DEV)
+    whole, some = torch.empty(640, 640, device=DEV), torch.empty(17, 640, device=DEV)
+    ops().gemm_reference(whole, x, w)
+    ops().gemm_reference(some, x[300:317].contiguous(), w)
+    assert rel(whole, f64(x) @ f64(w).T) < 2e-6
+    assert torch.equal(some, whole[300:317])
+
+
 def test_gemm_rows_do_not_depend_on_the_batch():
     x = torch.randn(70, 100, device=DEV)
     w = torch.randn(203, 100, device=DEV)
