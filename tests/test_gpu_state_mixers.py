@@ -90,7 +90,7 @@ def test_state_scan_in_portions_over_unequal_sequences(heads, qk_heads, dim, vdi
     assert bool((state[1] == 7.0).all()) and bool((state[4] == 7.0).all())
 
 
-@pytest.mark.parametrize("taps", [1, 2, 4])
+@pytest.mark.parametrize("taps", [1, 2, 3, 4, 6])
 def test_short_convolution_across_portions_shorter_than_its_reach(taps):
     from xeno_rt_b200.csrc import ops
     rng = np.random.default_rng(taps)

@@ -555,6 +555,45 @@ __global__ void short_conv_kernel(float* __restrict__ out, const float* __restri
   }
 }
 
+// The same for a number of taps known when compiling: the weights and the window of inputs stay in registers, and a tile's
+// inputs are asked for at once, so that an input is read once and not once a tap (and the taps' strided weights once a tile
+// and not once a token).  The sums are the same chains.
+// Measured, microseconds, 2,000 tokens, 4 taps: 4,096 channels 49 -> 21, 4,352 channels 52 -> 23 (3,050 GB/s).
+constexpr int CONV_TILE = 8;
+template <int TAPS>
+__global__ void __launch_bounds__(128)
+short_conv_taps_kernel(float* __restrict__ out, const float* __restrict__ x, int x_stride, const float* __restrict__ w,
+                       const float* __restrict__ bias, const float* __restrict__ in_bias, const float* __restrict__ state,
+                       const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, int channels, int act) {
+  constexpr int KEEP = TAPS - 1;
+  pdl_trigger();
+  pdl_wait(x, w, bias, in_bias, state, cu_seqlens, seq_slot);
+  const int s = blockIdx.x;
+  const int slot = seq_slot[s];
+  const int begin = cu_seqlens[s], len = cu_seqlens[s + 1] - begin;
+  const int l0 = blockIdx.y * CONV_TILE;
+  if (slot < 0 || l0 >= len) return;
+  const float* st = state + (size_t)slot * KEEP * channels;
+  for (int c = blockIdx.z * blockDim.x + threadIdx.x; c < channels; c += gridDim.z * blockDim.x) {
+    const float ib = in_bias != nullptr ? in_bias[c] : 0.f, b = bias != nullptr ? bias[c] : 0.f;
+    float wv[TAPS], in[KEEP + CONV_TILE];
+#pragma unroll
+    for (int i = 0; i < TAPS; ++i) wv[i] = w[c * TAPS + i];
+#pragma unroll
+    for (int i = 0; i < KEEP + CONV_TILE; ++i) {
+      const int src = l0 - KEEP + i;  // local index of the input
+      in[i] = src >= len ? 0.f : (src >= 0 ? x[(size_t)(begin + src) * x_stride + c] + ib : st[(size_t)(KEEP + src) * channels + c]);
+    }
+#pragma unroll
+    for (int t = 0; t < CONV_TILE; ++t) {
+      float acc = b;
+#pragma unroll
+      for (int i = 0; i < TAPS; ++i) acc = fmaf(wv[i], in[t + i], acc);
+      if (l0 + t < len) out[(size_t)(begin + l0 + t) * channels + c] = activate(acc, act);
+    }
+  }
+}
+
 // The state after the step: the last taps - 1 inputs of the sequence (older ones shift out).
 template <int MAX_KEEP>
 __global__ void short_conv_state_kernel(float* __restrict__ state, const float* __restrict__ x, int x_stride,
@@ -983,7 +1022,7 @@ XRT_EXPORT int xrt_short_conv(float* out, const float* x, int x_stride, const fl
   if (n_seqs < 0 || channels <= 0 || taps < 1 || max_new < 0) return XRT_ERR_ARGUMENT;
   if (taps > 9 || n_seqs > 65535) return XRT_ERR_UNSUPPORTED;
   if (n_seqs == 0 || max_new == 0) return XRT_OK;
-  const int tile_tokens = 8;
+  const int tile_tokens = xrt::CONV_TILE;
   const int threads = channels >= 128 ? 128 : 64;
   const int channel_blocks = (channels + threads - 1) / threads;
   if (max_new == 1 && taps > 1) {  // single tokens: one launch
@@ -992,10 +1031,15 @@ XRT_EXPORT int xrt_short_conv(float* out, const float* x, int x_stride, const fl
                        taps, act);
     return xrt::launch_status();
   }
-  xrt::launch_kernel(xrt::short_conv_kernel,
-                     dim3(n_seqs, (max_new + tile_tokens - 1) / tile_tokens, channel_blocks < 65535 ? channel_blocks : 65535),
-                     dim3(threads), 0, stream, out, x, x_stride, w, bias, in_bias, (const float*)state, cu_seqlens, seq_slot, channels, taps, tile_tokens,
-                     act);
+  const dim3 grid(n_seqs, (max_new + tile_tokens - 1) / tile_tokens, channel_blocks < 65535 ? channel_blocks : 65535);
+  if (taps >= 2 && taps <= 4) {
+    auto kernel = taps == 2 ? xrt::short_conv_taps_kernel<2> : (taps == 3 ? xrt::short_conv_taps_kernel<3> : xrt::short_conv_taps_kernel<4>);
+    xrt::launch_kernel(kernel, grid, dim3(threads), 0, stream, out, x, x_stride, w, bias, in_bias, (const float*)state, cu_seqlens,
+                       seq_slot, channels, act);
+  } else {
+    xrt::launch_kernel(xrt::short_conv_kernel, grid, dim3(threads), 0, stream, out, x, x_stride, w, bias, in_bias,
+                       (const float*)state, cu_seqlens, seq_slot, channels, taps, tile_tokens, act);
+  }
   if (taps > 1)
     xrt::launch_kernel(xrt::short_conv_state_kernel<8>, dim3(n_seqs, (channels + 255) / 256), dim3(256), 0, stream, state,
                        x, x_stride, in_bias, cu_seqlens, seq_slot, channels, taps);
