@@ -319,7 +319,7 @@ def test_experts_against_the_plain_experts(dtype, width, ff, experts, top, limit
 
 
 @pytest.mark.parametrize("width,ff,experts,top,n", [(64, 24, 6, 2, 230), (200, 72, 40, 1, 150), (256, 64, 8, 3, 333),
-                                                     (72, 136, 3, 3, 70)])
+                                                     (72, 136, 3, 3, 70), (328, 264, 3, 2, 300)])
 def test_experts_of_many_tokens_sorted_by_expert_in_one_launch_a_product(width, ff, experts, top, n):
     """The path of long steps in bfloat16: rows sorted by expert, both products for all experts in one launch each
     (experts without a row, row counts that are no multiple of the tile, widths that are no multiple of the K step)."""

@@ -477,7 +477,7 @@ def test_gelu_experts_against_the_plain_experts(dtype, width, ff, experts, top):
 
 
 @pytest.mark.parametrize("width,ff,experts,top,n", [(64, 24, 6, 2, 230), (200, 72, 40, 1, 150), (256, 64, 8, 3, 333),
-                                                     (72, 136, 3, 3, 70)])
+                                                     (72, 136, 3, 3, 70), (328, 264, 3, 2, 300)])
 def test_gelu_experts_of_many_tokens_sorted_by_expert(width, ff, experts, top, n):
     from xeno_rt_b200.csrc import ops
     rng = np.random.default_rng(9)

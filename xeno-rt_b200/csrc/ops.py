@@ -45,7 +45,7 @@ _SIGNATURES = {
     "xrt_moe_route": [_P, _P, _P, _P, _I, _I, _I, _P],
     "xrt_moe_experts": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _F, _F, _I, _I, _I, _P],
     "xrt_relu_squared": [_P, _P, _I, _I, _I, _P],
-    "xrt_moe_grouped_product": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _P],
+    "xrt_moe_grouped_product": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _P, _P],
     "xrt_moe_group": [_P, _P, _P, _P, _I, _I, _I, _P],
     "xrt_moe_gather": [_P, _P, _P, _I, _I, _I, _P],
     "xrt_moe_activation": [_P, _P, _I, _I, _F, _F, _I, _I, _P],
@@ -1274,7 +1274,7 @@ def moe_grouped_product(out, a, w, offsets, n_experts: int, ff: int = 0, limit: 
     _check(_kernels().xrt_moe_grouped_product(_ptr(out, "out", torch.bfloat16 if first else torch.float32),
                                              _ptr(a, "a", torch.bfloat16), _ptr(w, "w", torch.bfloat16),
                                              _ptr(offsets, "offsets", torch.int32), rows, int(n_experts), n, k, int(ff),
-                                             float(limit), float(alpha), first, _stream()),
+                                             float(limit), float(alpha), first, error_flag(a.device).data_ptr(), _stream()),
            "moe_grouped_product")
 
 
