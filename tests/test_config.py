@@ -151,22 +151,22 @@ def test_which_kernel_takes_a_decode_product_of_few_rows():
         assert choice(sms, rows, 5120, 8192, "accumulate") == (rows > 8)  # 320 blocks of 16 rows: one round
 
 
-def test_where_fixed_costs_decide_between_the_decode_kernels():
+def test_the_rounds_alone_decide_which_kernel_takes_a_decode_product(monkeypatch):
+    """Output matrices, long sums and narrow ones are no exceptions: which kernel adds up a product decides its last bits."""
     from xeno_rt_b200.core import KernelError
     from xeno_rt_b200.csrc import ops
-    from xeno_rt_b200.parts.linear_bf16 import few_rows_exception as choice
+    from xeno_rt_b200.parts import linear_bf16
     try:
         ops.library()
     except KernelError as exc:
         pytest.skip(f"the kernel library cannot be built here: {exc}")
+    monkeypatch.setattr(ops, "device_state", lambda device: (None, None, 148))
     for rows in (1, 8, 9, 16):
-        assert choice(148, rows, 4096, 14336, "accumulate") == choice(148, rows, 5120, 25600, "accumulate") == "tcgen05"
-        assert choice(148, rows, 2048, 8192, "accumulate") == "tcgen05"   # 256 blocks of 8 rows
-        assert choice(148, rows, 4096, 4096, "accumulate") is None
-        assert choice(148, rows, 5120, 8192, "accumulate") is None
-        assert choice(148, rows, 128256, 4096, "store") == ("stream" if rows <= 8 else None)
-        assert choice(148, rows, 5120, 4096, "store") is None             # one round
-        assert choice(148, rows, 25600, 5120, "swiglu") is None
+        many = "tcgen05" if rows > 8 else "stream"
+        for n, k, mode, kernel in ((128256, 4096, "store", "tcgen05"), (151936, 5120, "store", "tcgen05"),
+                                   (4096, 14336, "accumulate", many), (5120, 25600, "accumulate", many),
+                                   (2048, 8192, "accumulate", many), (2304, 9216, "accumulate", many)):
+            assert linear_bf16._decode_kernel(rows, n, k, mode, "cuda:0") == kernel, (rows, n, k, mode)
 
 
 def test_decode_attention_splits_cover_the_context_and_fill_the_rounds():

@@ -23,7 +23,6 @@ def aligned(x, weight) -> bool:
 
 
 ACCUMULATE_MIN_K_9_ROWS = 8192  # a product of 9 to 16 rows that adds into the residual stream takes the tcgen05 kernel from here on
-ACCUMULATE_LONG_K = 12288       # one of any number of rows does from here on
 STREAM_BLOCKS_PER_SM = 4        # blocks of the cp.async kernel that a multiprocessor holds at once (registers)
 
 
@@ -41,14 +40,16 @@ def stream_kernel_waves(sms: int, n: int, accumulate: bool = False) -> float:
 
 
 def tcgen05_for_few_rows(sms: int, rows: int, n: int, k: int, mode: str) -> bool:
-    """Up to 16 rows both decode kernels take the product; this is the choice by how full their rounds are
-    (``_decode_kernel`` makes two exceptions).  The tcgen05 kernel runs its items one a
+    """Up to 16 rows both decode kernels take the product.  The tcgen05 kernel runs its items one a
     multiprocessor in rounds: it wins where they fill the rounds (one round at least 0.6 full, or
     several at least 0.85 full).  Products that add into the residual stream stay on the cp.async
     kernel up to 8 rows, and from 9 rows on below K = 8,192 (its time grows with the rows, the tcgen05
     kernel's does not), unless its own rounds of blocks are badly filled.  Measured alone and back to
     back, cp.async against tcgen05 in microseconds at 1 / 8 / 16 rows: N 4,096, K 4,096: 7.8 / 8.2 / 9.8
-    against 10.0; N 5,120, K 8,192: 14.7 / 15.9 / 20.6 against 17.6."""
+    against 10.0; K 14,336: 22.7 / 24.7 / 26.9 against 21.8; N 5,120, K 8,192: 14.7 / 15.9 / 20.6 against
+    17.6; K 25,600: 44.0 / 46.6 / 63.6 against 43.9.  (Long sums of few rows would by now be a twentieth faster on the
+    tcgen05 kernel, and output matrices of up to 8 rows on the cp.async one; but with such exceptions short ones of 256
+    blocks, N 2,048, K 8,192, took 19.5 for 14.0, and which kernel adds up a product decides its last bits.)"""
     rounds, fill, reduction = ops.gemm_decode_tcgen05_plan(sms, rows, n, k, mode)
     fills = fill >= 0.6 and (rounds == 1 or fill >= 0.85)
     if mode == "accumulate" and (rows <= 8 or k < ACCUMULATE_MIN_K_9_ROWS):
@@ -62,24 +63,6 @@ def tcgen05_for_few_rows(sms: int, rows: int, n: int, k: int, mode: str) -> bool
     return fills
 
 
-def few_rows_exception(sms: int, rows: int, n: int, k: int, mode: str):
-    """Where the fixed costs of the two kernels decide and not how full their rounds are: the kernel, or None.  Products that
-    add into the residual stream take the tcgen05 kernel with any number of rows once K is so long that its ramp and its
-    meeting do not count (cp.async against tcgen05 in microseconds at 1 / 8 / 16 rows: N 4,096, K 12,288: 19.8 / 21.7 / 23.5
-    against 19.3; K 14,336: 22.7 / 24.7 / 26.9 against 21.8; N 5,120, K 25,600: 44.0 / 46.6 / 63.6 against 43.9), or earlier
-    where the cp.async kernel has fewer than two blocks a multiprocessor (N 2,048, K 8,192: 13.5 / 14.5 / 15.6 against 10.8).
-    Up to 8 rows of a product that is only stored and takes several rounds (an output matrix) take the cp.async kernel: it
-    reads whole rows of the weight, which the memory answers faster (N 128,256, K 4,096: 146 / 151 / 167 against 162 / 164 /
-    166; N 151,936: 173 / 178 / 198 against 196 / 196 / 202)."""
-    rounds, fill, _ = ops.gemm_decode_tcgen05_plan(sms, rows, n, k, mode)
-    if mode == "accumulate" and rounds == 1 and fill >= 0.6 and (
-            k >= ACCUMULATE_LONG_K or (k >= ACCUMULATE_MIN_K_9_ROWS and -(-n // 8) < 2 * sms)):
-        return "tcgen05"
-    if mode == "store" and rows <= 8 and rounds > 1:
-        return "stream"
-    return None
-
-
 def _decode_kernel(rows: int, n: int, k: int, mode: str, device) -> str:
     """Which of the two decode kernels takes a product of at most 128 rows: "stream" or "tcgen05"."""
     force = ops.tuning().decode_gemm
@@ -88,8 +71,7 @@ def _decode_kernel(rows: int, n: int, k: int, mode: str, device) -> str:
     if force == "tcgen05" or rows > STREAM_ROWS:
         return "tcgen05"
     sms = ops.device_state(device)[2]
-    return few_rows_exception(sms, rows, n, k, mode) or (
-        "tcgen05" if tcgen05_for_few_rows(sms, rows, n, k, mode) else "stream")
+    return "tcgen05" if tcgen05_for_few_rows(sms, rows, n, k, mode) else "stream"
 
 
 def _product(out, x, weight, mode: str, up_rows: int = 0, gate_act="silu") -> None:
