@@ -29,7 +29,7 @@ def close(got, want, tol=2e-5):
 
 # heads, q/k heads, key size, value size: key sizes on every lane layout of the kernel (8, 16 and 32 rows a
 # lane, 1 to 8 lanes a column), value sizes below, at and above a block's columns, sizes that are no power of two; the last
-# four: the kernel of four tokens at a time, with two columns a lane and (many heads) with four
+# four: the kernel of one chain a lane, with one column a lane and (many heads) with two
 SCAN_SIZES = [(2, 2, 8, 8), (3, 1, 16, 24), (4, 2, 48, 40), (1, 1, 130, 100), (2, 1, 256, 16), (2, 2, 32, 64),
               (2, 1, 128, 20), (4, 4, 64, 36), (20, 10, 128, 36), (20, 10, 64, 68)]
 
@@ -88,6 +88,43 @@ def test_state_scan_in_portions_over_unequal_sequences(heads, qk_heads, dim, vdi
         got[rows] = out.cpu().numpy()
     close(torch.from_numpy(got), want.reshape(total, -1), 3e-5)
     assert bool((state[1] == 7.0).all()) and bool((state[4] == 7.0).all())
+
+
+# blocks of one, two and four columns a lane (1, 12 and 40 sequences), single tokens on both kernels (1 and 80); columns beyond the last
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("heads,qk_heads,dim,vdim", [(4, 2, 128, 64), (8, 8, 128, 36), (4, 4, 64, 64), (8, 4, 64, 20)])
+def test_state_scan_is_the_same_bits_alone_and_in_a_batch_whole_and_cut(heads, qk_heads, dim, vdim, delta):
+    from xeno_rt_b200.csrc import ops
+    n, length = 80, 21
+    gen = torch.Generator(device=DEV).manual_seed(dim + vdim + delta)
+    rnd = lambda *shape: torch.randn(*shape, device=DEV, generator=gen)
+    q, k, v = rnd(n, length, qk_heads * dim), rnd(n, length, qk_heads * dim) * dim ** -0.5, rnd(n, length, heads * vdim)
+    decay = torch.rand(n, length, heads * dim, device=DEV, generator=gen) * 0.2 + 0.8
+    beta = rnd(n, length, heads)
+
+    def run(seqs, portions):
+        """Outputs [sequences, length, ...] and states of ``seqs``, brought in ``portions`` of tokens."""
+        m = len(seqs)
+        state = torch.zeros(m, heads, vdim, dim, device=DEV)
+        slots = torch.arange(m, dtype=torch.int32, device=DEV)
+        outs, at = [], 0
+        for part in portions:
+            take = lambda t: t[seqs, at:at + part].reshape(m * part, -1).contiguous()
+            out = torch.empty(m * part, heads * vdim, device=DEV)
+            cu = torch.arange(0, m * part + 1, part, dtype=torch.int32, device=DEV)
+            ops.state_scan(out, take(q), take(k), take(v), take(decay), take(beta) if delta else None, state, cu, slots, heads,
+                           qk_heads, dim, vdim, 0.5, delta, max_new=part)
+            outs.append(out.view(m, part, -1))
+            at += part
+        return torch.cat(outs, dim=1), state
+
+    singles = [1] * length
+    for seq in (0, 7):
+        want, want_state = run([seq], [length])
+        for seqs, portions in (([seq], [8, 1, 5, 7]), ([seq], singles), (list(range(12)), [length]), (list(range(40)), [length]),
+                               (list(range(n)), [length]), (list(range(n)), singles)):
+            got, state = run(seqs, portions)
+            assert torch.equal(got[seqs.index(seq)], want[0]) and torch.equal(state[seqs.index(seq)], want_state[0])
 
 
 @pytest.mark.parametrize("taps", [1, 2, 3, 4, 6])

@@ -2,6 +2,8 @@
 #pragma once
 
 #include <cuda_bf16.h>
+#include <atomic>
+
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdlib.h>
@@ -264,6 +266,18 @@ __device__ __forceinline__ void pdl_wait(P&... pointers) {
 }
 
 inline bool pdl_enabled() { return tuning().pdl; }
+
+// The current device's multiprocessors, asked once a device (0 if it cannot be asked).  What a rule of a dispatch compares
+// block counts with.
+inline int multiprocessors() {
+  static std::atomic<int> counts[64];
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 0;
+  int n = counts[device].load(std::memory_order_relaxed);
+  if (n == 0 && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess)
+    counts[device].store(n, std::memory_order_relaxed);
+  return n;
+}
 
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

@@ -44,7 +44,6 @@ struct ScanArgs {
   int n_heads, heads_per_qk, dim, vdim;
   float q_scale;
   int parts, cols, tile_tokens, stage_floats;
-  int stages;  // the wide kernel's ring
 };
 
 // VEC: 16-byte copies (dim, vdim, cols and every row stride are multiples of 4 floats, every base 16-byte aligned).
@@ -278,33 +277,46 @@ __global__ void __launch_bounds__(128) state_scan_kernel(const ScanArgs a) {
   }
 }
 
-// The scan for keys of 64 or 128 floats whose rows can be copied 16 bytes at a time; plain or delta rule.
-// What bounds the general kernel above is shared memory: every lane reads 12 bytes for each element of the state and token,
-// and a multiprocessor delivers 128 bytes a clock, whatever the lanes share.  Here a lane holds R rows of C2 neighbouring
-// columns, so that what it reads of q, k and a serves C2 columns, and what one prompt has of heads and columns is cut
-// finely enough to give every scheduler of the device a warp or two.  What is left is the chain from token to token, so
-// four tokens go together:
-//   the read-outs of four tokens are summed over the lanes in one go (lane_sums);
-//   with the delta rule, all the sums that four tokens' writes need are formed before the first write: with D_i the
-//   state decayed to token i without these writes, token i sees k_i^T D_i + sum over j < i of (k_i^T w_ij) u_j, where
-//   w_ij is k_j decayed from token j to i.  One round of shuffles instead of four.  The writes and read-outs then
-//   follow token by token as in the general kernel.
-// A ring of WIDE_STAGES tiles of WIDE_TOKENS tokens is filled by cp.async.
-// Measured, microseconds, general kernel -> this one: one prompt of 2,000 tokens, plain, 8 heads of 128 x 256 897 -> 281
-// (32 heads of 128 x 128 897 -> 400; 8 heads of 64 x 64 565 -> 216); delta rule, 16 heads of 128 x 128 1,046 -> 461 (four
-// prompts of 1,024 539 -> 433); 64 single tokens 27 -> 24.  Bound by the latency of its own chain of instructions: with two
-// warps a scheduler 0.4 instructions a clock, a third of the waiting for shared memory and shuffles.
-constexpr int WIDE_TOKENS = 8, WIDE_STAGES = 4, WIDE_GROUP = 4;
+// The scan for keys of 64 or 128 floats, plain or delta rule, with the same sums bit for bit.
+// The general kernel above gives a column few lanes with long chains each: one prompt of 8 heads of 128 x 256 is 32 blocks, and
+// a lane asks shared memory for 12 bytes an element of the state and token.  But a column's sums there are 4 * parts chains
+// over every (4 * parts)-th row (two chains of pairs a lane), added as a butterfly; here every chain has a lane of its own
+// (LANES of them, ROWS rows each) and the butterfly goes over the lanes in the same order, so a sequence's outputs and state do
+// not depend on which kernel took it, on how its tokens were cut into steps, nor on who else is in the step.  A lane's rows lie
+// next to one another in shared memory (brought there four bytes at a time by cp.async), so that it reads four at a time; the
+// read-outs of four tokens are summed over the lanes in one go (lane_sums).
+// A ring of SPREAD_STAGES tiles of SPREAD_TOKENS tokens is filled by cp.async.
+// Measured, microseconds, general kernel -> this one: one prompt of 2,000 tokens, plain, 8 heads of 128 x 256 899 -> 350 (8 heads of
+// 64 x 64 565 -> 193); delta rule, 16 heads of 128 x 128 1,046 -> 461; 64 prompts of 300 1,065 -> 757 and 1,332 -> 1,017.  One prompt
+// is bound by the chain of its own instructions, a warp a scheduler and 330 clocks a token; 64 prompts, by the count of the
+// instructions, by about half of what the schedulers issue.
+constexpr int SPREAD_TOKENS = 8, SPREAD_STAGES = 4, SPREAD_GROUP = 4, SPREAD_THREADS = 128;
 
-template <int R, int PARTS, int C2, int THREADS, bool DELTA>
-__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 3) state_scan_wide_kernel(const ScanArgs a) {
-  constexpr int P = R / 2, DIM = PARTS * R, COLS = THREADS / PARTS * C2, G = WIDE_GROUP;
+template <int LANES, int ROWS, int C2>
+struct SpreadShape {
+  static constexpr int THREADS = SPREAD_THREADS, DIM = LANES * ROWS, COLS = THREADS / LANES * C2;
+  // a vector in shared memory: a lane's rows together; the pitches put the lanes of a quarter warp on different banks
+  static constexpr int PITCH = ROWS == 16 ? 20 : 4, SKEW = LANES == 16 ? 4 : 0;
+  static constexpr int VECTOR = LANES * PITCH + SKEW;
+  static constexpr int STAGE = SPREAD_TOKENS * (3 * VECTOR + COLS + 1);  // q | k | a, then v [tokens][COLS], then b [tokens]
+  static constexpr int SMEM = SPREAD_STAGES * STAGE * (int)sizeof(float);
+  __device__ static constexpr int place(int residue) { return residue * PITCH + (residue >> 3) * SKEW; }
+  static_assert((ROWS == 16 && LANES == 8) || (ROWS == 4 && LANES == 16), "the pitches are for these");
+};
+
+template <int LANES, int ROWS, int C2, bool DELTA>
+__global__ void __launch_bounds__(SPREAD_THREADS) state_scan_spread_kernel(const ScanArgs a) {
+  using Shape = SpreadShape<LANES, ROWS, C2>;
+  constexpr int THREADS = SPREAD_THREADS, P = ROWS / 2, DIM = Shape::DIM, COLS = Shape::COLS, VECTOR = Shape::VECTOR, TT = SPREAD_TOKENS;
+  constexpr int G = SPREAD_GROUP * C2 <= LANES ? SPREAD_GROUP : LANES / C2;  // tokens whose read-outs are summed together
   extern __shared__ float4 tile4[];
   float* tile = reinterpret_cast<float*>(tile4);
   pdl_trigger();
-  const int TT = a.tile_tokens, vdim = a.vdim;
-  const int vec_floats = TT * DIM;  // a stage: q | k | a, each [TT][DIM]; v [TT][COLS]; b [TT], padded to 16 bytes
-  const int part = threadIdx.x % PARTS, jl = (threadIdx.x / PARTS) * C2;
+  const int vdim = a.vdim;
+  const int part = threadIdx.x % LANES, jl = (threadIdx.x / LANES) * C2;
+  // the lane's rows: residue, residue + LANES, ...; the bits of the lane's number from the highest down are those of the
+  // residue from the lowest up, since the butterfly of the general kernel adds neighbouring rows first
+  const int residue = (int)(__brev((unsigned)part) >> (LANES == 8 ? 29 : 28));
   pdl_wait();
   const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * COLS;
   const int slot = a.seq_slot[s];
@@ -313,215 +325,180 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 3) state_scan_wi
   const int j = col0 + jl, qh = h / a.heads_per_qk;
 
   auto issue = [&](int t0, int stage) {
-    float* sq = tile + stage * a.stage_floats;
+    float* sq = tile + stage * Shape::STAGE;
     const int nt = min(TT, end - t0);
-    constexpr int PER = DIM / 4;
-    const int d = (threadIdx.x % PER) * 4;
-    for (int tt = threadIdx.x / PER; tt < nt; tt += THREADS / PER) {
+    const int r = threadIdx.x % DIM;
+    const int at = Shape::place(r % LANES) + r / LANES;
+    for (int tt = threadIdx.x / DIM; tt < nt; tt += THREADS / DIM) {
       const size_t t = (size_t)(t0 + tt);
-      cp_async<16>(sq + tt * DIM + d, a.q + t * a.q_stride + qh * DIM + d);
-      cp_async<16>(sq + vec_floats + tt * DIM + d, a.k + t * a.k_stride + qh * DIM + d);
-      cp_async<16>(sq + 2 * vec_floats + tt * DIM + d, a.decay + t * a.decay_stride + h * DIM + d);
+      cp_async<4>(sq + tt * VECTOR + at, a.q + t * a.q_stride + qh * DIM + r);
+      cp_async<4>(sq + (TT + tt) * VECTOR + at, a.k + t * a.k_stride + qh * DIM + r);
+      cp_async<4>(sq + (2 * TT + tt) * VECTOR + at, a.decay + t * a.decay_stride + h * DIM + r);
     }
-    float* sv = sq + 3 * vec_floats;
-    constexpr int VPER = COLS / 4;
-    const int c = (threadIdx.x % VPER) * 4;
+    float* sv = sq + 3 * TT * VECTOR;
+    const int c = threadIdx.x % COLS;
     if (col0 + c < vdim)
-      for (int tt = threadIdx.x / VPER; tt < nt; tt += THREADS / VPER)
-        cp_async<16>(sv + tt * COLS + c, a.v + (size_t)(t0 + tt) * a.v_stride + h * vdim + col0 + c);
+      for (int tt = threadIdx.x / COLS; tt < nt; tt += THREADS / COLS)
+        cp_async<4>(sv + tt * COLS + c, a.v + (size_t)(t0 + tt) * a.v_stride + h * vdim + col0 + c);
     if (DELTA && (int)threadIdx.x < nt)
       cp_async<4>(sv + TT * COLS + threadIdx.x, a.beta + (size_t)(t0 + threadIdx.x) * a.beta_stride + h);
   };
 
-  // a lane's rows: every PARTS-th group of four, as in the general kernel
-  auto rows_of = [&](const float* row, float2 (&out)[P]) {
+  struct Token { float2 k[P], a[P], q[P]; float u[C2], b; };
+  auto load = [&](const float* sq, int tt, Token& t) {
+    auto rows_of = [&](const float* vector, float2 (&out)[P]) {
+      const float4* src = reinterpret_cast<const float4*>(vector + Shape::place(residue));
 #pragma unroll
-    for (int g = 0; g < R / 4; ++g) {
-      const float4 t = reinterpret_cast<const float4*>(row)[g * PARTS + part];
-      out[2 * g] = make_float2(t.x, t.y);
-      out[2 * g + 1] = make_float2(t.z, t.w);
-    }
+      for (int i = 0; i < ROWS / 4; ++i) {
+        const float4 f = src[i];
+        out[2 * i] = make_float2(f.x, f.y);
+        out[2 * i + 1] = make_float2(f.z, f.w);
+      }
+    };
+    rows_of(sq + (2 * TT + tt) * VECTOR, t.a);
+    rows_of(sq + (TT + tt) * VECTOR, t.k);
+    rows_of(sq + tt * VECTOR, t.q);
+    const float* sv = sq + 3 * TT * VECTOR;
+#pragma unroll
+    for (int c = 0; c < C2; ++c) t.u[c] = sv[tt * COLS + jl + c];
+    t.b = DELTA ? sv[TT * COLS + tt] : 0.f;
   };
-  auto dot = [](const float2 (&x)[P], const float2 (&y)[P]) {
-    float2 sum = __fmul2_rn(x[0], y[0]);
+  // one chain over the lane's rows
+  auto chain = [](const float2 (&x)[P], const float2 (&y)[P]) {
+    float sum = 0.f;
 #pragma unroll
-    for (int i = 1; i < P; ++i) sum = __ffma2_rn(x[i], y[i], sum);
-    return sum.x + sum.y;
+    for (int i = 0; i < P; ++i) sum = __fmaf_rn(x[i].y, y[i].y, __fmaf_rn(x[i].x, y[i].x, sum));
+    return sum;
   };
   float2 S[C2][P];
-  float* sp = a.state + (((size_t)slot * a.n_heads + h) * vdim + j) * DIM;
+  float* sp = a.state + (((size_t)slot * a.n_heads + h) * vdim + j) * DIM + residue;
 #pragma unroll
-  for (int c = 0; c < C2; ++c) {
-    if (j + c < vdim) {
-      rows_of(sp + (size_t)c * DIM, S[c]);
+  for (int c = 0; c < C2; ++c)
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+      S[c][i] = j + c < vdim ? make_float2(sp[(size_t)c * DIM + 2 * i * LANES], sp[(size_t)c * DIM + (2 * i + 1) * LANES])
+                             : make_float2(0.f, 0.f);
+
+  // a token's write into the state; `read` gets this lane's chains of what the token reads
+  auto work = [&](const Token& t, float* read) {
+    float u[C2];
+#pragma unroll
+    for (int c = 0; c < C2; ++c) u[c] = t.u[c];
+    if (DELTA) {
+      float seen[C2];
+#pragma unroll
+      for (int c = 0; c < C2; ++c) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) S[c][i] = __fmul2_rn(S[c][i], t.a[i]);
+        seen[c] = chain(S[c], t.k);
+      }
+#pragma unroll
+      for (int o = LANES / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < C2; ++c) seen[c] += __shfl_xor_sync(0xffffffffu, seen[c], o);
+#pragma unroll
+      for (int c = 0; c < C2; ++c) {
+        u[c] = t.b * (u[c] - seen[c]);
+#pragma unroll
+        for (int i = 0; i < P; ++i) S[c][i] = __ffma2_rn(t.k[i], make_float2(u[c], u[c]), S[c][i]);
+      }
     } else {
 #pragma unroll
-      for (int i = 0; i < P; ++i) S[c][i] = make_float2(0.f, 0.f);
+      for (int c = 0; c < C2; ++c)
+#pragma unroll
+        for (int i = 0; i < P; ++i) S[c][i] = __ffma2_rn(S[c][i], t.a[i], __fmul2_rn(t.k[i], make_float2(u[c], u[c])));
     }
-  }
-  // the write of u into the state decayed by `aa`
-  auto write = [&](const float2 (&aa)[P], const float2 (&kk)[P], const float (&u)[C2]) {
 #pragma unroll
-    for (int c = 0; c < C2; ++c)
-#pragma unroll
-      for (int i = 0; i < P; ++i) {
-        if (DELTA) S[c][i] = __ffma2_rn(kk[i], make_float2(u[c], u[c]), __fmul2_rn(S[c][i], aa[i]));
-        else S[c][i] = __ffma2_rn(S[c][i], aa[i], __fmul2_rn(kk[i], make_float2(u[c], u[c])));
-      }
+    for (int c = 0; c < C2; ++c) read[c] = chain(S[c], t.q);
   };
-  // sum number `value` of a group of tokens that begins at token t belongs to this lane
+  // sum number `value` of the tokens from t on belongs to this lane
   auto store = [&](int t, int value, int per_value, float sum) {
     const int tt = value / C2, c = value % C2;
     if (part % per_value == 0 && j + c < vdim)
       a.out[(size_t)(t + tt) * a.n_heads * vdim + h * vdim + j + c] = sum * a.q_scale;
   };
 
-  const int n_tiles = (end - begin + TT - 1) / TT, stages = a.stages;
-  for (int p = 0; p < stages - 1; ++p) {
+  const int n_tiles = (end - begin + TT - 1) / TT;
+  for (int p = 0; p < SPREAD_STAGES - 1; ++p) {
     if (p < n_tiles) issue(begin + p * TT, p);
     cp_async_commit();
   }
   for (int tile_i = 0; tile_i < n_tiles; ++tile_i) {
-    const int t0 = begin + tile_i * TT, nt = min(TT, end - t0), stage = tile_i % stages;
-    if (stages == 1) {
-      if (tile_i > 0) __syncthreads();  // (a sequence is longer than the caller said: one tile after another)
-      issue(t0, 0);
-      cp_async_commit();
-      cp_async_wait<0>();
-    } else {
-      cp_async_wait<WIDE_STAGES - 2>();
+    const int t0 = begin + tile_i * TT, nt = min(TT, end - t0);
+    cp_async_wait<SPREAD_STAGES - 2>();
+    float* sq = tile + (tile_i % SPREAD_STAGES) * Shape::STAGE;
+    if (DELTA && (int)threadIdx.x < nt) {  // b = sigmoid(raw), once a tile, by the thread whose own copy brought the raw value
+      float* b = sq + TT * (3 * VECTOR + COLS) + threadIdx.x;
+      *b = sigmoidf_(*b);
     }
-    const float* sq = tile + stage * a.stage_floats;
-    const float* sk = sq + vec_floats;
-    const float* sa = sk + vec_floats;
-    float* sv = tile + stage * a.stage_floats + 3 * vec_floats;
-    float* sb = sv + TT * COLS;
-    if (DELTA && (int)threadIdx.x < nt)  // b = sigmoid(raw), once a tile, by the thread whose own copy brought the raw value
-      sb[threadIdx.x] = sigmoidf_(sb[threadIdx.x]);
     __syncthreads();  // the tile is there, and everybody has left the stage that the next copies overwrite
-    if (stages > 1) {
-      if (tile_i + stages - 1 < n_tiles) issue(t0 + (stages - 1) * TT, (tile_i + stages - 1) % stages);
-      cp_async_commit();
-    }
-    auto group = [&](int tt) {
-      float2 kk[G][P], aa[G][P], qq[G][P];
-      float u[G][C2];
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        rows_of(sk + (tt + g) * DIM, kk[g]);
-        rows_of(sa + (tt + g) * DIM, aa[g]);
-#pragma unroll
-        for (int c = 0; c < C2; ++c) u[g][c] = sv[(tt + g) * COLS + jl + c];
-      }
-#pragma unroll
-      for (int g = 0; g < G; ++g) rows_of(sq + (tt + g) * DIM, qq[g]);
-      if (DELTA) {
-        constexpr int CROSS = G * (G - 1) / 2, N = G * C2 + CROSS;  // k_i^T D_i by token and column, then k_i^T w_ij
-        float sums[N];
-        float2 D[C2][P], w[G][P];
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-#pragma unroll
-          for (int c = 0; c < C2; ++c) {
-#pragma unroll
-            for (int i = 0; i < P; ++i) D[c][i] = __fmul2_rn(g == 0 ? S[c][i] : D[c][i], aa[g][i]);
-            sums[g * C2 + c] = dot(D[c], kk[g]);
-          }
-#pragma unroll
-          for (int e = 0; e < g; ++e) {
-#pragma unroll
-            for (int i = 0; i < P; ++i) w[e][i] = __fmul2_rn(w[e][i], aa[g][i]);
-            sums[G * C2 + g * (g - 1) / 2 + e] = dot(w[e], kk[g]);
-          }
-#pragma unroll
-          for (int i = 0; i < P; ++i) w[g][i] = kk[g][i];
-        }
-        all_lane_sums<PARTS>(sums, part);
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          const float b = sb[tt + g];
-#pragma unroll
-          for (int c = 0; c < C2; ++c) {
-            float seen = sums[g * C2 + c];
-#pragma unroll
-            for (int e = 0; e < g; ++e) seen = fmaf(sums[G * C2 + g * (g - 1) / 2 + e], u[e][c], seen);
-            u[g][c] = b * (u[g][c] - seen);
-          }
-        }
-      }
+    if (tile_i + SPREAD_STAGES - 1 < n_tiles) issue(t0 + (SPREAD_STAGES - 1) * TT, (tile_i + SPREAD_STAGES - 1) % SPREAD_STAGES);
+    cp_async_commit();
+    if (nt == TT) {  // the usual tile in one piece, the next token's vectors on their way to the registers
+      Token now, next;
+      load(sq, 0, now);
       float read[G * C2];
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        write(aa[g], kk[g], u[g]);
-#pragma unroll
-        for (int c = 0; c < C2; ++c) read[g * C2 + c] = dot(S[c], qq[g]);
+      for (int tt = 0; tt < TT; ++tt) {
+        if (tt + 1 < TT) load(sq, tt + 1, next);
+        work(now, read + (tt % G) * C2);
+        if (tt % G == G - 1)
+          store(t0 + tt - (G - 1), part * (G * C2) / LANES, LANES / (G * C2), lane_sums<LANES>(read, part));
+        now = next;
       }
-      store(t0 + tt, part * (G * C2) / PARTS, PARTS / (G * C2), lane_sums<PARTS>(read, part));
-    };
-    int tt = 0;
-    if (nt == WIDE_TOKENS) {  // the usual tile in one piece: the second group's loads do not wait for the first's sums
-#pragma unroll
-      for (; tt < WIDE_TOKENS; tt += G) group(tt);
     } else {
 #pragma unroll 1
-      for (; tt + G <= nt; tt += G) group(tt);
-    }
-#pragma unroll 1
-    for (; tt < nt; ++tt) {
-      float2 kk[P], aa[P], qq[P];
-      rows_of(sk + tt * DIM, kk);
-      rows_of(sa + tt * DIM, aa);
-      rows_of(sq + tt * DIM, qq);
-      float u[C2], read[C2];
-#pragma unroll
-      for (int c = 0; c < C2; ++c) u[c] = sv[tt * COLS + jl + c];
-      if (DELTA) {
-        float seen[C2];
-#pragma unroll
-        for (int c = 0; c < C2; ++c) {
-          float2 D[P];
-#pragma unroll
-          for (int i = 0; i < P; ++i) D[i] = __fmul2_rn(S[c][i], aa[i]);
-          seen[c] = dot(D, kk);
-        }
-#pragma unroll
-        for (int o = PARTS / 2; o > 0; o >>= 1)
-#pragma unroll
-          for (int c = 0; c < C2; ++c) seen[c] += __shfl_xor_sync(0xffffffffu, seen[c], o);
-        const float b = sb[tt];
-#pragma unroll
-        for (int c = 0; c < C2; ++c) u[c] = b * (u[c] - seen[c]);
+      for (int tt = 0; tt < nt; ++tt) {
+        Token now;
+        load(sq, tt, now);
+        float read[C2];
+        work(now, read);
+        store(t0 + tt, part * C2 / LANES, LANES / C2, lane_sums<LANES>(read, part));
       }
-      write(aa, kk, u);
-#pragma unroll
-      for (int c = 0; c < C2; ++c) read[c] = dot(S[c], qq);
-      store(t0 + tt, part * C2 / PARTS, PARTS / C2, lane_sums<PARTS>(read, part));
     }
   }
 #pragma unroll
   for (int c = 0; c < C2; ++c)
 #pragma unroll
-    for (int g = 0; g < R / 4; ++g)
-      if (j + c < vdim)
-        reinterpret_cast<float4*>(sp + (size_t)c * DIM)[g * PARTS + part] =
-            make_float4(S[c][2 * g].x, S[c][2 * g].y, S[c][2 * g + 1].x, S[c][2 * g + 1].y);
+    for (int i = 0; i < P; ++i)
+      if (j + c < vdim) {
+        sp[(size_t)c * DIM + 2 * i * LANES] = S[c][i].x;
+        sp[(size_t)c * DIM + (2 * i + 1) * LANES] = S[c][i].y;
+      }
 }
 
-template <int R, int PARTS, int C2, int THREADS, bool DELTA>
-int launch_state_scan_wide(ScanArgs a, int n_seqs, int max_new, cudaStream_t stream) {
-  constexpr int DIM = PARTS * R, COLS = THREADS / PARTS * C2;
-  auto kernel = state_scan_wide_kernel<R, PARTS, C2, THREADS, DELTA>;
-  a.tile_tokens = max_new < WIDE_TOKENS ? max_new : WIDE_TOKENS;
-  a.stages = max_new <= WIDE_TOKENS ? 1 : WIDE_STAGES;
-  a.stage_floats = 3 * a.tile_tokens * DIM + a.tile_tokens * COLS + ((a.tile_tokens + 3) & ~3);
-  const size_t smem = (size_t)a.stages * a.stage_floats * sizeof(float);
-  constexpr int most = WIDE_STAGES * (WIDE_TOKENS * (3 * DIM + COLS + 1)) * (int)sizeof(float);
-  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+template <int LANES, int ROWS, int C2, bool DELTA>
+int launch_state_scan_spread(const ScanArgs& a, int n_seqs, int max_new, cudaStream_t stream) {
+  using Shape = SpreadShape<LANES, ROWS, C2>;
+  auto kernel = state_scan_spread_kernel<LANES, ROWS, C2, DELTA>;
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
   if (err != cudaSuccess) return (int)err;
-  const dim3 grid(n_seqs, a.n_heads, (a.vdim + COLS - 1) / COLS);
-  if (max_new > 1) launch_kernel_alone(kernel, grid, dim3(THREADS), smem, stream, a);
-  else launch_kernel(kernel, grid, dim3(THREADS), smem, stream, a);
+  const dim3 grid(n_seqs, a.n_heads, (a.vdim + Shape::COLS - 1) / Shape::COLS);
+  if (max_new > 1) launch_kernel_alone(kernel, grid, dim3(SPREAD_THREADS), (size_t)Shape::SMEM, stream, a);
+  else launch_kernel(kernel, grid, dim3(SPREAD_THREADS), (size_t)Shape::SMEM, stream, a);
   return launch_status();
+}
+
+// Columns a lane: what it reads of q, k and a serves all of them, but the blocks get fewer.  As few as still let all blocks run
+// at once (microseconds at 1 / 2 / 4 columns, plain, 8 heads of 128 x 256: one prompt of 2,000 tokens 350 / 372 / 485, two 564 /
+// 382 / 487, three of 1,000 395 / 315 / 245, 64 of 300 2,186 / 1,139 / 757); for the delta rule, whose chain from token to token is
+// longer, two columns until its blocks are two a multiprocessor (16 heads of 128 x 128: three prompts of 1,000 433 / 362 / 424, eight
+// of 300 383 / 220 / 167).  Single tokens: two columns up to four blocks a multiprocessor (1 / 8 sequences 3.3 -> 2.4 / 6.5 -> 4.8),
+// then four (32 / 64 sequences 13.1 -> 11.8 / 24.2 -> 22.2); a state that the L2 does not hold is left to the general kernel, which
+// reads it in whole lines (128 sequences, 134 MB, 50.8 against 62.4).
+template <int LANES, int ROWS, bool DELTA>
+int state_scan_spread(const ScanArgs& a, int n_seqs, int max_new, bool& taken, cudaStream_t stream) {
+  const int sms = multiprocessors();
+  auto blocks = [&](int columns) {
+    const int cols = SPREAD_THREADS / LANES * columns;
+    return (long long)n_seqs * a.n_heads * ((a.vdim + cols - 1) / cols);
+  };
+  taken = max_new > 1 || (long long)n_seqs * a.n_heads * a.vdim * (LANES * ROWS * 4) <= (96ll << 20);
+  if (!taken) return XRT_OK;
+  if (max_new > 1 && blocks(1) <= sms) return launch_state_scan_spread<LANES, ROWS, 1, DELTA>(a, n_seqs, max_new, stream);
+  if (blocks(2) <= (max_new == 1 ? 4 : (DELTA ? 2 : 1)) * (long long)sms)
+    return launch_state_scan_spread<LANES, ROWS, 2, DELTA>(a, n_seqs, max_new, stream);
+  return launch_state_scan_spread<LANES, ROWS, 4, DELTA>(a, n_seqs, max_new, stream);
 }
 
 // ------------------------------------------------------------------------------------------ convolution
@@ -928,7 +905,7 @@ inline int grid_for(size_t total, int threads) {
 }  // namespace xrt
 
 // Rows of a column's state that one lane holds, for a key size.  Few lanes a column (4 up to a key size of 64,
-// 2 at 128) keep the butterflies short; measured at 32 heads of 128 x 128 (16 / 32 / 64 rows a lane): one prompt
+// 2 at 128) keep the butterflies short; the general kernel at 32 heads of 128 x 128 (16 / 32 / 64 rows a lane): one prompt
 // of 2,048 tokens 1.11 / 1.11 / 1.17 ms, four such prompts 2.1 / 2.05 / 1.64 ms, 64 single tokens 130 / 109 / 95 us.
 static int scan_rows_per_lane(int dim) { return dim <= 32 ? 8 : (dim <= 64 ? 16 : (dim <= 128 ? 64 : 32)); }
 
@@ -949,16 +926,12 @@ XRT_EXPORT int xrt_state_scan(float* out, const float* q, int q_stride, const fl
   const int R = scan_rows_per_lane(dim);
   int parts = 1;
   while (parts * R < dim) parts <<= 1;
-  // columns a lane holds: one.  (Several, so that what a lane reads of q, k and a serves more columns, was
-  // measured slower: 1.77 against 0.96 ms for 2,048 tokens of 32 heads of 128 x 128; a token's time is the
-  // chain of dependent instructions of ONE warp, and more columns a lane make that chain longer.)
-  const int per_lane = 1;
   // 128 threads a block at most, whole warps at least
   int groups = 128 / parts;
   if (groups < 1) groups = 1;
-  while (groups > 1 && (groups / 2) * per_lane >= vdim && (groups / 2) * parts >= 32) groups >>= 1;
+  while (groups > 1 && groups / 2 >= vdim && (groups / 2) * parts >= 32) groups >>= 1;
   if (groups * parts < 32) groups = 32 / parts;
-  const int cols = groups * per_lane;
+  const int cols = groups;  // one column a lane
   const int padded = parts * R;
   const int n_vec = mode == 2 ? 5 : 3;
   auto stage_floats = [&](int tt) { return n_vec * tt * padded + ((tt * cols + 3) & ~3) + ((tt + 3) & ~3); };
@@ -975,22 +948,14 @@ XRT_EXPORT int xrt_state_scan(float* out, const float* q, int q_stride, const fl
   xrt::ScanArgs a = {out, q, k, v, decay, beta, unit, removal, unit_stride, removal_stride,
                      q_stride, k_stride, v_stride, decay_stride, beta_stride, state,
                      cu_seqlens, seq_slot, n_heads, n_heads / n_qk_heads, dim, vdim, q_scale, parts, cols, tile_tokens,
-                     stage_floats(tile_tokens), 1};
-  if (vec && mode != 2 && (dim == 128 || dim == 64)) {
-    // four columns a lane once their blocks cover the multiprocessors (16 prompts of 500 tokens, 8 heads of 128 x 256, plain:
-    // 360 us against 370 with two columns); else two, and half the rows a lane (one prompt: 281 against 290)
-    const long long blocks_4 = (long long)n_seqs * n_heads * ((vdim + 31) / 32);
-    const bool four = blocks_4 >= 148;
-#define XRT_SCAN_WIDE(DD)                                                                                    \
-  do {                                                                                                       \
-    if (dim == 128 && four) return xrt::launch_state_scan_wide<8, 16, 4, 128, DD>(a, n_seqs, max_new, stream); \
-    if (dim == 128) return xrt::launch_state_scan_wide<4, 32, 2, 256, DD>(a, n_seqs, max_new, stream);         \
-    if (four) return xrt::launch_state_scan_wide<4, 16, 4, 128, DD>(a, n_seqs, max_new, stream);               \
-    return xrt::launch_state_scan_wide<4, 16, 2, 128, DD>(a, n_seqs, max_new, stream);                         \
-  } while (0)
-    if (delta) XRT_SCAN_WIDE(true);
-    XRT_SCAN_WIDE(false);
-#undef XRT_SCAN_WIDE
+                     stage_floats(tile_tokens)};
+  if (mode != 2 && (dim == 128 || dim == 64)) {
+    bool taken = false;
+    const int status = dim == 128 ? (delta ? xrt::state_scan_spread<8, 16, true>(a, n_seqs, max_new, taken, stream)
+                                           : xrt::state_scan_spread<8, 16, false>(a, n_seqs, max_new, taken, stream))
+                                  : (delta ? xrt::state_scan_spread<16, 4, true>(a, n_seqs, max_new, taken, stream)
+                                           : xrt::state_scan_spread<16, 4, false>(a, n_seqs, max_new, taken, stream));
+    if (taken) return status;
   }
   const dim3 grid(n_seqs, n_heads, (vdim + cols - 1) / cols), block(parts * groups);
 #define XRT_SCAN(RR, CC, DD, VV)                                                                                  \
