@@ -180,3 +180,20 @@ def test_rows_without_a_finite_maximum_and_with_nan():
         logits[5] = np.nan
         assert set(run_sampler(logits, 64, 1.0, 2, 1.0, 1.0).tolist()) == {7, vocab - 2}
         assert set(run_sampler(logits, 8, 0.0, 0, 1.0, 1.0).tolist()) == {7}
+
+
+@pytest.mark.parametrize("vocab", [300, 20001, 128256])
+def test_infinities_take_the_row_and_a_nan_is_never_drawn(vocab):
+    """The first infinity is the id, whatever else the row holds; beside finite values a NaN has no mass, with and without top_k
+    and top_p, on one block and on a team."""
+    rng = np.random.default_rng(vocab)
+    options = [(1.0, 0, 1.0), (1.0, 0, 0.9), (0.7, 40, 0.95), (0.7, 280, 1.0), (0.0, 0, 1.0)]
+    logits = rng.normal(size=vocab).astype(np.float32)
+    logits[[3, vocab // 2, vocab - 1]] = np.nan
+    for temperature, top_k, top_p in options:
+        got = run_sampler(logits, 64, temperature, top_k, top_p, 1.0)
+        assert np.isfinite(logits[got]).all()
+        for infinite in ([vocab // 3], [vocab - 2, vocab // 3], [7, 8, vocab - 2]):
+            row = logits.copy()
+            row[infinite] = np.inf
+            assert set(run_sampler(row, 8, temperature, top_k, top_p, 1.0).tolist()) == {min(infinite)}

@@ -120,7 +120,6 @@ struct SampleShared {
   int selected;
   int count;                           // this block's candidates, -1: too many
   int cut;
-  int irregular;                       // a NaN among this block's logits
   unsigned int draw;
   long long pick;
   int warp_count[SAMPLE_WARPS];
@@ -193,6 +192,12 @@ __device__ long long ordered_pick(F weight, int n, int base, uint64_t target, Te
   const long long found = team.sh->pick;
   __syncthreads();  // the next call resets it
   return found;
+}
+
+// The mass of a value: 2^32 times its probability over the largest value's, rounded down.  None for a NaN, and none for an
+// infinity against another (the row's first infinity is then its id, as the first maximum without any mass).
+__device__ __forceinline__ uint64_t probability_mass(float a, float row_max, float inv_temp) {
+  return (uint64_t)(fmaxf(expf((a - row_max) * inv_temp), 0.f) * 4294967296.0f);  // (the larger of a NaN and 0 is 0)
 }
 
 // Radix select from the top: the largest key K such that the weight of {key >= K} reaches `want` (>= 1).
@@ -290,7 +295,7 @@ __device__ long long sample_place(A adjusted, int n, int base, long long n_all, 
   auto mass_of = [&](int i, float a) -> uint64_t {
     const uint32_t key = order_key(a);
     if (key < k_key || (key == k_key && base + i > k_last)) return 0ull;
-    return (uint64_t)(expf((a - row_max) * inv_temp) * 4294967296.0f);
+    return probability_mass(a, row_max, inv_temp);
   };
   // top-p: threshold by probability mass
   uint32_t p_key = 0u; long long p_last = n_all;
@@ -393,7 +398,7 @@ __device__ long long ranked_place(float a, int n, int k, float temp, float p, fl
 #pragma unroll 4
     for (int j = 0; j < n; ++j) rank += order[j] > mine;
   }
-  const uint64_t m = i < n && rank < k ? (uint64_t)(expf((a - row_max) * (1.0f / temp)) * 4294967296.0f) : 0ull;
+  const uint64_t m = i < n && rank < k ? probability_mass(a, row_max, 1.0f / temp) : 0ull;
   if (i < n) mass[i] = m;
   uint64_t total;
   block_exclusive_scan(m, team.sh->scan, &total);
@@ -458,11 +463,10 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
   if (few)
     for (int b = threadIdx.x; b < SAMPLE_FINE_BINS; b += SAMPLE_THREADS) hist[b] = 0u;
   if (few) __syncthreads();
-  float best = -INFINITY; int best_i = -1, nan_seen = 0;
+  float best = -INFINITY; int best_i = -1;
   auto take = [&](int i, float a) {
     if (CACHED) values[i] = a;
     if (a > best) { best = a; best_i = i; }  // indices rise: the first maximum is kept
-    nan_seen |= a != a;
     if (few && !of_largest) atomicAdd(&hist[order_key(a) >> 20], 1u);
   };
   if (VEC) {
@@ -504,8 +508,7 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
     packed = other > packed ? other : packed;
   }
   if (lane == 0) sh.scan[warp] = packed;
-  const int irregular_here = __syncthreads_or(nan_seen);
-  if (threadIdx.x == 0) sh.irregular = irregular_here;
+  __syncthreads();
   if (threadIdx.x < SAMPLE_TEAM) {
     for (int w = 0; w < SAMPLE_WARPS; ++w) packed = sh.scan[w] > packed ? sh.scan[w] : packed;
   }
@@ -547,12 +550,9 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
   bool compact = few;
   int counts[SAMPLE_TEAM];
   int all = 0;
-  // masses beyond 2^32 (of a NaN, or of an infinity against another) are summed in 64 bits
-  bool wide = n > 65535 * SAMPLE_HIST_COPIES || !(fabsf(row_max) < INFINITY);
 #pragma unroll
   for (int r = 0; r < SAMPLE_TEAM; ++r) {
     counts[r] = (few && r < team_size) ? *of_block(&sh.count, r) : 0;
-    if (r < team_size) wide = wide || *of_block(&sh.irregular, r) != 0;
     compact = compact && counts[r] >= 0;
     all += counts[r];
   }
@@ -575,7 +575,7 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
         at += counts[r];
       }
       team_sync();  // the candidates are here: the other blocks may leave
-      if (all > SAMPLE_NARROW && k <= SAMPLE_THREADS / 2 && !wide) {
+      if (all > SAMPLE_NARROW && k <= SAMPLE_THREADS / 2) {
         for (int b = threadIdx.x; b < SAMPLE_FINE_BINS; b += SAMPLE_THREADS) hist[b] = 0u;
         __syncthreads();
         for (int i = threadIdx.x; i < all; i += SAMPLE_THREADS) atomicAdd(&hist[order_key(vals[i]) >> 20], 1u);
@@ -591,12 +591,12 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
         }
       }
       long long place;
-      if (all <= SAMPLE_THREADS && !wide) {
+      if (all <= SAMPLE_THREADS) {
         uint64_t* order = reinterpret_cast<uint64_t*>(hist) + SAMPLE_THREADS;  // beyond the candidates that may lie there
         place = ranked_place(threadIdx.x < all ? vals[threadIdx.x] : 0.f, all, k, temp, p, row_max, order,
                              order + SAMPLE_THREADS, team);
       } else {
-        place = sample_place<false>([&](int i) { return vals[i]; }, all, 0, all, k, temp, p, row_max, wide, team);
+        place = sample_place<false>([&](int i) { return vals[i]; }, all, 0, all, k, temp, p, row_max, false, team);
       }
       if (threadIdx.x == 0) out_ids[row] = place >= 0 ? ids[place] : row_arg;
     } else {
@@ -605,6 +605,7 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
     return;
   }
   team_sync();  // the counts are read; the histograms start anew
+  const bool wide = n > 65535 * SAMPLE_HIST_COPIES;
   const long long place = sample_place<true>(adjusted, n, base, vocab, k, temp, p, row_max, wide, team);
   if (rank == 0 && threadIdx.x == 0) out_ids[row] = place >= 0 ? (int)place : row_arg;
   team_sync();  // nobody leaves while its sums may still be read
