@@ -197,3 +197,24 @@ def test_infinities_take_the_row_and_a_nan_is_never_drawn(vocab):
             row = logits.copy()
             row[infinite] = np.inf
             assert set(run_sampler(row, 8, temperature, top_k, top_p, 1.0).tolist()) == {min(infinite)}
+
+
+# candidates that one block's room just holds and does not; values spread over the blocks of a team, and falling, so that one block has
+# all of them
+@pytest.mark.parametrize("falling", [False, True])
+@pytest.mark.parametrize("vocab", [4096, 20001, 128256, 400000])
+@pytest.mark.parametrize("top_k", [257, 500, 1900, 3500])
+def test_a_large_top_k_over_one_block_and_a_team(vocab, top_k, falling):
+    """Only ids of the k largest are drawn, and each half of their mass (by index) about as often as it says: 720 draws, most of
+    them from batches whose rows get the largest teams, six standard deviations."""
+    rng = np.random.default_rng(vocab + top_k)
+    logits = (rng.normal(size=vocab) * 0.5).astype(np.float32)
+    if falling:
+        logits = np.sort(logits)[::-1].copy()
+    ids, probs = ps.candidate_distribution(logits.astype(np.float64), (), 1.0, top_k, 1.0, 1.0)
+    got = np.concatenate([run_sampler(logits, n, 1.0, top_k, 1.0, 1.0, seed=i) for i, n in enumerate([300] + [70] * 6)])
+    assert set(got.tolist()) <= set(ids.tolist())
+    order = np.argsort(ids)
+    half = ids[order][np.searchsorted(np.cumsum(probs[order]), 0.5)]
+    share = probs[ids <= half].sum()
+    assert abs((got <= half).mean() - share) < 6 * np.sqrt(share * (1 - share) / len(got))

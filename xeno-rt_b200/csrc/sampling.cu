@@ -326,29 +326,37 @@ __device__ long long sample_place(A adjusted, int n, int base, long long n_all, 
   return total > 0 ? ordered_pick<TEAM>(kept_mass, n, base, target, team) : -1;
 }
 
-// `hist` holds, by the top 12 bits of their order keys, numbers that say: at least so many elements lie in this bin.  Cuts
-// at the bin where they reach k from the top (at 0 if they don't) and copies every element from there upwards to
-// out_id / out_val, in index order, if there are no more than `cap`.  Returns how many there are.  The outputs may be the
-// histogram's own room.
-template <typename A, typename I>
-__device__ int cut_and_gather(A adjusted, I id_of, int n, int k, int cap, const uint32_t* hist, SampleShared* sh, int* out_id,
-                              float* out_val) {
-  constexpr int BINS = SAMPLE_FINE_BINS / SAMPLE_THREADS;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// `hist` holds, by the top 12 bits of their order keys, numbers that say: at least so many elements lie in this bin; TEAM: the
+// numbers of all blocks together.  The bin at which they reach k from the top, 0 if they don't.
+template <bool TEAM>
+__device__ uint32_t find_cut(uint32_t* hist, int k, Team& team) {
+  const int blocks = TEAM ? team.size : 1;
+  const int bins = SAMPLE_FINE_BINS / (SAMPLE_THREADS * blocks);  // of a thread: the first block's first has the top ones
+  const int first = SAMPLE_FINE_BINS - bins * ((TEAM ? team.rank * SAMPLE_THREADS : 0) + (int)threadIdx.x + 1);
+  auto bin = [&](int i) {
+    uint32_t sum = 0;
+    for (int r = 0; r < blocks; ++r) sum += (TEAM ? of_block(hist, r) : hist)[i];
+    return sum;
+  };
   uint64_t local = 0, total;
-  if (threadIdx.x == 0) sh->cut = 0;
-#pragma unroll
-  for (int j = 0; j < BINS; ++j) local += hist[SAMPLE_FINE_BINS - 1 - BINS * (int)threadIdx.x - j];
-  uint64_t above = block_exclusive_scan(local, sh->scan, &total);
-  if (above < (uint64_t)k && (uint64_t)k <= above + local) {
-    for (int j = 0; j < BINS; ++j) {
-      const int bin = SAMPLE_FINE_BINS - 1 - BINS * (int)threadIdx.x - j;
-      above += hist[bin];
-      if (above >= (uint64_t)k) { sh->cut = bin; break; }
-    }
+  if (threadIdx.x == 0) team.sh->cut = 0;
+  for (int i = first; i < first + bins; ++i) local += bin(i);
+  uint64_t above = team_exclusive_scan<TEAM>(local, team, &total);
+  if (above < (uint64_t)k && (uint64_t)k <= above + local) {  // one thread
+    int cut = first + bins;
+    while (above < (uint64_t)k) above += bin(--cut);
+    for (int r = 0; r < blocks; ++r) *(TEAM ? of_block(&team.sh->cut, r) : &team.sh->cut) = cut;
   }
-  __syncthreads();
-  const uint32_t cut = (uint32_t)sh->cut;
+  if (TEAM) team_sync();  // (also: everybody is done with the others' histograms)
+  else __syncthreads();
+  return (uint32_t)team.sh->cut;
+}
+
+// Copies every element whose order key's top 12 bits are `cut` or more to out_id / out_val, in index order, if there are no
+// more than `cap`.  Returns how many there are.  The outputs may be the histogram's own room.
+template <typename A, typename I>
+__device__ int gather(A adjusted, I id_of, int n, uint32_t cut, int cap, SampleShared* sh, int* out_id, float* out_val) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (cut == 0 && n > cap) return n;
   const int run = ((n + SAMPLE_WARPS - 1) / SAMPLE_WARPS + 31) & ~31;
   const int lo = min(n, warp * run), hi = min(n, lo + run);
@@ -514,14 +522,24 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
   }
   __syncthreads();
 
-  // This block's candidates, in index order.  (What the row keeps lies at or above its k-th largest value, which is no
-  // smaller than any block's k-th largest.)
+  // This block's candidates, in index order.  Cut at its own k-th largest value (what the row keeps lies at or above the row's
+  // k-th largest, which is no smaller) where all blocks together then keep few; at the row's, by the histograms of all blocks, for
+  // a larger k: 500 of 128,256 at each of eight blocks' own leave more than there is room for, and the selects over the whole row
+  // took 195 us for 64 rows (now 91).
   int* my_id = reinterpret_cast<int*>(hist);
-  const int quota = min(SAMPLE_CANDIDATES / team_size, SAMPLE_HIST_BYTES / 8);
-  float* my_val = reinterpret_cast<float*>(hist) + quota;
+  float* my_val = reinterpret_cast<float*>(hist) + SAMPLE_HIST_BYTES / 8;
   if (few) {
-    const int count = cut_and_gather(adjusted, [&](int i) { return base + i; }, n, k, quota, hist, &sh, my_id, my_val);
-    if (threadIdx.x == 0) sh.count = count <= quota ? count : -1;
+    uint32_t cut;
+    if (of_largest || (long long)k * team_size <= SAMPLE_CANDIDATES / 4) {
+      cut = find_cut<false>(hist, k, team);
+    } else {
+      team_wait();
+      team_sync();  // every block's histogram is complete
+      cut = find_cut<true>(hist, k, team);
+      team_arrive();
+    }
+    const int count = gather(adjusted, [&](int i) { return base + i; }, n, cut, SAMPLE_HIST_BYTES / 8, &sh, my_id, my_val);
+    if (threadIdx.x == 0) sh.count = count <= SAMPLE_HIST_BYTES / 8 ? count : -1;
   }
 
   team_wait();  // every block of the team runs: its shared memory may be written
@@ -556,6 +574,7 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
     compact = compact && counts[r] >= 0;
     all += counts[r];
   }
+  compact = compact && all <= SAMPLE_CANDIDATES;
   const float p = top_p[row];
   if (compact) {
     if (rank == 0) {
@@ -582,8 +601,9 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
         __syncthreads();
         int* few_id = reinterpret_cast<int*>(hist);
         float* few_val = reinterpret_cast<float*>(hist) + SAMPLE_THREADS;
-        const int count = cut_and_gather([&](int i) { return vals[i]; }, [&](int i) { return ids[i]; }, all, k, SAMPLE_THREADS,
-                                         hist, &sh, few_id, few_val);
+        const uint32_t cut = find_cut<false>(hist, k, team);
+        const int count = gather([&](int i) { return vals[i]; }, [&](int i) { return ids[i]; }, all, cut, SAMPLE_THREADS, &sh,
+                                 few_id, few_val);
         if (count <= SAMPLE_THREADS) {
           ids = few_id;
           vals = few_val;
@@ -633,11 +653,13 @@ XRT_EXPORT int xrt_sample(int* out_ids, const float* logits, int n_rows, int voc
   if (n_rows < 0 || vocab <= 0) return XRT_ERR_ARGUMENT;
   if (seen != nullptr && seen_words * 32 < vocab) return XRT_ERR_ARGUMENT;
   if (n_rows == 0) return XRT_OK;
-  // blocks of a team: slices of 4,096 logits or more (smaller ones are read in less time than a team takes to meet); half as
-  // many while the rows alone bring more than four blocks a multiprocessor
+  // blocks of a team: as many as it takes to bring a slice to 4,096 logits (smaller ones are read in less time than a team takes
+  // to meet), or, where the rows alone occupy the multiprocessors, as keep it at 4,096 (256 rows of 5,000 logits, one block against
+  // two: 20.7 against 26.6 us); half as many while the rows alone bring more than four blocks a multiprocessor
+  const int sms = xrt::multiprocessors();
   int team = 1;
-  while (team < xrt::SAMPLE_TEAM && (long long)team * 4096 < vocab) team *= 2;
-  while (team > 2 && (long long)team * n_rows > 4 * 148) team /= 2;
+  while (team < xrt::SAMPLE_TEAM && (long long)team * (n_rows >= sms ? 2 * 4096 - 1 : 4096) < vocab) team *= 2;
+  while (team > 2 && (long long)team * n_rows > 4ll * sms) team /= 2;
   const long long per = ((long long)vocab + team * 32 - 1) / (team * 32) * 32;
   const bool cached = per * 4 <= xrt::SAMPLE_CACHED_BYTES;
   const bool vec = vocab % 4 == 0 && ((uintptr_t)logits & 15) == 0;
