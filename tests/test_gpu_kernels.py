@@ -744,6 +744,35 @@ def test_attention_prefill_tcgen05_kernel(nh, nkv):
         at += new[s]
 
 
+# even and odd numbers of query heads a kv head; whole prompts, a continued one, one of a single token, a skipped one; last tiles of few
+# rows, an odd number of tiles, more steps than the rings have stages
+@pytest.mark.parametrize("nh,nkv,window", [(8, 2, 0), (5, 1, 0), (4, 4, 0), (4, 2, 200), (3, 1, 150)])
+def test_attention_prefill_tcgen05_one_and_two_tiles_a_block_give_the_same_bits(nh, nkv, window):
+    hd = 128
+    torch.manual_seed(nh + nkv)
+    starts, new, slots = [0, 0, 700, 0, 0, 100], [150, 1, 70, 5, 700, 257], [1, 2, 3, -1, 5, 4]
+    totals = [s + n for s, n in zip(starts, new)]
+    k_pool, v_pool, table = _cache_for(totals, nkv, hd, torch.bfloat16, shuffle_seed=nh)
+    for s in range(6):
+        _fill_cache(k_pool, v_pool, table, s + 1, torch.randn(totals[s], nkv, hd, device=DEV),
+                    torch.randn(totals[s], nkv, hd, device=DEV))
+    one = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    q = torch.randn(sum(new), nh * hd, device=DEV).to(torch.bfloat16)
+    cu = one(np.concatenate([[0], np.cumsum(new)]).tolist())
+    sinks = torch.randn(nh, device=DEV)
+    slots = [s if s < 0 else i + 1 for i, s in enumerate(slots)]
+    got = []
+    for tiles in (1, 2):
+        out = torch.full_like(q, 5.0)
+        with ops().tuned(prefill_tiles=tiles):
+            ops().attention_prefill_tcgen05(out, q, k_pool, v_pool, cu, one(slots), one(starts), table, max(new), nh, nkv, hd,
+                                            1 / math.sqrt(hd), window, sinks)
+        got.append(out)
+    ops().check_error_flag(DEV)
+    assert torch.equal(got[0], got[1])
+    assert bool((got[0][221:226] == 5.0).all()) and bool((got[0][226:] != 5.0).any())
+
+
 @pytest.mark.parametrize("m", [1, 3, 8, 16])
 @pytest.mark.parametrize("width,inner,out_rows,norm_dtype", [(1032, 2760, 1536, torch.float32), (256, 520, 392, torch.bfloat16),
                                                             (4096, 1024, 4096, torch.bfloat16), (5120, 264, 5000, torch.float32)])

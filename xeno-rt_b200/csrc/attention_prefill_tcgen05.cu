@@ -4,16 +4,18 @@
 //
 // A block owns two tiles of 128 query rows that need the same keys: 128 consecutive new tokens of one sequence for two
 // query heads of one kv head, or, where a kv head's query heads are odd in number, 256 consecutive new tokens for one query
-// head.  It walks the sequence's keys in steps of 128 (two cache blocks of 64) from the cache block of the first row's
+// head; or one tile of 128 rows, where two would leave multiprocessors empty (two_tiles, below).  It walks the sequence's keys in steps of 128 (two cache blocks of 64) from the cache block of the first row's
 // first visible key (KeyRange in common.cuh: all keys, a window, or the query's own chunk of positions).  A head may have
-// a sink: one more term of the softmax's denominator, added to the row's sum at the end.  Ten warps:
+// a sink: one more term of the softmax's denominator, added to the row's sum at the end.  Ten warps (one tile: six):
 //   warp 0    TMA: the Q tiles once, then for each step its K and V tiles ([128 keys x 128], as boxes
-//             of 64 keys x 64 dims, 128-byte swizzle), fetched once for both query tiles, into rings of two stages.
+//             of 64 keys x 64 dims, 128-byte swizzle), fetched once for both query tiles, into rings of two stages
+//             (one tile: three).
 //   warp 1    owns TMEM and issues the MMAs: S = Q K^T (128 x 128, eight tcgen05.mma over the head
 //             size) and O += P V (128 x 128, eight tcgen05.mma over the step's keys) accumulated in TMEM over all
 //             steps.  K is a K-major operand as stored; V ([key][dim]) is an MN-major operand as stored: no
 //             transposition anywhere.  The two query tiles take turns: while one's softmax runs, the tensor core has
-//             the other's products (P V of a step, at once followed by Q K^T of the next).
+//             the other's products (P V of a step, at once followed by Q K^T of the next).  A single tile has two S of its
+//             own: while the softmax of a step runs, the tensor core has the Q K^T of the next.
 //   warps 2-9 softmax and output, four warps a query tile, one thread a query row (TMEM lane).  A thread reads its row
 //             of S (tcgen05.ld), masks (only steps that reach the diagonal), keeps the row's sum in 32-bit,
 //             and writes P as bfloat16 pairs over the S it has read (tcgen05.st), from where P V reads it as its A
@@ -37,13 +39,15 @@ namespace xrt {
 
 using namespace sm100;
 
-constexpr int FA_ROWS = 128, FA_KEYS = 128, FA_HD = 128, FA_STAGES = 2, FA_TILES = 2;
+constexpr int FA_ROWS = 128, FA_KEYS = 128, FA_HD = 128;
 constexpr int FA_Q_BYTES = FA_ROWS * FA_HD * 2;        // 32 KB (two halves of 16 KB)
 constexpr int FA_BOX = 64 * 64 * 2;                    // 8 KB: what one tensor copy brings, 64 keys x 64 dims
 constexpr int FA_KV_HALF = FA_KEYS * 64 * 2;           // 16 KB: 128 keys (two cache blocks) x 64 dims
 constexpr int FA_STAGE_BYTES = 4 * FA_KV_HALF;         // K halves, then V halves: 64 KB
-constexpr int FA_THREADS = 64 + 128 * FA_TILES;
-constexpr int FA_SMEM = FA_TILES * FA_Q_BYTES + FA_STAGES * FA_STAGE_BYTES + 512 + 1024;
+template <int TILES> struct FaShape {
+  static constexpr int STAGES = TILES == 2 ? 2 : 3, THREADS = 64 + 128 * TILES;
+  static constexpr int SMEM = TILES * FA_Q_BYTES + STAGES * FA_STAGE_BYTES + 512 + 1024;
+};
 
 // 2^x by the special-function unit; exp2(-inf) = 0.  Inputs are differences to a running maximum
 // (at most 0) and the result feeds a bfloat16 product or a 32-bit sum: the unit's 2 ulp are far
@@ -54,15 +58,19 @@ __device__ __forceinline__ float fa_exp2(float x) {
   return y;
 }
 
-// HEADS: the block's two tiles are the same rows of two query heads of one kv head; else 256 rows of one query head.
-template <bool HEADS>
-__global__ void __launch_bounds__(FA_THREADS, 1)
+// HEADS: the block's two tiles are the same rows of two query heads of one kv head; else its tiles are consecutive rows of one
+// query head.
+template <int TILES, bool HEADS>
+__global__ void __launch_bounds__(FaShape<TILES>::THREADS, 1)
 attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                  const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
                                  const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot,
                                  const int* __restrict__ seq_start, const int* __restrict__ block_table, int max_blocks,
                                  int n_heads, int n_kv_heads, float scale_log2, int* __restrict__ error_flag,
                                  const KeyRange range, const float* __restrict__ sinks) {
+  static_assert(TILES == 2 || !HEADS, "one tile is of one head");
+  constexpr int FA_TILES = TILES, FA_STAGES = FaShape<TILES>::STAGES;
+  constexpr int S_BUFFERS = TILES == 1 ? 2 : 1;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* q_tiles = smem;                                   // [FA_TILES] x 32 KB
@@ -73,9 +81,9 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   uint64_t* k_empty = k_full + FA_STAGES;  //   since a step's K is free again (after its QK^T) a whole step
   uint64_t* v_full = k_empty + FA_STAGES;  //   before its V (after its PV): the next K is fetched that much earlier
   uint64_t* v_empty = v_full + FA_STAGES;
-  uint64_t* s_full = v_empty + FA_STAGES;  // [FA_TILES]: once a step
-  uint64_t* p_full = s_full + FA_TILES;    // [FA_TILES]: once a step; also says that S was read
-  uint64_t* o_done = p_full + FA_TILES;    // [FA_TILES]: once, after the tile's last product
+  uint64_t* s_full = v_empty + FA_STAGES;  // [2]: of a tile, or of a single tile's buffer of S (whose next step but one comes
+  uint64_t* p_full = s_full + 2;           //   first when its waits have passed); p_full also says that S was read
+  uint64_t* o_done = p_full + 2;           // [FA_TILES]: once, after the tile's last product; one tile: after every step's
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + FA_TILES);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -101,12 +109,12 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   auto steps_of = [&](int u) {  // 0: the second tile lies beyond the sequence
     return row0_of(u) < n_new ? (start + last_row_of(u) + 1 - key_base + FA_KEYS - 1) / FA_KEYS : 0;
   };
-  const int steps0 = steps_of(0), steps1 = steps_of(1);
+  const int steps0 = steps_of(0), steps1 = TILES == 2 ? steps_of(1) : 0;
   const int n_steps = max(steps0, steps1);
   const int last_row = steps1 > 0 ? last_row_of(1) : last_row_of(0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int TMEM_COLS = FA_TILES * (FA_KEYS + FA_HD);  // S (and P over it) and O of every tile
-  static_assert(TMEM_COLS == 512, "all of TMEM");
+  constexpr int TMEM_COLS = 512;  // S (and P over it) and O of every tile: all of TMEM, or 384 columns of it
+  static_assert(FA_TILES * (S_BUFFERS * FA_KEYS + FA_HD) <= TMEM_COLS, "S and O must fit in TMEM");
 
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(q_full), 1);
@@ -114,13 +122,13 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       mbar_init(smem_u32(&k_full[s]), 1); mbar_init(smem_u32(&k_empty[s]), 1);
       mbar_init(smem_u32(&v_full[s]), 1); mbar_init(smem_u32(&v_empty[s]), 1);
     }
-    for (int u = 0; u < FA_TILES; ++u) {
+    for (int u = 0; u < 2; ++u) {
       mbar_init(smem_u32(&s_full[u]), 1);
       // the softmax warps arrive once each (lane 0, after the warp has synchronised): a hundred
       // arrivals on one shared-memory word would serialise
       mbar_init(smem_u32(&p_full[u]), 4);
-      mbar_init(smem_u32(&o_done[u]), 1);
     }
+    for (int u = 0; u < FA_TILES; ++u) mbar_init(smem_u32(&o_done[u]), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -132,8 +140,10 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   __syncthreads();
   fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s = tmem_base;                            // [tile] x 128 columns; P: the first 64 of them
-  const uint32_t tmem_o = tmem_base + FA_TILES * FA_KEYS;       // [tile] x 128 columns
+  const uint32_t tmem_s = tmem_base;                            // [tile or buffer] x 128 columns; P: the first 64 of them
+  const uint32_t tmem_o = tmem_base + 2 * FA_KEYS;              // [tile] x 128 columns
+  auto s_place = [](int j, int u) { return TILES == 2 ? u : j & 1; };  // which S (and barrier) tile u has at step j
+  auto s_parity = [](int j) { return (uint32_t)(TILES == 2 ? j : j >> 1) & 1u; };
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
@@ -196,9 +206,9 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         for (int ks = 0; ks < FA_HD / 16; ++ks) {  // 16 dims a step; 4 steps a 64-dim half
           const uint64_t a = desc_k_major(smem_u32(q_tiles + u * FA_Q_BYTES + (ks / 4) * (FA_Q_BYTES / 2))) + 2 * (ks % 4);
           const uint64_t bd = desc_k_major(smem_u32(stage + (ks / 4) * FA_KV_HALF)) + 2 * (ks % 4);
-          mma_f16(tmem_s + u * FA_KEYS, a, bd, idesc_qk, ks > 0);
+          mma_f16(tmem_s + s_place(j, u) * FA_KEYS, a, bd, idesc_qk, ks > 0);
         }
-        commit(smem_u32(&s_full[u]));
+        commit(smem_u32(&s_full[s_place(j, u)]));
         if (u == last_tile(j)) commit(smem_u32(&k_empty[s]));
         return true;
       };
@@ -208,22 +218,28 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       for (int j = 0; j < n_steps && ok; ++j) {
         const int s = j % FA_STAGES;
         unsigned char* stage = kv_ring + s * FA_STAGE_BYTES;
+        // one tile: the next S goes into the other buffer, whose P was used up by a product issued before
+        if (TILES == 1 && j + 1 < n_steps) {
+          ok = issue_qk(j + 1, 0);
+          if (!ok) break;
+        }
 #pragma unroll 1
         for (int u = 0; u < FA_TILES && ok; ++u) {
           const int steps = u == 0 ? steps0 : steps1;
           if (j >= steps) continue;
-          ok = mbar_wait(smem_u32(&p_full[u]), (uint32_t)j & 1u, abort_flag) &&  // P is written, and O rescaled if it had to be
+          ok = mbar_wait(smem_u32(&p_full[s_place(j, u)]), s_parity(j), abort_flag) &&  // P is written, and O rescaled if it had to be
                mbar_wait(smem_u32(&v_full[s]), (j / FA_STAGES) & 1, abort_flag);
           if (!ok) break;
           fence_after();
 #pragma unroll
           for (int ks = 0; ks < FA_KEYS / 16; ++ks) {  // 16 keys a step
             const uint64_t bd = desc_mn_major(smem_u32(stage + 2 * FA_KV_HALF + ks * 2048), FA_KV_HALF);
-            mma_f16_a_tmem(tmem_o + u * FA_HD, tmem_s + u * FA_KEYS + ks * 8, bd, idesc_pv, j > 0 || ks > 0);
+            mma_f16_a_tmem(tmem_o + u * FA_HD, tmem_s + s_place(j, u) * FA_KEYS + ks * 8, bd, idesc_pv,
+                           j > 0 || ks > 0);
           }
           if (u == last_tile(j)) commit(smem_u32(&v_empty[s]));
-          // the next S takes the place of this step's P: products run in the order in which they are issued
-          if (j + 1 < steps) ok = issue_qk(j + 1, u);
+          // two tiles: the next S takes the place of this step's P: products run in the order in which they are issued
+          if (TILES == 2 && j + 1 < steps) ok = issue_qk(j + 1, u);
           else commit(smem_u32(&o_done[u]));
         }
       }
@@ -242,20 +258,22 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     const int key_lo = range.first(start + row);
     const int all_lo = range.first(start + last_row_of(u));  // from here on no row's range has yet to begin
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    const uint32_t my_s = tmem_s + lane_base + u * FA_KEYS, my_o = tmem_o + lane_base + u * FA_HD;
+    const uint32_t my_o = tmem_o + lane_base + u * FA_HD;
     float m_ref = -INFINITY, l_run = 0.f;  // the reference value of the exponents (scaled, base 2) and the sum
     bool ok = true;
 
     for (int j = 0; j < n_tiles && ok; ++j) {
-      ok = mbar_wait(smem_u32(&s_full[u]), (uint32_t)j & 1u, abort_flag);
+      ok = mbar_wait(smem_u32(&s_full[s_place(j, u)]), s_parity(j), abort_flag);
       if (!ok) break;
       fence_after();
+      const uint32_t my_s = tmem_s + lane_base + s_place(j, u) * FA_KEYS;
       const int key0 = key_base + j * FA_KEYS;
       // Only steps that reach past the first row's last visible key, or begin before the last row's first one, can
       // hide a key from a row (uniform over the tile); every other step skips the comparisons.
       const bool early = key0 < all_lo, late = key0 + FA_KEYS > start + tile_row0 + 1;
       // Half of the row at a time, twice: for the maximum, and again from tensor memory for the exponents.  (The whole row
-      // in registers beside P does not fit the 168 that ten warps leave each thread.)
+      // in registers beside P does not fit the 168 that ten warps leave each thread; six warps keep it.)
+      float s[TILES == 2 ? 1 : 2][FA_KEYS / 2];
       auto read_half = [&](float (&s)[FA_KEYS / 2], int half) {
         uint32_t v0[32], v1[32];
         tmem_ld32(v0, my_s + half * 64);
@@ -276,12 +294,12 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       float part_max[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        float s[FA_KEYS / 2];
-        read_half(s, half);
+        float (&row)[FA_KEYS / 2] = s[TILES == 2 ? 0 : half];
+        read_half(row, half);
 #pragma unroll
         for (int i = 0; i < 64; i += 4) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) part_max[k] = fmaxf(part_max[k], s[i + k]);
+          for (int k = 0; k < 4; ++k) part_max[k] = fmaxf(part_max[k], row[i + k]);
         }
       }
       const float m_tile = fmaxf(fmaxf(part_max[0], part_max[1]), fmaxf(part_max[2], part_max[3])) * scale_log2;
@@ -289,7 +307,12 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       const bool moves = m_tile > m_ref + 8.0f || (m_ref == -INFINITY && m_tile != -INFINITY);
       if (__any_sync(0xffffffffu, moves)) {
         const float factor = (moves && m_ref != -INFINITY) ? fa_exp2(m_ref - m_tile) : 1.0f;
-        if (j > 0) {  // O holds the products of the steps so far: they were issued before this step's S, which is complete
+        if (j > 0) {  // O holds the products of the steps so far: two tiles' were issued before this step's S, which is complete
+          if (TILES == 1) {
+            ok = mbar_wait(smem_u32(&o_done[u]), (uint32_t)(j - 1) & 1u, abort_flag);
+            if (!ok) break;
+            fence_after();
+          }
           if (__any_sync(0xffffffffu, factor != 1.0f)) {
 #pragma unroll
             for (int c = 0; c < FA_HD; c += 32) {
@@ -314,13 +337,13 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       // columns that the first half has left behind)
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        float s[FA_KEYS / 2];
-        read_half(s, half);
+        float (&row)[FA_KEYS / 2] = s[TILES == 2 ? 0 : half];
+        if (TILES == 2) read_half(row, half);
         uint32_t packed[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          const float p0 = fa_exp2(fmaf(s[2 * i], scale_log2, neg_m));
-          const float p1 = fa_exp2(fmaf(s[2 * i + 1], scale_log2, neg_m));
+          const float p0 = fa_exp2(fmaf(row[2 * i], scale_log2, neg_m));
+          const float p1 = fa_exp2(fmaf(row[2 * i + 1], scale_log2, neg_m));
           part_sum[i & 3] += p0 + p1;
           __nv_bfloat162 pair = __floats2bfloat162_rn(p0, p1);
           packed[i] = *reinterpret_cast<uint32_t*>(&pair);
@@ -330,10 +353,10 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&p_full[u]));
+      if (lane == 0) mbar_arrive(smem_u32(&p_full[s_place(j, u)]));
       l_run += (part_sum[0] + part_sum[1]) + (part_sum[2] + part_sum[3]);
     }
-    if (ok && n_tiles > 0) ok = mbar_wait(smem_u32(&o_done[u]), 0, abort_flag);
+    if (ok && n_tiles > 0) ok = mbar_wait(smem_u32(&o_done[u]), TILES == 1 ? (uint32_t)(n_tiles - 1) & 1u : 0u, abort_flag);
     if (ok && n_tiles > 0) {
       fence_after();
       if (sinks != nullptr) l_run += exp2f(sinks[head] * 1.4426950408889634f - m_ref);
@@ -371,9 +394,42 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   }
 }
 
+// Whether blocks of two query tiles take the step.  A two-tile block's step takes 1.6 to 1.8 times a one-tile block's, so two
+// tiles a block are faster only while the blocks are many: not where the one-tile blocks all run at once (at most one a
+// multiprocessor; measured, microseconds, one tile -> two: 128 new tokens of 32 heads behind 8,000 keys 82 -> 149, 2,000 tokens of
+// 8 heads 27 -> 43, 512 of 32 heads 13.4 -> 18.4), nor where a long prompt's few blocks run at most about twice a
+// multiprocessor, since its last tiles, which are the longest, then decide (2,000 tokens of 16 heads 31 -> 43, 1,024 of 32 heads
+// 22.6 -> 26.7, 1,100 of 32 heads with a kv head each 24.7 -> 28.7; but 8 prompts of 128 tokens 16.4 -> 14.0, 600 tokens of 64
+// heads, 2.2 a multiprocessor, 26.7 -> 20.6).  Consecutive tiles of one head share their keys only where every row begins
+// at the first key: under a window or a chunk the second tile's steps would begin where the first's do, so that its sums could
+// depend on the form (and there is nothing to gain: 4,000 tokens of 24 + 8 heads in a window of 1,024 88 either way).
+static bool two_tiles(long long n_tokens, long long n_seqs, long long tiles, int n_heads, bool heads, bool bounded, int sms) {
+  if (!heads && bounded) return false;
+  if (tuning().prefill_tiles != 0) return tuning().prefill_tiles == 2;
+  const long long most = n_tokens / FA_ROWS + n_seqs;  // of sequences of unequal lengths
+  const long long blocks = (n_seqs * tiles < most ? n_seqs * tiles : most) * n_heads;
+  return blocks > (tiles >= 5 ? 2 : 1) * (long long)sms;
+}
+
 // A map over a row-major bfloat16 matrix [rows, cols], boxes of box_rows x 64 columns, 128-byte swizzle.
 static bool fa_make_map(CUtensorMap* map, const void* base, long long rows, int cols, int box_rows) {
   return sm100::make_map_bf16_2d(map, base, rows, cols, cols, box_rows);
+}
+
+template <int TILES, bool HEADS>
+static int launch_prefill(dim3 grid, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v,
+                          __nv_bfloat16* out, const int* cu_seqlens, const int* seq_slot, const int* seq_start,
+                          const int* block_table, int max_blocks, int n_heads, int n_kv_heads, float scale_log2,
+                          int* error_flag, KeyRange range, const float* sinks, cudaStream_t stream) {
+  constexpr auto kernel = attention_prefill_tcgen05_kernel<TILES, HEADS>;
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FaShape<TILES>::SMEM);
+  if (err != cudaSuccess) return (int)err;
+  // launched without programmatic dependent launch: a block needs a multiprocessor to itself, so nothing of it can
+  // run beside the kernel before it, and the early launch was measured slower (28.2 against 27.8 ms a prompt of 2,048)
+  kernel<<<grid, FaShape<TILES>::THREADS, FaShape<TILES>::SMEM, stream>>>(
+      map_q, map_k, map_v, out, cu_seqlens, seq_slot, seq_start, block_table, max_blocks, n_heads, n_kv_heads, scale_log2,
+      error_flag, range, sinks);
+  return launch_status();
 }
 
 }  // namespace xrt
@@ -402,20 +458,11 @@ XRT_EXPORT int xrt_attention_prefill_tcgen05(void* out, const void* q, const voi
       !xrt::fa_make_map(&map_k, k_pool, pool_rows, xrt::FA_HD, XRT_BLOCK_TOKENS) ||
       !xrt::fa_make_map(&map_v, v_pool, pool_rows, xrt::FA_HD, XRT_BLOCK_TOKENS))
     return XRT_ERR_UNSUPPORTED;
+  const int tiles = (max_new + xrt::FA_ROWS - 1) / xrt::FA_ROWS;
   const bool heads = (n_heads / n_kv_heads) % 2 == 0;
-  auto kernel = heads ? xrt::attention_prefill_tcgen05_kernel<true> : xrt::attention_prefill_tcgen05_kernel<false>;
-  static bool allowed[2] = {false, false};
-  if (!allowed[heads]) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, xrt::FA_SMEM);
-    if (err != cudaSuccess) return (int)err;
-    allowed[heads] = true;
-  }
-  const int rows = heads ? xrt::FA_ROWS : xrt::FA_TILES * xrt::FA_ROWS;
-  dim3 grid(heads ? n_heads / 2 : n_heads, n_seqs, (max_new + rows - 1) / rows);
-  // launched without programmatic dependent launch: a block needs a multiprocessor to itself, so nothing of it can
-  // run beside the kernel before it, and the early launch was measured slower (28.2 against 27.8 ms a prompt of 2,048)
-  kernel<<<grid, xrt::FA_THREADS, xrt::FA_SMEM, stream>>>(
-      map_q, map_k, map_v, (__nv_bfloat16*)out, cu_seqlens, seq_slot, seq_start, block_table, max_blocks, n_heads,
-      n_kv_heads, scale * 1.4426950408889634f, error_flag, xrt::key_range(window, mask_chunk), sinks);
-  return xrt::launch_status();
+  const bool two = xrt::two_tiles(n_tokens, n_seqs, tiles, n_heads, heads, window > 0 || mask_chunk > 0, xrt::multiprocessors());
+  auto launch = two ? (heads ? xrt::launch_prefill<2, true> : xrt::launch_prefill<2, false>) : xrt::launch_prefill<1, false>;
+  const dim3 grid(two && heads ? n_heads / 2 : n_heads, n_seqs, two && !heads ? (tiles + 1) / 2 : tiles);
+  return launch(grid, map_q, map_k, map_v, (__nv_bfloat16*)out, cu_seqlens, seq_slot, seq_start, block_table, max_blocks,
+                n_heads, n_kv_heads, scale * 1.4426950408889634f, error_flag, xrt::key_range(window, mask_chunk), sinks, stream);
 }

@@ -32,6 +32,7 @@ struct Tuning {
   int gemm_tile_rows = 0;           // 0 auto, 128 or 256: the prefill product's tile
   bool decode_gemm_clusters = true; // the decode product's splits meet through a cluster's shared memory
   int decode_cluster_pairs = 128;    // decode attention merges its splits as clusters up to so many (token, kv head) pairs
+  int prefill_tiles = 0;            // 0 auto, 1 or 2: query tiles a block of the prompt attention
 };
 const Tuning& tuning();
 

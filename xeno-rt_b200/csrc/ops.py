@@ -148,6 +148,7 @@ class Tuning:
     ``decode_gemm_clusters``  splits of K of the tcgen05 few-row product meet through a cluster
     ``decode_attention`` "auto", "rows" (query heads as MMA rows), "cp" (cp.async tiles), "nocluster"
     ``prefill_attention`` "auto" or "mma" (the mma.sync kernel also where the tcgen05 one applies)
+    ``prefill_tiles``    0 (auto), 1 or 2: query tiles a block of the tcgen05 prompt attention (2 only where they share keys)
     ``gemm_tile_rows``   0 (auto), 128 or 256: the tile of the prompt product
     ``pending_norm``     "auto": a few-row product that adds into the residual prepares the norm that follows
                          it where the next product runs on the kernel that can finish it; "off": never
@@ -161,6 +162,7 @@ class Tuning:
     decode_gemm_clusters: bool = True
     decode_attention: str = "auto"
     prefill_attention: str = "auto"
+    prefill_tiles: int = 0
     gemm_tile_rows: int = 0
     decode_cluster_pairs: int = 128
     pending_norm: str = "auto"
@@ -188,7 +190,7 @@ def set_tuning(new: Tuning) -> None:
     lib = library()
     for key, value in ((0, int(new.pdl)), (1, _DECODE_ATTENTION[new.decode_attention]),
                        (2, int(new.gemm_tile_rows)), (3, int(new.decode_gemm_clusters)),
-                       (4, int(new.decode_cluster_pairs))):
+                       (4, int(new.decode_cluster_pairs)), (5, int(new.prefill_tiles))):
         if lib.xrt_set_tuning(key, value) != 0:
             raise KernelError(f"tuning: value {value} of setting {key} was refused")
     _tuning = new

@@ -13,7 +13,7 @@ const Tuning& tuning() { return g_tuning; }
 
 // key: 0 pdl (1 on, 0 off); 1 decode_attention (0 auto, 1 heads as rows, 2 cp.async copies, 3 no
 // clusters); 2 gemm_tile_rows (0 auto, 128, 256); 3 decode_gemm_clusters (1 on, 0 off); 4 decode_cluster_pairs
-// (decode attention merges its splits as clusters up to so many (token, kv head) pairs).
+// (decode attention merges its splits as clusters up to so many (token, kv head) pairs); 5 prefill_tiles (0 auto, 1, 2).
 XRT_EXPORT int xrt_set_tuning(int key, int value) {
   using xrt::g_tuning;
   switch (key) {
@@ -22,6 +22,7 @@ XRT_EXPORT int xrt_set_tuning(int key, int value) {
     case 2: if (value != 0 && value != 128 && value != 256) return XRT_ERR_ARGUMENT; g_tuning.gemm_tile_rows = value; return XRT_OK;
     case 3: g_tuning.decode_gemm_clusters = value != 0; return XRT_OK;
     case 4: if (value < 0) return XRT_ERR_ARGUMENT; g_tuning.decode_cluster_pairs = value; return XRT_OK;
+    case 5: if (value < 0 || value > 2) return XRT_ERR_ARGUMENT; g_tuning.prefill_tiles = value; return XRT_OK;
     default: return XRT_ERR_ARGUMENT;
   }
 }
