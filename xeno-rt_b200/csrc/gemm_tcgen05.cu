@@ -391,7 +391,9 @@ int launch_tcgen05_tiled(void* out, const CUtensorMap& map_x, const CUtensorMap&
 // that a pair's round is shorter (600 rows, 14,336 gated outputs: 5 against 4, 155 us against 137; 7,999 rows: 49 against
 // 48, 1,402 against 1,430), or pad the rows by more than a tenth beyond tiles of 128 (600 rows, 6,144 outputs: 35
 // against 31), then only if single blocks would leave four multiprocessors in ten without a tile (600 rows, 4,096 outputs,
-// 14,336 inputs: 94 against 114).
+// 14,336 inputs: 94 against 114).  Nor where single blocks take one round and the sums are short, or the tiles so few that the L2
+// feeds each at its full rate: a pair's meeting then costs 2 us (microseconds, single against pairs: 256 rows of 3,072 outputs,
+// 2,048 inputs 18.6 / 20.6; 768 of 6,144, 4,096 38.5 / 41.1; 512 of 2,048, 8,192 49.3 / 51.4; but 512 of 4,096, 8,192 57.4 / 49.4).
 // Tuning::gemm_tile_rows = 128 or 256 forces one, for comparison.
 template <int MODE, typename TO>
 int launch_tcgen05(void* out, const CUtensorMap& map_x, const CUtensorMap& map_w, int M, int N, int K, int ldo,
@@ -403,7 +405,8 @@ int launch_tcgen05(void* out, const CUtensorMap& map_x, const CUtensorMap& map_w
   const long long tiles_128 = rows_128 / 128 * tiles_n, tiles_256 = rows_256 / 256 * tiles_n;
   auto rounds = [](long long tiles, int units) { return (tiles + units - 1) / units; };
   const int forced = tuning().gemm_tile_rows;
-  const bool pair = forced == 256 || (forced != 128 && M > 128 && sm_count >= 2 &&
+  const bool short_sums = tiles_128 <= sm_count && (K <= 4096 || tiles_128 * 5 < sm_count);
+  const bool pair = forced == 256 || (forced != 128 && M > 128 && sm_count >= 2 && !short_sums &&
                                       24 * rounds(tiles_256, sm_count / 2) <= 25 * rounds(tiles_128, sm_count) &&
                                       (rows_256 * 10 <= rows_128 * 11 || tiles_128 * 10 < 6ll * sm_count));
   if (pair)
