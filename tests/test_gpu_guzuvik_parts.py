@@ -4,6 +4,8 @@ stream), the short convolution with a bias, the scalar-decay state-space scan (p
 sizes), the gated group norm, the preparation of attention heads (biases, unit norms, blended values), the scores'
 options (window edges, kept first tokens, far keys made to stand out, the cap, the distance slope) in the 32-bit and
 the tensor-core kernel, the router and the experts."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -316,6 +318,35 @@ def test_experts_against_the_plain_experts(dtype, width, ff, experts, top, limit
     ops.moe_experts(out, _t(h).to(tdt), _t(w_in).to(tdt), _t(down.reshape(experts * width, ff)).to(tdt), _ints(ids),
                     _t(weights), ff, limit, 1.702)
     _close(out.sum(0).cpu().numpy(), want, 2e-5)  # the kernels keep 32-bit inside in both dtypes
+
+
+@pytest.mark.parametrize("n,k", [(202, 72), (33, 64), (260, 136)])
+def test_experts_products_over_ragged_rows_and_columns_write_nothing_else(n, k):
+    """Columns that are no multiple of four (stored one at a time) or of a tile, experts of no, one and more rows than a tile:
+    against float64, and the rows before and after the experts' stay as they are."""
+    from xeno_rt_b200.csrc import ops
+    rng = np.random.default_rng(n)
+    counts = [5, 0, 1, 130, 64]
+    offsets = np.concatenate([[0], np.cumsum(counts)])
+    rows, experts = int(offsets[-1]), len(counts)
+    a = _t(rng.normal(size=(rows, k))).to(torch.bfloat16)
+    f64 = lambda t: t.double().cpu().numpy()
+    for act, ff in ((None, 0), ("gelu", n), ("gated_silu", n)):
+        w = _t(rng.normal(size=(experts * n * (2 if act == "gated_silu" else 1), k)) * 0.2).to(torch.bfloat16)
+        whole = torch.full((rows + 2, n), 7.0, device="cuda", dtype=torch.bfloat16 if ff else torch.float32)
+        out = whole[1:-1]
+        ops.moe_grouped_product(out, a, w, _ints(offsets), experts, ff, act=act or "gated_sigmoid")
+        ops.check_error_flag("cuda:0")
+        assert bool((whole[0] == 7.0).all()) and bool((whole[-1] == 7.0).all())
+        for e in range(experts):
+            x = f64(a[offsets[e]:offsets[e + 1]]) @ f64(w.view(experts, -1, k)[e]).T
+            if act == "gelu":
+                x = x * 0.5 * (1 + np.vectorize(math.erf)(x / math.sqrt(2))) if x.size else x
+            elif act == "gated_silu":
+                x = x[:, :n] / (1 + np.exp(-x[:, :n])) * x[:, n:]
+            got = f64(out[offsets[e]:offsets[e + 1]])
+            if got.size:  # bfloat16 results: half a unit in the last of 8 bits; 32-bit sums else
+                assert np.linalg.norm(got - x) <= (4e-3 if ff else 2e-6) * np.linalg.norm(x)
 
 
 @pytest.mark.parametrize("width,ff,experts,top,n", [(64, 24, 6, 2, 230), (200, 72, 40, 1, 150), (256, 64, 8, 3, 333),
