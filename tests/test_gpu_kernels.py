@@ -773,6 +773,43 @@ def test_attention_prefill_tcgen05_one_and_two_tiles_a_block_give_the_same_bits(
     assert bool((got[0][221:226] == 5.0).all()) and bool((got[0][226:] != 5.0).any())
 
 
+def test_rotation_a_warp_a_token_and_a_block_a_token_give_the_same_bits():
+    """More tokens than the kernel of one warp a token begins at, and not eight times as many as it has blocks, against the same
+    tokens in pieces that the other kernel takes: head norms or none, no rotation, a query temperature, values from the keys'
+    columns, a reader that writes nothing, a 32-bit cache, padding rows."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n, nh, nkv, hd = 80 * sms + 5, 2, 1, 128
+    piece = 20 * sms
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    qkv = torch.randn(n, (nh + 2 * nkv) * hd, device=DEV, generator=gen)
+    cos_sin = torch.randn(n, hd // 2, 2, device=DEV, generator=gen)
+    weight = torch.randn(hd, device=DEV, generator=gen)
+    blocks = -(-n // 64)
+    slot = torch.zeros(n, dtype=torch.int32, device=DEV)
+    slot[n // 2:n // 2 + 11] = -1
+    slot[-3:] = -1
+    pos = torch.arange(n, dtype=torch.int32, device=DEV)
+    table = torch.randperm(blocks, device=DEV, generator=gen).to(torch.int32).view(1, blocks)
+    for dtype, norm, rotate, temp, tied, write in ((torch.bfloat16, True, True, None, False, True), (torch.float32, False, True, None, False, True),
+                                                   (torch.bfloat16, False, False, (0.1, 100), True, True),
+                                                   (torch.float32, True, True, (0.1, 100), False, False)):
+        got = []
+        for cuts in ([n], [piece] * (n // piece) + [n % piece]):
+            q_out = torch.full((n, nh * hd), 7.0, device=DEV, dtype=dtype)
+            k_pool, v_pool = (torch.full((blocks, nkv, 64, hd), 7.0, device=DEV, dtype=dtype) for _ in range(2))
+            at = 0
+            for m in cuts:
+                part = slice(at, at + m)
+                ops().qk_rope_kv_write(q_out[part], k_pool, v_pool, qkv[part], nh * hd, (nh if tied else nh + nkv) * hd,
+                                       weight if norm else None, weight if norm else None, 1e-6, cos_sin[part] if rotate else None,
+                                       slot[part], pos[part], table, nh, nkv, hd, write_kv=write, q_temp=temp)
+                at += m
+            got.append((q_out, k_pool, v_pool))
+        for large, small in zip(*got):
+            assert torch.equal(large, small)
+        assert bool((got[0][1] == 7.0).all()) == (not write) and bool((got[0][0][:100] != 7.0).any())
+
+
 @pytest.mark.parametrize("m", [1, 3, 8, 16])
 @pytest.mark.parametrize("width,inner,out_rows,norm_dtype", [(1032, 2760, 1536, torch.float32), (256, 520, 392, torch.bfloat16),
                                                             (4096, 1024, 4096, torch.bfloat16), (5120, 264, 5000, torch.float32)])

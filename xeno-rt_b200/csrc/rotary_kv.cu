@@ -246,8 +246,7 @@ __device__ __forceinline__ void store4_as(__nv_bfloat16* dst, const float (&v)[4
 
 // PROMPT: a warp walks all heads of a token of its own instead of every eighth head of the block's, so that what a warp has
 // to fetch before its first row (slot, position, cache block, angles: three trips to memory) is paid once for 48 rows and not
-// once for six, and the next rows are on their way while four are worked on.  From 32 tokens a multiprocessor on (2,048
-// tokens: 23.5 us against 21.7).
+// once for six, and the next rows are on their way while four are worked on.
 // Measured, microseconds, block a token -> warp a token, 32 + 8 + 8 heads: 7,999 tokens 98 -> 82,
 // 17,000 with head norms 275 -> 209 (3,000 GB/s).
 template <typename TN, typename TQ, typename TC, bool PROMPT>
@@ -410,7 +409,13 @@ static int qk_rope_kv_write(void* q_out, void* k_pool, void* v_pool, const float
     XRT_DISPATCH_DTYPE(norm_dtype, TN, {
       XRT_DISPATCH_DTYPE(q_dtype, TQ, {
         XRT_DISPATCH_DTYPE(cache_dtype, TC, {
-          const bool prompt = n_tokens >= 32 * 148;
+          // a warp a token from so many tokens a multiprocessor on; with head norms a warp's rows take it longer, and the more
+          // of them (microseconds, block a token -> warp a token: 16 + 8 heads 4,736 tokens 24.2 -> 22.1, with norms 29.2 -> 30.2, 5,000
+          // 32.6 -> 30.9; 32 + 16 heads with norms 5,000 56.7 -> 58.7, 6,001 67.2 -> 65.5; 64 + 16 heads 4,800 66.3 -> 68.4, 6,001 81.8 ->
+          // 78.7, with norms 8,000 131.7 -> 136.9, 17,000 273 -> 261; 2,048 tokens of 32 + 16 heads 21.7 -> 23.5)
+          const int heads = n_heads + 2 * n_kv_heads;
+          const int many = q_norm_w == nullptr ? (heads <= 48 ? 32 : 34) : (heads <= 24 ? 33 : (heads <= 48 ? 40 : 80));
+          const bool prompt = n_tokens >= (long long)many * xrt::multiprocessors();
           auto kernel = prompt ? xrt::qk_rope_kv_write_128_kernel<TN, TQ, TC, true> : xrt::qk_rope_kv_write_128_kernel<TN, TQ, TC, false>;
           xrt::launch_kernel(kernel, dim3(prompt ? (n_tokens + 7) / 8 : n_tokens), dim3(256), 0, stream,
               (TQ*)q_out, (TC*)k_pool, (TC*)v_pool, qkv, row_stride, k_offset, v_offset, (const TN*)q_norm_w,
