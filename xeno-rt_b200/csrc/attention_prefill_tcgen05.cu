@@ -422,7 +422,7 @@ static int launch_prefill(dim3 grid, const CUtensorMap& map_q, const CUtensorMap
                           const int* block_table, int max_blocks, int n_heads, int n_kv_heads, float scale_log2,
                           int* error_flag, KeyRange range, const float* sinks, cudaStream_t stream) {
   constexpr auto kernel = attention_prefill_tcgen05_kernel<TILES, HEADS>;
-  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FaShape<TILES>::SMEM);
+  const cudaError_t err = allow_shared_memory_once<kernel>(FaShape<TILES>::SMEM);
   if (err != cudaSuccess) return (int)err;
   // launched without programmatic dependent launch: a block needs a multiprocessor to itself, so nothing of it can
   // run beside the kernel before it, and the early launch was measured slower (28.2 against 27.8 ms a prompt of 2,048)

@@ -280,6 +280,21 @@ inline int multiprocessors() {
   return n;
 }
 
+// Lets a kernel have `bytes` of dynamic shared memory (always the same for one kernel), once a device: the call takes the
+// driver some tenths of a microsecond, and a launch of a few microseconds should not pay for it each time.
+template <auto KERNEL>
+inline cudaError_t allow_shared_memory_once(int bytes) {
+  static std::atomic<uint64_t> done{0};
+  int device = 0;
+  const cudaError_t asked = cudaGetDevice(&device);
+  if (asked != cudaSuccess) return asked;
+  const uint64_t bit = device < 64 ? (uint64_t)1 << device : 0;
+  if (bit != 0 && (done.load(std::memory_order_acquire) & bit) != 0) return cudaSuccess;
+  const cudaError_t err = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (err == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return err;
+}
+
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                           Args... args) {

@@ -140,7 +140,7 @@ XRT_EXPORT int xrt_gemm_reference(void* out, const void* x, const void* w, int M
   dim3 grid((N + xrt::RG_BN - 1) / xrt::RG_BN, (M + xrt::RG_BM - 1) / xrt::RG_BM);
   if (grid.y > 65535) return XRT_ERR_UNSUPPORTED;
   // small tiles while the large ones would occupy no more than half of the multiprocessors
-  const bool few = 2ll * grid.x * grid.y <= 148;
+  const bool few = 2ll * grid.x * grid.y <= xrt::multiprocessors();
   XRT_DISPATCH_DTYPE(x_dtype, TX, {
     XRT_DISPATCH_DTYPE(w_dtype, TW, {
       XRT_DISPATCH_DTYPE(out_dtype, TO, {

@@ -362,13 +362,9 @@ template <int MODE, bool PAIR, typename TO>
 int launch_tcgen05_tiled(void* out, const CUtensorMap& map_x, const CUtensorMap& map_w, int M, int N, int K, int ldo,
                          int up_rows, int* error_flag, int sm_count, const NormEmit& emit, const RowScale& scale,
                          cudaStream_t stream) {
-  auto kernel = gemm_tcgen05_kernel<MODE, PAIR, TO>;
-  static bool allowed = false;
-  if (!allowed) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TcShape<PAIR>::SMEM);
-    if (err != cudaSuccess) return (int)err;
-    allowed = true;
-  }
+  constexpr auto kernel = gemm_tcgen05_kernel<MODE, PAIR, TO>;
+  const cudaError_t err = allow_shared_memory_once<kernel>(TcShape<PAIR>::SMEM);
+  if (err != cudaSuccess) return (int)err;
   constexpr int n_per_tile = MODE == 2 ? TC_BN / 2 : TC_BN, tile_rows = (PAIR ? 2 : 1) * TC_BM;
   const int tiles = ((M + tile_rows - 1) / tile_rows) * ((N + n_per_tile - 1) / n_per_tile);
   const int units = PAIR ? sm_count / 2 : sm_count;

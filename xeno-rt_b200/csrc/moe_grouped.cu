@@ -237,8 +237,7 @@ moe_grouped_product_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
 template <int MODE>
 static int launch_moe_grouped(const CUtensorMap& map_a, const CUtensorMap& map_w, const MoeTiles& g, int blocks, int* error_flag,
                               cudaStream_t stream) {
-  const cudaError_t err =
-      cudaFuncSetAttribute(moe_grouped_product_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM);
+  const cudaError_t err = allow_shared_memory_once<moe_grouped_product_kernel<MODE>>(MG_SMEM);
   if (err != cudaSuccess) return (int)err;
   launch_kernel_alone(moe_grouped_product_kernel<MODE>, dim3(blocks), dim3(MG_THREADS), (size_t)MG_SMEM, stream, map_a, map_w, g,
                       error_flag);
@@ -266,10 +265,8 @@ XRT_EXPORT int xrt_moe_grouped_product(void* out, const void* a, const void* w, 
   if (rows < 0 || n_experts <= 0 || n <= 0 || k <= 0 || (first == 1 && (ff <= 0 || n != 2 * ff))) return XRT_ERR_ARGUMENT;
   if (k % 8 || (((uintptr_t)a | (uintptr_t)w) & 15)) return XRT_ERR_UNSUPPORTED;
   if (rows == 0) return XRT_OK;
-  int device = 0, sms = 0;
-  if (cudaGetDevice(&device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
-    return XRT_ERR_UNSUPPORTED;
+  const int sms = xrt::multiprocessors();
+  if (sms <= 0) return XRT_ERR_UNSUPPORTED;
   CUtensorMap map_a, map_w;
   if (!xrt::sm100::make_map_bf16_2d(&map_a, a, rows, k, k, xrt::MG_ROWS) ||
       !xrt::sm100::make_map_bf16_2d(&map_w, w, (long long)n_experts * n, k, k, 128))

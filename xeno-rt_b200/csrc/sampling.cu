@@ -666,12 +666,15 @@ XRT_EXPORT int xrt_sample(int* out_ids, const float* logits, int n_rows, int voc
   int values_bytes = cached ? (int)per * 4 : 0;
   if (values_bytes < xrt::SAMPLE_CANDIDATES * 8) values_bytes = xrt::SAMPLE_CANDIDATES * 8;
   const size_t smem = (size_t)values_bytes + xrt::SAMPLE_HIST_BYTES;
+  // one limit for every launch: setting a smaller one beside a launch of another thread would take it its room
+  constexpr int most = xrt::SAMPLE_CACHED_BYTES + xrt::SAMPLE_HIST_BYTES;
+  const cudaError_t err = cached ? (vec ? xrt::allow_shared_memory_once<xrt::sample_kernel<true, true>>(most)
+                                        : xrt::allow_shared_memory_once<xrt::sample_kernel<true, false>>(most))
+                                 : (vec ? xrt::allow_shared_memory_once<xrt::sample_kernel<false, true>>(most)
+                                        : xrt::allow_shared_memory_once<xrt::sample_kernel<false, false>>(most));
+  if (err != cudaSuccess) return (int)err;
   auto kernel = cached ? (vec ? xrt::sample_kernel<true, true> : xrt::sample_kernel<true, false>)
                        : (vec ? xrt::sample_kernel<false, true> : xrt::sample_kernel<false, false>);
-  // one limit for every launch: setting a smaller one beside a launch of another thread would take it its room
-  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               xrt::SAMPLE_CACHED_BYTES + xrt::SAMPLE_HIST_BYTES);
-  if (err != cudaSuccess) return (int)err;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3((unsigned)n_rows * team);
   config.blockDim = dim3(xrt::SAMPLE_THREADS);

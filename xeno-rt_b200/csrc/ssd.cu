@@ -307,7 +307,7 @@ template <int C2>
 int launch_ssd_scan_wide(const SsdArgs& a, int n_seqs, cudaStream_t stream) {
   constexpr int COLS = 8 * C2;
   constexpr size_t smem = (size_t)SSD_STAGES * (2 * SSD_TOKENS * 128 + SSD_TOKENS * COLS + SSD_TOKENS) * sizeof(float);
-  const cudaError_t err = cudaFuncSetAttribute(ssd_scan_wide_kernel<C2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t err = allow_shared_memory_once<ssd_scan_wide_kernel<C2>>((int)smem);
   if (err != cudaSuccess) return (int)err;
   launch_kernel_alone(ssd_scan_wide_kernel<C2>, dim3(n_seqs, a.n_heads, (a.vdim + COLS - 1) / COLS), dim3(128), smem, stream, a);
   return launch_status();
@@ -374,7 +374,7 @@ XRT_EXPORT int xrt_ssd_scan(float* out, const float* x, int x_stride, const floa
                    (((uintptr_t)x | (uintptr_t)b | (uintptr_t)c) & 15) == 0;
   if (max_new > 1 && vec && n_state == 128 && ((uintptr_t)state & 15) == 0) {
     // four columns a lane where their blocks still reach two thirds of the multiprocessors, two else
-    if ((long long)n_seqs * n_heads * ((vdim + 31) / 32) >= 100) return xrt::launch_ssd_scan_wide<4>(a, n_seqs, stream);
+    if (3ll * n_seqs * n_heads * ((vdim + 31) / 32) >= 2ll * xrt::multiprocessors()) return xrt::launch_ssd_scan_wide<4>(a, n_seqs, stream);
     return xrt::launch_ssd_scan_wide<2>(a, n_seqs, stream);
   }
   dim3 grid(n_seqs, n_heads, (vdim + a.cols - 1) / a.cols);

@@ -470,8 +470,8 @@ __global__ void __launch_bounds__(SPREAD_THREADS) state_scan_spread_kernel(const
 template <int LANES, int ROWS, int C2, bool DELTA>
 int launch_state_scan_spread(const ScanArgs& a, int n_seqs, int max_new, cudaStream_t stream) {
   using Shape = SpreadShape<LANES, ROWS, C2>;
-  auto kernel = state_scan_spread_kernel<LANES, ROWS, C2, DELTA>;
-  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
+  constexpr auto kernel = state_scan_spread_kernel<LANES, ROWS, C2, DELTA>;
+  const cudaError_t err = allow_shared_memory_once<kernel>(Shape::SMEM);
   if (err != cudaSuccess) return (int)err;
   const dim3 grid(n_seqs, a.n_heads, (a.vdim + Shape::COLS - 1) / Shape::COLS);
   if (max_new > 1) launch_kernel_alone(kernel, grid, dim3(SPREAD_THREADS), (size_t)Shape::SMEM, stream, a);
