@@ -170,7 +170,7 @@ def test_a_draw_lands_where_the_mass_says(vocab, temperature, top_k, top_p):
 
 
 def test_rows_without_a_finite_maximum_and_with_nan():
-    """Only ids above minus infinity are drawn; one infinity takes the row; a row without any value gives its first id."""
+    """Only ids above minus infinity are drawn, also beside a NaN (a small top_k, greedy); a row without any value gives its first id."""
     for vocab in (300, 20001):
         logits = np.full(vocab, -np.inf, dtype=np.float32)
         assert set(run_sampler(logits, 8, 1.0, 40, 0.9, 1.0).tolist()) == {0}

@@ -27,10 +27,13 @@
 //             precision at any magnitude), and the accumulated O in TMEM has to be rescaled (read,
 //             multiplied, written back by the row's thread) only on those rare moves instead of once a step.
 // What bounds a step of one tile is the chain of its softmax (the exponentials alone take 1,024 clocks of the special-function
-// units, as long as the tile's products take the tensor core): with one tile a block that chain was all a multiprocessor
-// did, 2,600 clocks a step.  Measured, microseconds a layer of 32 + 8 heads, one tile a block -> two: a prompt of 7,999
-// tokens 814 -> 714 (734 TFLOP/s), 16 prompts of 64 to 2,047 582 -> 404, one of 2,048 58 -> 50.  Two threads a row
-// (eight warps a tile, halves of the keys) were no faster (718 and 420): what is left is the products' own time.
+// units, as long as the tile's products take the tensor core): with one tile a block that chain is all a multiprocessor
+// does.  Measured, microseconds a layer of 32 + 8 heads, one tile a block -> two: a prompt of 7,999
+// tokens 814 -> 714 (734 TFLOP/s), 16 prompts of 64 to 2,047 582 -> 404, one of 2,048 58 -> 50.  With two tiles neither unit is
+// the bound yet: the products of 7,999 tokens are 333 us at the burst rate and the exponentials 235, and a prompt of 4,096 keeps
+// the tensor core busy 43 percent of the clocks, the special-function units 43 and the issue slots 34, so the two tiles' chains
+// overlap only in part.  What a step waits for is not known; two threads a row (eight warps a tile, halves of the keys) were no
+// faster (718 and 420), so it is not the length of one thread's chain.
 // Every mbarrier wait is bounded; a wait that runs out raises the error flag and an abort flag, all
 // roles leave their loops, TMEM is freed and the block returns.
 #include "tcgen05.cuh"

@@ -22,9 +22,11 @@
 // A block reads its slice once, applies the penalty and keeps the values in shared memory.  A small top_k leaves few
 // candidates, which the first block finishes by itself; without one, the team goes through the
 // selects together, meeting once a pass.
-// Measured, microseconds, one block a row -> teams: 128,256 logits, top_k 40, top_p 0.95, 1 row 137 -> 22, 64 rows 145 -> 59; top_p
-// alone 463 -> 58 and 483 -> 162; greedy 16 -> 5 and 17 -> 14; 4 rows of 256 logits 45 -> 10.  64 rows: bound by the
-// multiprocessors' instructions (16,032 logits a block, three and a half blocks on each); memory would take 5.
+// Measured, microseconds, one block a row -> teams: 128,256 logits, top_k 40, top_p 0.95, 1 row 136 -> 21, 64 rows 145 -> 57; top_p
+// 0.9 alone 559 -> 62 and 571 -> 169; greedy 32 -> 6 and 34 -> 14; top_k 500 136 -> 33 and 151 -> 91.  Memory would take 5 for 64 rows.
+// One row is a chain of latencies: the pass over the slice, the team's meetings, the ranking.  64 rows run it twice, since two blocks
+// fill a multiprocessor (64 registers a thread of 512; 85 KB) and there are 512; the schedulers then issue on half of the clocks, and
+// a warp waits for its block or its team a quarter of the time.
 #include "common.cuh"
 
 namespace xrt {

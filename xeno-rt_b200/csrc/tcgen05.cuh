@@ -2,8 +2,8 @@
 // wrappers over inline PTX: mbarriers with bounded waits, TMA tensor copies, shared-memory and
 // instruction descriptors of tcgen05.mma (kind::f16, bfloat16 operands, float32 accumulators in tensor
 // memory), commits, fences, tensor-memory loads and stores, and the driver's tensor-map encoder.
-// Used by gemm_tcgen05.cu (prompt products), gemm_decode_tcgen05.cu (few-row products) and
-// attention_prefill_tcgen05.cu (prompt attention).
+// Used by gemm_tcgen05.cu (prompt products), gemm_decode_tcgen05.cu (few-row products), moe_grouped.cu (experts'
+// products) and attention_prefill_tcgen05.cu (prompt attention).
 #pragma once
 
 #include <cuda.h>
