@@ -102,14 +102,16 @@ def test_state_scan_is_the_same_bits_alone_and_in_a_batch_whole_and_cut(heads, q
     decay = torch.rand(n, length, heads * dim, device=DEV, generator=gen) * 0.2 + 0.8
     beta = rnd(n, length, heads)
 
-    def run(seqs, portions):
-        """Outputs [sequences, length, ...] and states of ``seqs``, brought in ``portions`` of tokens."""
+    def run(seqs, portions, odd=False):
+        """Outputs [sequences, length, ...] and states of ``seqs``, brought in ``portions`` of tokens; ``odd``: operands in wider rows,
+        at no multiple of 16 bytes."""
         m = len(seqs)
+        place = (lambda t: torch.cat([t[:, :1], t, t[:, :2]], dim=1)[:, 1:-2]) if odd else (lambda t: t)
         state = torch.zeros(m, heads, vdim, dim, device=DEV)
         slots = torch.arange(m, dtype=torch.int32, device=DEV)
         outs, at = [], 0
         for part in portions:
-            take = lambda t: t[seqs, at:at + part].reshape(m * part, -1).contiguous()
+            take = lambda t: place(t[seqs, at:at + part].reshape(m * part, -1).contiguous())
             out = torch.empty(m * part, heads * vdim, device=DEV)
             cu = torch.arange(0, m * part + 1, part, dtype=torch.int32, device=DEV)
             ops.state_scan(out, take(q), take(k), take(v), take(decay), take(beta) if delta else None, state, cu, slots, heads,
@@ -121,6 +123,8 @@ def test_state_scan_is_the_same_bits_alone_and_in_a_batch_whole_and_cut(heads, q
     singles = [1] * length
     for seq in (0, 7):
         want, want_state = run([seq], [length])
+        for got in (run([seq], [length], odd=True), run([seq], singles, odd=True)):
+            assert torch.equal(got[0], want) and torch.equal(got[1], want_state)
         for seqs, portions in (([seq], [8, 1, 5, 7]), ([seq], singles), (list(range(12)), [length]), (list(range(40)), [length]),
                                (list(range(n)), [length]), (list(range(n)), singles)):
             got, state = run(seqs, portions)
