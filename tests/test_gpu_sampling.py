@@ -218,3 +218,52 @@ def test_a_large_top_k_over_one_block_and_a_team(vocab, top_k, falling):
     half = ids[order][np.searchsorted(np.cumsum(probs[order]), 0.5)]
     share = probs[ids <= half].sum()
     assert abs((got <= half).mean() - share) < 6 * np.sqrt(share * (1 - share) / len(got))
+
+
+# a slice of the smallest size, of an odd one, rows of whole 16 bytes or not; teams of eight, four and two blocks; a top_k of one, the
+# usual ones, the largest that each team serves and one more
+@pytest.mark.parametrize("rows", [1, 37, 64, 149])
+@pytest.mark.parametrize("vocab", [4096, 16385, 32000, 128256, 151937])
+def test_the_small_form_gives_the_same_ids(rows, vocab):
+    """Every id is the one that the kernel gives without being told the largest top_k: kept sets, masses and draws are whole numbers
+    there.  Rows: plain logits, few different values (ties at the cut, also more than there is room for), both zeros, infinities
+    and NaN, fewer finite values than top_k, falling values, greedy rows and padding among them, with a history."""
+    from xeno_rt_b200.csrc import ops
+    rng = np.random.default_rng(rows * 7 + vocab)
+    logits = (rng.normal(size=(rows, vocab)) * 3.0).astype(np.float32)
+    for i in range(rows):
+        kind = (i + vocab) % 9 if rows > 1 else 0
+        if kind == 1:
+            logits[i] = np.round(logits[i])
+        elif kind == 2:
+            logits[i] = np.where(rng.random(vocab) < 0.5, -0.0, 0.0)
+        elif kind == 3:
+            logits[i, rng.choice(vocab, 3)] = np.inf
+        elif kind == 4:
+            logits[i, rng.random(vocab) < 0.5] = np.nan
+        elif kind == 5:
+            logits[i] = -np.inf
+            logits[i, rng.choice(vocab, 11)] = 1.0
+        elif kind == 6:
+            logits[i] = np.sort(logits[i])[::-1]
+        elif kind == 7:
+            logits[i] = -np.inf
+    logits = torch.from_numpy(logits).to(DEV)
+    seen = torch.from_numpy(rng.integers(0, 2 ** 31, size=(rows, (vocab + 31) // 32), dtype=np.int32)).to(DEV)
+    slots = torch.arange(rows, dtype=torch.int32, device=DEV)
+    if rows > 1:
+        slots[rows // 2] = -1
+    as_rows = lambda v: torch.from_numpy(np.resize(np.asarray(v), rows)).to(DEV)
+    key = torch.from_numpy(rng.integers(0, 2 ** 62, size=rows)).to(DEV)
+    for top_k in (1, 40, 64, 65, 128, 129, 256, 257):
+        ks = as_rows(np.array([top_k, max(1, top_k // 2), top_k, 1, top_k], dtype=np.int32))
+        temps = as_rows(np.array([0.8, 1.0, 0.7, 1.3, 0.9, 0.8, 0.0] if rows > 1 else [0.8], dtype=np.float32))
+        for top_p, penalty in ((0.95, 1.1), (1.0, 1.0), (0.5, 1.3)):
+            args = (temps, ks, as_rows(np.array([top_p], dtype=np.float32)), as_rows(np.array([penalty], dtype=np.float32)), seen, key)
+            got = []
+            for told in (0, top_k):
+                out = torch.full((rows,), -7, dtype=torch.int32, device=DEV)
+                counter = torch.arange(rows, dtype=torch.int32, device=DEV)
+                ops.sample(out, logits, slots, *args, counter, largest_top_k=told)
+                got.append((out.tolist(), counter.tolist()))
+            assert got[0] == got[1]

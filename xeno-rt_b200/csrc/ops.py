@@ -92,7 +92,7 @@ _SIGNATURES = {
     "xrt_recurrence_scan": [_P, _P, _I, _I, _P],
     "xrt_recurrence_step": [_P, _P, _P, _P, _P, _P, _I, _P],
     "xrt_fill_normal": [_P, ctypes.c_longlong, ctypes.c_ulonglong, ctypes.c_double, ctypes.c_double, _I, _P],
-    "xrt_sample": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P],
+    "xrt_sample": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _P],
     "xrt_mark_seen": [_P, _I, _P, _P, _I, _I, _P],
 }
 
@@ -859,8 +859,10 @@ def fill_normal(out, key: int, mean: float, std: float) -> None:
                                      float(std), _code(out.dtype), _stream()), "fill_normal")
 
 
-def sample(out_ids, logits, row_slot, temperature, top_k, top_p, penalty, seen, rng_key, rng_counter) -> None:
-    """One token id per row of float32 logits; see sampling.cu for the conventions."""
+def sample(out_ids, logits, row_slot, temperature, top_k, top_p, penalty, seen, rng_key, rng_counter,
+           largest_top_k: int = 0) -> None:
+    """One token id per row of float32 logits; see sampling.cu for the conventions.  ``largest_top_k``: the largest of
+    ``top_k`` where every row is greedy or has one (0: not known, or some row has none); the same ids, by a faster form."""
     n, vocab = logits.shape
     seen_words = 0 if seen is None else seen.shape[1]
     _check(_kernels().xrt_sample(
@@ -868,7 +870,8 @@ def sample(out_ids, logits, row_slot, temperature, top_k, top_p, penalty, seen, 
         _ptr(row_slot, "row_slot", torch.int32), _ptr(temperature, "temperature", torch.float32),
         _ptr(top_k, "top_k", torch.int32), _ptr(top_p, "top_p", torch.float32),
         _ptr(penalty, "penalty", torch.float32), _ptr(seen, "seen", torch.int32), seen_words,
-        _ptr(rng_key, "rng_key", torch.int64), _ptr(rng_counter, "rng_counter", torch.int32), _stream()), "sample")
+        _ptr(rng_key, "rng_key", torch.int64), _ptr(rng_counter, "rng_counter", torch.int32), int(largest_top_k), _stream()),
+        "sample")
 
 
 def mark_seen(seen, slots, ids, vocab: int) -> None:

@@ -24,9 +24,13 @@
 // selects together, meeting once a pass.
 // Measured, microseconds, one block a row -> teams: 128,256 logits, top_k 40, top_p 0.95, 1 row 136 -> 21, 64 rows 145 -> 57; top_p
 // 0.9 alone 559 -> 62 and 571 -> 169; greedy 32 -> 6 and 34 -> 14; top_k 500 136 -> 33 and 151 -> 91.  Memory would take 5 for 64 rows.
-// One row is a chain of latencies: the pass over the slice, the team's meetings, the ranking.  64 rows run it twice, since two blocks
-// fill a multiprocessor (64 registers a thread of 512; 85 KB) and there are 512; the schedulers then issue on half of the clocks, and
-// a warp waits for its block or its team a quarter of the time.
+// One row is a chain of latencies: the pass over the slice, the team's meetings, the ranking.  64 rows of that kernel run it twice, since
+// two blocks fill a multiprocessor (64 registers a thread of 512; 85 KB) and there are 512.
+//
+// Batches whose rows all have a small top_k (the usual options; the caller says so) or are greedy take the SMALL form (64 rows of 128,256
+// with top_k 40, top_p 0.95: 63 -> 27 us a call, of which the kernel is no longer the larger part): no values kept,
+// so that four blocks of 32,064 logits a row run all at once, and one cut for the whole team, so that hardly more than top_k
+// candidates remain and only the threads that hold one look at the logits again.
 #include "common.cuh"
 
 namespace xrt {
@@ -39,6 +43,8 @@ constexpr int SAMPLE_HIST_BYTES = SAMPLE_FINE_BINS * 4;    // also room for the 
 constexpr int SAMPLE_CANDIDATES = 4096;                    // of a small top_k, all blocks together
 constexpr int SAMPLE_NARROW = 192;                         // so many candidates are cut down once more
 constexpr int SAMPLE_CACHED_BYTES = 160 * 1024;            // of logits a block keeps at most
+constexpr int SAMPLE_GROUPS = SAMPLE_THREADS / 8;          // of a block in the SMALL form: eight lanes each
+constexpr uint32_t SAMPLE_LOWEST_KEY = 0x007fffffu;        // the order key of minus infinity
 static_assert(SAMPLE_HIST_COPIES * 256 * 8 <= SAMPLE_HIST_BYTES && SAMPLE_CANDIDATES * 8 <= 32 * 1024, "the regions hold");
 
 __device__ __forceinline__ uint64_t sm64(uint64_t x) {
@@ -125,6 +131,16 @@ struct SampleShared {
   unsigned int draw;
   long long pick;
   int warp_count[SAMPLE_WARPS];
+};
+
+// What the SMALL form has beside: the largest order keys of every group of every block, the cut, and the first block's candidates.
+struct SmallShared {
+  alignas(16) uint32_t group_key[SAMPLE_TEAM * SAMPLE_GROUPS];
+  uint32_t own_key[SAMPLE_GROUPS];
+  uint32_t cut;
+  int count;
+  int id[SAMPLE_THREADS];
+  float value[SAMPLE_THREADS];
 };
 
 struct Team {
@@ -430,15 +446,70 @@ __device__ long long ranked_place(float a, int n, int k, float temp, float p, fl
   return team.sh->pick;
 }
 
+// The same choice for candidates in any order (ids[i], vals[i], no more than threads, all of the row's values at or above its
+// k-th largest among them): places are compared by id.  Returns the id.  `order`, `mass`: shared memory for SAMPLE_THREADS numbers each.
+__device__ int ranked_id(const int* ids, const float* vals, int n, int k, float temp, float p, float row_max, int row_arg,
+                         uint64_t* order, uint64_t* mass, Team& team) {
+  const int i = threadIdx.x;
+  const bool live = i < n, warp_live = (i & ~31) < n;
+  const int id = live ? ids[i] : 0;
+  const float a = live ? vals[i] : 0.f;
+  const uint64_t mine = ((uint64_t)order_key(a) << 32) | (uint32_t)~(uint32_t)id;
+  if (live) order[i] = mine;
+  if (i == 0) team.sh->pick = -1;
+  __syncthreads();
+  int rank = n;
+  if (warp_live) {
+    rank = 0;
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) rank += order[j] > mine;
+  }
+  const uint64_t m = live && rank < k ? probability_mass(a, row_max, 1.0f / temp) : 0ull;
+  if (live) mass[i] = m;
+  uint64_t total;
+  block_exclusive_scan(m, team.sh->scan, &total);
+  uint64_t kept = m;
+  if (p < 1.0f) {
+    uint64_t want = (uint64_t)ceil((double)p * (double)total);
+    if (want < 1) want = 1;
+    uint64_t before = 0;
+    if (warp_live) {
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) before += order[j] > mine ? mass[j] : 0ull;
+    }
+    if (before >= want) kept = 0;
+    __syncthreads();  // the masses are read: what is kept of them takes their place
+    if (live) mass[i] = kept;
+  }
+  block_exclusive_scan(kept, team.sh->scan, &total);  // (its barriers: the kept masses are there)
+  uint64_t below = 0;
+  if (warp_live) {
+    const uint32_t place = (uint32_t)mine;  // falls as the id rises
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) below += (uint32_t)order[j] > place ? mass[j] : 0ull;
+  }
+  const uint64_t target = __umul64hi((uint64_t)team.sh->draw << 32, total);  // floor(u / 2^32 * total)
+  if (total > 0 && below <= target && target < below + kept) team.sh->pick = id;
+  __syncthreads();
+  return team.sh->pick >= 0 ? (int)team.sh->pick : row_arg;
+}
+
 // CACHED: a block's slice of the row fits its shared memory (else the passes read it from the L2 again).
 // VEC: rows are whole 16 bytes.
-template <bool CACHED, bool VEC>
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+// SMALL (not CACHED): for batches whose rows have a small top_k or are greedy.  The row's cut is the k-th largest of the largest values
+// of all groups of eight lanes of the team (64 a block): k values lie at or above it, and with twice as many groups as k hardly more.
+// Every block gets every group's value (one meeting) and finds the cut by itself; a thread whose own largest value reaches it
+// looks at its logits again and sends what lies at or above the cut to the first block, which ranks the candidates.  A row that
+// this does not serve (a larger k, more equal values than there is room for, fewer than k values above minus infinity) goes
+// through the selects over the whole row, as without a small top_k.
+template <bool CACHED, bool VEC, bool SMALL>
+__global__ void __launch_bounds__(SAMPLE_THREADS, 2)
 sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int vocab, int per_block, int values_bytes,
               const int* __restrict__ row_slot, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
               const float* __restrict__ penalty, const uint32_t* __restrict__ seen, int seen_words,
               const unsigned long long* __restrict__ rng_key, unsigned int* __restrict__ rng_counter, int team_size) {
+  static_assert(!(CACHED && SMALL), "the small form keeps no values");
   __shared__ SampleShared sh;
   extern __shared__ __align__(16) unsigned char dynamic[];
   float* values = reinterpret_cast<float*>(dynamic);  // the slice; in the first block later the candidates' ids and values
@@ -464,7 +535,8 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
   view.seen = (seen != nullptr && view.penalty > 1.0f) ? seen + (size_t)slot * seen_words + base / 32 : nullptr;
   const float temp = temperature[row];
   const int k = top_k[row];
-  const bool few = temp > 1e-5f && k > 0 && k < vocab;  // candidates are gathered first
+  const bool few = !SMALL && temp > 1e-5f && k > 0 && k < vocab;  // candidates are gathered first
+  SmallShared* small = reinterpret_cast<SmallShared*>(dynamic);   // SMALL: where the others keep values
 
   // The one pass over the logits: penalty, and every thread's largest value (the first of equals).  For a small top_k a
   // histogram of the order keys' top 12 bits says where to cut: of the threads' largest values if they are at least twice
@@ -479,34 +551,38 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
     if (a > best) { best = a; best_i = i; }  // indices rise: the first maximum is kept
     if (few && !of_largest) atomicAdd(&hist[order_key(a) >> 20], 1u);
   };
-  if (VEC) {
-    constexpr int UNROLL = 4;  // loads in flight a thread
-    const int quads = n / 4;
-    const float4* src = reinterpret_cast<const float4*>(view.logits);
-    for (int q0 = threadIdx.x; q0 < quads; q0 += UNROLL * SAMPLE_THREADS) {
-      float4 v[UNROLL]; uint32_t bits[UNROLL];
+  // every element of this thread, with the penalty
+  auto visit = [&](auto&& f) {
+    if (VEC) {
+      constexpr int UNROLL = 4;  // loads in flight a thread
+      const int quads = n / 4;
+      const float4* src = reinterpret_cast<const float4*>(view.logits);
+      for (int q0 = threadIdx.x; q0 < quads; q0 += UNROLL * SAMPLE_THREADS) {
+        float4 v[UNROLL]; uint32_t bits[UNROLL];
 #pragma unroll
-      for (int u = 0; u < UNROLL; ++u) {
-        const int q = q0 + u * SAMPLE_THREADS;
-        v[u] = q < quads ? src[q] : make_float4(0.f, 0.f, 0.f, 0.f);
-        bits[u] = (q < quads && view.seen != nullptr) ? view.seen[q >> 3] >> (4 * (q & 7)) : 0u;
-      }
+        for (int u = 0; u < UNROLL; ++u) {
+          const int q = q0 + u * SAMPLE_THREADS;
+          v[u] = q < quads ? src[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+          bits[u] = (q < quads && view.seen != nullptr) ? view.seen[q >> 3] >> (4 * (q & 7)) : 0u;
+        }
 #pragma unroll
-      for (int u = 0; u < UNROLL; ++u) {
-        const int q = q0 + u * SAMPLE_THREADS;
-        if (q < quads) {
-          float a[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+        for (int u = 0; u < UNROLL; ++u) {
+          const int q = q0 + u * SAMPLE_THREADS;
+          if (q < quads) {
+            float a[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if ((bits[u] >> e) & 1u) a[e] = a[e] > 0.f ? a[e] / view.penalty : a[e] * view.penalty;
-            take(4 * q + e, a[e]);
+            for (int e = 0; e < 4; ++e) {
+              if ((bits[u] >> e) & 1u) a[e] = a[e] > 0.f ? a[e] / view.penalty : a[e] * view.penalty;
+              f(4 * q + e, a[e]);
+            }
           }
         }
       }
+    } else {
+      for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) f(i, view.adjusted(i));
     }
-  } else {
-    for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) take(i, view.adjusted(i));
-  }
+  };
+  visit(take);
   auto adjusted = [&](int i) { return CACHED ? values[i] : view.adjusted(i); };
 
   if (few && of_largest) atomicAdd(&hist[best_i < 0 ? 0 : order_key(best) >> 20], 1u);
@@ -518,6 +594,14 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
     packed = other > packed ? other : packed;
   }
   if (lane == 0) sh.scan[warp] = packed;
+  const uint32_t own_key = best_i < 0 ? 0u : order_key(best + 0.0f);  // (both zeros alike: which of them is first in `best` is chance)
+  if (SMALL) {
+    uint32_t group = own_key;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) group = max(group, __shfl_xor_sync(0xffffffffu, group, o));
+    if ((lane & 7) == 0) small->own_key[threadIdx.x >> 3] = group;
+    if (threadIdx.x == 0) small->count = 0;
+  }
   __syncthreads();
   if (threadIdx.x < SAMPLE_TEAM) {
     for (int w = 0; w < SAMPLE_WARPS; ++w) packed = sh.scan[w] > packed ? sh.scan[w] : packed;
@@ -545,6 +629,9 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
   }
 
   team_wait();  // every block of the team runs: its shared memory may be written
+  if (SMALL)
+    for (int e = threadIdx.x; e < SAMPLE_GROUPS * team_size; e += SAMPLE_THREADS)
+      of_block(small->group_key, e / SAMPLE_GROUPS)[rank * SAMPLE_GROUPS + e % SAMPLE_GROUPS] = small->own_key[e % SAMPLE_GROUPS];
   if ((int)threadIdx.x < team_size) {
     of_block(sh.best, threadIdx.x)[rank] = packed;
     if (rank == 0) {
@@ -567,6 +654,51 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
     return;
   }
 
+  const float p = top_p[row];
+  if (SMALL) {
+    const int groups = SAMPLE_GROUPS * team_size;
+    bool served = k > 0 && k < vocab && 2 * k <= groups;
+    if (served) {
+      if ((int)threadIdx.x < groups) {
+        const uint32_t key = small->group_key[threadIdx.x];
+        int above = 0, equal = 0;
+#pragma unroll 4
+        for (int j = 0; j < groups; j += 4) {
+          const uint4 other = *reinterpret_cast<const uint4*>(&small->group_key[j]);
+          above += (other.x > key) + (other.y > key) + (other.z > key) + (other.w > key);
+          equal += (other.x == key) + (other.y == key) + (other.z == key) + (other.w == key);
+        }
+        if (above < k && k <= above + equal) small->cut = key;  // (all who write it write the same)
+      }
+      __syncthreads();
+      const uint32_t cut = small->cut;
+      served = cut > SAMPLE_LOWEST_KEY;
+      if (served) {
+        if (own_key >= cut)
+          visit([&](int i, float a) {
+            if (order_key(a + 0.0f) >= cut) {
+              SmallShared* first = of_block(small, 0);
+              const int place = atomicAdd(&first->count, 1);
+              if (place < SAMPLE_THREADS) {
+                first->id[place] = base + i;
+                first->value[place] = a;
+              }
+            }
+          });
+        team_sync();  // the candidates are there
+        const int count = of_block(small, 0)->count;
+        served = count <= SAMPLE_THREADS;
+        team_sync();  // everybody has read how many they are: the other blocks may leave
+        if (served) {
+          if (rank != 0) return;
+          uint64_t* order = reinterpret_cast<uint64_t*>(hist);
+          const int id = ranked_id(small->id, small->value, count, k, temp, p, row_max, row_arg, order, order + SAMPLE_THREADS, team);
+          if (threadIdx.x == 0) out_ids[row] = id;
+          return;
+        }
+      }
+    }
+  }
   bool compact = few;
   int counts[SAMPLE_TEAM];
   int all = 0;
@@ -577,7 +709,6 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
     all += counts[r];
   }
   compact = compact && all <= SAMPLE_CANDIDATES;
-  const float p = top_p[row];
   if (compact) {
     if (rank == 0) {
       int* ids = reinterpret_cast<int*>(values);
@@ -645,38 +776,55 @@ __global__ void mark_seen_kernel(uint32_t* __restrict__ seen, int seen_words, co
 
 }  // namespace xrt
 
+namespace xrt {
+
+// One limit for every launch of a form: setting a smaller one beside a launch of another thread would take it its room.
+template <bool CACHED, bool VEC, bool SMALL>
+static auto sample_form(cudaError_t& err) {
+  err = allow_shared_memory_once<sample_kernel<CACHED, VEC, SMALL>>(SAMPLE_CACHED_BYTES + SAMPLE_HIST_BYTES);
+  return sample_kernel<CACHED, VEC, SMALL>;
+}
+
+}  // namespace xrt
+
 // logits: [n_rows, vocab] 32-bit.  Per row: its slot (< 0 = padding, id -1), temperature, top_k
 // (0 = all), top_p (>= 1 = all), repetition penalty (<= 1 = none).  seen: [slots, seen_words]
-// bitmaps or null.  rng_key / rng_counter: per slot.
+// bitmaps or null.  rng_key / rng_counter: per slot.  largest_top_k: where the caller knows that every row is greedy or has a
+// top_k of at least 1, the largest of those, else 0; it chooses the form of the kernel and changes no result.
 XRT_EXPORT int xrt_sample(int* out_ids, const float* logits, int n_rows, int vocab, const int* row_slot,
                           const float* temperature, const int* top_k, const float* top_p, const float* penalty,
                           const unsigned int* seen, int seen_words, const unsigned long long* rng_key,
-                          unsigned int* rng_counter, cudaStream_t stream) {
+                          unsigned int* rng_counter, int largest_top_k, cudaStream_t stream) {
   if (n_rows < 0 || vocab <= 0) return XRT_ERR_ARGUMENT;
   if (seen != nullptr && seen_words * 32 < vocab) return XRT_ERR_ARGUMENT;
   if (n_rows == 0) return XRT_OK;
-  // blocks of a team: as many as it takes to bring a slice to 4,096 logits (smaller ones are read in less time than a team takes
-  // to meet), or, where the rows alone occupy the multiprocessors, as keep it at 4,096 (256 rows of 5,000 logits, one block against
-  // two: 20.7 against 26.6 us); half as many while the rows alone bring more than four blocks a multiprocessor
   const int sms = xrt::multiprocessors();
-  int team = 1;
-  while (team < xrt::SAMPLE_TEAM && (long long)team * (n_rows >= sms ? 2 * 4096 - 1 : 4096) < vocab) team *= 2;
-  while (team > 2 && (long long)team * n_rows > 4ll * sms) team /= 2;
+  // The SMALL form: as many blocks a row as run all at once (two a multiprocessor), where slices are then no smaller than 2,048
+  // logits and the team has at least twice as many groups of lanes as the largest top_k.
+  int team = xrt::SAMPLE_TEAM;
+  while (team > 2 && ((long long)team * n_rows > 2ll * sms || (long long)team * 2048 > vocab)) team /= 2;
+  const bool small = largest_top_k > 0 && largest_top_k < vocab && 2 * largest_top_k <= team * xrt::SAMPLE_GROUPS &&
+                     (long long)team * 2048 <= vocab;
+  if (!small) {
+    // blocks of a team: as many as it takes to bring a slice to 4,096 logits (smaller ones are read in less time than a team takes
+    // to meet), or, where the rows alone occupy the multiprocessors, as keep it at 4,096 (256 rows of 5,000 logits, one block against
+    // two: 20.7 against 26.6 us); half as many while the rows alone bring more than four blocks a multiprocessor
+    team = 1;
+    while (team < xrt::SAMPLE_TEAM && (long long)team * (n_rows >= sms ? 2 * 4096 - 1 : 4096) < vocab) team *= 2;
+    while (team > 2 && (long long)team * n_rows > 4ll * sms) team /= 2;
+  }
   const long long per = ((long long)vocab + team * 32 - 1) / (team * 32) * 32;
-  const bool cached = per * 4 <= xrt::SAMPLE_CACHED_BYTES;
+  const bool cached = !small && per * 4 <= xrt::SAMPLE_CACHED_BYTES;
   const bool vec = vocab % 4 == 0 && ((uintptr_t)logits & 15) == 0;
   int values_bytes = cached ? (int)per * 4 : 0;
-  if (values_bytes < xrt::SAMPLE_CANDIDATES * 8) values_bytes = xrt::SAMPLE_CANDIDATES * 8;
+  if (small) values_bytes = (int)((sizeof(xrt::SmallShared) + 15) / 16 * 16);
+  else if (values_bytes < xrt::SAMPLE_CANDIDATES * 8) values_bytes = xrt::SAMPLE_CANDIDATES * 8;
   const size_t smem = (size_t)values_bytes + xrt::SAMPLE_HIST_BYTES;
-  // one limit for every launch: setting a smaller one beside a launch of another thread would take it its room
-  constexpr int most = xrt::SAMPLE_CACHED_BYTES + xrt::SAMPLE_HIST_BYTES;
-  const cudaError_t err = cached ? (vec ? xrt::allow_shared_memory_once<xrt::sample_kernel<true, true>>(most)
-                                        : xrt::allow_shared_memory_once<xrt::sample_kernel<true, false>>(most))
-                                 : (vec ? xrt::allow_shared_memory_once<xrt::sample_kernel<false, true>>(most)
-                                        : xrt::allow_shared_memory_once<xrt::sample_kernel<false, false>>(most));
+  cudaError_t err = cudaSuccess;
+  auto kernel = small ? (vec ? xrt::sample_form<false, true, true>(err) : xrt::sample_form<false, false, true>(err))
+                : cached ? (vec ? xrt::sample_form<true, true, false>(err) : xrt::sample_form<true, false, false>(err))
+                         : (vec ? xrt::sample_form<false, true, false>(err) : xrt::sample_form<false, false, false>(err));
   if (err != cudaSuccess) return (int)err;
-  auto kernel = cached ? (vec ? xrt::sample_kernel<true, true> : xrt::sample_kernel<true, false>)
-                       : (vec ? xrt::sample_kernel<false, true> : xrt::sample_kernel<false, false>);
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3((unsigned)n_rows * team);
   config.blockDim = dim3(xrt::SAMPLE_THREADS);
