@@ -20,8 +20,12 @@ constexpr int PRE_ROWS = PRE_WARPS * 16;
 
 // SCORED: the layer's score options (common.cuh) are on: kept first keys behind the window, a tanh cap, a distance
 // slope.  The tiles of the kept keys are walked before the window's.
-template <int HD_MAX, bool SCORED>
-__global__ void __launch_bounds__(PRE_WARPS * 32)
+// HEADS: query heads of one kv head a block, four warps each, that share every tile.  Rows of more than 128 dims fill a
+// multiprocessor's shared memory with one block: with one head it was four warps that waited for their own loads and products
+// in turn (16 heads on rows of 256 dims, windows of 1,024, prompts of 3,598 tokens together: 354 us; 197 in this form).  Where the values are the keys'
+// own rows (latent attention) a tile is brought once.
+template <int HD_MAX, bool SCORED, int HEADS>
+__global__ void __launch_bounds__(HEADS * PRE_WARPS * 32)
 attention_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ q,
                          const __nv_bfloat16* __restrict__ k_pool, const __nv_bfloat16* __restrict__ v_pool,
                          const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot,
@@ -32,7 +36,8 @@ attention_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* _
   extern __shared__ __align__(16) unsigned char smem[];
   // later query tiles walk more keys: they are scheduled first, the longest tiles of all heads and of all the step's
   // prompts before any shorter one (heads are the grid's fastest dimension, query tiles its slowest)
-  const int q_tile = gridDim.z - 1 - blockIdx.z, head = blockIdx.x, seq = blockIdx.y;
+  const int all_warps = threadIdx.x >> 5;
+  const int q_tile = gridDim.z - 1 - blockIdx.z, head = blockIdx.x * HEADS + all_warps / PRE_WARPS, seq = blockIdx.y;
   const int slot = seq_slot[seq];
   if (slot < 0) return;
   const int tok0 = cu_seqlens[seq];
@@ -40,12 +45,13 @@ attention_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* _
   const int row0 = q_tile * PRE_ROWS;
   if (row0 >= n_new) return;
   const int start = seq_start[seq];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int warp = all_warps % PRE_WARPS, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int kv_head = head / (n_heads / n_kv_heads);
   const int row_bytes = tile_row_bytes(head_dim);
   const int tile_bytes = XRT_BLOCK_TOKENS * row_bytes;
+  const bool own_values = v_pool != k_pool;
   unsigned char* k_tiles = smem;
-  unsigned char* v_tiles = smem + 2 * tile_bytes;
+  unsigned char* v_tiles = own_values ? smem + 2 * tile_bytes : k_tiles;
 
   // this lane's two query rows (new-token indices) and their key ranges
   const int rows[2] = {row0 + warp * 16 + g, row0 + warp * 16 + g + 8};
@@ -102,7 +108,7 @@ attention_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* _
     const size_t base = ((size_t)block * n_kv_heads + kv_head) * head_stride;
     const int live = min(XRT_BLOCK_TOKENS, block_hi - key0);
     copier.copy(k_tiles + buffer * tile_bytes, k_pool + base, XRT_BLOCK_TOKENS, live);
-    copier.copy(v_tiles + buffer * tile_bytes, v_pool + base, XRT_BLOCK_TOKENS, live);
+    if (own_values) copier.copy(v_tiles + buffer * tile_bytes, v_pool + base, XRT_BLOCK_TOKENS, live);
     cp_async_commit();
   };
 
@@ -146,24 +152,38 @@ attention_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* _
   }
 }
 
+template <int HD_MAX, bool SCORED, int HEADS>
+int launch_prefill_heads(__nv_bfloat16* out, const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __nv_bfloat16* v_pool,
+                   const int* cu_seqlens, const int* seq_slot, const int* seq_start, const int* block_table,
+                   int max_blocks, int n_seqs, int max_new, int n_heads, int n_kv_heads, int head_dim, float scale,
+                   const KeyRange& range, const ScoreOptions& opt, cudaStream_t stream) {
+  const int smem = (v_pool == k_pool ? 2 : 4) * XRT_BLOCK_TOKENS * (head_dim * 2 + 16);
+  // (one limit for every launch of a form, the largest it can need)
+  const cudaError_t err = allow_shared_memory_once<attention_prefill_kernel<HD_MAX, SCORED, HEADS>>(4 * XRT_BLOCK_TOKENS * (HD_MAX * 2 + 16));
+  if (err != cudaSuccess) return (int)err;
+  auto kernel = attention_prefill_kernel<HD_MAX, SCORED, HEADS>;
+  dim3 grid(n_heads / HEADS, n_seqs, (max_new + PRE_ROWS - 1) / PRE_ROWS);
+  kernel<<<grid, HEADS * PRE_WARPS * 32, smem, stream>>>(out, q, k_pool, v_pool, cu_seqlens, seq_slot, seq_start, block_table,
+                                                max_blocks, n_heads, n_kv_heads, head_dim,
+                                                SCORED ? scale : scale * 1.4426950408889634f, range, opt);
+  return launch_status();
+}
+
 template <int HD_MAX, bool SCORED>
 int launch_prefill_of(__nv_bfloat16* out, const __nv_bfloat16* q, const __nv_bfloat16* k_pool, const __nv_bfloat16* v_pool,
                    const int* cu_seqlens, const int* seq_slot, const int* seq_start, const int* block_table,
                    int max_blocks, int n_seqs, int max_new, int n_heads, int n_kv_heads, int head_dim, float scale,
                    const KeyRange& range, const ScoreOptions& opt, cudaStream_t stream) {
-  const int smem = 4 * XRT_BLOCK_TOKENS * (head_dim * 2 + 16);
-  auto kernel = attention_prefill_kernel<HD_MAX, SCORED>;
-  static int smem_allowed = 0;
-  if (smem > 48 * 1024 && smem > smem_allowed) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (err != cudaSuccess) return (int)err;
-    smem_allowed = smem;
+  // two heads a block for the wide rows, unless blocks of one head leave multiprocessors empty (each holds one of them)
+  const bool two = HD_MAX > 128 && n_heads / n_kv_heads % 2 == 0 &&
+                   (long long)n_heads * n_seqs * ((max_new + PRE_ROWS - 1) / PRE_ROWS) > multiprocessors();
+  if constexpr (HD_MAX > 128) {
+    if (two)
+      return launch_prefill_heads<HD_MAX, SCORED, 2>(out, q, k_pool, v_pool, cu_seqlens, seq_slot, seq_start, block_table, max_blocks,
+                                                     n_seqs, max_new, n_heads, n_kv_heads, head_dim, scale, range, opt, stream);
   }
-  dim3 grid(n_heads, n_seqs, (max_new + PRE_ROWS - 1) / PRE_ROWS);
-  kernel<<<grid, PRE_WARPS * 32, smem, stream>>>(out, q, k_pool, v_pool, cu_seqlens, seq_slot, seq_start, block_table,
-                                                max_blocks, n_heads, n_kv_heads, head_dim,
-                                                SCORED ? scale : scale * 1.4426950408889634f, range, opt);
-  return launch_status();
+  return launch_prefill_heads<HD_MAX, SCORED, 1>(out, q, k_pool, v_pool, cu_seqlens, seq_slot, seq_start, block_table, max_blocks,
+                                                 n_seqs, max_new, n_heads, n_kv_heads, head_dim, scale, range, opt, stream);
 }
 
 template <int HD_MAX>
