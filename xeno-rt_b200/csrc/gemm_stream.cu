@@ -300,6 +300,10 @@ int launch_stream(void* out, const void* x, const void* w, int M, int N, int K, 
                   const NormEmit& emit, const RowScale& scale, cudaStream_t stream) {
   // more than 32 batch rows: two row groups a block halve the X traffic per weight byte
   constexpr int RG = M_TILES >= 4 ? 2 : 1;
+  // No more than two blocks a multiprocessor: they are the only ones to keep bytes in flight, so their rings are deep (eight stages,
+  // 70 KB a block; the same sums).  With four, N 2,048 / K 8,192 at one row took 14 us of a decode step, with eight 11 to 12.
+  if (MODE != 2 && M_TILES == 1 && K > 4 * GS_SLAB && (N + GS_ROWS - 1) / GS_ROWS <= stream_sm_count() * 2)
+    return launch_stream_staged<M_TILES, MODE, 8, 1, TO>(out, x, w, M, N, K, ldx, ldo, up_offset, emit, scale, stream);
   // products that add into the residual stream (long K, few blocks a multiprocessor): four stages
   if (MODE == 1 && M_TILES == 1) {
     if (stream_row_groups_accumulate(N) == 2)
