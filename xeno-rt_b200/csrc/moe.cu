@@ -96,9 +96,54 @@ __global__ void moe_route_scores_kernel(int* __restrict__ ids, float* __restrict
       if (e < n_experts) z[i] += opt.correction[e];
     }
   }
+  const int size = n_experts / groups;
+  if (PER_LANE == 1 && (keep == groups || (opt.group_best == 1 && (size & (size - 1)) == 0))) {
+    // One score a lane and every score a number: a lane counts who comes before it.  The shuffles don't wait for one another, as
+    // the searches one choice at a time below do (4 tokens, 16 experts in 4 groups: 5.0 us of a decode step -> 1.7).
+    const bool in = lane < n_experts;
+    if (__all_sync(0xffffffffu, !in || fabsf(z[0]) < INFINITY)) {
+      const float own = in ? z[0] : -INFINITY;
+      bool allowed = in;
+      if (keep < groups) {
+        float worth = own;
+        for (int o = 1; o < size; o <<= 1) worth = fmaxf(worth, __shfl_xor_sync(0xffffffffu, worth, o));
+        const int group = lane / size;
+        int before = 0;
+#pragma unroll 4
+        for (int g = 0; g < groups; ++g) {
+          const float other = __shfl_sync(0xffffffffu, worth, g * size);
+          before += other > worth || (other == worth && g < group);
+        }
+        allowed = in && before < keep;
+      }
+      const float choice = allowed ? own : -INFINITY;
+      int rank = 0;
+#pragma unroll 8
+      for (int e = 0; e < n_experts; ++e) {
+        const float other = __shfl_sync(0xffffffffu, choice, e);
+        rank += other > choice || (other == choice && e < lane);
+      }
+      const bool chosen = allowed && rank < top;
+      float weight = chosen ? score[0] : 0.f;
+      if (opt.normalize) {  // the sum in the order of the choices
+        float sum = 0.f;
+        for (int c = 0; c < top; ++c) {
+          const unsigned who = __ballot_sync(0xffffffffu, chosen && rank == c);
+          sum += __shfl_sync(0xffffffffu, weight, __ffs(who) - 1);
+        }
+        weight *= opt.scale / (sum + opt.sum_eps);
+      } else if (opt.scale != 1.f) {
+        weight *= opt.scale;
+      }
+      if (chosen) {
+        ids[(size_t)t * top + rank] = lane;
+        weights[(size_t)t * top + rank] = weight;
+      }
+      return;
+    }
+  }
   if (keep < groups) {
     float* best_of = group_best + (size_t)warp * groups;
-    const int size = n_experts / groups;
     for (int g = 0; g < groups; ++g) {
       // the sum of the group's `group_best` largest choice scores (one: the largest), taken one at a time
       float worth = 0.f;
