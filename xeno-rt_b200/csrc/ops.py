@@ -31,7 +31,7 @@ _SIGNATURES = {
     "xrt_layernorm": [_P, _P, _P, _P, _I, _I, _F, _I, _I, _P],
     "xrt_swiglu": [_P, _P, _I, _I, _I, _I, _I, _P, _P],
     "xrt_rotation_table": [_P, _P, _P, _P, _F, _I, _I, _P],
-    "xrt_state_scan": [_P, _P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
+    "xrt_state_scan": [_P, _P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P],
     "xrt_head_scan": [_P, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _I, _P, _P],
     "xrt_stream_add": [_P, _P, ctypes.c_longlong, _I, _P, _P, _P, _P, _F, _F, _P, _P, _F, _I, _I, _I, _I, _P],
     "xrt_removal_gates": [_P, _I, _P, _P, _I, _P, _P, _I, _P, _I, _I, _I, _I, _F, _F, _P],
@@ -39,8 +39,8 @@ _SIGNATURES = {
     "xrt_add_row": [_P, _P, _I, _I, _I, _P],
     "xrt_act_cast": [_P, _P, _I, _I, _I, _I, _I, _P],
     "xrt_add_scaled_parts": [_P, _P, _P, ctypes.c_longlong, _I, _P],
-    "xrt_short_conv": [_P, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "xrt_ssd_scan": [_P, _P, _I, _P, _P, _I, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
+    "xrt_short_conv": [_P, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
+    "xrt_ssd_scan": [_P, _P, _I, _P, _P, _I, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "xrt_gated_group_norm": [_P, _P, _P, _I, _P, _I, _I, _I, _F, _I, _P],
     "xrt_moe_route": [_P, _P, _P, _P, _I, _I, _I, _P],
     "xrt_moe_experts": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _F, _F, _I, _I, _I, _P],
@@ -910,7 +910,8 @@ def rotation_table(cos_sin, positions, freq, magnitude: float = 1.0, freq_lo=Non
 
 
 def state_scan(out, q, k, v, decay, beta, state, cu_seqlens, seq_slot, n_heads: int, n_qk_heads: int, dim: int,
-               vdim: int, q_scale: float = 1.0, delta: bool = False, max_new: int = 0, unit=None, removal=None) -> None:
+               vdim: int, q_scale: float = 1.0, delta: bool = False, max_new: int = 0, unit=None, removal=None,
+               zero_padding: bool = False) -> None:
     """The scan of a matrix state over the step's tokens, a sequence after the other in parallel:
     S <- diag(decay_t) S + k_t u_t^T and out_t = S^T (q_t * q_scale), with u_t = v_t, or with ``delta``
     u_t = sigmoid(beta_t) (v_t - S^T k_t) taken after the decay.  q, k [T, n_qk_heads * dim], v [T, n_heads * vdim],
@@ -919,7 +920,8 @@ def state_scan(out, q, k, v, decay, beta, state, cu_seqlens, seq_slot, n_heads: 
     ``max_new`` (0: not known): the most tokens a sequence brings, from which the kernel sizes its tiles.
     With ``unit`` and ``removal`` (float32 rows of n_heads * dim, n_t and e_t) the state instead loses what it answers
     along n_t: S <- diag(decay_t) S - e_t (n_t^T S) + k_t v_t^T, both corrections from the state as the token found
-    it, and out_t = S^T q_t (no ``delta`` then)."""
+    it, and out_t = S^T q_t (no ``delta`` then).  ``zero_padding``: in a step of single tokens (``max_new`` 1) whose ``out`` has a
+    row for every sequence, the rows beyond the step's tokens are cleared (else rows of no sequence are left alone)."""
     if (unit is None) != (removal is None) or (unit is not None and delta):
         raise KernelError("state_scan: unit and removal come together, and without the delta rule")
     n = out.shape[0]
@@ -946,7 +948,7 @@ def state_scan(out, q, k, v, decay, beta, state, cu_seqlens, seq_slot, n_heads: 
                                     _ptr(cu_seqlens, "cu_seqlens", torch.int32), _ptr(seq_slot, "seq_slot", torch.int32),
                                     n_seqs, n_heads, n_qk_heads, dim, vdim, float(q_scale),
                                     2 if unit is not None else (1 if delta else 0), int(max_new),
-                                    _stream()),
+                                    _clears_padding(zero_padding, out, n_seqs), _stream()),
            "state_scan")
 
 
@@ -1025,12 +1027,20 @@ def stream_add(residual, y, factor: float = 1.0, rows=None, row_scales=None, sca
         _code(then_out.dtype if then is not None else torch.float32), _stream()), "stream_add")
 
 
-def short_conv(out, x, weight, state, cu_seqlens, seq_slot, max_new: int, act: str = "silu", bias=None, in_bias=None) -> None:
+def _clears_padding(asked: bool, out, n_seqs: int) -> int:
+    if asked and out.shape[0] < n_seqs:
+        raise KernelError("zero_padding needs a row of the output for every sequence")
+    return int(asked)
+
+
+def short_conv(out, x, weight, state, cu_seqlens, seq_slot, max_new: int, act: str = "silu", bias=None, in_bias=None,
+               zero_padding: bool = False) -> None:
     """out[t, c] = act(bias[c] + sum_j weight[c, j] * x[t - (taps - 1) + j, c]) inside each sequence (no bias: 0); inputs before the
     step come from ``state`` [slots, taps - 1, channels] (zeros at a sequence's start), which is left holding
     the sequence's last taps - 1 inputs.  x: float32 rows of at least ``channels`` columns; all float32.
     ``in_bias`` (float32 [channels]): every input inside a sequence is x + in_bias (the bias of the product that gave
-    x, added here); the state holds such sums, and what stands before a sequence's start stays zero."""
+    x, added here); the state holds such sums, and what stands before a sequence's start stays zero.  ``zero_padding``: as in
+    ``state_scan`` (with more than one tap)."""
     n, channels = out.shape
     taps = weight.shape[1]
     if weight.shape[0] != channels or x.shape[0] != n or out.dtype != torch.float32:
@@ -1045,7 +1055,8 @@ def short_conv(out, x, weight, state, cu_seqlens, seq_slot, max_new: int, act: s
                                     _ptr(bias, "bias", torch.float32), _ptr(in_bias, "in_bias", torch.float32),
                                     _ptr(state if taps > 1 else None, "state", torch.float32),
                                     _ptr(cu_seqlens, "cu_seqlens", torch.int32), _ptr(seq_slot, "seq_slot", torch.int32),
-                                    n_seqs, int(max_new), channels, taps, _ACTS[act], _stream()), "short_conv")
+                                    n_seqs, int(max_new), channels, taps, _ACTS[act],
+                                    _clears_padding(zero_padding, out, n_seqs), _stream()), "short_conv")
     if taps > 1 and int(max_new) != 1:  # longer portions leave the state in a second launch
         add_launches(1)
 
@@ -1125,10 +1136,11 @@ def scale_softcap(x, scale: float, cap: float | None) -> None:
 # The scalar-decay state-space scan and its group norm (csrc/ssd.cu), routed experts (csrc/moe.cu), and the small
 # steps of layers that norm a sublayer's result before adding it
 def ssd_scan(out, x, b, c, dt, dt_bias, a_log, d_skip, state, cu_seqlens, seq_slot, n_heads: int, n_groups: int,
-             n_state: int, vdim: int, max_new: int = 0) -> None:
+             n_state: int, vdim: int, max_new: int = 0, zero_padding: bool = False) -> None:
     """S <- exp(-exp(a_log) dt) S + dt b x^T, out = S^T c + d_skip x per head, dt = softplus(raw + dt_bias); x rows of
     heads * vdim, b and c rows of groups * n_state (one stride), dt rows of one raw step a head (all float32, rows may
-    be slices of wider rows); ``state`` float32 [slots, heads, vdim, n_state] is read and left as the last state."""
+    be slices of wider rows); ``state`` float32 [slots, heads, vdim, n_state] is read and left as the last state.  ``zero_padding``: as in
+    ``state_scan``."""
     n = out.shape[0]
     if out.shape != (n, n_heads * vdim) or out.dtype != torch.float32 or not out.is_contiguous():
         raise KernelError("ssd_scan: out must be float32 [T, heads * vdim]")
@@ -1149,7 +1161,8 @@ def ssd_scan(out, x, b, c, dt, dt_bias, a_log, d_skip, state, cu_seqlens, seq_sl
     _check(_kernels().xrt_ssd_scan(_ptr(out, "out"), xp, xs, bp, cp, bs, dp, ds, _ptr(dt_bias, "dt_bias"),
                                   _ptr(a_log, "a_log"), _ptr(d_skip, "d_skip"), _ptr(state, "state"),
                                   _ptr(cu_seqlens, "cu_seqlens", torch.int32), _ptr(seq_slot, "seq_slot", torch.int32),
-                                  n_seqs, n_heads, n_groups, n_state, vdim, int(max_new), _stream()), "ssd_scan")
+                                  n_seqs, n_heads, n_groups, n_state, vdim, int(max_new),
+                                  _clears_padding(zero_padding, out, n_seqs), _stream()), "ssd_scan")
 
 
 def gated_group_norm(out, y, z, weight, groups: int, eps: float) -> None:

@@ -44,7 +44,18 @@ struct ScanArgs {
   int n_heads, heads_per_qk, dim, vdim;
   float q_scale;
   int parts, cols, tile_tokens, stage_floats;
+  int zero_padding;  // rows beyond the step's tokens, one a sequence that brings none, are cleared
 };
+
+// What a block of a scan does for a sequence without tokens: a captured step of single tokens has a row for each of its padding
+// sequences, which the products after it read.  (A fill of the whole buffer ahead of the kernel took 1.4 us and kept it from
+// starting early.)
+template <typename Args>
+__device__ __forceinline__ void clear_padding(const Args& a, int s, int h, int col0, int cols) {
+  if (!a.zero_padding || s < a.cu_seqlens[gridDim.x]) return;
+  for (int c = col0 + threadIdx.x; c < min(col0 + cols, a.vdim); c += blockDim.x)
+    a.out[((size_t)s * a.n_heads + h) * a.vdim + c] = 0.f;
+}
 
 // VEC: 16-byte copies (dim, vdim, cols and every row stride are multiples of 4 floats, every base 16-byte aligned).
 // C2: value columns a lane holds (C2 * R state registers): what a lane reads of q, k and a serves C2 columns, and
@@ -67,7 +78,7 @@ __global__ void __launch_bounds__(128) state_scan_kernel(const ScanArgs a) {
   const int s = blockIdx.x, h = blockIdx.y;
   const int slot = a.seq_slot[s];
   const int begin = a.cu_seqlens[s], end = a.cu_seqlens[s + 1];
-  if (slot < 0 || end <= begin) return;
+  if (slot < 0 || end <= begin) return clear_padding(a, s, h, blockIdx.z * cols, cols);
   const int part = threadIdx.x % parts, jl = (threadIdx.x / parts) * C2;  // the lane's first column in the block
   const int col0 = blockIdx.z * cols;
   const int j = col0 + jl;
@@ -321,7 +332,7 @@ __global__ void __launch_bounds__(SPREAD_THREADS) state_scan_spread_kernel(const
   const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * COLS;
   const int slot = a.seq_slot[s];
   const int begin = a.cu_seqlens[s], end = a.cu_seqlens[s + 1];
-  if (slot < 0 || end <= begin) return;
+  if (slot < 0 || end <= begin) return clear_padding(a, s, h, col0, COLS);
   const int j = col0 + jl, qh = h / a.heads_per_qk;
 
   auto issue = [&](int t0, int stage) {
@@ -609,13 +620,17 @@ __global__ void short_conv_single_kernel(float* __restrict__ out, const float* _
                                          const float* __restrict__ w, const float* __restrict__ bias,
                                          const float* __restrict__ in_bias, float* __restrict__ state,
                                          const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot,
-                                         int channels, int taps, int act) {
+                                         int channels, int taps, int act, int zero_padding) {
   pdl_trigger();
   pdl_wait(x, w, bias, in_bias, cu_seqlens, seq_slot);
   const int s = blockIdx.x;
   const int slot = seq_slot[s];
   const int begin = cu_seqlens[s], len = cu_seqlens[s + 1] - begin;
-  if (slot < 0 || len <= 0) return;
+  if (slot < 0 || len <= 0) {  // (see clear_padding)
+    if (zero_padding && s >= cu_seqlens[gridDim.x])
+      for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < channels; c += gridDim.y * blockDim.x) out[(size_t)s * channels + c] = 0.f;
+    return;
+  }
   const int keep = taps - 1;
   float* st = state + (size_t)slot * keep * channels;
   for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < channels; c += gridDim.y * blockDim.x) {
@@ -696,25 +711,42 @@ __global__ void removal_gates_kernel(float* __restrict__ decay, int decay_stride
   }
 }
 
-// One warp a (token, head): y = o / sqrt(mean(o^2) + eps) * w * act(gate).
-template <typename TO>
-__global__ void head_norm_gate_kernel(TO* __restrict__ y, const float* __restrict__ o, const float* __restrict__ w,
-                                      const float* __restrict__ gate, int gate_stride, int n_tokens, int n_heads,
-                                      int vdim, float eps, int act, int w_per_head) {
+// One warp a (token, head): y = o / sqrt(mean(o^2) + eps) * w * act(gate).  PER numbers a lane, all asked for at once (the
+// weights before the wait): reading the row twice, a few numbers at a time, was 4 to 5 us of a decode step for one token; this is 1.6 to 2.0.
+template <typename TO, int PER>
+__global__ void __launch_bounds__(256)
+head_norm_gate_kernel(TO* __restrict__ y, const float* __restrict__ o, const float* __restrict__ w,
+                      const float* __restrict__ gate, int gate_stride, int n_tokens, int n_heads,
+                      int vdim, float eps, int act, int w_per_head) {
   pdl_trigger();
-  pdl_wait(o, w, gate);
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= n_tokens * n_heads) return;
+  const bool live = warp < n_tokens * n_heads;
   const int t = warp / n_heads, head = warp - t * n_heads;
+  const float* wh = w + (w_per_head ? head * vdim : 0);  // one weight a column of all heads, or one shared by the heads
+  float wv[PER], ov[PER], gv[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) wv[i] = live && lane + 32 * i < vdim ? wh[lane + 32 * i] : 0.f;
+  pdl_wait(o, w, gate);
+  if (!live) return;
   const float* p = o + ((size_t)t * n_heads + head) * vdim;
   const float* g = gate + (size_t)t * gate_stride + head * vdim;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int d = lane + 32 * i;
+    ov[i] = d < vdim ? p[d] : 0.f;
+    gv[i] = d < vdim ? g[d] : 0.f;
+  }
   float sum = 0.f;
-  for (int d = lane; d < vdim; d += 32) sum = fmaf(p[d], p[d], sum);
+#pragma unroll
+  for (int i = 0; i < PER; ++i) sum = fmaf(ov[i], ov[i], sum);
   sum = warp_sum(sum);
   const float inv = 1.0f / sqrtf(sum / (float)vdim + eps);
   TO* dst = y + ((size_t)t * n_heads + head) * vdim;
-  const float* wh = w + (w_per_head ? head * vdim : 0);  // one weight a column of all heads, or one shared by the heads
-  for (int d = lane; d < vdim; d += 32) dst[d] = from_float<TO>((p[d] * inv) * wh[d] * activate(g[d], act));
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int d = lane + 32 * i;
+    if (d < vdim) dst[d] = from_float<TO>((ov[i] * inv) * wv[i] * activate(gv[i], act));
+  }
 }
 
 // The same with a block of 256 threads a (token, head), for heads as wide as a model; PER columns a thread are asked for
@@ -914,7 +946,7 @@ XRT_EXPORT int xrt_state_scan(float* out, const float* q, int q_stride, const fl
                               const float* unit, int unit_stride, const float* removal, int removal_stride,
                               float* state, const int* cu_seqlens, const int* seq_slot, int n_seqs, int n_heads,
                               int n_qk_heads, int dim, int vdim, float q_scale, int mode, int max_new,
-                              cudaStream_t stream) {
+                              int zero_padding, cudaStream_t stream) {
   const bool delta = mode == 1;
   if (mode < 0 || mode > 2 || (mode == 2 && (unit == nullptr || removal == nullptr))) return XRT_ERR_ARGUMENT;
   if (max_new < 1) max_new = 1 << 30;
@@ -948,7 +980,7 @@ XRT_EXPORT int xrt_state_scan(float* out, const float* q, int q_stride, const fl
   xrt::ScanArgs a = {out, q, k, v, decay, beta, unit, removal, unit_stride, removal_stride,
                      q_stride, k_stride, v_stride, decay_stride, beta_stride, state,
                      cu_seqlens, seq_slot, n_heads, n_heads / n_qk_heads, dim, vdim, q_scale, parts, cols, tile_tokens,
-                     stage_floats(tile_tokens)};
+                     stage_floats(tile_tokens), zero_padding != 0 && max_new == 1};
   if (mode != 2 && (dim == 128 || dim == 64)) {
     bool taken = false;
     const int status = dim == 128 ? (delta ? xrt::state_scan_spread<8, 16, true>(a, n_seqs, max_new, taken, stream)
@@ -983,7 +1015,7 @@ XRT_EXPORT int xrt_state_scan(float* out, const float* q, int q_stride, const fl
 
 XRT_EXPORT int xrt_short_conv(float* out, const float* x, int x_stride, const float* w, const float* bias,
                               const float* in_bias, float* state, const int* cu_seqlens, const int* seq_slot, int n_seqs, int max_new, int channels,
-                              int taps, int act, cudaStream_t stream) {
+                              int taps, int act, int zero_padding, cudaStream_t stream) {
   if (n_seqs < 0 || channels <= 0 || taps < 1 || max_new < 0) return XRT_ERR_ARGUMENT;
   if (taps > 9 || n_seqs > 65535) return XRT_ERR_UNSUPPORTED;
   if (n_seqs == 0 || max_new == 0) return XRT_OK;
@@ -993,7 +1025,7 @@ XRT_EXPORT int xrt_short_conv(float* out, const float* x, int x_stride, const fl
   if (max_new == 1 && taps > 1) {  // single tokens: one launch
     xrt::launch_kernel(xrt::short_conv_single_kernel<8>, dim3(n_seqs, channel_blocks < 65535 ? channel_blocks : 65535),
                        dim3(threads), 0, stream, out, x, x_stride, w, bias, in_bias, state, cu_seqlens, seq_slot, channels,
-                       taps, act);
+                       taps, act, zero_padding);
     return xrt::launch_status();
   }
   const dim3 grid(n_seqs, (max_new + tile_tokens - 1) / tile_tokens, channel_blocks < 65535 ? channel_blocks : 65535);
@@ -1063,8 +1095,12 @@ XRT_EXPORT int xrt_head_norm_gate(void* y, const float* o, const float* w, const
   }
   const size_t warps = (size_t)n_tokens * n_heads;
   XRT_DISPATCH_DTYPE(out_dtype, TO, {
-    xrt::launch_kernel(xrt::head_norm_gate_kernel<TO>, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, stream, (TO*)y, o,
-                       w, gate, gate_stride, n_tokens, n_heads, vdim, eps, act, w_per_head);
+    auto kernel = vdim <= 64    ? xrt::head_norm_gate_kernel<TO, 2>
+                  : vdim <= 128 ? xrt::head_norm_gate_kernel<TO, 4>
+                  : vdim <= 256 ? xrt::head_norm_gate_kernel<TO, 8>
+                                : xrt::head_norm_gate_kernel<TO, 16>;
+    xrt::launch_kernel(kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, stream, (TO*)y, o, w, gate, gate_stride, n_tokens,
+                       n_heads, vdim, eps, act, w_per_head);
   });
   return xrt::launch_status();
 }

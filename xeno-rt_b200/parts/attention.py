@@ -313,8 +313,9 @@ class GroupedQueryAttention:
         pairing = getattr(self.position, "pairing", "split_half")
         cos_sin = self.position.tables(ctx)
         # padding rows belong to no sequence: kernels that walk sequences leave them unwritten
-        # a captured step is replayed with padding rows, which the kernel of the scored layers leaves unwritten
-        padded = (getattr(ctx, "captured", False) and not self.plain_scores) or sum(ctx.new_lens) < ctx.n_tokens
+        # (a captured step's padding rows too: the kernels of single tokens in bfloat16 clear them, the others may not)
+        clears = self.dtype is DType.BF16 and ctx.all_single and self.n_heads // self.n_kv_heads <= 16
+        padded = (getattr(ctx, "captured", False) and not self.plain_scores and not clears) or sum(ctx.new_lens) < ctx.n_tokens
         attended = (torch.zeros if padded else torch.empty)((n, self.q_width), dtype=self.act_dtype, device=h.device)
         if self.dtype is DType.BF16 and self.plain_heads and self.plain_scores:
             from . import attention_bf16
@@ -337,7 +338,7 @@ class GroupedQueryAttention:
                     if v_first is not None and v_first.shape[1] != self.n_kv_heads * self.true_vdim:
                         raise ConfigError("layers that blend their values must have the same kv heads and value size")
                     if v_first is None:  # the first layer of this name in the step: its values are the ones blended in
-                        v_keep = torch.zeros((n, self.n_kv_heads * self.true_vdim), dtype=torch.float32, device=h.device)
+                        v_keep = torch.empty((n, self.n_kv_heads * self.true_vdim), dtype=torch.float32, device=h.device)
                         ctx.shared[("value_blend", self.value_blend)] = v_keep
                 ops.qkv_heads_write(q, store.k, store.v, qkv, self.q_width, self.v_offset, bias,
                                     self.unit_norm, self.true_dim, self.eps, ctx.tok_slot, ctx.tok_pos, store.block_table,

@@ -70,14 +70,15 @@ class ScalarDecayStateSpace(_StateMixer):
         self._owning(owns_cache)
         n, inner, gn = h.shape[0], self.inner, self.gn
         p = linear(h, self.w_in, out_dtype=torch.float32)   # z | x | B | C | dt
-        xbc = self._rows(ctx)((n, self.channels), dtype=torch.float32, device=h.device)
+        clears = self._clears(ctx)
+        xbc = (self._rows_of if self.taps > 1 else self._rows)(ctx)((n, self.channels), dtype=torch.float32, device=h.device)
         conv_state = store[1].state if self.taps > 1 else None
         ops.short_conv(xbc, p[:, inner:], self.conv, conv_state, ctx.cu_seqlens, ctx.seq_slot, ctx.max_new, "silu",
-                       bias=self.conv_bias)
-        y = self._rows(ctx)((n, inner), dtype=torch.float32, device=h.device)
+                       bias=self.conv_bias, zero_padding=clears and self.taps > 1)
+        y = self._rows_of(ctx)((n, inner), dtype=torch.float32, device=h.device)
         ops.ssd_scan(y, xbc, xbc[:, inner:], xbc[:, inner + gn:], p[:, inner + self.channels:], self.dt_bias, self.a_log,
                      self.d_skip, store[0].state, ctx.cu_seqlens, ctx.seq_slot, self.n_heads, self.n_groups, self.state,
-                     self.value_dim, max_new=ctx.max_new)
+                     self.value_dim, max_new=ctx.max_new, zero_padding=clears)
         out = torch.empty((n, inner), dtype=self.act_dtype, device=h.device)
         ops.gated_group_norm(out, y, p, self.norm, self.norm_groups, self.eps)
         return out

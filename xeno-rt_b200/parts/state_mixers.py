@@ -49,6 +49,16 @@ class _StateMixer:
         return torch.zeros if padded else torch.empty
 
     @staticmethod
+    def _clears(ctx) -> bool:
+        """Whether the kernels that take ``zero_padding`` clear those rows themselves: the padding rows of a captured step, one a
+        sequence that brings no token."""
+        return bool(getattr(ctx, "captured", False)) and ctx.max_new == 1 and ctx.n_tokens == ctx.seq_slot.numel()
+
+    def _rows_of(self, ctx):
+        """``_rows`` for a buffer that such a kernel fills."""
+        return torch.empty if self._clears(ctx) else self._rows(ctx)
+
+    @staticmethod
     def _owning(owns_cache):
         if not owns_cache:
             raise ConfigError("a mixer with a state cannot read another place's: the state is what the tokens left there")
@@ -95,9 +105,9 @@ class GatedLinearAttention(_StateMixer):
         p = linear(h, self.w_in, out_dtype=torch.float32)
         decay = linear(linear(h, self.w_a1, out_dtype=self.act_dtype), self.w_a2, out_dtype=torch.float32)
         ops.decay_from_gate(decay, self.a2_bias, nh, kd, self.tau)
-        o = self._rows(ctx)((n, nh * vd), dtype=torch.float32, device=h.device)
+        o = self._rows_of(ctx)((n, nh * vd), dtype=torch.float32, device=h.device)
         ops.state_scan(o, p, p[:, nh * kd:], p[:, 2 * nh * kd:], decay, None, store.state, ctx.cu_seqlens, ctx.seq_slot,
-                       nh, nh, kd, vd, q_scale=kd ** -0.5, max_new=ctx.max_new)
+                       nh, nh, kd, vd, q_scale=kd ** -0.5, max_new=ctx.max_new, zero_padding=self._clears(ctx))
         y = torch.empty((n, nh * vd), dtype=self.act_dtype, device=h.device)
         ops.head_norm_gate(y, o, self.norm, p[:, 2 * nh * kd + nh * vd:], nh, vd, self.eps, "silu")
         return y
@@ -198,13 +208,15 @@ class GatedDeltaRule(_StateMixer):
         decay = linear(low[:, :self.decay_rank], self.w_a2, out_dtype=torch.float32)
         gate = linear(low[:, self.decay_rank:], self.w_g2, out_dtype=torch.float32)
         ops.decay_from_step(decay, self.dt_bias, self.a_log, nh, kd)
-        qkv = self._rows(ctx)((n, self.channels), dtype=torch.float32, device=h.device)
+        qkv = (self._rows_of if self.taps > 1 else self._rows)(ctx)((n, self.channels), dtype=torch.float32, device=h.device)
         conv_state = store[1].state if self.taps > 1 else None
-        ops.short_conv(qkv, p, self.conv, conv_state, ctx.cu_seqlens, ctx.seq_slot, ctx.max_new, "silu")
+        clears = self._clears(ctx)
+        ops.short_conv(qkv, p, self.conv, conv_state, ctx.cu_seqlens, ctx.seq_slot, ctx.max_new, "silu",
+                       zero_padding=clears and self.taps > 1)
         ops.unit_heads(qkv, 2 * nq, kd, self.UNIT_EPS, scaled_heads=nq, scale=kd ** -0.5)
-        o = self._rows(ctx)((n, nh * vd), dtype=torch.float32, device=h.device)
+        o = self._rows_of(ctx)((n, nh * vd), dtype=torch.float32, device=h.device)
         ops.state_scan(o, qkv, qkv[:, nq * kd:], qkv[:, 2 * nq * kd:], decay, p[:, self.channels:], store[0].state,
-                       ctx.cu_seqlens, ctx.seq_slot, nh, nq, kd, vd, delta=True, max_new=ctx.max_new)
+                       ctx.cu_seqlens, ctx.seq_slot, nh, nq, kd, vd, delta=True, max_new=ctx.max_new, zero_padding=clears)
         y = torch.empty((n, nh * vd), dtype=self.act_dtype, device=h.device)
         ops.head_norm_gate(y, o, self.norm, gate, nh, vd, self.eps, self.gate_act)
         return y
@@ -325,9 +337,9 @@ class DecayRemovalRule(_StateMixer):
         unit = torch.empty((n, w), dtype=torch.float32, device=h.device)
         removal = p[:, 4 * w:5 * w]
         ops.removal_gates(decay, self.w0, removal, self.a_bias, unit, p[:, w:2 * w], nh, hd, self.decay_rate, self.unit_eps)
-        o = self._rows(ctx)((n, w), dtype=torch.float32, device=h.device)
+        o = self._rows_of(ctx)((n, w), dtype=torch.float32, device=h.device)
         ops.state_scan(o, p, p[:, w:], p[:, 2 * w:], decay, None, store.state, ctx.cu_seqlens, ctx.seq_slot, nh, nh, hd, hd,
-                       max_new=ctx.max_new, unit=unit, removal=removal)
+                       max_new=ctx.max_new, unit=unit, removal=removal, zero_padding=self._clears(ctx))
         y = torch.empty((n, w), dtype=self.act_dtype, device=h.device)
         ops.head_norm_gate(y, o, self.norm, p[:, 3 * w:], nh, hd, self.eps, "sigmoid")
         return y
