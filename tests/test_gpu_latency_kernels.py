@@ -161,3 +161,40 @@ def test_padding_rows_are_cleared():
         outs.append((out, state))
     assert torch.equal(outs[0][0][:live], outs[1][0][:live]) and torch.equal(outs[0][1], outs[1][1])
     assert outs[0][0][live:].isnan().all() and (outs[1][0][live:] == 0).all()
+
+
+@pytest.mark.parametrize("width", [33, 1024, 1500, 2048, 2049, 4096])
+@pytest.mark.parametrize("top", [1, 2, 5])
+def test_norms_of_gathered_parts(width, top):
+    """The same bits as from parts written out by moe_combine; more rows than blocks run at once give what a few at a time give."""
+    from xeno_rt_b200.csrc import ops
+    n = 1000
+    y, x0 = _rand(n * top, width), _rand(n, width, seed=1)
+    rows = torch.randperm(n * top, device=DEV).to(torch.int32)
+    scales = torch.rand(n, top, device=DEV)
+    w, b, w2, b2 = (_rand(width, seed=s) for s in (2, 3, 4, 5))
+    parts = torch.empty(top, n, width, device=DEV)
+    ops.moe_combine(parts, y, rows, scales)
+    plain = parts if top > 1 else parts[0]
+    results = []
+    for form in ("parts", "gathered", "a few at a time"):
+        x, out = x0.clone(), torch.empty(n, width, dtype=torch.bfloat16, device=DEV)
+        r, copy = x0.clone(), torch.empty(n, width, dtype=torch.bfloat16, device=DEV)
+        if form == "parts":
+            ops.layernorm_affine(plain, w, b, 1e-5, out=out, residual=x, n_parts=top, then=(w2, b2))
+            ops.rmsnorm_add(r, plain, w, 1e-6, copy=copy)
+        elif form == "gathered":
+            ops.layernorm_affine(y, w, b, 1e-5, out=out, residual=x, then=(w2, b2), gather=(rows, scales))
+            ops.rmsnorm_add(r, y, w, 1e-6, copy=copy, gather=(rows, scales))
+        else:
+            for a in range(0, n, 100):
+                some = parts[:, a:a + 100].contiguous()
+                ops.layernorm_affine(some if top > 1 else some[0], w, b, 1e-5, out=out[a:a + 100], residual=x[a:a + 100],
+                                     n_parts=top, then=(w2, b2))
+            ops.rmsnorm_add(r, plain, w, 1e-6, copy=copy)
+        results.append((x, out, r, copy))
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))
+    v = parts.double().sum(0)
+    v = (v - v.mean(-1, keepdim=True)) / torch.sqrt(v.var(-1, unbiased=False, keepdim=True) + 1e-5) * w.double() + b.double()
+    _close(results[0][0], x0.double() + v, width)

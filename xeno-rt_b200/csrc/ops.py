@@ -51,10 +51,10 @@ _SIGNATURES = {
     "xrt_moe_activation": [_P, _P, _I, _I, _F, _F, _I, _I, _P],
     "xrt_moe_combine": [_P, _P, _P, _P, _I, _I, _I, _P],
     "xrt_embedding_pair": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
-    "xrt_layernorm_affine": [_P, _P, _P, _I, ctypes.c_longlong, _P, _P, _P, _I, _I, _F, _I, _P, _P, _P],
+    "xrt_layernorm_affine": [_P, _P, _P, _I, ctypes.c_longlong, _P, _P, _P, _I, _I, _F, _I, _P, _P, _P, _P, _P],
     "xrt_qkv_heads_write": [_P, _P, _P, _P, _I, _I, _I, _P, _I, _I, _F, _P, _P, _I, _I, _I, _P, _I, _I,
                             _P, _I, _P, _I, _F, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P],
-    "xrt_rmsnorm_add": [_P, _P, ctypes.c_longlong, _I, _P, _P, _I, _I, _F, _I, _I, _P, _P, _F, _P, _P, _F, _P],
+    "xrt_rmsnorm_add": [_P, _P, ctypes.c_longlong, _I, _P, _P, _I, _I, _F, _I, _I, _P, _P, _F, _P, _P, _F, _P, _P, _P],
     "xrt_cast_rows": [_P, _P, ctypes.c_longlong, _I, _P],
     "xrt_latent_prepare": [_P, _P, _P, _I, _I, _P, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     "xrt_head_product": [_P, _I, _I, _I, _P, _I, _I, _I, _P, _I, _I, _I, _I, _I, _I, _I, _P],
@@ -1323,11 +1323,23 @@ def embedding_pair(out, table, pairs, ids, tok_slot, tok_pos, last_token, cu_seq
     add_launches(1)
 
 
-def layernorm_affine(x, weight, bias, eps: float, out=None, residual=None, rows=None, n_parts: int = 1, then=None) -> None:
+def _gathered(gather, y, n_rows: int, width: int):
+    """(parts a row, pointer of the rows, pointer of their factors) of gathered parts."""
+    rows, scales = gather
+    if (scales.dim() != 2 or scales.shape[0] != n_rows or rows.numel() != scales.numel() or y.dim() != 2 or y.shape[1] != width
+            or y.dtype != torch.float32 or scales.dtype != torch.float32):
+        raise KernelError("gathered parts: rows int32 [T * n] and factors float32 [T, n] of rows [any, width] are needed")
+    return scales.shape[1], _ptr(rows, "part rows", torch.int32), _ptr(scales, "part scales")
+
+
+def layernorm_affine(x, weight, bias, eps: float, out=None, residual=None, rows=None, n_parts: int = 1, then=None,
+                     gather=None) -> None:
     """y = (x - mean) / sqrt(variance + eps) * weight + bias over float32 rows; written to ``out`` (any dtype), or
     added into ``residual`` (float32) when that is given.  With ``residual``, ``out`` and ``then`` = (weight2, bias2)
     the new residual rows are normed once more, with those, into ``out`` (the norm the next sublayer begins with).
-    ``x`` may be [n_parts, T, width]: the parts are added in index order first.  ``rows`` gathers rows of x."""
+    ``x`` may be [n_parts, T, width]: the parts are added in index order first.  ``rows`` gathers rows of x.
+    ``gather`` = (rows int32 [T * n], factors float32 [T, n]): ``x`` is [any, width] and part p of row t is its row rows[t * n + p]
+    times factors[t, p] (widths up to 4,096)."""
     width = x.shape[-1]
     target = residual if residual is not None else out
     both = out is not None and residual is not None
@@ -1335,21 +1347,26 @@ def layernorm_affine(x, weight, bias, eps: float, out=None, residual=None, rows=
         raise KernelError("layernorm_affine: give out or residual of x's width, or both with the second norm")
     if both and (out.shape != residual.shape or rows is not None or then[0].numel() != width):
         raise KernelError("layernorm_affine: the second norm needs rows of the residual's shape")
+    gather_rows = gather_scales = 0
+    if gather is not None:
+        if rows is not None or n_parts != 1:
+            raise KernelError("layernorm_affine: gathered parts come without rows and parts of their own")
+        parts, gather_rows, gather_scales = _gathered(gather, x, target.shape[0], width)
     if x.dim() != (3 if n_parts > 1 else 2) or (n_parts > 1 and x.shape[0] != n_parts) or not x.is_contiguous():
         raise KernelError("layernorm_affine: x must be [T, width] or [parts, T, width]")
     n_rows = target.shape[0]
-    if rows is not None and rows.numel() != n_rows or rows is None and x.shape[-2] != n_rows:
+    if rows is not None and rows.numel() != n_rows or rows is None and gather is None and x.shape[-2] != n_rows:
         raise KernelError("layernorm_affine: rows do not fit")
     if weight.numel() != width or (bias is not None and bias.numel() != width):
         raise KernelError("layernorm_affine: weight and bias must be [width]")
     _check(_kernels().xrt_layernorm_affine(_ptr(out, "out"), _ptr(residual, "residual", torch.float32), _ptr(x, "x"),
-                                          int(n_parts), x.shape[-2] * width if n_parts > 1 else 0,
+                                          int(parts if gather is not None else n_parts), x.shape[-2] * width if n_parts > 1 else 0,
                                           _ptr(weight, "weight", torch.float32), _ptr(bias, "bias", torch.float32),
                                           _ptr(rows, "rows", torch.int32), n_rows, width, float(eps),
                                           _code(out.dtype) if out is not None else 0,
                                           _ptr(then[0] if then else None, "weight2", torch.float32),
-                                          _ptr(then[1] if then else None, "bias2", torch.float32), _stream()),
-           "layernorm_affine")
+                                          _ptr(then[1] if then else None, "bias2", torch.float32), gather_rows, gather_scales,
+                                          _stream()), "layernorm_affine")
 
 
 def qkv_heads_write(q_out, k_pool, v_pool, qkv, k_offset: int, v_offset: int, bias, unit_norm: bool, norm_dim: int,
@@ -1408,14 +1425,18 @@ def qkv_heads_write(q_out, k_pool, v_pool, qkv, k_offset: int, v_offset: int, bi
 
 
 def rmsnorm_add(residual, y, weight, eps: float, copy=None, factor: float = 1.0, part_scales=None, bias=None,
-                then=None) -> None:
+                then=None, gather=None) -> None:
     """residual += factor * RMSNorm(y) * weight, 32-bit; ``y`` float32 [T, width] or [parts, T, width] (added in index
     order first, part p times ``part_scales[p]`` (float32 on the device) where given, plus the row ``bias`` (float32
     [width])); ``copy`` (optional, [T, width] in the compute dtype) receives the new residual as well; ``then`` =
-    (weight2, eps2, out2): out2 [T, width] receives RMSNorm(new residual) * weight2 (weight2 of ``weight``'s dtype)."""
+    (weight2, eps2, out2): out2 [T, width] receives RMSNorm(new residual) * weight2 (weight2 of ``weight``'s dtype).
+    ``gather``: the parts are gathered from ``y`` [any, width], as for ``layernorm_affine`` (without ``part_scales``)."""
     n, width = residual.shape
     parts = y.shape[0] if y.dim() == 3 else 1
-    if tuple(y.shape[-2:]) != (n, width) or weight.numel() != width or residual.dtype != torch.float32:
+    gather_rows = gather_scales = 0
+    if gather is not None:
+        parts, gather_rows, gather_scales = _gathered(gather, y, n, width)
+    if (gather is None and tuple(y.shape[-2:]) != (n, width)) or weight.numel() != width or residual.dtype != torch.float32:
         raise KernelError("rmsnorm_add: shapes do not fit")
     if copy is not None and tuple(copy.shape) != (n, width):
         raise KernelError("rmsnorm_add: the copy does not fit")
@@ -1434,7 +1455,7 @@ def rmsnorm_add(residual, y, weight, eps: float, copy=None, factor: float = 1.0,
                                      _code(side.dtype if side is not None else torch.float32),
                                      _ptr(part_scales, "part_scales", torch.float32), _ptr(bias, "bias", torch.float32),
                                      float(factor), _ptr(then_w, "then weight"), _ptr(then_out, "then out"),
-                                     float(then_eps), _stream()), "rmsnorm_add")
+                                     float(then_eps), gather_rows, gather_scales, _stream()), "rmsnorm_add")
 
 
 def cast_rows(out, x) -> None:

@@ -21,10 +21,15 @@ struct PostNormExtras {
   const void* then_w = nullptr;        // [width] in the first weight's dtype: a second norm over the new row ...
   void* then_out = nullptr;            // ... written here in the copy's dtype
   float then_eps = 0.f;
+  // the parts are gathered: part p of token t is row rows[t * n_parts + p] of y, times row_scales[t * n_parts + p] (the experts'
+  // results where they lie, sorted by expert; each product is rounded before it is added)
+  const int* rows = nullptr;
+  const float* row_scales = nullptr;
 };
 
-template <typename TW, typename TC, int PER>
-__global__ void rmsnorm_add_kernel(float* __restrict__ residual, const float* __restrict__ y, size_t part_stride,
+// GATHER: the parts are gathered (PostNormExtras::rows).
+template <typename TW, typename TC, int PER, bool GATHER>
+__global__ void __launch_bounds__(512) rmsnorm_add_kernel(float* __restrict__ residual, const float* __restrict__ y, size_t part_stride,
                                    int n_parts, const TW* __restrict__ w, TC* __restrict__ copy, int width, float eps,
                                    const PostNormExtras ex) {
   __shared__ float scratch[33];
@@ -36,7 +41,7 @@ __global__ void rmsnorm_add_kernel(float* __restrict__ residual, const float* __
     wv[i] = c < width ? to_float(w[c]) : 0.f;
   }
   pdl_wait(y, w);
-  const float* p = y + (size_t)blockIdx.x * width;
+  const float* p = y + (size_t)(GATHER ? ex.rows[(size_t)blockIdx.x * n_parts] : (int)blockIdx.x) * width;
   float* r = residual + (size_t)blockIdx.x * width;
   float sum = 0.f;
 #pragma unroll
@@ -49,6 +54,21 @@ __global__ void rmsnorm_add_kernel(float* __restrict__ residual, const float* __
     const float s0 = ex.part_scales[0];
 #pragma unroll
     for (int i = 0; i < PER; ++i) yv[i] *= s0;
+  }
+  if (GATHER) {
+    const float s0 = ex.row_scales[(size_t)blockIdx.x * n_parts];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) yv[i] = __fmul_rn(yv[i], s0);
+    for (int part = 1; part < n_parts; ++part) {
+      const float sp = ex.row_scales[(size_t)blockIdx.x * n_parts + part];
+      const float* q = y + (size_t)ex.rows[(size_t)blockIdx.x * n_parts + part] * width;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        if (c < width) yv[i] = __fadd_rn(yv[i], __fmul_rn(q[c], sp));
+      }
+    }
+    n_parts = 1;
   }
   for (int part = 1; part < n_parts; ++part) {
     const float sp = ex.part_scales != nullptr ? ex.part_scales[part] : 1.0f;
@@ -108,7 +128,8 @@ __global__ void cast_rows_kernel(TC* __restrict__ out, const float* __restrict__
 XRT_EXPORT int xrt_rmsnorm_add(float* residual, const float* y, long long part_stride, int n_parts, const void* weight,
                                void* copy, int n_tokens, int width, float eps, int weight_dtype, int copy_dtype,
                                const float* part_scales, const float* bias, float factor, const void* then_weight,
-                               void* then_out, float then_eps, cudaStream_t stream) {
+                               void* then_out, float then_eps, const int* rows, const float* row_scales,
+                               cudaStream_t stream) {
   if (n_tokens < 0 || width <= 0 || n_parts <= 0) return XRT_ERR_ARGUMENT;
   if ((then_weight == nullptr) != (then_out == nullptr)) return XRT_ERR_ARGUMENT;
   xrt::PostNormExtras ex;
@@ -118,12 +139,15 @@ XRT_EXPORT int xrt_rmsnorm_add(float* residual, const float* y, long long part_s
   ex.then_w = then_weight;
   ex.then_out = then_out;
   ex.then_eps = then_eps;
+  if ((rows == nullptr) != (row_scales == nullptr) || (rows != nullptr && part_scales != nullptr)) return XRT_ERR_ARGUMENT;
+  ex.rows = rows;
+  ex.row_scales = row_scales;
   if (n_tokens == 0) return XRT_OK;
   const int threads = width >= 4096 ? 512 : (width >= 1024 ? 256 : (width >= 256 ? 128 : 64));
   const int per = (width + threads - 1) / threads;
   if (per > 32) return XRT_ERR_UNSUPPORTED;
 #define XRT_POST(PER)                                                                                                   \
-  xrt::launch_kernel(xrt::rmsnorm_add_kernel<TW, TC, PER>, dim3(n_tokens), dim3(threads), 0, stream, residual, y,       \
+  xrt::launch_kernel(rows != nullptr ? xrt::rmsnorm_add_kernel<TW, TC, PER, true> : xrt::rmsnorm_add_kernel<TW, TC, PER, false>, dim3(n_tokens), dim3(threads), 0, stream, residual, y,       \
                      (size_t)part_stride, n_parts, (const TW*)weight, (TC*)copy, width, eps, ex)
   XRT_DISPATCH_DTYPE(weight_dtype, TW, {
     XRT_DISPATCH_DTYPE(copy_dtype, TC, {

@@ -73,6 +73,12 @@ def parallel_residual(parts: LayerParts, x, ctx, stores, owns_cache: bool) -> No
         ctx.then_norm = ctx.pending = None
 
 
+def _result_for(ffn, post):
+    """How a feed-forward hands its result to the norm after it: with its parts where they lie (``apply_rows``) if it can and the norm
+    gathers them, else ``apply``."""
+    return getattr(ffn, "apply_rows", ffn.apply) if getattr(post, "takes_rows", False) else ffn.apply
+
+
 def sandwich_residual(parts: LayerParts, x, ctx, stores, owns_cache: bool) -> None:
     """x += post_norm(mixer(norm(x))); x += post_norm(feed_forward(norm(x))): a norm before and after each sublayer.
     The layer's parts are ``mixer_norm``, ``mixer``, ``mixer_post`` and, if it has a feed-forward, ``ffn_norm``,
@@ -98,7 +104,7 @@ def sandwich_residual(parts: LayerParts, x, ctx, stores, owns_cache: bool) -> No
         if h is None:
             h = parts.ffn_norm.forward(x)
         following = after[0] if after else None
-        h = parts.ffn_post.add_into(x, parts.ffn.apply(h, ctx), then=following)
+        h = parts.ffn_post.add_into(x, _result_for(parts.ffn, parts.ffn_post)(h, ctx), then=following)
     if h is not None:
         ctx.pending = ReadyNorm(following, h)
 
@@ -151,7 +157,7 @@ def postnorm_residual(parts: LayerParts, x, ctx, stores, owns_cache: bool) -> No
                                   copy=rounds and (has_ffn or follows))
     ctx.then_norm = ctx.pending = None
     if has_ffn:
-        h = parts.ffn_post.add_into(x, parts.ffn.apply(x if not rounds else h, ctx), copy=rounds and follows)
+        h = parts.ffn_post.add_into(x, _result_for(parts.ffn, parts.ffn_post)(x if not rounds else h, ctx), copy=rounds and follows)
     if rounds and h is not None:
         ctx.pending = StreamCopy(x, h)
 

@@ -44,7 +44,7 @@ class WeightedParts:
     parts[p] + bias being the result (``scales`` float32 [n] on the device or None for ones, ``bias`` float32 [width] or
     None; a result in one piece may be [T, width]).  The
     norm that follows the sublayer adds them up in its own pass over the row.
-    Two more forms, which only ``parts/stream_add.py:ScaledAdd`` takes: ``norms`` (float32 [n, width], with ``eps``): part
+    Two more forms: ``norms`` (float32 [n, width], with ``eps``; only ``parts/stream_add.py:ScaledAdd`` takes it): part
     p counts as RMSNorm(parts[p]) * norms[p]; ``rows`` and ``row_scales`` (int32 [T * n], float32 [T, n]): ``parts`` is
     [any, width] and part p of token t is its row rows[t * n + p] times row_scales[t, p] (experts' results where they lie)."""
     parts: torch.Tensor
@@ -62,6 +62,7 @@ class RMSNorm:
     not use it).  weights: ``weight`` [width]."""
 
     graph_safe = True
+    takes_rows = True  # ``add_into`` takes a ``WeightedParts`` with ``rows``
 
     @classmethod
     def weight_shapes(cls, params):
@@ -94,10 +95,11 @@ class RMSNorm:
         row added to their sum).  ``copy``: the new residual is also returned in the compute dtype, written in the
         same pass (what the next sublayer's products read), else None.  ``then``: another RMSNorm of this width whose
         weight has this one's dtype; its result over the new residual is returned, computed in the same pass (else None)."""
-        scales = bias = None
+        scales = bias = gather = None
         if isinstance(y, WeightedParts):
-            if y.norms is not None or y.rows is not None:
-                raise ConfigError("a norm after a sublayer takes parts that are neither normed one by one nor gathered")
+            if y.norms is not None:
+                raise ConfigError("a norm after a sublayer takes parts that are not normed one by one")
+            gather = None if y.rows is None else (y.rows, y.row_scales)
             y, scales, bias = y.parts, y.scales, y.bias
         if y.dim() == 3 and y.shape[0] == 1 and scales is None:
             y = y[0]
@@ -108,7 +110,7 @@ class RMSNorm:
             out = torch.empty(residual.shape, dtype=then.out_dtype, device=residual.device)
             following = (then.weight, then.eps, out)
         ops.rmsnorm_add(residual, y, self.weight, self.eps, copy=out if copy else None, factor=self.gain,
-                        part_scales=scales, bias=bias, then=following)
+                        part_scales=scales, bias=bias, then=following, gather=gather)
         return out
 
 
@@ -135,6 +137,10 @@ class LayerNorm:
         self.weight32 = None
         self.out_dtype = torch_dtype(dtype)
 
+    @property
+    def takes_rows(self) -> bool:
+        return self.width <= 4096  # what the kernel that keeps a row in registers holds
+
     def _weight32(self):
         if self.weight32 is None:
             self.weight32 = self.weight.to(torch.float32).contiguous()
@@ -151,16 +157,23 @@ class LayerNorm:
 
     def add_into(self, residual, y, then=None):
         """residual += norm(y).  ``then``: another LayerNorm of the same width and eps; its result over the new
-        residual is returned (computed in the same pass), else None."""
+        residual is returned (computed in the same pass), else None.  ``y`` may be a ``WeightedParts`` whose parts have no
+        factors, norms or bias of their own (gathered ones where ``takes_rows``)."""
+        gather = None
+        if isinstance(y, WeightedParts):
+            if y.norms is not None or y.scales is not None or y.bias is not None:
+                raise ConfigError("a layer norm after a sublayer takes plain or gathered parts")
+            gather = None if y.rows is None else (y.rows, y.row_scales)
+            y = y.parts
         if y.dim() == 3 and y.shape[0] == 1:
             y = y[0]
         parts = y.shape[0] if y.dim() == 3 else 1
         if isinstance(then, LayerNorm) and then.width == self.width and then.eps == self.eps:
             out = torch.empty(residual.shape, dtype=then.out_dtype, device=residual.device)
             ops.layernorm_affine(y, self._weight32(), self.bias, self.eps, out=out, residual=residual, n_parts=parts,
-                                 then=(then._weight32(), then.bias))
+                                 then=(then._weight32(), then.bias), gather=gather)
             return out
-        ops.layernorm_affine(y, self._weight32(), self.bias, self.eps, residual=residual, n_parts=parts)
+        ops.layernorm_affine(y, self._weight32(), self.bias, self.eps, residual=residual, n_parts=parts, gather=gather)
         return None
 
 
