@@ -121,12 +121,16 @@ def build_context(entries, cache: Cache, vocab_size: int, dtype, device, pad_to:
     padded = max(sum(new_lens), pad_to or 0)
     n = len(entries)
     size = layout(padded, n)["size"]
+    n_wanted = sum(len(e.want) for e in entries)
     staging = staging or PinnedRing(device, count=1)
-    turn, host = staging.take(size)
-    wanted = fill_arrays(host.numpy(), entries, starts, padded, n)
+    turn, host = staging.take(size + n_wanted)
+    arrays = host.numpy()
+    # the wanted rows go along behind the step's arrays: a tensor made from a list of their own would be a copy from
+    # pageable memory, which waits for everything the device still has to do (a millisecond between two prompts)
+    arrays[size:] = fill_arrays(arrays, entries, starts, padded, n)
     dev = host.to(device, non_blocking=True)
     staging.copied(turn)
-    want_rows = torch.tensor(wanted, dtype=torch.int32, device=device) if wanted else None
+    want_rows = dev[size:] if n_wanted else None
     return context_from(dev, padded, n, new_lens, starts, dtype), want_rows
 
 
@@ -280,4 +284,8 @@ class Engine:
             return None
         if wanted == list(range(n)):
             return logits.clone()
-        return g.logits[torch.tensor(wanted, dtype=torch.int64, device=model.device)]
+        turn, host = self.staging.take(len(wanted))
+        host.numpy()[:] = wanted
+        rows = host.to(model.device, non_blocking=True)
+        self.staging.copied(turn)
+        return g.logits[rows]
