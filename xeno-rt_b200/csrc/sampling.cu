@@ -28,7 +28,7 @@
 // two blocks fill a multiprocessor (64 registers a thread of 512; 85 KB) and there are 512.
 //
 // Batches whose rows all have a small top_k (the usual options; the caller says so) or are greedy take the SMALL form (64 rows of 128,256
-// with top_k 40, top_p 0.95: 63 -> 27 us a call, of which the kernel is no longer the larger part): no values kept,
+// with top_k 40, top_p 0.95: 63 -> 27 us a call): no values kept,
 // so that four blocks of 32,064 logits a row run all at once, and one cut for the whole team, so that hardly more than top_k
 // candidates remain and only the threads that hold one look at the logits again.
 #include "common.cuh"
