@@ -267,3 +267,93 @@ def test_the_small_form_gives_the_same_ids(rows, vocab):
                 ops.sample(out, logits, slots, *args, counter, largest_top_k=told)
                 got.append((out.tolist(), counter.tolist()))
             assert got[0] == got[1]
+
+
+def _sampler_of(slots, vocab):
+    from xeno_rt_b200.cache import Cache
+    from xeno_rt_b200.core import DType
+    from xeno_rt_b200.sampling import Sampler
+    cache = Cache([], slots * 64, 1024, DType.BF16, DEV, slots)
+    sampler, opened = Sampler(cache, vocab), [cache.open_slot() for _ in range(slots)]
+    sampler.begin(opened, list(range(slots)))
+    return sampler, opened, torch.tensor(opened, dtype=torch.int32, device=DEV)
+
+
+def test_options_that_one_stream_brought_serve_another():
+    """The options of a batch are kept from call to call: a call on a second stream, while the first is still busy, finds them."""
+    from xeno_rt_b200.sampling import SamplerConfig
+    logits = torch.zeros(2, 5000, device=DEV)
+    greedy, hot = [SamplerConfig(0.0)] * 2, [SamplerConfig(1.0, 0, 1.0, 1.0)] * 2
+    sampler, _, rows = _sampler_of(2, 5000)
+    want = sampler.sample(logits, rows, hot).tolist()
+    assert want != [0, 0]  # (what greedy rows give)
+    sampler, _, rows = _sampler_of(2, 5000)
+    nobody = torch.full_like(rows, -1)
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(first):
+        sampler.sample(logits, nobody, greedy)  # what the room of the next options may still hold
+        sampler.sample(logits, nobody, [SamplerConfig(0.5), SamplerConfig(0.7)])
+        torch.cuda._sleep(500_000_000)
+        sampler.sample(logits, nobody, hot)
+    with torch.cuda.stream(second):
+        got = sampler.sample(logits, rows, hot)
+    torch.cuda.synchronize()
+    assert got.tolist() == want
+
+
+@pytest.mark.parametrize("call", ["sample", "begin"])
+def test_new_options_and_seeds_are_refused_inside_a_capture(call):
+    """They come from the host: a graph would replay whatever the host's buffer holds then.  Known options may be captured."""
+    from xeno_rt_b200.sampling import SamplerConfig
+    logits = torch.zeros(2, 5000, device=DEV)
+    sampler, slots, rows = _sampler_of(2, 5000)
+    known = [SamplerConfig(0.9)] * 2
+    sampler.sample(logits, rows, known)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            if call == "begin":
+                sampler.begin(slots, [5, 6])
+            else:
+                sampler.sample(logits, rows, [SamplerConfig(0.6)] * 2)
+    for turn in range(6):  # and all goes on
+        sampler.begin(slots, [turn, turn])
+        sampler.sample(logits, rows, [SamplerConfig(0.3 + turn)] * 2)
+    sampler.sample(logits, rows, known)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        out = sampler.sample(logits, rows, known)
+    sampler.begin(slots, [1, 2])
+    sampler.rng_counter.zero_()
+    graph.replay()
+    got = out.tolist()
+    sampler.rng_counter.zero_()
+    assert got == sampler.sample(logits, rows, known).tolist()
+
+
+def test_sequences_begun_by_several_threads_keep_their_seeds(monkeypatch):
+    """``begin`` of other slots at the same time, the device busy: no thread's seeds pass through a buffer that another one writes."""
+    import threading
+    import time
+    from xeno_rt_b200.core import staging
+    from xeno_rt_b200.sampling.sampler import sequence_key
+    take = staging.PinnedRing.take
+
+    def slow_take(self, n):  # every thread has its buffer before the first one fills it
+        got = take(self, n)
+        time.sleep(0.05)
+        return got
+
+    sampler, slots, _ = _sampler_of(12, 100)
+    torch.cuda.synchronize()
+    monkeypatch.setattr(staging.PinnedRing, "take", slow_take)
+    torch.cuda._sleep(500_000_000)
+    threads = [threading.Thread(target=sampler.begin, args=([s], [1000 + s])) for s in slots]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    want = [k - (1 << 64) if k >> 63 else k for k in (sequence_key(1000 + s) for s in slots)]
+    assert sampler.rng_key[torch.tensor(slots, device=DEV)].tolist() == want

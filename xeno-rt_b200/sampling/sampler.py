@@ -14,8 +14,6 @@ import numpy as np
 import torch
 
 from ..cache import Cache
-from ..core import ConfigError
-from ..core.staging import PinnedRing
 from ..csrc import ops
 from ..weights.random_init import _splitmix64_int
 from .params import SamplerConfig
@@ -41,27 +39,15 @@ class Sampler:
         self.rng_key = cache.register_sequence_state("sampler.rng_key", (), torch.int64)
         self.rng_counter = cache.register_sequence_state("sampler.rng_counter", (), torch.int32)
         self.seen = cache.register_sequence_state("sampler.seen", (words,), torch.int32)
-        self._staging = PinnedRing(self.device)
         self._options_key = None
         self._options = None
         self._largest_top_k = 0
 
     def begin(self, slots: list, seeds: list) -> None:
         """Sets the random stream of freshly opened slots (their counters and bitmaps are zero)."""
-        n = len(slots)
-        if len(seeds) != n:
-            raise ConfigError(f"{len(seeds)} seeds for {n} slots")
-        keys = np.array([sequence_key(s) for s in seeds], dtype=np.uint64).view(np.int32)
-        dev = self._to_device(np.concatenate([keys, np.array(slots, dtype=np.int32)]))
-        self.rng_key.index_copy_(0, dev[2 * n:].to(torch.int64), dev[:2 * n].view(torch.int64))
-
-    def _to_device(self, values: np.ndarray) -> torch.Tensor:
-        """32-bit values as an int32 tensor on the device, without a wait for what the device still has to do."""
-        turn, host = self._staging.take(values.size)
-        host.numpy()[:] = values.reshape(-1).view(np.int32)
-        dev = host.to(self.device, non_blocking=True, copy=True)
-        self._staging.copied(turn)
-        return dev
+        keys = np.array([sequence_key(s) for s in seeds], dtype=np.uint64).view(np.int64)
+        idx = torch.tensor(slots, dtype=torch.int64, device=self.device)
+        self.rng_key.index_copy_(0, idx, torch.from_numpy(keys).to(self.device))
 
     def observe(self, slots: torch.Tensor, ids: torch.Tensor) -> None:
         """Adds ids[i] to the history of slots[i] (int32 device tensors; slot -1 is skipped)."""
@@ -83,8 +69,9 @@ class Sampler:
                 params[1, i] = np.int32(c.top_k).view(np.float32)
                 params[2, i] = c.top_p
                 params[3, i] = c.repetition_penalty
-            dev = self._to_device(params).view(4, n)
-            self._options = (dev[0].view(torch.float32), dev[1], dev[2].view(torch.float32), dev[3].view(torch.float32))
+            # a copy that has ended when this returns: the options are kept, and the next call may come on any stream
+            dev = torch.from_numpy(params).to(self.device)
+            self._options = (dev[0], dev[1].view(torch.int32), dev[2], dev[3])
             self._options_key = key
             # what the batch's rows have in common, for the choice of the kernel's form
             ks = [c.top_k for c in configs if not c.greedy]
