@@ -375,3 +375,28 @@ def test_full_width_layers_agree_between_the_32_bit_and_the_bfloat16_path():
     # the 32-bit result does not depend on the batch at all
     for a, b in zip(results["float32"][3], results["float32"][20][:3]):
         assert np.array_equal(a, b)
+
+
+def test_wanted_rows_from_the_host_are_refused_inside_a_capture(setups, engines):
+    """Their copy would be replayed from a buffer that later steps write; nothing is reserved and all goes on as before."""
+    from xeno_rt_b200.core import RuntimeFault
+    from xeno_rt_b200.engine import StepEntry
+    engine = engines("tiny-llama", "float32")
+    prompt = setups["tiny-llama"][1][1]
+    a, b = engine.open_slot(), engine.open_slot()
+    engine.step([StepEntry(a, prompt, [0]), StepEntry(b, prompt, [0])])
+    engine.step([StepEntry(a, [1], [0]), StepEntry(b, [2], [0])])
+    engine.step([StepEntry(a, [1], []), StepEntry(b, [2], [0])])
+    held = list(engine.cache.lengths)
+    for entries in ([StepEntry(a, [1, 2], [1])], [StepEntry(a, [1], []), StepEntry(b, [2], [0])]):
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeFault):
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                engine.step(entries)
+        assert engine.cache.lengths == held
+    got = [engine.step([StepEntry(a, [1], []), StepEntry(b, [2], [0])]) for _ in range(6)]
+    engine.close_slot(a)
+    engine.close_slot(b)
+    whole = _whole(engine, prompt + [2] * 8)
+    for i, logits in enumerate(got):
+        assert scaled_error(logits.cpu().numpy(), whole[len(prompt) + 2 + i:][:1]) < 1e-5

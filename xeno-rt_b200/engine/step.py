@@ -116,12 +116,14 @@ def build_context(entries, cache: Cache, vocab_size: int, dtype, device, pad_to:
     Returns (context, wanted rows as a device tensor or None).  ``pad_to`` appends padding rows
     (slot -1) up to that many tokens; padding changes no result."""
     _check_entries(entries, vocab_size)
+    n_wanted = sum(len(e.want) for e in entries)
+    if n_wanted:
+        _refuse_capture(device)
     new_lens = [len(e.tokens) for e in entries]
     starts = cache.reserve_all([e.slot for e in entries], new_lens)
     padded = max(sum(new_lens), pad_to or 0)
     n = len(entries)
     size = layout(padded, n)["size"]
-    n_wanted = sum(len(e.want) for e in entries)
     staging = staging or PinnedRing(device, count=1)
     turn, host = staging.take(size + n_wanted)
     arrays = host.numpy()
@@ -132,6 +134,13 @@ def build_context(entries, cache: Cache, vocab_size: int, dtype, device, pad_to:
     staging.copied(turn)
     want_rows = dev[size:] if n_wanted else None
     return context_from(dev, padded, n, new_lens, starts, dtype), want_rows
+
+
+def _refuse_capture(device) -> None:
+    """Raises where the current stream is being captured: rows that come from the host are copied from a buffer that later steps
+    write again, so a graph would replay other rows."""
+    if torch.device(device).type == "cuda" and torch.cuda.is_current_stream_capturing():
+        raise RuntimeFault("a step whose wanted rows come from the host cannot be captured in a graph")
 
 
 class _DecodeGraph:
@@ -252,6 +261,9 @@ class Engine:
     def _graph_step(self, slots, tokens, wanted, ids_device=None):
         """One token for each of ``slots`` (checked by the caller); ``wanted``: the rows whose logits are returned."""
         model, n = self.model, len(slots)
+        every_row = wanted == list(range(n))
+        if wanted and not every_row:
+            _refuse_capture(model.device)
         bucket = batch_bucket(n)
         starts = self.cache.reserve_all(slots, [1] * n)
         # launch shapes follow the longest context and, where lengths are unequal, the mean one (both by
@@ -282,7 +294,7 @@ class Engine:
             self.cache.advance(slot, 1)
         if not wanted:
             return None
-        if wanted == list(range(n)):
+        if every_row:
             return logits.clone()
         turn, host = self.staging.take(len(wanted))
         host.numpy()[:] = wanted
