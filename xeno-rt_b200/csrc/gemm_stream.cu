@@ -251,12 +251,10 @@ int launch_stream_staged(void* out, const void* x, const void* w, int M, int N, 
   constexpr int RING_BYTES = GS_STAGES * GROUPS * GS_ROWS * GS_ROW_BYTES;
   constexpr int PARTIAL_BYTES = GS_WARPS * GROUPS * M_TILES * 16 * (GS_ROWS + 1) * (int)sizeof(float);
   constexpr int SMEM = RING_BYTES > PARTIAL_BYTES ? RING_BYTES : PARTIAL_BYTES;
-  auto kernel = gemm_stream_kernel<M_TILES, MODE, GS_STAGES, ROW_GROUPS, TO>;
-  static bool allowed = false;
-  if (SMEM > 48 * 1024 && !allowed) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  constexpr auto kernel = gemm_stream_kernel<M_TILES, MODE, GS_STAGES, ROW_GROUPS, TO>;
+  if (SMEM > 48 * 1024) {
+    const cudaError_t err = allow_shared_memory_once<kernel>(SMEM);
     if (err != cudaSuccess) return (int)err;
-    allowed = true;
   }
   const int blocks = (N + ROW_GROUPS * GS_ROWS - 1) / (ROW_GROUPS * GS_ROWS);
   // the weight is read once a step (cp.async carries no cache hint here): marked as streaming in the L2
