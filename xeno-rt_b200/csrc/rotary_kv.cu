@@ -137,7 +137,6 @@ __global__ void qk_rope_kv_write_kernel(
     const float* all = qkv + (size_t)t * row_stride + (kind == 0 ? 0 : k_offset);
     const int n_all = (kind == 0 ? n_heads : n_kv_heads) * head_dim;
     float total = 0.f;
-#pragma unroll 16  // the row's numbers in flight together: each warp walks all heads' (16 heads of 128, four tokens: 6 us of a decode step)
     for (int c = lane; c < n_all; c += 32) {
       const float a = all[c] + (ex.bias != nullptr ? ex.bias[(kind == 0 ? 0 : k_offset) + c] : 0.f);
       total = fmaf(a, a, total);
