@@ -279,6 +279,33 @@ def test_gemm_stream(m, n, k):
     assert torch.equal(one[0], out[m - 1])
 
 
+# the first and the last number of weight rows whose added products have rings of eight stages on 148 multiprocessors, and their
+# neighbours; K of more slabs (of 512) than stages, so that every stage is used again, the last slab not whole; the last number of
+# rows and one more
+@pytest.mark.parametrize("m", [1, 3, 12, 13, 16])
+@pytest.mark.parametrize("n,k", [(1256, 4616), (1264, 4616), (2048, 8192), (2357, 5128), (2368, 5128)])
+def test_gemm_stream_rings_that_are_used_again(m, n, k):
+    """Bounds as above: the operands are exact in float64, the sums' order differs.  A row is the same whatever the batch, that is
+    in the deep ring and in the other; and with a norm to prepare."""
+    x = torch.randn(m, k, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(n, k, device=DEV) * 0.1).to(torch.bfloat16)
+    base = torch.randn(m, n, device=DEV)
+    want = f64(x) @ f64(w).T
+    out, acc = torch.empty(m, n, device=DEV), base.clone()
+    ops().gemm_stream(out, x, w)
+    ops().gemm_stream(acc, x, w, "accumulate")
+    assert rel(out, want) < 1e-5 and rel(acc, f64(base) + want) < 1e-5
+    many = base[m - 1:m].repeat(16, 1)
+    ops().gemm_stream(many, x[m - 1:m].repeat(16, 1), w, "accumulate")
+    assert torch.equal(many, acc[m - 1:m].expand(16, n))
+    normed, scaled = base.clone(), torch.empty(m, n, device=DEV, dtype=torch.bfloat16)
+    squares = torch.empty((ops().gemm_stream_norm_parts(m, n), m), device=DEV)
+    weight = torch.ones(n, device=DEV)
+    ops().gemm_stream(normed, x, w, "accumulate", norm=(scaled, weight, squares))
+    assert torch.equal(normed, acc) and torch.equal(scaled, acc.to(torch.bfloat16))
+    assert rel(squares.sum(0), (f64(acc) ** 2).sum(1)) < 1e-5
+
+
 @pytest.mark.parametrize("m,inner,k", [(1, 136, 96), (9, 203, 104), (33, 64, 4096)])
 def test_gemm_stream_swiglu(m, inner, k):
     x = torch.randn(m, k, device=DEV).to(torch.bfloat16)

@@ -8,7 +8,7 @@
 // bytes in flight: a block of eight warps owns 8 weight rows (SwiGLU: 8 gate rows and the 8 matching
 // up rows); for each 512-wide slab of K every thread issues 16-byte asynchronous copies (a warp
 // covers 512 contiguous bytes of one row) into one of three stages, so two slabs are always in
-// flight per block, and the small footprint (26 KB) lets eight blocks share a multiprocessor.
+// flight per block, and the small footprint (26 KB) leaves the number of blocks a multiprocessor to their registers (four).
 // Warp w then takes k in [64w, 64w + 64) of the slab: lane (g = lane / 4, t = lane % 4) reads the
 // 16 bytes W[row g][k0 + 8t ..] from shared memory and the matching 16 bytes of up to two X rows
 // from global memory (X is small and stays in L1/L2).  A dot product does not care in which order
@@ -20,8 +20,8 @@
 //
 // A product that adds into the residual stream can also prepare the RMSNorm that follows it (NormEmit,
 // common.cuh): here the parts of a row's sum of squares are one a block (its 8 or 16 weight rows); and
-// the kernel can finish a norm that the product before prepared (RowScale).  Those products keep four
-// stages.  Every 64 weight rows start their walk over K at another slab, and the weight is marked as
+// the kernel can finish a norm that the product before prepared (RowScale).  Products that add keep four
+// stages or eight (stream_deep_ring).  Every 64 weight rows start their walk over K at another slab, and the weight is marked as
 // streaming in the L2 by the launch's access-policy window (it is read once a step).
 #include "common.cuh"
 
@@ -268,7 +268,9 @@ int launch_stream_staged(void* out, const void* x, const void* w, int M, int N, 
 // stages were measured: they help single shapes (the output matrix at one row reaches 6.7 TB/s with
 // 5) and lose on others; over a whole decode step of 8 sequences 3 stages is the fastest, except for the
 // products that add into the residual stream, where 4 stages with the rotated walk are (alone, 8 rows:
-// K 4,096 9.2 -> 8.6 us, K 14,336 26.6 -> 26.1, N 5,120 / K 25,600 85.0 -> 68.4; whole steps 1 % faster).
+// K 4,096 9.2 -> 8.6 us, K 14,336 26.6 -> 26.1, N 5,120 / K 25,600 85.0 -> 68.4; whole steps 1 % faster), and those of
+// few blocks among them, where 8 are (stream_deep_ring).
+
 // Multiprocessors of the current device (148 where there is none to ask: host arithmetic only).
 inline int stream_sm_count() {
   static const int count = [] {
@@ -293,17 +295,26 @@ inline int stream_row_groups_accumulate(int N) {
   return (N + 2 * GS_ROWS - 1) / (2 * GS_ROWS) <= sms * 3 ? 2 : 1;
 }
 
+// Eight stages (70 KB a block, the same sums) for a product of up to 12 rows that adds into the residual stream and has more than one
+// block a multiprocessor but less than two: they are the only ones to keep bytes in flight.  Alone, four stages -> eight, by which
+// number the time shrinks: N 2,048 / K 8,192 at 1 row 13.3 -> 10.8 us, at 8 14.4 -> 11.9, at 12 1.18; N 1,280 / K 8,192 1.07 to 1.17, N 2,304
+// 1.13 to 1.19 (of the 42 points between at K 2,560 to 14,336 only N 1,664 / K 14,336 at 1 and 2 rows lost, 16.1 -> 16.8).  Outside: N 1,216
+// 0.95 to 1.05, N 2,368 9.95 -> 11.6 us; N 2,048 / K 25,600 at 16 rows 42.8 -> 45.4 (the rows of X no longer fit beside the rings in the L1).
+// Stored products gained less and lost more (K 14,336 at 4 rows: N 2,048 19.4 -> 18.5, N 1,792 15.9 -> 18.2).
+inline bool stream_deep_ring(int M, int N, int K) {
+  const int blocks = (N + GS_ROWS - 1) / GS_ROWS, sms = stream_sm_count();
+  return M <= 12 && K > 4 * GS_SLAB && 16 * blocks > 17 * sms && blocks < 2 * sms;
+}
+
 template <int M_TILES, int MODE, typename TO>
 int launch_stream(void* out, const void* x, const void* w, int M, int N, int K, int ldx, int ldo, long long up_offset,
                   const NormEmit& emit, const RowScale& scale, cudaStream_t stream) {
   // more than 32 batch rows: two row groups a block halve the X traffic per weight byte
   constexpr int RG = M_TILES >= 4 ? 2 : 1;
-  // No more than two blocks a multiprocessor: they are the only ones to keep bytes in flight, so their rings are deep (eight stages,
-  // 70 KB a block; the same sums).  With four, N 2,048 / K 8,192 at one row took 14 us of a decode step, with eight 11 to 12.
-  if (MODE != 2 && M_TILES == 1 && K > 4 * GS_SLAB && (N + GS_ROWS - 1) / GS_ROWS <= stream_sm_count() * 2)
-    return launch_stream_staged<M_TILES, MODE, 8, 1, TO>(out, x, w, M, N, K, ldx, ldo, up_offset, emit, scale, stream);
   // products that add into the residual stream (long K, few blocks a multiprocessor): four stages
   if (MODE == 1 && M_TILES == 1) {
+    if (stream_deep_ring(M, N, K))
+      return launch_stream_staged<M_TILES, MODE, 8, 1, TO>(out, x, w, M, N, K, ldx, ldo, up_offset, emit, scale, stream);
     if (stream_row_groups_accumulate(N) == 2)
       return launch_stream_staged<M_TILES, MODE, 4, 2, TO>(out, x, w, M, N, K, ldx, ldo, up_offset, emit, scale, stream);
     return launch_stream_staged<M_TILES, MODE, 4, RG, TO>(out, x, w, M, N, K, ldx, ldo, up_offset, emit, scale, stream);
