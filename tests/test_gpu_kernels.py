@@ -623,6 +623,50 @@ def test_attention_prefill_window_edge():
     assert np.abs(want[150] - full[150]).max() > 0.05  # the window matters in this case
 
 
+@pytest.mark.parametrize("options", [{}, {"window": 70}, {"window": 70, "keep_first": 3}, {"softcap": 20.0}, {"distance_rate": 8.0},
+                                     {"sink": 0.5}, {"mask_chunk": 96}], ids=lambda o: "-".join(o) or "plain")
+@pytest.mark.parametrize("nh,nkv,hd,latent", [(16, 8, 256, False), (16, 2, 192, False), (16, 1, 208, False), (18, 9, 240, False),
+                                              (15, 5, 256, False), (16, 8, 176, False), (16, 1, 256, True), (16, 1, 144, True)])
+def test_attention_prefill_several_heads_a_block(nh, nkv, hd, latent, options):
+    """A step whose blocks of one head would take more than two rounds (two heads a block where the rows are wide and the group is
+    even) gives the bits that each sequence gives by itself, where a block has one head; and what the kernel for any case gives.  Prompts
+    of unequal lengths, one token, continuations across a block's edge, skipped sequences; values in the keys' rows (one tile for
+    both) or in their own."""
+    torch.manual_seed(nh * hd + len(options))
+    totals, starts = [150, 1, 170, 64, 130, 65, 190, 64, 33, 128], [0, 0, 100, 0, 0, 1, 62, 0, 0, 64]
+    new = [t - s for t, s in zip(totals, starts)]
+    skipped = (3, 7)
+    assert nh * len(new) * 3 > 2 * torch.cuda.get_device_properties(0).multi_processor_count >= nh * 3
+    k_pool, v_pool, table = _cache_for(totals, nkv, hd, torch.bfloat16, shuffle_seed=hd + 1)
+    for s, n in enumerate(totals):
+        _fill_cache(k_pool, v_pool, table, s + 1, torch.randn(n, nkv, hd, device=DEV), torch.randn(n, nkv, hd, device=DEV))
+    if latent:
+        v_pool = k_pool
+    ints = lambda v: torch.tensor(list(v), dtype=torch.int32, device=DEV)
+    q = torch.randn(sum(new), nh * hd, device=DEV).to(torch.bfloat16)
+    cu = np.concatenate([[0], np.cumsum(new)])
+    slots = [-1 if s in skipped else s + 1 for s in range(len(new))]
+    kw = dict(options)
+    window = kw.pop("window", 0)
+    rest = (table, nh, nkv, hd, 1 / math.sqrt(hd), window)
+    out = torch.full_like(q, 5.0)
+    ops().attention_prefill(out, q, k_pool, v_pool, ints(cu), ints(slots), ints(starts), table, max(new), *rest[1:], **kw)
+    tok_slot = ints(np.repeat(slots, new))
+    tok_pos = ints(np.concatenate([np.arange(a, a + n) for a, n in zip(starts, new)]))
+    ref = torch.empty_like(q)
+    ops().attention_reference(ref, q, k_pool, v_pool, tok_slot, tok_pos, *rest, **kw)
+    for s, n in enumerate(new):
+        rows = slice(int(cu[s]), int(cu[s]) + n)
+        if s in skipped:
+            assert bool((out[rows] == 5.0).all())
+            continue
+        alone = torch.empty(n, nh * hd, device=DEV, dtype=torch.bfloat16)
+        ops().attention_prefill(alone, q[rows].contiguous(), k_pool, v_pool, ints([0, n]), ints([slots[s]]), ints([starts[s]]), table, n,
+                                *rest[1:], **kw)
+        assert torch.equal(out[rows], alone), s
+        assert torch.allclose(out[rows].float(), ref[rows].float(), atol=3e-2), s
+
+
 @pytest.mark.parametrize("m,n,k", [(128, 256, 64), (65, 8, 8), (200, 300, 136), (129, 513, 1032), (1000, 136, 96)])
 def test_gemm_tcgen05(m, n, k):
     """Sizes that are no multiple of the 128 x 256 x 64 tile: TMA zero-fills what reaches beyond."""

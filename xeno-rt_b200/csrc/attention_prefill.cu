@@ -3,8 +3,8 @@
 // (The reference's prefill form: crates/xrt-models/src/llama.rs:728-770: for token t the keys
 // 0 .. start + t, read from the cache so that earlier context is included.)
 //
-// Grid (query tiles, heads, sequences).  A block of four warps owns 64 consecutive new tokens of one
-// sequence for one query head, 16 rows a warp, and walks the sequence's cache blocks (64 keys each,
+// Grid (heads, sequences, query tiles).  Four warps own 64 consecutive new tokens of one
+// sequence for one query head, 16 rows a warp; a block has one head, or two of wide rows, and walks the sequence's cache blocks (64 keys each,
 // contiguous in memory) from the first visible key to the last row's own position; tiles are
 // copied to shared memory with cp.async, double-buffered, and every warp runs the same online
 // softmax (32-bit maxima, sums and accumulators) over all keys of a tile.  The keys of this step
@@ -20,10 +20,10 @@ constexpr int PRE_ROWS = PRE_WARPS * 16;
 
 // SCORED: the layer's score options (common.cuh) are on: kept first keys behind the window, a tanh cap, a distance
 // slope.  The tiles of the kept keys are walked before the window's.
-// HEADS: query heads of one kv head a block, four warps each, that share every tile.  Rows of more than 128 dims fill a
-// multiprocessor's shared memory with one block: with one head it was four warps that waited for their own loads and products
-// in turn (16 heads on rows of 256 dims, windows of 1,024, prompts of 3,598 tokens together: 354 us; 197 in this form).  Where the values are the keys'
-// own rows (latent attention) a tile is brought once.
+// HEADS: query heads of one kv head a block, four warps each, that share every tile.  Wide rows fill a multiprocessor's shared memory
+// with one block: with one head it was four warps that waited for their own loads and products in turn.  Where the values are the
+// keys' own rows (latent attention) a tile is brought once, and two blocks of one head have room (16 heads on 1 of 256 dims, windows of
+// 1,024, a prompt of 2,560 tokens: 384 -> 219 us).
 template <int HD_MAX, bool SCORED, int HEADS>
 __global__ void __launch_bounds__(HEADS * PRE_WARPS * 32)
 attention_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ q,
@@ -174,9 +174,16 @@ int launch_prefill_of(__nv_bfloat16* out, const __nv_bfloat16* q, const __nv_bfl
                    const int* cu_seqlens, const int* seq_slot, const int* seq_start, const int* block_table,
                    int max_blocks, int n_seqs, int max_new, int n_heads, int n_kv_heads, int head_dim, float scale,
                    const KeyRange& range, const ScoreOptions& opt, cudaStream_t stream) {
-  // two heads a block for the wide rows, unless blocks of one head leave multiprocessors empty (each holds one of them)
-  const bool two = HD_MAX > 128 && n_heads / n_kv_heads % 2 == 0 &&
-                   (long long)n_heads * n_seqs * ((max_new + PRE_ROWS - 1) / PRE_ROWS) > multiprocessors();
+  // Two heads a block from 192 dims on, where blocks of one head take more than two rounds of one a multiprocessor (what their shared
+  // memory leaves room for above 208 dims) and the values have rows of their own.  Microseconds, one head -> two, 16 heads on 8, one
+  // prompt: 256 dims, 1,024 tokens (256 blocks) 105 -> 118, 1,152 (288) 128 -> 131, 1,216 (304) 147 -> 138, 1,900 340 -> 227, 3,500
+  // 1,033 -> 640; 192 dims, 640 tokens 73 -> 75, 1,216 139 -> 134, 3,500 668 -> 621; 144 dims, 1,216 tokens 123 -> 123, 1,900 209 -> 209.
+  // Capped scores, bound by their tanh, gain nothing up to 208 dims: 192 dims, 1,216 tokens 173 -> 180, 3,500 517 -> 528 (kept first keys
+  // 137 -> 131, 410 -> 379; 256 dims, capped 195 -> 183, 809 -> 541).  With values in the keys' rows two blocks of one head share a
+  // multiprocessor: 256 dims, 16 heads on 1, 640 tokens 66 -> 73, 1,900 204 -> 216, 3,500 571 -> 601.
+  const long long blocks = (long long)n_heads * n_seqs * ((max_new + PRE_ROWS - 1) / PRE_ROWS);
+  const bool two = head_dim >= (opt.softcap > 0.f ? 224 : 192) && v_pool != k_pool && n_heads / n_kv_heads % 2 == 0 &&
+                   blocks > 2ll * multiprocessors();
   if constexpr (HD_MAX > 128) {
     if (two)
       return launch_prefill_heads<HD_MAX, SCORED, 2>(out, q, k_pool, v_pool, cu_seqlens, seq_slot, seq_start, block_table, max_blocks,
