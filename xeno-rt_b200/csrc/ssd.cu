@@ -448,7 +448,10 @@ XRT_EXPORT int xrt_gated_group_norm(void* out, const float* y, const float* z, i
   const int per = width / groups;
   const int threads = per >= 1024 ? 256 : (per >= 256 ? 128 : 64);
   XRT_DISPATCH_DTYPE(out_dtype, TO, {
-    auto kernel = per <= 4 * threads    ? xrt::gated_group_norm_rows_kernel<TO, 4>
+    // as many numbers a thread as a stretch has: 64 tokens of 16 stretches of 64 took 2.2 us before and 2.8 with room for four
+    auto kernel = per <= threads        ? xrt::gated_group_norm_rows_kernel<TO, 1>
+                  : per <= 2 * threads  ? xrt::gated_group_norm_rows_kernel<TO, 2>
+                  : per <= 4 * threads  ? xrt::gated_group_norm_rows_kernel<TO, 4>
                   : per <= 8 * threads  ? xrt::gated_group_norm_rows_kernel<TO, 8>
                   : per <= 16 * threads ? xrt::gated_group_norm_rows_kernel<TO, 16>
                                         : xrt::gated_group_norm_kernel<TO>;
