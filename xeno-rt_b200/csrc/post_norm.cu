@@ -29,9 +29,9 @@ struct PostNormExtras {
 
 // GATHER: the parts are gathered (PostNormExtras::rows).
 template <typename TW, typename TC, int PER, bool GATHER>
-__global__ void __launch_bounds__(512) rmsnorm_add_kernel(float* __restrict__ residual, const float* __restrict__ y, size_t part_stride,
-                                   int n_parts, const TW* __restrict__ w, TC* __restrict__ copy, int width, float eps,
-                                   const PostNormExtras ex) {
+__device__ __forceinline__ void rmsnorm_add_row(float* __restrict__ residual, const float* __restrict__ y, size_t part_stride,
+                                                int n_parts, const TW* __restrict__ w, TC* __restrict__ copy, int width,
+                                                float eps, const PostNormExtras& ex) {
   __shared__ float scratch[33];
   pdl_trigger();
   float wv[PER], yv[PER], rv[PER];
@@ -113,6 +113,22 @@ __global__ void __launch_bounds__(512) rmsnorm_add_kernel(float* __restrict__ re
   }
 }
 
+template <typename TW, typename TC, int PER>
+__global__ void rmsnorm_add_kernel(float* __restrict__ residual, const float* __restrict__ y, size_t part_stride, int n_parts,
+                                   const TW* __restrict__ w, TC* __restrict__ copy, int width, float eps,
+                                   const PostNormExtras ex) {
+  rmsnorm_add_row<TW, TC, PER, false>(residual, y, part_stride, n_parts, w, copy, width, eps, ex);
+}
+
+// Gathered parts, and rows of more than 8,192 (32 numbers a thread of 512, which only run with no more than 128 registers).  Others go
+// without the bound: with it, 4,096 rows of 8,192 took 141 us for 136.
+template <typename TW, typename TC, int PER, bool GATHER>
+__global__ void __launch_bounds__(512)
+rmsnorm_add_bounded_kernel(float* __restrict__ residual, const float* __restrict__ y, size_t part_stride, int n_parts,
+                           const TW* __restrict__ w, TC* __restrict__ copy, int width, float eps, const PostNormExtras ex) {
+  rmsnorm_add_row<TW, TC, PER, GATHER>(residual, y, part_stride, n_parts, w, copy, width, eps, ex);
+}
+
 template <typename TC>
 __global__ void cast_rows_kernel(TC* __restrict__ out, const float* __restrict__ x, size_t total) {
   pdl_trigger();
@@ -146,18 +162,23 @@ XRT_EXPORT int xrt_rmsnorm_add(float* residual, const float* y, long long part_s
   const int threads = width >= 4096 ? 512 : (width >= 1024 ? 256 : (width >= 256 ? 128 : 64));
   const int per = (width + threads - 1) / threads;
   if (per > 32) return XRT_ERR_UNSUPPORTED;
+#define XRT_POST_KERNEL(...)                                                                                            \
+  xrt::launch_kernel((__VA_ARGS__), dim3(n_tokens), dim3(threads), 0, stream, residual, y, (size_t)part_stride, n_parts, \
+                     (const TW*)weight, (TC*)copy, width, eps, ex)
 #define XRT_POST(PER)                                                                                                   \
-  xrt::launch_kernel(rows != nullptr ? xrt::rmsnorm_add_kernel<TW, TC, PER, true> : xrt::rmsnorm_add_kernel<TW, TC, PER, false>, dim3(n_tokens), dim3(threads), 0, stream, residual, y,       \
-                     (size_t)part_stride, n_parts, (const TW*)weight, (TC*)copy, width, eps, ex)
+  XRT_POST_KERNEL(rows != nullptr ? xrt::rmsnorm_add_bounded_kernel<TW, TC, PER, true> : xrt::rmsnorm_add_kernel<TW, TC, PER>)
   XRT_DISPATCH_DTYPE(weight_dtype, TW, {
     XRT_DISPATCH_DTYPE(copy_dtype, TC, {
       if (per <= 4) XRT_POST(4);
       else if (per <= 8) XRT_POST(8);
       else if (per <= 16) XRT_POST(16);
-      else XRT_POST(32);
+      else
+        XRT_POST_KERNEL(rows != nullptr ? xrt::rmsnorm_add_bounded_kernel<TW, TC, 32, true>
+                                        : xrt::rmsnorm_add_bounded_kernel<TW, TC, 32, false>);
     });
   });
 #undef XRT_POST
+#undef XRT_POST_KERNEL
   return xrt::launch_status();
 }
 
