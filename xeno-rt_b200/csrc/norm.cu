@@ -266,10 +266,12 @@ struct GatheredParts {
 
 // The same for rows of up to 256 * ITEMS floats, held in registers: the weights and biases of both norms are asked
 // for before the wait for the kernel before, the row and the residual together after it, so that a row of a decode
-// step costs two trips to memory instead of six in a row.  Of many rows a block takes every gridDim.x-th
-// (2,126 rows of 2,048: 31 -> 20 us).
-template <typename TO, int ITEMS>
-__global__ void __launch_bounds__(256, ITEMS <= 8 ? 3 : 2)
+// step costs two trips to memory instead of six in a row.  A part's numbers are on their way together (item by item, 4 rows of
+// two parts with both norms: width 1,024 4.1 -> 2.7 us, 2,048 5.3 -> 3.3, 4,096 9.2 -> 4.3).
+// PARTS: 0 one, 1 several, 2 they lie in rows of their own (GatheredParts).  MANY: with more than 1,024 columns a block takes every
+// gridDim.x-th row, so that its weights serve several (4,096 rows, both norms: width 2,048 43 -> 35, 4,096 84 -> 70).
+template <typename TO, int ITEMS, int PARTS, bool MANY>
+__global__ void __launch_bounds__(256, ITEMS > 8 ? 2 : !MANY ? 1 : ITEMS > 4 ? 3 : 5)
 layernorm_affine_rows_kernel(TO* __restrict__ out, float* __restrict__ residual, const float* __restrict__ x, int n_parts,
                              size_t part_stride, const float* __restrict__ w, const float* __restrict__ b,
                              const int* __restrict__ rows, int n_rows, int width, float eps, const float* __restrict__ w2,
@@ -287,13 +289,11 @@ layernorm_affine_rows_kernel(TO* __restrict__ out, float* __restrict__ residual,
     b2v[i] = in && b2 != nullptr ? b2[c] : 0.f;
   }
   pdl_wait(x, w, b, rows, w2, b2);
-  for (int r = blockIdx.x; r < n_rows; r += gridDim.x) {
-    const int src = rows != nullptr ? rows[r] : r;
-    auto part_of = [&](int p) {
-      return gathered.rows != nullptr ? x + (size_t)gathered.rows[(size_t)r * n_parts + p] * width : x + p * part_stride + (size_t)src * width;
-    };
-    const float* xr = part_of(0);
-    const float first = gathered.rows != nullptr ? gathered.scales[(size_t)r * n_parts] : 1.0f;
+  constexpr bool GATHER = PARTS == 2;
+  int r = blockIdx.x;
+  do {
+    const int src = GATHER ? gathered.rows[(size_t)r * n_parts] : (rows != nullptr ? rows[r] : r);
+    const float* xr = x + (size_t)src * width;
     float v[ITEMS], res[ITEMS];
     float acc = 0.f;
 #pragma unroll
@@ -306,11 +306,14 @@ layernorm_affine_rows_kernel(TO* __restrict__ out, float* __restrict__ residual,
         if (residual != nullptr) res[i] = residual[(size_t)r * width + c];
       }
     }
+    if (GATHER) {
+      const float scale = gathered.scales[(size_t)r * n_parts];
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) v[i] = __fmul_rn(v[i], first);
-    for (int p = 1; p < n_parts; ++p) {  // a part's numbers are on their way together (item by item a row of two parts took 7 to 8 us of a decode step, for 3.4 to 4.9)
-      const float* pr = part_of(p);
-      const float scale = gathered.rows != nullptr ? gathered.scales[(size_t)r * n_parts + p] : 1.0f;
+      for (int i = 0; i < ITEMS; ++i) v[i] = __fmul_rn(v[i], scale);
+    }
+    for (int p = 1; PARTS != 0 && p < n_parts; ++p) {
+      const float* pr = GATHER ? x + (size_t)gathered.rows[(size_t)r * n_parts + p] * width : xr + p * part_stride;
+      const float scale = GATHER ? gathered.scales[(size_t)r * n_parts + p] : 1.0f;
       float more[ITEMS];
 #pragma unroll
       for (int i = 0; i < ITEMS; ++i) {
@@ -318,7 +321,7 @@ layernorm_affine_rows_kernel(TO* __restrict__ out, float* __restrict__ residual,
         more[i] = c < width ? pr[c] : 0.f;
       }
 #pragma unroll
-      for (int i = 0; i < ITEMS; ++i) v[i] = __fadd_rn(v[i], __fmul_rn(more[i], scale));
+      for (int i = 0; i < ITEMS; ++i) v[i] = __fadd_rn(v[i], GATHER ? __fmul_rn(more[i], scale) : more[i]);
     }
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) acc += v[i];
@@ -360,7 +363,7 @@ layernorm_affine_rows_kernel(TO* __restrict__ out, float* __restrict__ residual,
       const int c = threadIdx.x + i * 256;
       if (c < width) out[(size_t)r * width + c] = from_float<TO>(((v[i] - mean) * inv) * w2v[i] + b2v[i]);
     }
-  }
+  } while (MANY && ITEMS > 4 && (r += gridDim.x) < n_rows);
 }
 
 }  // namespace xrt
@@ -381,16 +384,34 @@ XRT_EXPORT int xrt_layernorm_affine(void* out, float* residual, const float* x, 
     xrt::GatheredParts gathered;
     gathered.rows = part_rows;
     gathered.scales = part_scales;
-    // as many blocks as run at once where the rows are more: a block's weights then serve several rows
-    const int resident = (width <= 256 * 8 ? 3 : 2) * xrt::multiprocessors();
-    const int blocks = n_rows < resident || resident <= 0 ? n_rows : resident;
+    // Several rows a block: from more rows on than two blocks a multiprocessor hold, for widths above 1,024.  (Up to there a row a
+    // block is one round, and the bound of three blocks a multiprocessor costs registers: 296 rows of 2,048 3.2 us against 4.2, 444 5.8
+    // against 4.4.)  Narrower rows fill a multiprocessor with more blocks than that (4,096 rows of 1,024 as three blocks a multiprocessor
+    // 22.1 us, as a block each 18.9): they only get the form of fewer registers where the other one's four blocks a multiprocessor are not
+    // all (600 rows of 512, 4.3 us against 3.8; of 148 rows it takes 2.5 against 2.4).
+    const int sms = xrt::multiprocessors();
+    const bool many = sms > 0 && n_rows > (width > 256 * 4 ? 2 : 4) * sms;
+    const int resident = (width <= 256 * 8 ? 3 : 2) * sms;
+    const int blocks = many && width > 256 * 4 && n_rows > resident ? resident : n_rows;
+#define XRT_LAYERNORM(ITEMS, MANY)                                                                                           \
+  xrt::launch_kernel(part_rows != nullptr ? xrt::layernorm_affine_rows_kernel<TO, ITEMS, 2, MANY>                            \
+                     : n_parts > 1        ? xrt::layernorm_affine_rows_kernel<TO, ITEMS, 1, MANY>                            \
+                                          : xrt::layernorm_affine_rows_kernel<TO, ITEMS, 0, MANY>,                           \
+                     dim3(blocks), dim3(256), 0, stream, (TO*)out, residual, x, n_parts, (size_t)part_stride, weight, bias,  \
+                     rows, n_rows, width, eps, weight2, bias2, gathered)
     XRT_DISPATCH_DTYPE(out_dtype, TO, {
-      auto kernel = width <= 256 * 4   ? xrt::layernorm_affine_rows_kernel<TO, 4>
-                    : width <= 256 * 8 ? xrt::layernorm_affine_rows_kernel<TO, 8>
-                                       : xrt::layernorm_affine_rows_kernel<TO, 16>;
-      xrt::launch_kernel(kernel, dim3(blocks), dim3(256), 0, stream, (TO*)out, residual, x, n_parts, (size_t)part_stride, weight, bias,
-                         rows, n_rows, width, eps, weight2, bias2, gathered);
+      if (width <= 256 * 4) {
+        if (many) XRT_LAYERNORM(4, true);
+        else XRT_LAYERNORM(4, false);
+      } else if (width <= 256 * 8) {
+        if (many) XRT_LAYERNORM(8, true);
+        else XRT_LAYERNORM(8, false);
+      } else {
+        if (many) XRT_LAYERNORM(16, true);
+        else XRT_LAYERNORM(16, false);
+      }
     });
+#undef XRT_LAYERNORM
     return xrt::launch_status();
   }
   XRT_DISPATCH_DTYPE(out_dtype, TO, {
