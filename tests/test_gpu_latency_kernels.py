@@ -81,8 +81,11 @@ def test_route_scores(experts, groups, keep, top, scores, normalize):
             allowed = [e for e in range(experts) if e // (experts // groups) in order]
             want = sorted(allowed, key=lambda e: (-round(float(choice[t, e]), 12), e))[:top]
             got = ids[t].tolist()
-            # a difference below the rounding of 32 bits may decide otherwise
-            assert all(a == b or abs(float(choice[t, a] - choice[t, b])) < 1e-6 for a, b in zip(got, want)), (t, got, want)
+            # a difference below the rounding of 32 bits may decide otherwise, but equal logits (and corrections) are a tie: the lower number
+            stands_for = lambda e: (logits[t, e], 0.0 if fix is None else fix[e])
+            assert len(set(got)) == top, (t, got)
+            assert all(a == b or (abs(float(choice[t, a] - choice[t, b])) < 1e-6 and stands_for(a) != stands_for(b))
+                       for a, b in zip(got, want)), (t, got, want)
             w = s[t, ids[t].long()]
             w = w / (w.sum() + 1e-9) if normalize else w
             assert torch.allclose(weights[t].double(), 2.5 * w, rtol=2e-6, atol=1e-12)
@@ -92,6 +95,7 @@ def test_route_scores(experts, groups, keep, top, scores, normalize):
     bad[4] = float("-inf")
     ops.moe_route_scores(ids, weights, bad, top, groups, keep, scores=scores, normalize=normalize)
     assert ((ids >= 0) & (ids < experts)).all()
+    assert all(len(set(row)) == top for row in ids.tolist())  # (rows that are no numbers too)
     good = torch.tensor([i for i in range(n) if i not in (0, 2, 4)], device=DEV)
     again, _ = torch.empty_like(ids), None
     ops.moe_route_scores(again, torch.empty_like(weights), torch.from_numpy(logits).to(DEV), top, groups, keep, scores=scores, normalize=normalize)
