@@ -269,6 +269,58 @@ def test_the_small_form_gives_the_same_ids(rows, vocab):
             assert got[0] == got[1]
 
 
+# teams of four and of two blocks, rows of whole 16 bytes or not
+@pytest.mark.parametrize("rows,vocab", [(40, 32000), (76, 20001), (152, 9000)])
+def test_rows_whose_first_cut_leaves_too_few_or_too_many(rows, vocab):
+    """The small form gives the ids of the other one: rows masked down to fewer ids than top_k, to a run of neighbours that few groups
+    of lanes hold, to as many as are ranked at once and one more, with the lowest number; more than that above the cut (values in order);
+    equal values at the cut, as many as are listed, one more, and all of them; zeros of both signs there."""
+    from xeno_rt_b200.csrc import ops
+    rng = np.random.default_rng(vocab)
+    logits = (rng.normal(size=(rows, vocab)) * 3.0).astype(np.float32)
+
+    def masked(row, kept, lowest=-np.inf):
+        values = row[kept].copy()
+        row[:] = lowest
+        row[kept] = values
+
+    for i in range(rows):
+        row, kind = logits[i], i % 18
+        if kind in (0, 1, 2, 3):
+            masked(row, rng.choice(vocab, (1, 11, 512, 513)[kind], replace=False))
+        elif kind in (4, 5, 6):
+            masked(row, slice(vocab // 3, vocab // 3 + (39, 400, 2500)[kind - 4]))
+        elif kind == 7:
+            row.sort()
+        elif kind == 8:
+            row[:] = np.sort(row)[::-1]
+        elif kind in (9, 10, 11):  # equal values at the cut
+            row[rng.choice(vocab, (600, 4096, 4097)[kind - 9], replace=False)] = 20.0
+            row[rng.choice(vocab, 5, replace=False)] = 21.0
+        elif kind == 12:
+            row[:] = 1.0
+        elif kind in (13, 14, 15):  # all zeros without a sign, few, half
+            row[:] = np.where(rng.random(vocab) < (1.0, 0.001, 0.5)[kind - 13], 0.0, -0.0)
+            row[rng.choice(vocab, 7, replace=False)] = 1.0
+        elif kind == 16:
+            masked(row, rng.choice(vocab, 11, replace=False), np.finfo(np.float32).min)
+    logits = torch.from_numpy(logits).to(DEV)
+    full = lambda v, dtype: torch.full((rows,), v, dtype=dtype, device=DEV)
+    slots = torch.arange(rows, dtype=torch.int32, device=DEV)
+    seen = torch.from_numpy(rng.integers(0, 2 ** 31, size=(rows, (vocab + 31) // 32), dtype=np.int32)).to(DEV)
+    key = torch.from_numpy(rng.integers(0, 2 ** 62, size=rows)).to(DEV)
+    for top_k in (1, 40, 64):
+        for top_p, penalty in ((0.95, 1.0), (1.0, 1.2), (0.3, 1.0)):
+            got = []
+            for told in (0, top_k):
+                out, counter = full(-7, torch.int32), torch.arange(rows, dtype=torch.int32, device=DEV)
+                for draw in range(4):
+                    ops.sample(out, logits, slots, full(0.9, torch.float32), full(top_k, torch.int32), full(top_p, torch.float32),
+                               full(penalty, torch.float32), seen, key, counter, largest_top_k=told)
+                    got.append(out.tolist())
+            assert got[:4] == got[4:]
+
+
 def _sampler_of(slots, vocab):
     from xeno_rt_b200.cache import Cache
     from xeno_rt_b200.core import DType

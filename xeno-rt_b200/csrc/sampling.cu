@@ -31,6 +31,8 @@
 // with top_k 40, top_p 0.95: 63 -> 27 us a call): no values kept,
 // so that four blocks of 32,064 logits a row run all at once, and one cut for the whole team, so that hardly more than top_k
 // candidates remain and only the threads that hold one look at the logits again.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace xrt {
@@ -139,8 +141,9 @@ struct SmallShared {
   uint32_t own_key[SAMPLE_GROUPS];
   uint32_t cut;
   int count;
-  int id[SAMPLE_THREADS];
-  float value[SAMPLE_THREADS];
+  int ties[SAMPLE_TEAM];  // of every block
+  int id[SAMPLE_CANDIDATES];
+  float value[SAMPLE_CANDIDATES];
 };
 
 struct Team {
@@ -222,9 +225,9 @@ __device__ __forceinline__ uint64_t probability_mass(float a, float row_max, flo
 // Returns the key; *inside gets want minus the weight of {key > K} (what the keys equal to K still
 // have to supply) and *at_key the weight of {key == K}.  If the whole weight is below `want`, returns 0 with *inside = 0.
 // weight <= 2^32.  `wide`: so many elements that a bin's sum of 16-bit halves could pass 32 bits.
-template <bool TEAM, typename A, typename F>
-__device__ uint32_t radix_select(A adjusted, F weight, int n, uint64_t want, bool wide, Team& team, uint64_t* inside,
-                                 uint64_t* at_key) {
+// each(f): f(i, value) for every element of this thread, in any order.
+template <bool TEAM, typename E, typename F>
+__device__ uint32_t radix_select(E each, F weight, uint64_t want, bool wide, Team& team, uint64_t* inside, uint64_t* at_key) {
   SampleShared* sh = team.sh;
   uint32_t prefix = 0, mask = 0;
   uint64_t remaining = want;
@@ -236,8 +239,7 @@ __device__ uint32_t radix_select(A adjusted, F weight, int n, uint64_t want, boo
     for (int b = threadIdx.x; b < SAMPLE_HIST_COPIES * 512; b += SAMPLE_THREADS) team.hist[b] = 0u;
     if (threadIdx.x == 0) sh->selected = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) {
-      const float a = adjusted(i);
+    each([&](int i, float a) {
       const uint32_t k = order_key(a);
       if ((k & mask) == prefix) {
         const uint64_t w = weight(i, a);
@@ -250,7 +252,7 @@ __device__ uint32_t radix_select(A adjusted, F weight, int n, uint64_t want, boo
           if (high) atomicAdd(&mine[2 * bin + 1], high);
         }
       }
-    }
+    });
     __syncthreads();
     unsigned long long* merged = sh->merged[pass & 1];
     unsigned long long sum = 0ull;
@@ -294,16 +296,17 @@ __device__ uint32_t radix_select(A adjusted, F weight, int n, uint64_t want, boo
 }
 
 // From the values to the id: top_k, top_p and the draw over `n` elements of this block, whose places count from `base`.
-// TEAM: over the elements of all blocks.  Returns the place of the id, -1 if no mass was left.
-template <bool TEAM, typename A>
-__device__ long long sample_place(A adjusted, int n, int base, long long n_all, int k, float temp, float p, float row_max,
+// TEAM: over the elements of all blocks.  adjusted(i): element i; each(f): see radix_select.  Returns the place of the id, -1 if no
+// mass was left.
+template <bool TEAM, typename A, typename E>
+__device__ long long sample_place(A adjusted, E each, int n, int base, long long n_all, int k, float temp, float p, float row_max,
                                   bool wide, Team& team) {
   // top-k: threshold key and the last place kept among equal keys
   uint32_t k_key = 0u; long long k_last = n_all;  // kept: key > k_key, or key == k_key and place <= k_last
   if (k > 0 && k < n_all) {
     uint64_t inside, at_key;
     auto one = [&](int, float) { return (uint64_t)1; };
-    k_key = radix_select<TEAM>(adjusted, one, n, (uint64_t)k, wide, team, &inside, &at_key);
+    k_key = radix_select<TEAM>(each, one, (uint64_t)k, wide, team, &inside, &at_key);
     if (at_key > inside) {
       auto tie = [&](int i) { return (uint64_t)(order_key(adjusted(i)) == k_key); };
       k_last = ordered_pick<TEAM>(tie, n, base, inside - 1, team);
@@ -319,26 +322,26 @@ __device__ long long sample_place(A adjusted, int n, int base, long long n_all, 
   uint32_t p_key = 0u; long long p_last = n_all;
   if (p < 1.0f) {
     uint64_t local = 0, total;
-    for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) local += mass_of(i, adjusted(i));
+    each([&](int i, float a) { local += mass_of(i, a); });
     team_exclusive_scan<TEAM>(local, team, &total);
     uint64_t want = (uint64_t)ceil((double)p * (double)total);
     if (want < 1) want = 1;
     uint64_t inside, at_key;
-    p_key = radix_select<TEAM>(adjusted, mass_of, n, want, wide, team, &inside, &at_key);
+    p_key = radix_select<TEAM>(each, mass_of, want, wide, team, &inside, &at_key);
     if (at_key > inside) {
       // equal keys have equal mass: how many of them the remaining mass needs
       auto tie_mass = [&](int i) { const float a = adjusted(i); return order_key(a) == p_key ? mass_of(i, a) : 0ull; };
       p_last = ordered_pick<TEAM>(tie_mass, n, base, inside - 1, team);
     }
   }
-  auto kept_mass = [&](int i) -> uint64_t {
-    const float a = adjusted(i);
+  auto kept_of = [&](int i, float a) -> uint64_t {
     const uint32_t key = order_key(a);
     if (key < p_key || (key == p_key && base + i > p_last)) return 0ull;
     return mass_of(i, a);
   };
+  auto kept_mass = [&](int i) { return kept_of(i, adjusted(i)); };
   uint64_t local = 0, total;
-  for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) local += kept_mass(i);
+  each([&](int i, float a) { local += kept_of(i, a); });
   team_exclusive_scan<TEAM>(local, team, &total);
   const uint64_t target = __umul64hi((uint64_t)team.sh->draw << 32, total);  // floor(u / 2^32 * total)
   return total > 0 ? ordered_pick<TEAM>(kept_mass, n, base, target, team) : -1;
@@ -494,14 +497,54 @@ __device__ int ranked_id(const int* ids, const float* vals, int n, int k, float 
   return team.sh->pick >= 0 ? (int)team.sh->pick : row_arg;
 }
 
+// Lists the first `want` places, in index order over the team's blocks, where tie(i) holds, behind the first `at` entries of the
+// first block's candidates.  `ties`: every block's count, in every block.  Returns whether so many places hold.  Ends with a meeting.
+template <typename P, typename A>
+__device__ bool send_ties(P tie, A adjusted, int n, int base, int want, SmallShared* first, int at, int* warp_count, int* ties,
+                          Team& team) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int run = ((n + SAMPLE_WARPS - 1) / SAMPLE_WARPS + 31) & ~31;
+  const int lo = min(n, warp * run), hi = min(n, lo + run);
+  int mine = 0;  // (counted no further than matters)
+  for (int i0 = lo; i0 < hi && mine < want; i0 += 32) mine += __popc(__ballot_sync(0xffffffffu, i0 + lane < hi && tie(i0 + lane)));
+  if (lane == 0) warp_count[warp] = mine;
+  __syncthreads();
+  int place = 0, all = 0;
+  for (int w = 0; w < SAMPLE_WARPS; ++w) {
+    if (w < warp) place += warp_count[w];
+    all += warp_count[w];
+  }
+  if ((int)threadIdx.x < team.size) of_block(ties, threadIdx.x)[team.rank] = all;
+  team_sync();
+  all = 0;
+  for (int r = 0; r < team.size; ++r) {
+    if (r < team.rank) place += ties[r];
+    all += ties[r];
+  }
+  for (int i0 = lo; i0 < hi && place < want; i0 += 32) {
+    const int i = i0 + lane;
+    const bool in = i < hi && tie(i);
+    const unsigned mask = __ballot_sync(0xffffffffu, in);
+    const int here = place + __popc(mask & ((1u << lane) - 1u));
+    if (in && here < want) {
+      first->id[at + here] = base + i;
+      first->value[at + here] = adjusted(i);
+    }
+    place += __popc(mask);
+  }
+  team_sync();
+  return all >= want;
+}
+
 // CACHED: a block's slice of the row fits its shared memory (else the passes read it from the L2 again).
 // VEC: rows are whole 16 bytes.
 // SMALL (not CACHED): for batches whose rows have a small top_k or are greedy.  The row's cut is the k-th largest of the largest values
 // of all groups of eight lanes of the team (64 a block): k values lie at or above it, and with twice as many groups as k hardly more.
 // Every block gets every group's value (one meeting) and finds the cut by itself; a thread whose own largest value reaches it
-// looks at its logits again and sends what lies at or above the cut to the first block, which ranks the candidates.  A row that
-// this does not serve (a larger k, more equal values than there is room for, fewer than k values above minus infinity) goes
-// through the selects over the whole row, as without a small top_k.
+// looks at its logits again and lists what lies at or above the cut in the first block, which ranks the candidates.  Where more than
+// that is at the cut (rows masked with a lowest value, or whose values are equal), what lies above it is listed, and the first of its equals; more
+// than are ranked at once are cut once more.  A row that this does not serve (a larger k, thousands above the cut, too many in the bin
+// of the second one, a cut at zero with too few zeros without a sign) goes through the selects over the whole row.
 template <bool CACHED, bool VEC, bool SMALL>
 __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
 sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int vocab, int per_block, int values_bytes,
@@ -551,10 +594,10 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
     if (a > best) { best = a; best_i = i; }  // indices rise: the first maximum is kept
     if (few && !of_largest) atomicAdd(&hist[order_key(a) >> 20], 1u);
   };
-  // every element of this thread, with the penalty
-  auto visit = [&](auto&& f) {
+  // every element of this thread, with the penalty; `ahead` loads in flight
+  auto visit_by = [&](auto ahead, auto&& f) {
     if (VEC) {
-      constexpr int UNROLL = 4;  // loads in flight a thread
+      constexpr int UNROLL = decltype(ahead)::value;
       const int quads = n / 4;
       const float4* src = reinterpret_cast<const float4*>(view.logits);
       for (int q0 = threadIdx.x; q0 < quads; q0 += UNROLL * SAMPLE_THREADS) {
@@ -582,8 +625,16 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
       for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) f(i, view.adjusted(i));
     }
   };
+  auto visit = [&](auto&& f) { visit_by(std::integral_constant<int, 4>(), f); };
   visit(take);
   auto adjusted = [&](int i) { return CACHED ? values[i] : view.adjusted(i); };
+  auto each = [&](auto&& f) {  // (for the selects)
+    if constexpr (CACHED) {
+      for (int i = threadIdx.x; i < n; i += SAMPLE_THREADS) f(i, values[i]);
+    } else {
+      visit_by(std::integral_constant<int, 2>(), f);
+    }
+  };
 
   if (few && of_largest) atomicAdd(&hist[best_i < 0 ? 0 : order_key(best) >> 20], 1u);
   // (larger value, smaller place) as one number; 0 where nothing lies above minus infinity
@@ -671,31 +722,66 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
         if (above < k && k <= above + equal) small->cut = key;  // (all who write it write the same)
       }
       __syncthreads();
-      const uint32_t cut = small->cut;
-      served = cut > SAMPLE_LOWEST_KEY;
-      if (served) {
-        if (own_key >= cut)
-          visit([&](int i, float a) {
-            if (order_key(a + 0.0f) >= cut) {
-              SmallShared* first = of_block(small, 0);
-              const int place = atomicAdd(&first->count, 1);
-              if (place < SAMPLE_THREADS) {
-                first->id[place] = base + i;
-                first->value[place] = a;
-              }
+      const uint32_t cut = max(small->cut, SAMPLE_LOWEST_KEY + 1);  // fewer values than k groups: all that have a mass are kept
+      SmallShared* first = of_block(small, 0);
+      auto list = [&](uint32_t low) {  // of this block, what lies at or above `low`
+        if (own_key < low) return;
+        bool room = true;
+        visit([&](int i, float a) {
+          if (room && order_key(a + 0.0f) >= low) {
+            const int place = atomicAdd(&first->count, 1);
+            room = place < SAMPLE_CANDIDATES;
+            if (room) {
+              first->id[place] = base + i;
+              first->value[place] = a;
             }
-          });
-        team_sync();  // the candidates are there
-        const int count = of_block(small, 0)->count;
-        served = count <= SAMPLE_THREADS;
-        team_sync();  // everybody has read how many they are: the other blocks may leave
-        if (served) {
-          if (rank != 0) return;
-          uint64_t* order = reinterpret_cast<uint64_t*>(hist);
-          const int id = ranked_id(small->id, small->value, count, k, temp, p, row_max, row_arg, order, order + SAMPLE_THREADS, team);
-          if (threadIdx.x == 0) out_ids[row] = id;
-          return;
+          }
+        });
+      };
+      list(cut);
+      team_sync();  // the candidates are there
+      int count = first->count;
+      served = count <= SAMPLE_THREADS;
+      team_sync();  // everybody has read how many they are
+      if (!served) {
+        if (rank == 0 && threadIdx.x == 0) small->count = 0;
+        team_sync();
+        list(cut + 1);
+        team_sync();
+        count = first->count;
+        if (count < k) {  // the rest are the first values equal to the cut (of zeros, those without a sign come first)
+          served = send_ties([&](int i) { return order_key(adjusted(i)) == cut; }, adjusted, n, base, k - count, first, count,
+                             sh.warp_count, small->ties, team);
+          count = k;
+        } else if (count <= SAMPLE_CANDIDATES) {  // the first block cuts once more, by the top 12 bits of the keys
+          if (rank == 0 && count > SAMPLE_THREADS) {
+            int* few_id = reinterpret_cast<int*>(hist);
+            float* few_val = reinterpret_cast<float*>(hist) + SAMPLE_THREADS;
+            for (int b = threadIdx.x; b < SAMPLE_FINE_BINS; b += SAMPLE_THREADS) hist[b] = 0u;
+            __syncthreads();
+            for (int i = threadIdx.x; i < count; i += SAMPLE_THREADS) atomicAdd(&hist[order_key(small->value[i]) >> 20], 1u);
+            __syncthreads();
+            const uint32_t fine = find_cut<false>(hist, k, team);
+            const int left = gather([&](int i) { return small->value[i]; }, [&](int i) { return small->id[i]; }, count, fine,
+                                    SAMPLE_THREADS, &sh, few_id, few_val);
+            if (left <= SAMPLE_THREADS && (int)threadIdx.x < left) {
+              small->id[threadIdx.x] = few_id[threadIdx.x];
+              small->value[threadIdx.x] = few_val[threadIdx.x];
+            }
+            if (threadIdx.x == 0) small->count = left;
+          }
+          team_sync();
+          count = first->count;
+          served = count <= SAMPLE_THREADS;
         }
+        team_sync();
+      }
+      if (served) {
+        if (rank != 0) return;
+        uint64_t* order = reinterpret_cast<uint64_t*>(hist);
+        const int id = ranked_id(small->id, small->value, count, k, temp, p, row_max, row_arg, order, order + SAMPLE_THREADS, team);
+        if (threadIdx.x == 0) out_ids[row] = id;
+        return;
       }
     }
   }
@@ -749,7 +835,9 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
         place = ranked_place(threadIdx.x < all ? vals[threadIdx.x] : 0.f, all, k, temp, p, row_max, order,
                              order + SAMPLE_THREADS, team);
       } else {
-        place = sample_place<false>([&](int i) { return vals[i]; }, all, 0, all, k, temp, p, row_max, false, team);
+        auto value = [&](int i) { return vals[i]; };
+        auto every = [&](auto&& f) { for (int i = threadIdx.x; i < all; i += SAMPLE_THREADS) f(i, vals[i]); };
+        place = sample_place<false>(value, every, all, 0, all, k, temp, p, row_max, false, team);
       }
       if (threadIdx.x == 0) out_ids[row] = place >= 0 ? ids[place] : row_arg;
     } else {
@@ -759,7 +847,7 @@ sample_kernel(int* __restrict__ out_ids, const float* __restrict__ logits, int v
   }
   team_sync();  // the counts are read; the histograms start anew
   const bool wide = n > 65535 * SAMPLE_HIST_COPIES;
-  const long long place = sample_place<true>(adjusted, n, base, vocab, k, temp, p, row_max, wide, team);
+  const long long place = sample_place<true>(adjusted, each, n, base, vocab, k, temp, p, row_max, wide, team);
   if (rank == 0 && threadIdx.x == 0) out_ids[row] = place >= 0 ? (int)place : row_arg;
   team_sync();  // nobody leaves while its sums may still be read
 }
@@ -799,20 +887,19 @@ XRT_EXPORT int xrt_sample(int* out_ids, const float* logits, int n_rows, int voc
   if (seen != nullptr && seen_words * 32 < vocab) return XRT_ERR_ARGUMENT;
   if (n_rows == 0) return XRT_OK;
   const int sms = xrt::multiprocessors();
-  // The SMALL form: as many blocks a row as run all at once (two a multiprocessor), where slices are then no smaller than 2,048
-  // logits and the team has at least twice as many groups of lanes as the largest top_k.
-  int team = xrt::SAMPLE_TEAM;
-  while (team > 2 && ((long long)team * n_rows > 2ll * sms || (long long)team * 2048 > vocab)) team /= 2;
-  const bool small = largest_top_k > 0 && largest_top_k < vocab && 2 * largest_top_k <= team * xrt::SAMPLE_GROUPS &&
-                     (long long)team * 2048 <= vocab;
-  if (!small) {
-    // blocks of a team: as many as it takes to bring a slice to 4,096 logits (smaller ones are read in less time than a team takes
-    // to meet), or, where the rows alone occupy the multiprocessors, as keep it at 4,096 (256 rows of 5,000 logits, one block against
-    // two: 20.7 against 26.6 us); half as many while the rows alone bring more than four blocks a multiprocessor
-    team = 1;
-    while (team < xrt::SAMPLE_TEAM && (long long)team * (n_rows >= sms ? 2 * 4096 - 1 : 4096) < vocab) team *= 2;
-    while (team > 2 && (long long)team * n_rows > 4ll * sms) team /= 2;
-  }
+  // blocks of a team: as many as it takes to bring a slice to 4,096 logits (smaller ones are read in less time than a team takes
+  // to meet), or, where the rows alone occupy the multiprocessors, as keep it at 4,096 (256 rows of 5,000 logits, one block against
+  // two: 20.7 against 26.6 us); half as many while the rows alone bring more than four blocks a multiprocessor
+  int team = 1;
+  while (team < xrt::SAMPLE_TEAM && (long long)team * (n_rows >= sms ? 2 * 4096 - 1 : 4096) < vocab) team *= 2;
+  while (team > 2 && (long long)team * n_rows > 4ll * sms) team /= 2;
+  // The SMALL form where those blocks would take more than one round (two run on a multiprocessor at a time): a team of no more than
+  // four, as run all at once, with at least twice as many groups of lanes as the largest top_k.
+  int small_team = team < 4 ? team : 4;
+  while (small_team > 2 && (long long)small_team * n_rows > 2ll * sms) small_team /= 2;
+  const bool small = (long long)team * n_rows > 2ll * sms && largest_top_k > 0 && largest_top_k < vocab && small_team > 1 &&
+                     2 * largest_top_k <= small_team * xrt::SAMPLE_GROUPS;
+  if (small) team = small_team;
   const long long per = ((long long)vocab + team * 32 - 1) / (team * 32) * 32;
   const bool cached = !small && per * 4 <= xrt::SAMPLE_CACHED_BYTES;
   const bool vec = vocab % 4 == 0 && ((uintptr_t)logits & 15) == 0;
