@@ -202,3 +202,25 @@ def test_norms_of_gathered_parts(width, top):
     v = parts.double().sum(0)
     v = (v - v.mean(-1, keepdim=True)) / torch.sqrt(v.var(-1, unbiased=False, keepdim=True) + 1e-5) * w.double() + b.double()
     _close(results[0][0], x0.double() + v, width)
+
+
+# the edges of the rules on 148 multiprocessors: rows of one part and of two in one round, in two, and several a block
+@pytest.mark.parametrize("rows", [296, 297, 444, 445, 592, 593, 1500])
+@pytest.mark.parametrize("width", [1000, 1024, 1025, 2048, 2049])
+def test_layer_norm_of_many_rows_gives_the_bits_of_few(rows, width):
+    from xeno_rt_b200.csrc import ops
+    x, x2, r0 = _rand(rows, width), _rand(2, rows, width, seed=1), _rand(rows, width, seed=2)
+    w, b, w2, b2 = (_rand(width, seed=s) for s in (3, 4, 5, 6))
+
+    def all_forms(a, e):
+        n, residuals = e - a, [r0[a:e].clone() for _ in range(3)]
+        outs = [torch.empty(n, width, dtype=torch.bfloat16, device=DEV) for _ in range(3)]
+        ops.layernorm_affine(x[a:e], w, b, 1e-5, out=outs[0])
+        ops.layernorm_affine(x[a:e], w, b, 1e-5, residual=residuals[0])
+        ops.layernorm_affine(x[a:e], w, b, 1e-5, out=outs[1], residual=residuals[1], then=(w2, b2))
+        ops.layernorm_affine(x2[:, a:e].contiguous(), w, b, 1e-5, out=outs[2], residual=residuals[2], n_parts=2, then=(w2, b2))
+        return outs + residuals
+
+    some = [all_forms(a, min(rows, a + 100)) for a in range(0, rows, 100)]
+    for whole, parts in zip(all_forms(0, rows), zip(*some)):
+        assert torch.equal(whole, torch.cat(parts))

@@ -303,6 +303,10 @@ layernorm_affine_rows_kernel(TO* __restrict__ out, float* __restrict__ residual,
       res[i] = 0.f;
       if (c < width) {
         v[i] = xr[c];
+        // (Never entered: n_parts is 1.  It keeps the loads of the four numbers apart, which then need no more than the 48 registers of
+        // five blocks a multiprocessor: 1,000 rows of 512 5.6 us against 5.75.)
+        if (PARTS == 0 && ITEMS <= 4 && MANY)
+          for (int p = 1; p < n_parts; ++p) v[i] += xr[p * part_stride + c];
         if (residual != nullptr) res[i] = residual[(size_t)r * width + c];
       }
     }
@@ -384,14 +388,18 @@ XRT_EXPORT int xrt_layernorm_affine(void* out, float* residual, const float* x, 
     xrt::GatheredParts gathered;
     gathered.rows = part_rows;
     gathered.scales = part_scales;
-    // Several rows a block: from more rows on than two blocks a multiprocessor hold, for widths above 1,024.  (Up to there a row a
-    // block is one round, and the bound of three blocks a multiprocessor costs registers: 296 rows of 2,048 3.2 us against 4.2, 444 5.8
-    // against 4.4.)  Narrower rows fill a multiprocessor with more blocks than that (4,096 rows of 1,024 as three blocks a multiprocessor
-    // 22.1 us, as a block each 18.9): they only get the form of fewer registers where the other one's four blocks a multiprocessor are not
-    // all (600 rows of 512, 4.3 us against 3.8; of 148 rows it takes 2.5 against 2.4).
+    // Several rows a block, three blocks a multiprocessor, for widths above 1,024 where that takes fewer rounds than a row a block with two
+    // (whose registers are not bounded): 296 rows of 2,048 3.2 us against 4.2, 444 5.8 against 4.4, 592 6.0 against 7.2, 600 7.5 against 7.3,
+    // 4,096 43 against 35.  Above 2,048 either form has two blocks a multiprocessor.  Narrower rows fill a multiprocessor with more
+    // blocks than that (4,096 rows of 1,024 as three blocks a multiprocessor 22.1 us, as a block each 18.9): they only get the form of fewer
+    // registers where the other one's four blocks a multiprocessor are not all (600 rows of 512, 4.3 us against 3.9; of 148 rows it
+    // takes 2.5 against 2.4).
     const int sms = xrt::multiprocessors();
-    const bool many = sms > 0 && n_rows > (width > 256 * 4 ? 2 : 4) * sms;
     const int resident = (width <= 256 * 8 ? 3 : 2) * sms;
+    const auto rounds = [&](int at_once) { return (n_rows + at_once - 1) / at_once; };
+    const bool many = sms > 0 && (width <= 256 * 4   ? n_rows > 4 * sms
+                                  : width <= 256 * 8 ? rounds(resident) < rounds(2 * sms)
+                                                     : n_rows > resident);
     const int blocks = many && width > 256 * 4 && n_rows > resident ? resident : n_rows;
 #define XRT_LAYERNORM(ITEMS, MANY)                                                                                           \
   xrt::launch_kernel(part_rows != nullptr ? xrt::layernorm_affine_rows_kernel<TO, ITEMS, 2, MANY>                            \
