@@ -296,10 +296,10 @@ inline int stream_row_groups_accumulate(int N) {
 }
 
 // Eight stages (70 KB a block, the same sums) for a product of up to 12 rows that adds into the residual stream and has more than one
-// block a multiprocessor but less than two: they are the only ones to keep bytes in flight.  Alone, four stages -> eight, by which
-// number the time shrinks: N 2,048 / K 8,192 at 1 row 13.3 -> 10.8 us, at 8 14.4 -> 11.9, at 12 1.18; N 1,280 / K 8,192 1.07 to 1.17, N 2,304
-// 1.13 to 1.19 (of the 42 points between at K 2,560 to 14,336 only N 1,664 / K 14,336 at 1 and 2 rows lost, 16.1 -> 16.8).  Outside: N 1,216
-// 0.95 to 1.05, N 2,368 9.95 -> 11.6 us; N 2,048 / K 25,600 at 16 rows 42.8 -> 45.4 (the rows of X no longer fit beside the rings in the L1).
+// block a multiprocessor but less than two: they are the only ones to keep bytes in flight.  Alone, four stages -> eight: N 2,048 /
+// K 8,192 at 1 row 13.4 -> 10.9 us, at 8 14.4 -> 11.9, at 12 14.9 -> 12.7; N 1,280 / K 8,192 1.07 to 1.17 times as fast, N 2,304 1.13 to
+// 1.19 (of 9 N between, K 2,560 to 14,336, only N 1,664 / K 14,336 at 1 and 2 rows lost, 15.8 -> 16.8).  Outside: N 1,216
+// 0.95 to 1.05 times, N 2,368 / K 8,192 9.95 -> 11.6 us; N 2,048 / K 25,600 at 16 rows 42.8 -> 45.4 (the rows of X no longer fit beside the rings in the L1).
 // Stored products gained less and lost more (K 14,336 at 4 rows: N 2,048 19.4 -> 18.5, N 1,792 15.9 -> 18.2).
 inline bool stream_deep_ring(int M, int N, int K) {
   const int blocks = (N + GS_ROWS - 1) / GS_ROWS, sms = stream_sm_count();

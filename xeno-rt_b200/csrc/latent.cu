@@ -22,7 +22,7 @@ namespace xrt {
 
 // gridDim.y blocks a token.  Warp 0 of the first writes the cache row; all warps walk the heads' rotated query parts, which the blocks of
 // a token share: a step of few tokens has so many blocks that a thread has one number of them, since a thread's numbers come one
-// after the other (4 tokens of 16 heads with 64 rotated dims: 9.7 us of a decode step with one block a token, 3.3 to 4.3 with eight).
+// after the other (alone, 4 tokens of 16 heads with 64 rotated dims: one block a token 5.9 us, eight 2.7; 147 tokens 6.2 and 2.9).
 // qd row: [heads x (dim | rot)] then, at down_offset, [rank | rot].  q_rows row: heads x [rank | rot | padding]
 // of head_size.  cos_sin [T, rot / 2, 2]; pairs are (2i, 2i + 1) with `interleaved`, else (i, i + rot / 2).
 template <typename TN, typename TQ, typename TC>

@@ -27,10 +27,12 @@
 // One row is a chain of latencies: the pass over the slice, the team's meetings, the ranking.  64 rows of that kernel run it twice, since
 // two blocks fill a multiprocessor (64 registers a thread of 512; 85 KB) and there are 512.
 //
-// Batches whose rows all have a small top_k (the usual options; the caller says so) or are greedy take the SMALL form (64 rows of 128,256
-// with top_k 40, top_p 0.95: 63 -> 27 us a call): no values kept,
-// so that four blocks of 32,064 logits a row run all at once, and one cut for the whole team, so that hardly more than top_k
-// candidates remain and only the threads that hold one look at the logits again.
+// Batches that would take two rounds and whose rows all have a small top_k (the usual options; the caller says so) or are greedy take
+// the SMALL form: no values kept, so that four blocks of 32,064 logits a row run all at once, and one cut for the whole team, so that hardly more
+// than top_k candidates remain and only the threads that hold one look at the logits again.  64 rows of 128,256, top_k 40, top_p 0.95,
+// the kernel alone, values kept -> SMALL: normal logits 63 -> 27 us; all rows masked to 11 ids 192 -> 25, with the lowest number for a mask 199 -> 37,
+// in falling order 171 -> 42, of one value 212 -> 31; one such row among them 78 -> 27, 81 -> 32, 72 -> 35, 84 -> 28.  Of fewer rows the values
+// are worth their place (16 rows of 32,000: 18.9, SMALL with eight blocks a row 27.3).
 #include <type_traits>
 
 #include "common.cuh"

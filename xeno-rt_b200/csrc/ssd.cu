@@ -321,7 +321,8 @@ int launch_ssd_scan_wide(const SsdArgs& a, int n_seqs, cudaStream_t stream) {
 
 // v = y * silu(z); each of `groups` stretches of the row by its own root mean square; times w.  One block a
 // (token, group).  A row's numbers are all asked for at once (PER a thread, the weights before the wait) and v is kept: the
-// kernel is a chain of latencies in a decode step, where the loop over memory below took 10.8 us for 2 rows of 2 x 2,048 and this takes 3.6.
+// kernel is a chain of latencies in a decode step (alone, the loop over memory below -> this: 4 tokens of 2 x 2,048 5.2 -> 2.2 us, of
+// 2 x 4,096 9.1 -> 3.2; 4,000 tokens of 2 x 2,048 66 -> 43).
 template <typename TO, int PER>
 __global__ void __launch_bounds__(256)
 gated_group_norm_rows_kernel(TO* __restrict__ out, const float* __restrict__ y, const float* __restrict__ z, int z_stride,
@@ -448,7 +449,8 @@ XRT_EXPORT int xrt_gated_group_norm(void* out, const float* y, const float* z, i
   const int per = width / groups;
   const int threads = per >= 1024 ? 256 : (per >= 256 ? 128 : 64);
   XRT_DISPATCH_DTYPE(out_dtype, TO, {
-    // as many numbers a thread as a stretch has: 64 tokens of 16 stretches of 64 took 2.2 us before and 2.8 with room for four
+    // no more numbers a thread than a stretch has: with room for four, 64 tokens of 16 stretches of 64 took 2.8 us (the loop 2.2, one
+    // number 1.8), 4,000 tokens of 4 of 256 24.4 (19.6, two numbers 17.1)
     auto kernel = per <= threads        ? xrt::gated_group_norm_rows_kernel<TO, 1>
                   : per <= 2 * threads  ? xrt::gated_group_norm_rows_kernel<TO, 2>
                   : per <= 4 * threads  ? xrt::gated_group_norm_rows_kernel<TO, 4>
