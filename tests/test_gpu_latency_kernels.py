@@ -224,3 +224,21 @@ def test_layer_norm_of_many_rows_gives_the_bits_of_few(rows, width):
     some = [all_forms(a, min(rows, a + 100)) for a in range(0, rows, 100)]
     for whole, parts in zip(all_forms(0, rows), zip(*some)):
         assert torch.equal(whole, torch.cat(parts))
+
+
+@pytest.mark.parametrize("width", [4097, 8192, 8193, 16384])
+def test_norm_after_a_sublayer_of_wide_rows(width):
+    """The last width of every form beyond 4,096 and the widest: gathered parts give the bits of parts written out, and both the norm."""
+    from xeno_rt_b200.csrc import ops
+    n, top = 20, 2
+    y, x0, w = _rand(n * top, width), _rand(n, width, seed=1), _rand(width, seed=2)
+    rows, scales = torch.randperm(n * top, device=DEV).to(torch.int32), torch.rand(n, top, device=DEV)
+    parts = torch.empty(top, n, width, device=DEV)
+    ops.moe_combine(parts, y, rows, scales)
+    plain, gathered = x0.clone(), x0.clone()
+    ops.rmsnorm_add(plain, parts, w, 1e-6)
+    ops.rmsnorm_add(gathered, y, w, 1e-6, gather=(rows, scales))
+    assert torch.equal(plain, gathered)
+    v = parts.double().sum(0)
+    v = x0.double() + v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-6) * w.double()
+    _close(plain, v, width)
